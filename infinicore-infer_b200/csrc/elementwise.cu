@@ -1,6 +1,6 @@
 // Row-wise kernels of the step: embedding gather, residual add + RMSNorm, rotary position
-// encoding fused with the write of keys and values into cache pages, SwiGLU, and a
-// float32 matrix product on the CUDA cores (the true 32-bit path).
+// encoding fused with the write of keys and values into cache pages, and SwiGLU (the module's
+// float32 matrix product is gemm_f32.cu).
 //
 // The residual stream is float32 in both precisions; products, norms and rotations are
 // computed in float32 and rounded once when they are stored as bfloat16.
@@ -410,67 +410,5 @@ JK_EXPORT int jk_rope_kv(const void *qkv, int in_dtype, int ld_qkv, const float 
     else
         JK_FAIL(JK_UNSUPPORTED, "rope_kv: dtypes %d -> %d", in_dtype, out_dtype);
     JK_CHECK_LAUNCH("rope_kv");
-    return JK_OK;
-}
-
-// ---------------------------------------------------------------------------------------
-// float32 matrix product on the CUDA cores:  C[M, N] = A[M, K] * W[N, K]^T (+ bias[N]).
-// Plain fused multiply-adds in float32: no tensor cores, hence no TF32 rounding of the
-// operands.  Each output element sums over k in ascending order whatever M and N are, so a
-// row's result does not depend on what else is in the batch.
-// (reference: the products at jiuge.cpp:200, :236, :247, :249, :264 go to a library.)
-// ---------------------------------------------------------------------------------------
-constexpr int GF_BM = 64, GF_BN = 64, GF_BK = 16;
-
-__global__ void __launch_bounds__(256)
-gemm_f32_kernel(const float *__restrict__ A, const float *__restrict__ W,
-                const float *__restrict__ bias, float *__restrict__ C, int M, int N, int K,
-                int lda, int ldw, int ldc) {
-    pdl_trigger();
-    pdl_wait();
-    __shared__ float As[GF_BK][GF_BM + 1];
-    __shared__ float Ws[GF_BK][GF_BN + 1];
-    const int m0 = blockIdx.y * GF_BM, n0 = blockIdx.x * GF_BN;
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += GF_BK) {
-        for (int i = threadIdx.x; i < GF_BM * GF_BK; i += 256) {
-            const int r = i / GF_BK, c = i % GF_BK;
-            As[c][r] = (m0 + r < M && k0 + c < K) ? A[(size_t)(m0 + r) * lda + k0 + c] : 0.f;
-            Ws[c][r] = (n0 + r < N && k0 + c < K) ? W[(size_t)(n0 + r) * ldw + k0 + c] : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < GF_BK; ++k) {
-            float a[4], w[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) { a[i] = As[k][ty * 4 + i]; w[i] = Ws[k][tx * 4 + i]; }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + ty * 4 + i;
-        if (m >= M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx * 4 + j;
-            if (n < N) C[(size_t)m * ldc + n] = acc[i][j] + (bias ? bias[n] : 0.f);
-        }
-    }
-}
-
-JK_EXPORT int jk_gemm_f32(const float *A, int lda, const float *W, int ldw, const float *bias,
-                          float *C, int ldc, int M, int N, int K, cudaStream_t stream) {
-    if (M == 0 || N == 0) return JK_OK;
-    JK_REQUIRE(M > 0 && N > 0 && K > 0, "gemm_f32: M %d N %d K %d", M, N, K);
-    dim3 grid((N + GF_BN - 1) / GF_BN, (M + GF_BM - 1) / GF_BM);
-    JK_REQUIRE(grid.y <= 65535, "gemm_f32: M %d is too large for one launch", M);
-    jk_launch(gemm_f32_kernel, grid, dim3(256), 0, stream, A, W, bias, C, M, N, K, lda, ldw, ldc);
-    JK_CHECK_LAUNCH("gemm_f32");
     return JK_OK;
 }

@@ -110,6 +110,23 @@ def test_gemm_f32_is_a_true_float32_product(K, M, N, K_):
         assert torch.equal(one[0], out[M - 1])
 
 
+@pytest.mark.parametrize("M,N,K_", [(1, 1, 1), (8, 64, 16), (9, 65, 17), (16, 33, 63), (33, 2049, 64), (65, 130, 66), (301, 1536, 132), (129, 9601, 20)])
+def test_gemm_f32_tiles_agree_bit_for_bit(K, M, N, K_):
+    """Every tile size at its edges and with rows that do not start on 16 bytes: the sums' order depends on K alone."""
+    g = torch.Generator().manual_seed(M + N + K_)
+    a, w = torch.randn(M, K_, generator=g).to(DEV), torch.randn(N, K_, generator=g).to(DEV)
+    out = torch.full((M, N), 7.0, device=DEV)
+    K.gemm_f32(a, w, out)
+    want = a.double() @ w.double().T
+    # a product's rounding is below 2^-24 of |a||w| < 25 here, and K of them add up
+    assert (out.double() - want).abs().max() <= 2.0 ** -24 * 25 * max(4, K_)
+    for rows, cols in ((slice(0, 1), slice(None)), (slice(M // 2, None), slice(0, (N + 1) // 2))):
+        part_a, part_w = a[rows].contiguous(), w[cols].contiguous()
+        part = torch.full((part_a.shape[0], part_w.shape[0]), 7.0, device=DEV)
+        K.gemm_f32(part_a, part_w, part)
+        assert torch.equal(part, out[rows, cols])
+
+
 def _scatter_pages(k, v, tables, page, num_pages, dtype, junk=7.0):
     """Dense per-request keys/values [len, nkvh, dh] -> pages [num_pages, nkvh, page, dh]."""
     nkvh, dh = k[0].shape[1:]
