@@ -17,6 +17,8 @@
 #include "common.cuh"
 #include "host_rules.h"
 
+#include <type_traits>
+
 JK_DEFINE_ERROR_BUFFER(jk_attention)
 
 struct AttnArgs {
@@ -42,102 +44,239 @@ struct AttnArgs {
     int keep_first;
     const float *sink_w;
     int gate_elem;
+    // the row kernel's cut: rows and heads of a block, and whether key and value rows are read 16 bytes at a time
+    // chunks of keys in shared memory (1 or 2), and the logarithm of the lanes that read a row
+    int tile_rows, tile_heads, vec, stages, lanes, page_shift;      // page_shift: log2(page_size), or -1
 };
 
 // ---------------------------------------------------------------------------------------
-// Row kernel: one warp per (row, query head).  Lanes take one key each for the scores, then
-// one slice of the head each for the weighted values.  Any head size, any page size, both
-// element types; the result for a row does not depend on what else is in the batch.
+// Row kernel: any head size, any page size, both element types, everything in float32.  A block of eight warps takes the
+// (row, query head) pairs of up to a.tile_rows neighbouring rows of one request and up to ROW_PAIRS / rows of the heads that
+// share a key/value head, and walks the request's keys 32 at a time through shared memory.  A warp has up to four pairs at
+// once: lanes take one key each for the scores (a key's vector is read once for all four), then one slice of the head each
+// for the weighted values.  Chunks of keys start at multiples of 32 positions, so the result for a row does not depend on
+// what else is in the batch or on how its prompt was cut.
+//
+// Every row starts a block; the block of a row that neither begins a request's rows nor a tile of a.tile_rows returns at
+// once, so a launch needs no list of tiles, and a request with one row has a block of its own.
+//
+// What bounds it: instructions and, in small launches, a chunk's chain of copies, barriers and shuffles.  A warp a pair, each lane
+// with a key row of its own in memory, waited for 32 cache lines a load.  B200, float32, before and after (us): 24 heads of 64
+// over 8, a prompt of 301 rows 375 -> 62, one row over 1,000 keys 293 -> 72, 8 rows over 4,000 keys each 2,072 -> 279; 36
+// heads, a prompt of 512 rows 1,554 -> 168; bfloat16, 16 heads of 256, a prompt of 1,024 rows 9,515 -> 1,369.
 // ---------------------------------------------------------------------------------------
-constexpr int ROW_WARPS = 4;
+constexpr int ROW_WARPS = 8, ROW_SLOTS = 4, ROW_PAIRS = ROW_WARPS * ROW_SLOTS, ROW_KEYS = 32;
 constexpr int ROW_MAX_DH = 512;
+
+// 32 rows of `size` elements as floats into rows of `ld`, four rows a warp, 2^`lanes` lanes a row.  `row`: the number of this
+// lane's row among the rows of `pages`, or -1 for a key that no row of the block sees (zeros).  Float rows of whole vectors
+// come by asynchronous copies.
+template <typename T>
+__device__ __forceinline__ void row_load_tile(float *tile, int ld, const T *pages, bool vec, int lanes, long long row, int size) {
+    constexpr int VEC = 16 / sizeof(T), ROWS = ROW_KEYS / ROW_WARPS;
+    const int lane = threadIdx.x & 31, per = vec ? VEC : 1, step = 32 >> lanes;
+    for (int i = lane >> lanes; i - (lane >> lanes) < ROWS; i += step) {
+        const int r = (threadIdx.x >> 5) * ROWS + i;
+        const long long from = __shfl_sync(0xffffffffu, row, r & 31);
+        if (i >= ROWS) continue;
+        const T *src = pages + (size_t)(from < 0 ? 0 : from) * size;
+        float *dst = tile + r * ld;
+        for (int c = (lane & ((1 << lanes) - 1)) * per; c < size; c += per << lanes) {
+            if (!vec) {
+                dst[c] = from >= 0 ? to_f32(src[c]) : 0.f;
+            } else if (sizeof(T) == 4) {
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst + c)), "l"(src + c), "r"(from >= 0 ? 16 : 0) : "memory");
+            } else {
+                const uint4 raw = from >= 0 ? *reinterpret_cast<const uint4 *>(src + c) : make_uint4(0u, 0u, 0u, 0u);
+                const T *v = reinterpret_cast<const T *>(&raw);
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) dst[c + e] = to_f32(v[e]);
+            }
+        }
+    }
+}
+
+// One chunk of keys for the SLOTS pairs of a warp: the weights p go through shared memory, m, l and acc move on.
+template <int SLOTS, int NS>
+__device__ __forceinline__ void row_chunk(const AttnArgs &a, const float *ks, const float *vs, const float *q, float *ps, int ldk, int ldv, int j0,
+                                          const int (&pos)[ROW_SLOTS], const int (&lo)[ROW_SLOTS], float (&m)[ROW_SLOTS], float (&l)[ROW_SLOTS],
+                                          float (&acc)[ROW_SLOTS][NS]) {
+    const int lane = threadIdx.x & 31, j = j0 + lane, width = (a.dh + 3) / 4 * 4;
+    float dot[SLOTS] = {};
+    const float *kr = ks + lane * ldk;
+#pragma unroll 4
+    for (int e = 0; e < width; e += 4) {
+        const float4 k = *reinterpret_cast<const float4 *>(kr + e);
+#pragma unroll
+        for (int i = 0; i < SLOTS; ++i) {
+            const float4 x = *reinterpret_cast<const float4 *>(q + i * ROW_WARPS * width + e);
+            dot[i] = fmaf(x.w, k.w, fmaf(x.z, k.z, fmaf(x.y, k.y, fmaf(x.x, k.x, dot[i]))));
+        }
+    }
+    // keys that a slot does not see have weight 0, but their values are other rows' business: what is not finite there must not
+    // come through as 0 x inf, so a chunk with such keys and values adds the seen keys only
+    unsigned mask[SLOTS], live = 0, whole = 1;
+#pragma unroll
+    for (int i = 0; i < SLOTS; ++i) {
+        const bool seen = j <= pos[i] && (j >= lo[i] || j < a.keep_first);
+        mask[i] = __ballot_sync(0xffffffffu, seen);
+        live |= mask[i];
+        whole &= mask[i] == 0xffffffffu || pos[i] < 0;
+        float s = dot[i] * a.scale;
+        if (a.cap > 0.f) s = a.cap * tanhf(s / a.cap);
+        if (mask[i] == 0) {
+            ps[i * ROW_KEYS + lane] = 0.f;
+            continue;
+        }
+        const float m_new = fmaxf(m[i], warp_max(seen ? s : -INFINITY)), p = seen ? expf(s - m_new) : 0.f, corr = expf(m[i] - m_new);
+        l[i] = l[i] * corr + warp_sum(p);
+        m[i] = m_new;
+#pragma unroll
+        for (int n = 0; n < NS; ++n) acc[i][n] *= corr;
+        ps[i * ROW_KEYS + lane] = p;
+    }
+    __syncwarp();
+    auto add = [&](auto all) {
+        for (int jj = 0; jj < ROW_KEYS; jj += 4) {
+            float4 p[SLOTS];
+#pragma unroll
+            for (int i = 0; i < SLOTS; ++i) p[i] = *reinterpret_cast<const float4 *>(ps + i * ROW_KEYS + jj);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int n = 0; n < NS; ++n) {
+                    const int e = lane + 32 * n;
+                    const float v = e < a.dv ? vs[(jj + k) * ldv + e] : 0.f;
+#pragma unroll
+                    for (int i = 0; i < SLOTS; ++i) {
+                        const float w = k == 0 ? p[i].x : k == 1 ? p[i].y : k == 2 ? p[i].z : p[i].w;
+                        if (decltype(all)::value || (mask[i] >> (jj + k) & 1)) acc[i][n] = fmaf(w, v, acc[i][n]);
+                    }
+                }
+        }
+    };
+    if (live != 0 && !whole) {
+        float sum = 0.f;                 // stays 0 unless a value is infinite or not a number
+#pragma unroll 8
+        for (int jj = 0; jj < ROW_KEYS; ++jj)
+#pragma unroll
+            for (int n = 0; n < NS; ++n)
+                if (lane + 32 * n < a.dv) sum = fmaf(vs[jj * ldv + lane + 32 * n], 0.f, sum);
+        whole = __all_sync(0xffffffffu, sum == 0.f);
+    }
+    if (live == 0) ;
+    else if (whole) add(std::true_type());
+    else add(std::false_type());
+    __syncwarp();
+}
 
 template <typename T, int NS>     // NS: slices of 32 elements that cover one head's values
 __global__ void __launch_bounds__(ROW_WARPS * 32)
 attention_row_kernel(AttnArgs a) {
     pdl_trigger();
     pdl_wait();
-    extern __shared__ float q_smem[];          // [ROW_WARPS][dh]
+    const int t0 = blockIdx.x, req = a.row_req[t0];
+    if (t0 % a.tile_rows != 0 && a.row_req[t0 - 1] == req) return;
+    int rows = 1;
+    while ((t0 + rows) % a.tile_rows != 0 && t0 + rows < a.T && a.row_req[t0 + rows] == req) ++rows;
+    extern __shared__ __align__(16) float row_smem[];
+    const int width = (a.dh + 3) / 4 * 4, ldk = width + 4, ldv = (a.dv + 3) / 4 * 4, tile = ROW_KEYS * (ldk + ldv);
+    float *ring = row_smem, *qs = ring + a.stages * tile, *ps = qs + ROW_PAIRS * width;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int t = blockIdx.y;
-    const int h = blockIdx.x * ROW_WARPS + warp;
-    if (h >= a.nh) return;
-    const int dh = a.dh, dv = a.dv;
-    const int hk = h / (a.nh / a.nkvh);
-    const int pos = a.positions[t];
-    const int *bt = a.block_table + (size_t)a.row_req[t] * a.max_blocks;
-    const int lo = jk_mask_lo(pos, a.window);
-
-    float *qs = q_smem + warp * dh;
-    const T *qrow = (const T *)a.q + ((size_t)t * a.nh + h) * dh;
-    for (int e = lane; e < dh; e += 32) qs[e] = to_f32(qrow[e]);
-    __syncwarp();
-
-    const T *kp = (const T *)a.k_pages;
-    const T *vp = (const T *)a.v_pages;
-    // offsets are counted in rows of a key/value head: a key row has dh elements, a value row dv
-    const size_t head_off = (size_t)hk * a.page_size;
-    const size_t page_stride = (size_t)a.nkvh * a.page_size;
-
-    float m = -INFINITY, l = 0.f;
-    float acc[NS];
+    const int group = a.nh / a.nkvh, parts = (group + a.tile_heads - 1) / a.tile_heads;
+    const int hk = blockIdx.y / parts, h0 = hk * group + blockIdx.y % parts * a.tile_heads, heads = min(a.tile_heads, (hk + 1) * group - h0);
+    const int pairs = rows * heads;
+    // pair number p = row * heads + head belongs to warp p % ROW_WARPS, slot p / ROW_WARPS
+    for (int i = threadIdx.x; i < ROW_PAIRS * width; i += ROW_WARPS * 32) {
+        const int p = i / width, e = i % width;
+        qs[i] = p < pairs && e < a.dh ? to_f32(((const T *)a.q)[((size_t)(t0 + p / heads) * a.nh + h0 + p % heads) * a.dh + e]) : 0.f;
+    }
+    const int *bt = a.block_table + (size_t)req * a.max_blocks;
+    int pos[ROW_SLOTS], lo[ROW_SLOTS];
+    float m[ROW_SLOTS], l[ROW_SLOTS], acc[ROW_SLOTS][NS];
 #pragma unroll
-    for (int i = 0; i < NS; ++i) acc[i] = 0.f;
-
-    // two ranges of keys: the kept first ones that the window has passed, then the window
-    const int kept = min(a.keep_first, lo);
-    for (int range = kept > 0 ? 0 : 1; range < 2; ++range) {
-    const int begin = range == 0 ? 0 : lo, end = range == 0 ? kept - 1 : pos;
-    for (int j0 = begin; j0 <= end; j0 += 32) {
-        const int j = j0 + lane;
-        const bool valid = j <= end;
-        size_t row_off = 0;
-        float s = -INFINITY;
-        if (valid) {
-            const int page = bt[j / a.page_size];
-            row_off = (size_t)page * page_stride + head_off + (size_t)(j % a.page_size);
-            const T *kr = kp + row_off * dh;
-            float dot = 0.f;
-            for (int e = 0; e < dh; ++e) dot = fmaf(qs[e], to_f32(kr[e]), dot);
-            s = dot * a.scale;
-            if (a.cap > 0.f) s = a.cap * tanhf(s / a.cap);
+    for (int i = 0; i < ROW_SLOTS; ++i) {
+        const int p = warp + i * ROW_WARPS;
+        pos[i] = p < pairs ? a.positions[t0 + p / heads] : -1;
+        lo[i] = jk_mask_lo(max(pos[i], 0), a.window);
+        m[i] = -INFINITY;
+        l[i] = 0.f;
+#pragma unroll
+        for (int n = 0; n < NS; ++n) acc[i][n] = 0.f;
+    }
+    // the keys that some row of the block sees: [0, kept) and [first, last]
+    int first = 0x7fffffff, last = 0;
+    for (int r = 0; r < rows; ++r) {
+        first = min(first, jk_mask_lo(a.positions[t0 + r], a.window));
+        last = max(last, a.positions[t0 + r]);
+    }
+    const int kept = min(a.keep_first, last + 1);
+    const float *q = qs + warp * width;
+    float *p = ps + warp * ROW_SLOTS * ROW_KEYS;
+    // chunks in order: those that hold kept keys, then those from the first seen key's on
+    auto after = [&](int j) { return j + ROW_KEYS < kept ? j + ROW_KEYS : max(j + ROW_KEYS, first / ROW_KEYS * ROW_KEYS); };
+    // this lane's key of the chunk at j: its row among all rows of the pages (looked up a chunk ahead of its copy)
+    auto row_of = [&](int j) {
+        j += lane;
+        if (j > last || (j >= kept && j < first)) return -1ll;
+        const int block = a.page_shift >= 0 ? j >> a.page_shift : j / a.page_size;
+        return ((long long)bt[block] * a.nkvh + hk) * a.page_size + (j - block * a.page_size);
+    };
+    auto fetch = [&](int stage, long long row) {
+        row_load_tile<T>(ring + stage * tile, ldk, (const T *)a.k_pages, a.vec, a.lanes, row, a.dh);
+        row_load_tile<T>(ring + stage * tile + ROW_KEYS * ldk, ldv, (const T *)a.v_pages, a.vec, a.lanes, row, a.dv);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    if (a.dh % 4 != 0)          // the columns that fill a key up to whole vectors
+        for (int i = threadIdx.x; i < a.stages * ROW_KEYS; i += ROW_WARPS * 32)
+            for (int e = a.dh; e < width; ++e) ring[i / ROW_KEYS * tile + i % ROW_KEYS * ldk + e] = 0.f;
+    int j0 = kept > 0 ? 0 : first / ROW_KEYS * ROW_KEYS, stage = 0;
+    long long row = row_of(j0);
+    if (a.stages > 1) {
+        fetch(0, row);
+        row = row_of(after(j0));
+    }
+    for (; j0 <= last; j0 = after(j0)) {
+        if (a.stages > 1) {       // the chunk after this one is on its way while this one is at work
+            if (after(j0) <= last) fetch(stage ^ 1, row);
+            else asm volatile("cp.async.commit_group;\n" ::: "memory");
+            row = row_of(after(after(j0)));
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        } else {
+            fetch(0, row);
+            row = row_of(after(j0));
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         }
-        const float m_new = fmaxf(m, warp_max(s));
-        const float p = valid ? expf(s - m_new) : 0.f;
-        const float corr = expf(m - m_new);          // exp(-inf) = 0 on the first chunk
-        l = l * corr + warp_sum(p);
-        m = m_new;
+        __syncthreads();
+        const float *ks = ring + stage * tile, *vs = ks + ROW_KEYS * ldk;
+        if (pairs > 2 * ROW_WARPS) row_chunk<ROW_SLOTS, NS>(a, ks, vs, q, p, ldk, ldv, j0, pos, lo, m, l, acc);
+        else if (pairs > ROW_WARPS) row_chunk<2, NS>(a, ks, vs, q, p, ldk, ldv, j0, pos, lo, m, l, acc);
+        else if (warp < pairs) row_chunk<1, NS>(a, ks, vs, q, p, ldk, ldv, j0, pos, lo, m, l, acc);
+        __syncthreads();
+        stage ^= a.stages - 1;
+    }
 #pragma unroll
-        for (int i = 0; i < NS; ++i) acc[i] *= corr;
-        const int n = min(32, end - j0 + 1);
-        for (int jj = 0; jj < n; ++jj) {
-            const float pj = __shfl_sync(0xffffffffu, p, jj);
-            const unsigned long long off = __shfl_sync(0xffffffffu, (unsigned long long)row_off, jj);
-            const T *vr = vp + off * dv;
+    for (int i = 0; i < ROW_SLOTS; ++i) {
+        const int pair = warp + i * ROW_WARPS;
+        if (pair >= pairs) continue;
+        const int t = t0 + pair / heads, h = h0 + pair % heads;
+        if (a.sink) {       // one more key that brings no value
+            const float sink = a.sink_w != nullptr ? a.sink_w[h] : 0.f;
+            const float m_new = fmaxf(m[i], sink);
+            const float corr = expf(m[i] - m_new);
+            l[i] = l[i] * corr + expf(sink - m_new);
 #pragma unroll
-            for (int i = 0; i < NS; ++i) {
-                const int e = lane + 32 * i;
-                if (e < dv) acc[i] = fmaf(pj, to_f32(vr[e]), acc[i]);
-            }
+            for (int n = 0; n < NS; ++n) acc[i][n] *= corr;
         }
-    }
-    }
-    if (a.sink) {       // one more key that brings no value
-        const float sink = a.sink_w != nullptr ? a.sink_w[h] : 0.f;
-        const float m_new = fmaxf(m, sink);
-        const float corr = expf(m - m_new);
-        l = l * corr + expf(sink - m_new);
+        T *orow = (T *)a.out + ((size_t)t * a.nh + h) * a.dv;
+        float inv = 1.f / l[i];
+        const float *gate = a.gate != nullptr ? a.gate + (size_t)t * a.gate_ld + (size_t)h * (a.gate_elem ? a.dv : 1) : nullptr;
+        if (gate != nullptr && !a.gate_elem) inv *= jk_sigmoid(gate[0]);
 #pragma unroll
-        for (int i = 0; i < NS; ++i) acc[i] *= corr;
-    }
-    T *orow = (T *)a.out + ((size_t)t * a.nh + h) * dv;
-    float inv = 1.f / l;
-    const float *gate = a.gate != nullptr ? a.gate + (size_t)t * a.gate_ld + (size_t)h * (a.gate_elem ? dv : 1) : nullptr;
-    if (gate != nullptr && !a.gate_elem) inv *= jk_sigmoid(gate[0]);
-#pragma unroll
-    for (int i = 0; i < NS; ++i) {
-        const int e = lane + 32 * i;
-        if (e < dv) orow[e] = from_f32<T>(acc[i] * inv * (a.gate_elem && gate != nullptr ? jk_sigmoid(gate[e]) : 1.f));
+        for (int n = 0; n < NS; ++n) {
+            const int e = lane + 32 * n;
+            if (e < a.dv) orow[e] = from_f32<T>(acc[i][n] * inv * (a.gate_elem && gate != nullptr ? jk_sigmoid(gate[e]) : 1.f));
+        }
     }
 }
 
@@ -162,9 +301,32 @@ JK_EXPORT int jk_attention_rows(const void *q, const void *k_pages, const void *
     JK_REQUIRE(dh <= ROW_MAX_DH && dv <= ROW_MAX_DH, "attention: head size %d / %d exceeds %d", dh, dv, ROW_MAX_DH);
     JK_REQUIRE(gate == nullptr || gate_ld >= nh * (gate_elem ? dv : 1), "attention: a gate row of %d holds no %d heads", gate_ld, nh);
     JK_REQUIRE(T <= 65535, "attention: %d rows exceed one launch (65535)", T);
-    dim3 grid((nh + ROW_WARPS - 1) / ROW_WARPS, T);
-    const size_t smem = (size_t)ROW_WARPS * dh * sizeof(float);
-#define LAUNCH_ROWS(T, NS) jk_launch(attention_row_kernel<T, NS>, grid, dim3(ROW_WARPS * 32), smem, stream, a)
+    // A block's pairs: as many heads of one key/value head as there are, then rows until the pairs are full (every row alike: the
+    // cut does not change a row's result)
+    const int group = nh / nkvh, elem = dtype == JK_F32 ? 4 : 2;
+    a.tile_heads = group < ROW_PAIRS ? group : ROW_PAIRS;
+    a.tile_rows = ROW_PAIRS / a.tile_heads;
+    a.page_shift = -1;
+    for (int i = 0; i < 31; ++i)
+        if (page_size == 1 << i) a.page_shift = i;
+    a.vec = dh * elem % 16 == 0 && dv * elem % 16 == 0 && (((uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0;
+    const int vectors = std::max(dh, dv) * elem / (a.vec ? 16 : elem);
+    for (a.lanes = 2; a.lanes < 5 && (1 << a.lanes) < vectors;) ++a.lanes;
+    const long long parts = (group + a.tile_heads - 1) / a.tile_heads;
+    JK_REQUIRE(parts * nkvh <= 65535, "attention: %d heads exceed one launch", nh);
+    // fewer rows a block until there are three blocks for every SM: a block alone there waits for its chunks and its barriers
+    while (a.tile_rows > 1 && (T + a.tile_rows - 1) / a.tile_rows * parts * nkvh < 3 * 148) a.tile_rows = (a.tile_rows + 1) / 2;
+    dim3 grid(T, (unsigned)(parts * nkvh));
+    const int width = (dh + 3) / 4 * 4;
+    // two chunks of keys as long as two blocks fit an SM with them
+    const size_t tile = (size_t)ROW_KEYS * (width + 4 + (dv + 3) / 4 * 4), fixed = (size_t)ROW_PAIRS * (width + ROW_KEYS);
+    a.stages = sizeof(float) * (2 * tile + fixed) <= 112 * 1024 ? 2 : 1;
+    const size_t smem = sizeof(float) * (a.stages * tile + fixed);
+#define LAUNCH_ROWS(T, NS)                                                                                                              \
+    do {                                                                                                                                \
+        if (smem > 46 * 1024) cudaFuncSetAttribute(attention_row_kernel<T, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        jk_launch(attention_row_kernel<T, NS>, grid, dim3(ROW_WARPS * 32), smem, stream, a);                                            \
+    } while (0)
 #define LAUNCH_ROWS_T(T)                                \
     do {                                                \
         if (dv <= 32) LAUNCH_ROWS(T, 1);                \

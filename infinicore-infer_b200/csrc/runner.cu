@@ -268,7 +268,7 @@ int run_attention(Run &r, const RunnerOp &op) {
     if (dv != dh && !jk::attention_unlike_heads(dh, dv)) fast = false;
     if (fast && n_tiles > 0 && !(tc || (dv == dh && g_fns.attention_prefill_supports(dh)))) fast = false;
     if (!fast) {
-        // one warp per (row, head): float32, and every shape the tensor-core kernels are not built for
+        // float32 arithmetic throughout: float32 mode, and every shape the tensor-core kernels are not built for
         RUN(attention, g_fns.attention_rows(q, op.k_pages, op.v_pages, o, r.env.dtype, r.st.positions, r.st.row_req, table,
                                             r.env.max_blocks, page, T, nh, nkvh, dh, op.softmax_scale, op.window, dv, op.sink, gate, op.ld,
                                             op.cap, op.keep_first, op.sink_w, op.gated == 2, r.stream));

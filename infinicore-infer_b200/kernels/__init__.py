@@ -456,7 +456,7 @@ def attention_rows(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor
                    nh: int, scale: float, window: int = 0, sink: bool = False,
                    gate: Optional[torch.Tensor] = None, cap: float = 0.0, keep_first: int = 0,
                    sink_w: Optional[torch.Tensor] = None, gate_elem: bool = False) -> torch.Tensor:
-    """Causal attention of ``ntok`` query rows over the paged cache, one warp per (row, head).  Values may have
+    """Causal attention of ``ntok`` query rows over the paged cache, float32 arithmetic.  Values may have
     another size than keys (``v_pages [..., dv]``, ``out [ntok, nh, dv]``); ``sink`` adds a key of score 0 without a
     value; ``gate`` (float32 ``[ntok, >= nh]``, a view of wider rows is fine) multiplies head h's output by
     sigmoid(gate[t, h]); ``cap`` > 0 caps the scores by cap tanh(s / cap); keys at positions below ``keep_first`` stay

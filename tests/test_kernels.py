@@ -456,6 +456,20 @@ def test_attention_rows_over_pages(K, dtype, nh, nkvh, dh, page, window):
     _close(got, want, dtype, scale=2.0)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("nh,nkvh,dh,page,window", [(1, 1, 4, 16, None), (40, 1, 20, 8, None), (6, 2, 6, 4, 50), (3, 3, 512, 16, 33), (16, 1, 130, 16, 31)])
+def test_attention_rows_tiles(K, dtype, nh, nkvh, dh, page, window):
+    """Tiles of rows at their edges (32, 16, 10 and 2 rows of a request a block, more heads than a block takes), the rest of the
+    cache not a number, and every row alone: the same bits."""
+    lens = [70, 33, 1, 65]
+    queries = [list(range(3, 70)), [32], [0], list(range(31, 65))]
+    got, want, _ = _attention_case(K, dtype, nh, nkvh, dh, page, window, lens, queries, seed=dh, junk=float("nan"))
+    _close(got, want, dtype, scale=2.0)
+    # the same rows as other tiles: one request less ahead of them
+    less, _, _ = _attention_case(K, dtype, nh, nkvh, dh, page, window, lens, [list(range(5, 70)), [], [0], list(range(31, 65))], seed=dh, junk=float("nan"))
+    assert torch.equal(torch.cat([got[2:67], got[68:]]), less)
+
+
 # grouped heads of 64 or 128: the decode kernel that puts the group on the tensor cores (16 heads fill a tile;
 # 20 need a second one; 2 to 7 leave most of it empty)
 GROUPED = [(32, 2, 128, 16, None), (10, 2, 64, 16, 70), (40, 2, 128, 8, None), (6, 1, 64, 32, 33), (7, 1, 128, 5, None),
