@@ -622,6 +622,21 @@ def test_sample_matches_the_plain_rule(K, V):
     assert not miss, miss[:5]
 
 
+@pytest.mark.parametrize("V", [1, 384, 2048, 5000])
+def test_sample_with_ties_and_long_candidate_lists(K, V):
+    """Equal logits at the cut, more of them than the kernel's list holds, cuts at and beyond the threads of a block, masses that
+    round to nothing.  Whole numbers: the running masses are far from any pick's edge."""
+    g = torch.Generator().manual_seed(V)
+    cases = [(t, k, p, u) for t in (0.5, 2.0) for k in (0, 2, 50, 1024, 1025, V) for p in (1.0, 0.7, 0.0) for u in (0.0, 0.4001, 0.9003)]
+    rows = [torch.zeros(V), torch.randint(0, 4, (V,), generator=g).float(), torch.randint(-40, 4, (V,), generator=g).float()]
+    for row in rows:
+        f = lambda j, dt: torch.tensor([c[j] for c in cases], dtype=dt, device=DEV)
+        out = torch.empty(len(cases), dtype=torch.int32, device=DEV)
+        K.sample(row.repeat(len(cases), 1).to(DEV), f(0, torch.float32), f(1, torch.int32), f(2, torch.float32), f(3, torch.float32), out)
+        want = [plain_sample(row, *c) for c in cases]
+        assert out.tolist() == want, [(c, a, b) for c, a, b in zip(cases, out.tolist(), want) if a != b][:5]
+
+
 def test_sample_is_reproducible_and_follows_the_distribution(K):
     V, n = 50, 4000
     g = torch.Generator().manual_seed(1)
