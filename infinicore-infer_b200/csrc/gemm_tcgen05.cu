@@ -10,7 +10,7 @@
 //              accumulator to the epilogue;
 //   tiles      a block is persistent: it walks over output tiles with two accumulators in tensor
 //              memory, so that the epilogue of one tile runs while the next tile's products are issued;
-//   epilogue   four warps read the accumulator with tcgen05.ld (each warp its quarter of the
+//   epilogue   eight warps read the accumulator with tcgen05.ld (two warps a quarter of the
 //              lanes; a thread holds 32 consecutive columns of one row), stage 32 rows x 128 bytes in
 //              swizzled shared memory and hand them to TMA (a store, or a reduce-add for the residual:
 //              the memory system does x += value, the SM never reads x) and apply one of
@@ -26,7 +26,7 @@
 //                              float32 copy of the product in between: src/models/jiuge/jiuge.cpp:200-218).
 // Rows, columns and the K range that a tile has beyond the matrices are zero-filled by TMA and
 // never stored.  Warp roles: warp 0 TMA, warp 1 MMA (and owner of the tensor-memory allocation),
-// warps 2..5 epilogue.  Every wait on an mbarrier is bounded; a wait that runs out records a code in
+// warps 2..9 epilogue.  Every wait on an mbarrier is bounded; a wait that runs out records a code in
 // `status`, the roles drain what is in flight, tensor memory is freed and the kernel returns.
 //
 // (The reference sends these products to a library: src/models/inference_context.cpp:59-79; the
@@ -61,11 +61,15 @@ struct TgArgs {
     int gate_act;      // EPI_SWIGLU: JkGateAct of the gate
 };
 
+// Eight epilogue warps: two share the 32 rows of a lane quarter and take turns at the tile's passes of columns.  With four, a
+// tile of 128 x 128 gated units or 128 x 256 rotated columns took longer to finish than the products of the next one.
+constexpr int TG_EPI_WARPS = 8, TG_GEMM_THREADS = 64 + 32 * TG_EPI_WARPS;
+
 template <int BN, int CTAS> struct TgSmem {
     static constexpr int STAGES = CTAS == 2 ? 6 : TG_STAGES;
     __nv_bfloat16 a[STAGES][TG_BM * TG_BK];          // 16 KB each, 1024-byte aligned
     __nv_bfloat16 b[STAGES][BN / CTAS * TG_BK];
-    unsigned char stage_out[4][4096];                // per epilogue warp: 32 rows x 128 bytes, swizzled
+    unsigned char stage_out[TG_EPI_WARPS][4096];     // per epilogue warp: 32 rows x 128 bytes, swizzled
     unsigned long long full[STAGES], empty[STAGES], acc_full[2], acc_empty[2];
     unsigned tmem_base;
 };
@@ -90,7 +94,7 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
 }
 
 template <int BN, int EPI, int CTAS>
-__global__ void __launch_bounds__(TG_THREADS)
+__global__ void __launch_bounds__(TG_GEMM_THREADS)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ CUtensorMap map_out, TgArgs a) {
     extern __shared__ unsigned char tg_raw[];
@@ -115,7 +119,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < STAGES; ++i) { mbar_init(&s.full[i], 1); mbar_init(&s.empty[i], 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(&s.acc_full[i], 1); mbar_init(&s.acc_empty[i], 4 * CTAS); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&s.acc_full[i], 1); mbar_init(&s.acc_empty[i], TG_EPI_WARPS * CTAS); }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == 1) {
@@ -219,10 +223,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (failed) atomicExch(a.status, 2);
         }
     } else {
-        // ---- epilogue: warps 2..5, each owns the 32 lanes (rows) warp % 4 of the accumulator ----
+        // ---- epilogue: warps 2..9; warp w has the 32 lanes (rows) w % 4 of the accumulator and every second pass of columns ----
         pdl_wait();                       // what follows reads and writes what earlier kernels wrote
-        const int quarter = warp & 3;
-        unsigned char *stage = s.stage_out[quarter];
+        const int quarter = warp & 3, turn = (warp - 2) >> 2;
+        unsigned char *stage = s.stage_out[warp - 2];
         int j = 0;
         // handing an accumulator back: the issuing block's barrier counts the epilogue warps of the whole pair
         auto release_accumulator = [&](int buf) {
@@ -269,7 +273,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 };
                 if (cs != nullptr && half == 32) load_angles(0);
 #pragma unroll 1
-                for (int c0 = 0; c0 < OUT_COLS; c0 += d.dh) {
+                for (int c0 = turn * d.dh; c0 < OUT_COLS; c0 += 2 * d.dh) {
                     if (n0 + c0 >= a.N) break;                             // warp-uniform
                     const int h = (n0 + c0) / d.dh;
                     __nv_bfloat16 *dst;
@@ -313,7 +317,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             // columns per pass: a staging row is 128 bytes = 32 floats or 64 bfloat16
             constexpr int PASS = (EPI == EPI_F32 || EPI == EPI_RESIDUAL) ? 32 : 64;
 #pragma unroll 1
-            for (int c0 = 0; c0 < OUT_COLS; c0 += PASS) {
+            for (int c0 = turn * PASS; c0 < OUT_COLS; c0 += 2 * PASS) {
                 const int col = n0 + c0;
                 if (col >= a.N) break;                                     // warp-uniform
                 if (!a.direct) {
@@ -405,7 +409,7 @@ static int launch_tg(const CUtensorMap &ma, const CUtensorMap &mw, const CUtenso
     if (e != cudaSuccess) JK_FAIL(JK_CUDA_ERROR, "gemm_tcgen05: %s", cudaGetErrorString(e));
     const int out_cols = EPI == EPI_SWIGLU ? BN / 2 : BN;
     const int tiles = ((a.N + out_cols - 1) / out_cols) * ((a.M + TG_BM - 1) / TG_BM) * (a.ksplit > 1 ? a.ksplit : 1);
-    jk_launch(gemm_tcgen05_kernel<BN, EPI, 1>, dim3(tiles < sms ? tiles : sms), dim3(TG_THREADS), smem, stream, ma, mw, mo, a);
+    jk_launch(gemm_tcgen05_kernel<BN, EPI, 1>, dim3(tiles < sms ? tiles : sms), dim3(TG_GEMM_THREADS), smem, stream, ma, mw, mo, a);
     JK_CHECK_LAUNCH("gemm_tcgen05");
     return JK_OK;
 }
@@ -424,7 +428,7 @@ static int launch_tg_pair(const CUtensorMap &ma, const CUtensorMap &mw, const CU
     static int resident = 0;
     if (resident == 0) {
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * (sms / 2)); cfg.blockDim = dim3(TG_THREADS); cfg.dynamicSmemBytes = smem;
+        cfg.gridDim = dim3(2 * (sms / 2)); cfg.blockDim = dim3(TG_GEMM_THREADS); cfg.dynamicSmemBytes = smem;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
@@ -437,7 +441,7 @@ static int launch_tg_pair(const CUtensorMap &ma, const CUtensorMap &mw, const CU
         resident = n < sms / 2 ? n : sms / 2;
     }
     const int pairs = tiles < resident ? tiles : resident;
-    e = jk_launch_clusters(kernel, 2, dim3(2 * pairs), dim3(TG_THREADS), smem, stream, ma, mw, mo, a);
+    e = jk_launch_clusters(kernel, 2, dim3(2 * pairs), dim3(TG_GEMM_THREADS), smem, stream, ma, mw, mo, a);
     if (e != cudaSuccess) JK_FAIL(JK_CUDA_ERROR, "gemm_tcgen05 (pairs): %s", cudaGetErrorString(e));
     return JK_OK;
 }
