@@ -53,7 +53,8 @@ constexpr int AT_POLY_OF_8 = 2;
 
 struct AtArgs {
     __nv_bfloat16 *out;       // [T, nh, dv]
-    const int *tiles;         // [ntiles][2]: batch entry, first row of the tile (row index in the step); most keys first
+    const int *tiles;         // [ntiles][2]: batch entry, first row of the tile (row index in the step); most keys first.
+                              // LAID heads: [ntiles][3], with the row of `k` and `v` that holds the request's position 0; entry < 0: no tile
     const int *req_start;     // [nreq + 1]
     const int *req_pos;       // [nreq]
     const int *block_table;   // [nreq, max_blocks]
@@ -67,7 +68,13 @@ struct AtArgs {
     int keep_first;           // with a window: keys at positions below this stay visible when the window has passed them
     const float *sink_w;
     int dk, dv;               // sizes of a key and of a value head (DK and DV are these rounded up to 64 or 128)
+    int rot_ld, rot_off;      // LAID_ROT: columns between two heads of the queries' rotated parts, and before the first one
 };
+
+// Where a tile's keys and values come from.  PAGED: cached heads, page by page.  LAID: heads made for this step, rows of all
+// requests' positions one after the other (csrc/blocks.cu: latent_gather), a head's keys and values side by side columns of
+// these rows.  LAID_ROT: the same, and 64 elements more that all heads share, in rows of their own.
+enum { AT_PAGED = 0, AT_LAID = 1, AT_LAID_ROT = 2 };
 
 // ---- PTX wrappers (see gemm_tcgen05.cu for the same set) -----------------------------------------
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -222,9 +229,10 @@ __host__ __device__ constexpr unsigned instr_desc(int n, bool b_mn) {
 
 template <int DK, int DV> struct AtSmem {
     static constexpr int SUB_K = DK / 64, SUB_V = DV / 64;    // 64-wide sub-tiles along the head
+    static constexpr int STAGES_V = DK > 128 ? 1 : 2;         // keys of 192 leave room for one tile of values of 128
     __nv_bfloat16 q[SUB_K][AT_BM * 64];                       // K-major, per sub-tile [128 rows][64]
     __nv_bfloat16 k[2][SUB_K][AT_BN * 64];                    // two stages
-    __nv_bfloat16 v[2][SUB_V][AT_BN * 64];
+    __nv_bfloat16 v[STAGES_V][SUB_V][AT_BN * 64];
     __nv_bfloat16 p[2][AT_BM * 64];                           // [128 rows][128 keys] as two sub-tiles of 64 keys
     unsigned long long q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full, s_free, p_ready, pv_done, met[4];
     unsigned tmem_base;
@@ -235,11 +243,13 @@ template <int DK, int DV> struct AtSmem {
 // Keys and values may differ in size.  Heads of dk or dv elements that are no multiple of 64 run as ones of DK or DV: TMA fills what
 // lies beyond a cached row with zeros (of a query row it brings the next head's elements, which meet the keys' zeros), and columns
 // of the output beyond dv are not written.
-template <int DK, int DV, bool ELEM>
+template <int DK, int DV, bool ELEM, int FROM = AT_PAGED>
 __global__ void __launch_bounds__(AT_THREADS, DK <= 64 && DV <= 64 ? 2 : 1)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                         const __grid_constant__ CUtensorMap map_v, AtArgs a) {
-    constexpr int SUB_K = DK / 64, SUB_V = DV / 64;
+                         const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_q_rot,
+                         const __grid_constant__ CUtensorMap map_k_rot, AtArgs a) {
+    constexpr int SUB_K = DK / 64, SUB_V = DV / 64, SUB_PLAIN = FROM == AT_LAID_ROT ? SUB_K - 1 : SUB_K;
+    constexpr int STAGES_V = AtSmem<DK, DV>::STAGES_V;
     constexpr unsigned TMEM_COLS = DV <= 64 ? 256 : 512;      // S: 128 columns; two accumulators of DV columns
     extern __shared__ __align__(1024) unsigned char at_raw[];      // swizzled tiles need 1024-byte alignment
     AtSmem<DK, DV> &s = *reinterpret_cast<AtSmem<DK, DV> *>(at_raw);
@@ -271,8 +281,14 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     pdl_trigger();
     pdl_wait();
 
-    const int r = a.tiles[2 * tile];
-    const int row0 = a.tiles[2 * tile + 1];
+    const int r = a.tiles[(FROM == AT_PAGED ? 2 : 3) * tile];
+    if (FROM != AT_PAGED && r < 0) {                           // the list is shorter than the launch
+        __syncthreads();
+        if (warp == 1) tmem_dealloc(s.tmem_base, TMEM_COLS);
+        return;
+    }
+    const int row0 = a.tiles[(FROM == AT_PAGED ? 2 : 3) * tile + 1];
+    const int base = FROM == AT_PAGED ? 0 : a.tiles[3 * tile + 2];
     const int nrows = min(AT_BM, a.req_start[r + 1] - row0);
     const int p0 = a.req_pos[r] + (row0 - a.req_start[r]);    // position of the tile's first row
     const int p_last = p0 + nrows - 1;
@@ -283,15 +299,16 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     const int n_kept = a.keep_first > 0 ? (min(a.keep_first, kv_first) + AT_BN - 1) / AT_BN : 0;
     const int n_kv = n_kept + (p_last - kv_first) / AT_BN + 1;
     auto tile_at = [&](int i) { return i < n_kept ? i * AT_BN : kv_first + (i - n_kept) * AT_BN; };
-    const int *bt = a.block_table + (size_t)r * a.max_blocks;
-    const int pages_per_tile = AT_BN / a.page_size;
+    const int *bt = FROM == AT_PAGED ? a.block_table + (size_t)r * a.max_blocks : nullptr;
+    const int pages_per_tile = FROM == AT_PAGED ? AT_BN / a.page_size : 1;
     int failed = 0;
 
     if (warp == 0) {
         // ---- TMA producer: the whole warp; lane = (page of the tile, 64-wide part of the head) ----
         if (lane == 0) {
             mbar_expect_tx(&s.q_full, AT_BM * DK * 2);
-            for (int u = 0; u < SUB_K; ++u) tma_load_2d(s.q[u], &map_q, &s.q_full, h * a.dk + u * 64, row0);
+            for (int u = 0; u < SUB_PLAIN; ++u) tma_load_2d(s.q[u], &map_q, &s.q_full, h * a.dk + u * 64, row0);
+            if (FROM == AT_LAID_ROT) tma_load_2d(s.q[SUB_K - 1], &map_q_rot, &s.q_full, h * a.rot_ld + a.rot_off, row0);
         }
         for (int i = 0; i < n_kv && !failed; ++i) {
             const int st = i & 1, kv0 = tile_at(i);
@@ -299,6 +316,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             // a page beyond what the request holds is never looked at: its keys are masked
             int pg = lane / SUB_K, u = lane % SUB_K;
             auto first_row = [&]() {
+                if (FROM != AT_PAGED) return base + kv0;
                 const int blk = kv0 / a.page_size + pg;
                 const int page = (pg < pages_per_tile && blk < a.max_blocks) ? bt[blk] : 0;
                 return (page * a.nkvh + hk) * a.page_size;
@@ -306,19 +324,28 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             int grow = first_row();
             for (int kind = 0; kind < 2; ++kind) {               // 0: keys, 1: values
                 if (SUB_K != SUB_V && kind == 1) { pg = lane / SUB_V; u = lane % SUB_V; grow = first_row(); }
-                unsigned long long *empty = kind ? &s.v_empty[st] : &s.k_empty[st];
-                unsigned long long *full = kind ? &s.v_full[st] : &s.k_full[st];
+                const int stages = kind ? STAGES_V : 2, sk = kind ? i % STAGES_V : st;
+                unsigned long long *empty = kind ? &s.v_empty[sk] : &s.k_empty[sk];
+                unsigned long long *full = kind ? &s.v_full[sk] : &s.k_full[sk];
                 int ok = 1;
-                if (i >= 2) {
-                    if (lane == 0) ok = mbar_wait(empty, ((i >> 1) - 1) & 1) ? 1 : 0;
+                if (i >= stages) {
+                    if (lane == 0) ok = mbar_wait(empty, (i / stages - 1) & 1) ? 1 : 0;
                     ok = __shfl_sync(0xffffffffu, ok, 0);
                 }
                 if (!ok) { failed = 1; break; }
                 if (lane == 0) mbar_expect_tx(full, AT_BN * (kind ? DV : DK) * 2);
                 __syncwarp();
                 if (pg < pages_per_tile) {                       // at most 16 pages x 2 parts
-                    __nv_bfloat16 *dst = (kind ? s.v[st][u] : s.k[st][u]) + pg * a.page_size * 64;
-                    tma_load_2d(dst, kind ? &map_v : &map_k, full, u * 64, grow);
+                    if (FROM == AT_PAGED) {
+                        __nv_bfloat16 *dst = (kind ? s.v[sk][u] : s.k[sk][u]) + pg * a.page_size * 64;
+                        tma_load_2d(dst, kind ? &map_v : &map_k, full, u * 64, grow);
+                    } else if (kind) {
+                        tma_load_2d(s.v[sk][u], &map_v, full, h * a.dv + u * 64, grow);
+                    } else if (u < SUB_PLAIN) {
+                        tma_load_2d(s.k[sk][u], &map_k, full, h * a.dk + u * 64, grow);
+                    } else {
+                        tma_load_2d(s.k[sk][u], &map_k_rot, full, 0, grow);
+                    }
                 }
             }
         }
@@ -332,11 +359,11 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             constexpr unsigned desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
             auto lo_k = [](const void *tile) { return ((smem_u32(tile) & 0x3FFFFu) >> 4) | (1u << 16); };
             auto lo_mn = [](const void *tile) { return ((smem_u32(tile) & 0x3FFFFu) >> 4) | ((unsigned)((AT_BN * 64 * 2) >> 4) << 16); };
-            unsigned q_lo[SUB_K], k_lo[2][SUB_K], p_lo[2], v_lo[2];
+            unsigned q_lo[SUB_K], k_lo[2][SUB_K], p_lo[2], v_lo[2];       // one stage of values: both the same
 #pragma unroll
             for (int u = 0; u < SUB_K; ++u) { q_lo[u] = lo_k(s.q[u]); k_lo[0][u] = lo_k(s.k[0][u]); k_lo[1][u] = lo_k(s.k[1][u]); }
             p_lo[0] = lo_k(s.p[0]); p_lo[1] = lo_k(s.p[1]);
-            v_lo[0] = lo_mn(s.v[0][0]); v_lo[1] = lo_mn(s.v[1][0]);
+            v_lo[0] = lo_mn(s.v[0][0]); v_lo[1] = lo_mn(s.v[STAGES_V - 1][0]);
             auto issue_qk = [&](int st) {
 #pragma unroll
                 for (int u = 0; u < SUB_K; ++u)
@@ -365,7 +392,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 }
                 if (!mbar_wait(&s.p_ready, i & 1)) { failed = 2; break; }          // P_i is written
                 tc_fence_after();
-                if (!mbar_wait(&s.v_full[st], (i >> 1) & 1)) { failed = 2; break; }
+                if (!mbar_wait(&s.v_full[i % STAGES_V], (i / STAGES_V) & 1)) { failed = 2; break; }
                 tc_fence_after();
 #pragma unroll
                 for (int k = 0; k < AT_BN / 16; ++k) {   // 16 keys per instruction
@@ -375,7 +402,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                                     (st ? v_lo[1] : v_lo[0]) + ((k * 16 * 128) >> 4), desc_hi, idesc_pv, (i | (k % 4)) ? 1u : 0u);
                 }
                 umma_commit(&s.pv_done);
-                umma_commit(&s.v_empty[st]);
+                umma_commit(&s.v_empty[i % STAGES_V]);
             }
             if (failed) atomicExch(a.status, 12);
         }
@@ -485,11 +512,11 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             // holder of the page left there.  Those rows become zeros before the product reads them (only the last
             // tile of keys has any; the first half's threads take one key row each).
             if (i == n_kv - 1 && half == 0 && tile_at(i) + AT_BN - 1 > p_last) {
-                if (!__all_sync(0xffffffffu, mbar_wait(&s.v_full[i & 1], (i >> 1) & 1))) { alive = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(&s.v_full[i % STAGES_V], (i / STAGES_V) & 1))) { alive = false; break; }
                 if (tile_at(i) + row > p_last) {
 #pragma unroll
                     for (int u = 0; u < SUB_V; ++u) {
-                        uint4 *vrow = reinterpret_cast<uint4 *>(s.v[i & 1][u] + row * 64);      // 128 bytes; the swizzle stays inside
+                        uint4 *vrow = reinterpret_cast<uint4 *>(s.v[i % STAGES_V][u] + row * 64);      // 128 bytes; the swizzle stays inside
 #pragma unroll
                         for (int c = 0; c < 8; ++c) vrow[c] = make_uint4(0u, 0u, 0u, 0u);
                     }
@@ -563,7 +590,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     // a role that gave up may leave copies in flight: bounded time to land before memory is released
     if (failed && lane == 0) {
         mbar_wait(&s.q_full, 0);
-        for (int st = 0; st < 2; ++st) { mbar_wait(&s.k_full[st], 0); mbar_wait(&s.v_full[st], 0); }
+        for (int st = 0; st < 2; ++st) { mbar_wait(&s.k_full[st], 0); mbar_wait(&s.v_full[st % STAGES_V], 0); }
     }
     tc_fence_before();
     __syncthreads();
@@ -587,19 +614,21 @@ static EncodeTiledFn encode_fn() {
     });
     return fn;
 }
-// A 2-D bfloat16 tensor map [rows, cols] with boxes of 64 columns x box_rows, 128-byte swizzle; cached.
-static int tensor_map(const void *ptr, long long rows, int cols, int box_rows, CUtensorMap *out) {
-    using Key = std::tuple<const void *, long long, int, int>;
+// A 2-D bfloat16 tensor map [rows, cols], rows `ld` elements apart (0: cols), with boxes of 64 columns x box_rows, 128-byte
+// swizzle; cached.
+static int tensor_map(const void *ptr, long long rows, int cols, int box_rows, CUtensorMap *out, int ld = 0) {
+    if (ld <= 0) ld = cols;
+    using Key = std::tuple<const void *, long long, int, int, int>;
     static std::map<Key, CUtensorMap> cache;
     static std::mutex mu;
     std::lock_guard<std::mutex> lock(mu);
-    const Key key(ptr, rows, cols, box_rows);
+    const Key key(ptr, rows, cols, box_rows, ld);
     auto it = cache.find(key);
     if (it != cache.end()) { *out = it->second; return JK_OK; }
     EncodeTiledFn fn = encode_fn();
     if (!fn) JK_FAIL(JK_CUDA_ERROR, "attention_tcgen05: the driver has no cuTensorMapEncodeTiled");
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+    const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
     const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
     const cuuint32_t elem[2] = {1, 1};
     CUtensorMap m;
@@ -619,12 +648,15 @@ JK_EXPORT int jk_attention_tcgen05_supports(int dh, int page_size) {
     return (dh == 64 || dh == 128) && (page_size == 8 || page_size == 16 || page_size == 32 || page_size == 64 || page_size == 128);
 }
 
-template <int DK, int DV, bool ELEM>
-static int launch_at(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const AtArgs &a, cudaStream_t stream) {
+template <int DK, int DV, bool ELEM, int FROM = AT_PAGED>
+static int launch_at(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const CUtensorMap &mqr, const CUtensorMap &mkr,
+                     const AtArgs &a, cudaStream_t stream) {
     const size_t smem = sizeof(AtSmem<DK, DV>);
-    cudaError_t e = cudaFuncSetAttribute(attention_tcgen05_kernel<DK, DV, ELEM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static_assert(sizeof(AtSmem<DK, DV>) <= 227 * 1024, "shared memory");
+    auto kernel = attention_tcgen05_kernel<DK, DV, ELEM, FROM>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) JK_FAIL(JK_CUDA_ERROR, "attention_tcgen05: %s", cudaGetErrorString(e));
-    jk_launch(attention_tcgen05_kernel<DK, DV, ELEM>, dim3(a.nh, a.ntiles), dim3(AT_THREADS), smem, stream, mq, mk, mv, a);
+    jk_launch(kernel, dim3(a.nh, a.ntiles), dim3(AT_THREADS), smem, stream, mq, mk, mv, mqr, mkr, a);
     JK_CHECK_LAUNCH("attention_tcgen05");
     return JK_OK;
 }
@@ -646,10 +678,10 @@ JK_EXPORT int jk_attention_tcgen05(const void *q, const void *k_pages, const voi
     if (int rc = tensor_map(v_pages, (long long)num_pages * nkvh * page_size, dv, page_size, &mv)) return rc;
     AtArgs a{(__nv_bfloat16 *)out, tiles, req_start, req_pos, block_table, status,
              ntiles, nh, nkvh, page_size, max_blocks, window, scale * 1.4426950408889634f, sink, gate, gate_ld,
-             cap > 0.f ? cap / scale : 0.f, window > 0 ? keep_first : 0, sink_w, dh, dv};
+             cap > 0.f ? cap / scale : 0.f, window > 0 ? keep_first : 0, sink_w, dh, dv, 0, 0};
     JK_REQUIRE(cap >= 0.f && keep_first >= 0 && scale > 0.f, "attention_tcgen05: cap %g, %d kept keys, scale %g", cap, keep_first, scale);
     const bool elem = gate != nullptr && gate_elem;
-#define LAUNCH_AT(DK, DV) return elem ? launch_at<DK, DV, true>(mq, mk, mv, a, stream) : launch_at<DK, DV, false>(mq, mk, mv, a, stream)
+#define LAUNCH_AT(DK, DV) return elem ? launch_at<DK, DV, true>(mq, mk, mv, mq, mk, a, stream) : launch_at<DK, DV, false>(mq, mk, mv, mq, mk, a, stream)
     if (dh <= 64) {
         if (dv <= 64) LAUNCH_AT(64, 64);
         LAUNCH_AT(64, 128);
@@ -657,4 +689,40 @@ JK_EXPORT int jk_attention_tcgen05(const void *q, const void *k_pages, const voi
     if (dv <= 64) LAUNCH_AT(128, 64);
     LAUNCH_AT(128, 128);
 #undef LAUNCH_AT
+}
+
+// Attention over heads that were made for this step from latent rows (csrc/blocks.cu): `kv` [rows, nh dh | nh dh] keys and
+// values of all requests' positions one after the other, `k_rot` [rows, 64] the part of a key that all heads share (null:
+// none).  `q` [ntok, nh dh], and with `k_rot` the queries' rotated parts at columns h * rot_ld + rot_off of rows of q_rot
+// [ntok, nh rot_ld].  `tiles` [ntiles][3] as in AtArgs.  out [ntok, nh dh].
+JK_EXPORT int jk_attention_laid_tcgen05(const void *q, const void *q_rot, int rot_ld, int rot_off, const void *kv, const void *k_rot, long long rows,
+                                        void *out, const int *tiles, int ntiles, int ntok, const int *req_start, const int *req_pos, int nh,
+                                        int dh, float scale, int window, int *status, const float *sink_w, const float *gate, int gate_ld,
+                                        int gate_elem, cudaStream_t stream) {
+    if (ntiles == 0 || ntok == 0) return JK_OK;
+    JK_REQUIRE(dh == 64 || dh == 128, "attention_laid: heads of %d are not built", dh);
+    JK_REQUIRE(q && kv && out && tiles && req_start && req_pos && status && (k_rot == nullptr || q_rot != nullptr), "attention_laid: an argument is missing");
+    JK_REQUIRE(ntiles > 0 && ntiles <= 65535 && nh > 0 && rows > 0 && scale > 0.f && window >= 0, "attention_laid: tiles %d, heads %d", ntiles, nh);
+    JK_REQUIRE(k_rot == nullptr || (rot_ld % 8 == 0 && rot_off % 8 == 0 && rot_off + 64 <= rot_ld), "attention_laid: rotated parts at %d of %d", rot_off, rot_ld);
+    JK_REQUIRE(gate == nullptr || gate_ld >= nh * (gate_elem ? dh : 1), "attention_laid: a gate row of %d holds no %d heads", gate_ld, nh);
+    CUtensorMap mq, mk, mv, mqr, mkr;
+    if (int rc = tensor_map(q, ntok, nh * dh, AT_BM, &mq)) return rc;
+    if (int rc = tensor_map(kv, rows, nh * dh, AT_BN, &mk, 2 * nh * dh)) return rc;
+    if (int rc = tensor_map((const __nv_bfloat16 *)kv + nh * dh, rows, nh * dh, AT_BN, &mv, 2 * nh * dh)) return rc;
+    mqr = mq, mkr = mk;
+    if (k_rot != nullptr) {
+        if (int rc = tensor_map(q_rot, ntok, nh * rot_ld, AT_BM, &mqr)) return rc;
+        if (int rc = tensor_map(k_rot, rows, 64, AT_BN, &mkr)) return rc;
+    }
+    AtArgs a{(__nv_bfloat16 *)out, tiles, req_start, req_pos, nullptr, status, ntiles, nh, nh, 1, 1, window, scale * 1.4426950408889634f,
+             sink_w != nullptr, gate, gate_ld, 0.f, 0, sink_w, dh, dh, rot_ld, rot_off};
+    const bool elem = gate != nullptr && gate_elem;
+#define LAUNCH_LAID(DK, DV, FROM) return elem ? launch_at<DK, DV, true, FROM>(mq, mk, mv, mqr, mkr, a, stream) : launch_at<DK, DV, false, FROM>(mq, mk, mv, mqr, mkr, a, stream)
+    if (dh == 64) {
+        if (k_rot != nullptr) LAUNCH_LAID(128, 64, AT_LAID_ROT);
+        LAUNCH_LAID(64, 64, AT_LAID);
+    }
+    if (k_rot != nullptr) LAUNCH_LAID(192, 128, AT_LAID_ROT);
+    LAUNCH_LAID(128, 128, AT_LAID);
+#undef LAUNCH_LAID
 }

@@ -1229,6 +1229,83 @@ __global__ void __launch_bounds__(256) latent_attention_tc_kernel(LatentTcArgs a
     }
 }
 
+// ---- heads made from the latent rows, for steps of many rows ---------------------------------------------------------
+// Between `rows` query rows and the same positions the attention over the latent rows themselves does R + dr + R multiply-adds
+// a pair and head, the one over heads made from them dn + dr + dv, at the price of one product [R] -> [H (dn + dv)] per
+// position: the cheaper way from some rows a request on (jk::latent_takes_heads).  This kernel lays the positions of all requests
+// one after the other: their latent vectors [C, R] (the product's operand), their shared key parts [C, dr], and the list of query
+// tiles, the ones that see most keys first: (request, first row, row of the request's position 0), filled up with request -1.
+struct GatherArgs {
+    const __nv_bfloat16 *pages;
+    const int *block_table, *req_start, *req_pos;
+    __nv_bfloat16 *latent, *rot;
+    int *tiles;
+    int nreq, R, dr, page_size, max_blocks, keys, ntiles, tile_rows;
+};
+constexpr int LG_THREADS = 256, LG_ROWS = 8;
+__global__ void __launch_bounds__(LG_THREADS) latent_gather_kernel(GatherArgs a) {
+    pdl_trigger();
+    pdl_wait();
+    const int D = a.R + a.dr;
+    if (blockIdx.x == 0) {          // the list: a tile's place is the number of tiles that see more keys, or as many and come before it
+        for (int i = threadIdx.x; i < a.ntiles; i += LG_THREADS) {
+            int n = 0, base = 0, mine[4] = {-1, 0, 0, 0};
+            for (int r = 0; r < a.nreq && mine[0] < 0; ++r) {
+                const int len = a.req_start[r + 1] - a.req_start[r], tiles = (len + a.tile_rows - 1) / a.tile_rows;
+                if (i < n + tiles) { mine[0] = r; mine[1] = a.req_start[r] + (i - n) * a.tile_rows; mine[2] = base; mine[3] = a.req_pos[r] + (i - n) * a.tile_rows; }
+                n += tiles;
+                base += a.req_pos[r] + len;
+            }
+            int place = 0;
+            if (mine[0] < 0) {
+                place = i;
+            } else {
+                int at = 0;
+                for (int r = 0; r < a.nreq; ++r) {
+                    const int tiles = (a.req_start[r + 1] - a.req_start[r] + a.tile_rows - 1) / a.tile_rows;
+                    for (int t = 0; t < tiles; ++t, ++at) {
+                        const int keys = a.req_pos[r] + t * a.tile_rows;
+                        place += keys > mine[3] || (keys == mine[3] && at < i);
+                    }
+                }
+            }
+            a.tiles[3 * place] = mine[0];
+            a.tiles[3 * place + 1] = mine[1];
+            a.tiles[3 * place + 2] = mine[2];
+        }
+        return;
+    }
+    const int vectors = D / 8;
+    for (int k = 0; k < LG_ROWS; ++k) {
+        const int row = ((int)blockIdx.x - 1) * LG_ROWS + k;
+        if (row >= a.keys) return;
+        int base = 0, r = 0;
+        for (; r < a.nreq; ++r) {
+            const int n = a.req_pos[r] + a.req_start[r + 1] - a.req_start[r];
+            if (row < base + n) break;
+            base += n;
+        }
+        if (r == a.nreq) return;
+        const int j = row - base, page = a.block_table[(size_t)r * a.max_blocks + j / a.page_size];
+        const __nv_bfloat16 *src = a.pages + ((size_t)page * a.page_size + (size_t)(j % a.page_size)) * D;
+        for (int v = threadIdx.x; v < vectors; v += LG_THREADS) {
+            const uint4 x = *reinterpret_cast<const uint4 *>(src + v * 8);
+            if (v * 8 < a.R) *reinterpret_cast<uint4 *>(a.latent + (size_t)row * a.R + v * 8) = x;
+            else *reinterpret_cast<uint4 *>(a.rot + (size_t)row * a.dr + v * 8 - a.R) = x;
+        }
+    }
+}
+JK_EXPORT int jk_latent_gather(const void *pages, const int *block_table, int max_blocks, int page_size, const int *req_start, const int *req_pos,
+                               int nreq, int R, int dr, void *latent, void *rot, int keys, int *tiles, int ntiles, int tile_rows, cudaStream_t stream) {
+    JK_REQUIRE(pages && block_table && req_start && req_pos && latent && tiles && (rot || dr == 0), "latent_gather: an argument is missing");
+    JK_REQUIRE(R > 0 && R % 8 == 0 && dr % 8 == 0 && keys > 0 && ntiles > 0 && nreq > 0 && page_size > 0, "latent_gather: rows of %d + %d", R, dr);
+    GatherArgs a{(const __nv_bfloat16 *)pages, block_table, req_start, req_pos, (__nv_bfloat16 *)latent, (__nv_bfloat16 *)rot, tiles,
+                 nreq, R, dr, page_size, max_blocks, keys, ntiles, tile_rows};
+    jk_launch(latent_gather_kernel, dim3((keys + LG_ROWS - 1) / LG_ROWS + 1), dim3(LG_THREADS), 0, stream, a);
+    JK_CHECK_LAUNCH("latent_gather");
+    return JK_OK;
+}
+
 static bool latent_tc_enabled() {
     static const bool on = [] { const char *e = std::getenv("JK_LATENT_NO_TC"); return !(e && e[0] == '1'); }();
     return on;

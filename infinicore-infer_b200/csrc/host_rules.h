@@ -252,6 +252,20 @@ inline bool attention_tcgen05_takes(int dh, int page_size, int dv = 0) {
     return size && (page_size == 8 || page_size == 16 || page_size == 32 || page_size == 64 || page_size == 128);
 }
 
+// Whether a latent attention over `rows` query rows of `nreq` requests makes the heads' keys and values from the latent rows
+// (one product per cached position) instead of running over the latent rows: heads of 64 or 128 for keys and values alike, a
+// rotated part of 64 or none, whole vectors; `keys`: positions of all requests, or 0 when a request brings few rows.  The line, 16
+// rows for each position within reach, lies where the product per position is shared by enough rows (B200, 16 heads of 128 + 64 and 128
+// over a latent of 512; over the latent rows -> over heads): 4 requests of 17 rows after 0 positions 37 -> 25 us, after 512
+// 102 -> 41; 64 rows after 2,048 297 -> 64; 2,048 rows after 0 887 -> 74.  Below it the way over heads costs 24 us at the least, while
+// 8 requests of one row over the latent rows take 17.
+inline bool latent_heads_fit(int dn, int dr, int dv, int R) { return dn == dv && (dn == 64 || dn == 128) && (dr == 0 || dr == 64) && R % 8 == 0 && R >= 64; }
+inline bool latent_takes_heads(int rows, int nreq, long long keys, int window, int dn, int dr, int dv, int R) {
+    if (keys <= 0 || rows < 32 || nreq <= 0 || !latent_heads_fit(dn, dr, dv, R)) return false;
+    const long long reach = window > 0 ? std::min<long long>(window, keys / nreq) : keys / nreq;
+    return rows * reach >= 16LL * keys;
+}
+
 // ---- which kernel takes a bfloat16 product ------------------------------------------------------------------------
 struct Routing {
     int sms = 148;

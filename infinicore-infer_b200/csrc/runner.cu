@@ -586,8 +586,56 @@ int run_latent_qkv(Run &r, const RunnerOp &op) {
     return JK_OK;
 }
 
+// Where the parts of a latent attention over heads made for the step lie in SLOT_HEADS (bytes, each on 256).
+struct HeadsLayout {
+    long long rot, kv, tiles, total;
+    int ntiles;
+    HeadsLayout(const RunnerOp &op, long long keys, long long rows, long long nreq) {
+        auto up = [](long long b) { return (b + 255) / 256 * 256; };
+        ntiles = (int)(rows / jk::TILE_ROWS + nreq);
+        rot = up(2 * keys * op.rank);
+        kv = up(rot + 2 * keys * op.rot_width);
+        tiles = up(kv + 2 * keys * op.heads * (op.head_dim + op.v_head_dim));
+        total = up(tiles + 12LL * ntiles);
+    }
+};
+// The three records of a latent attention ask this with the same sizes, so all run one way or the other.
+bool latent_over_heads(const Run &r, const RunnerOp &op) {
+    return op.fold != 0 && r.env.dtype == JK_BF16 && !r.env.plain_attention && !r.env.legacy_tensor_cores && !r.env.routing.library_only &&
+           g_fns.attention_laid != nullptr && g_fns.latent_gather != nullptr && r.tcgen05_bound() &&
+           jk::latent_takes_heads(r.st.ntok, r.st.nreq, r.st.tile_keys, op.window, op.head_dim, op.rot_width, op.v_head_dim, op.rank) &&
+           r.buf.slot[SLOT_HEADS] != nullptr && HeadsLayout(op, r.st.tile_keys, r.st.ntok, r.st.nreq).total <= r.buf.bytes[SLOT_HEADS];
+}
+
+int run_latent_over_heads(Run &r, const RunnerOp &op) {
+    const int T = r.st.ntok, H = op.heads, C = r.st.tile_keys, dh = op.head_dim, D = op.rank + op.rot_width;
+    void *q, *plain, *out;
+    if (int rc = r.slot(op.in_slot, 2LL * T * H * D, &q, "the queries")) return rc;
+    if (int rc = r.slot(op.in2_slot, 2LL * T * H * dh, &plain, "the queries' plain parts")) return rc;
+    if (int rc = r.slot(op.out2_slot, 2LL * T * H * dh, &out, "a latent attention's value heads")) return rc;
+    const float *gate = nullptr;
+    if (op.gated) {
+        void *u;
+        if (int rc = r.slot(SLOT_TMP, 4LL * T * op.ld, &u, "the projection that holds the gate")) return rc;
+        gate = (const float *)u + op.g_off;
+    }
+    const int *table = r.st.block_tables[op.cache_group];
+    JK_REQUIRE(table != nullptr, "runner: a latent attention reads the cache of group %d, whose block table the step lacks", op.cache_group);
+    const HeadsLayout at(op, C, T, r.st.nreq);
+    unsigned char *base = (unsigned char *)r.buf.slot[SLOT_HEADS];
+    void *rot = op.rot_width > 0 ? base + at.rot : nullptr;
+    RUN(blocks, g_fns.latent_gather(op.k_pages, table, r.env.max_blocks, r.env.page_size, r.st.req_start, r.st.req_pos, r.st.nreq, op.rank, op.rot_width,
+                                    base, rot, C, (int *)(base + at.tiles), at.ntiles, jk::TILE_ROWS, r.stream));
+    RUN(gemm_tcgen05, g_fns.gemm_tcgen05(base, op.w_heads, base + at.kv, C, 2 * H * dh, op.rank, 2 * H * dh, 1, 1.f, r.env.status, r.env.routing.sms, r.stream));
+    RUN(attention_tcgen05, g_fns.attention_laid(plain, q, D, op.rank, base + at.kv, rot, C, out, (const int *)(base + at.tiles), at.ntiles, T, r.st.req_start,
+                                                r.st.req_pos, H, dh, op.softmax_scale, op.window, r.env.status, op.sink_w, gate, op.ld, op.gated == 1,
+                                                r.stream));
+    return JK_OK;
+}
+
 int run_head_linear(Run &r, const RunnerOp &op) {
     if (int rc = need_blocks("a product per head")) return rc;
+    if (latent_over_heads(r, op)) return JK_OK;
     const int T = r.st.ntok;
     void *in, *out;
     if (int rc = r.slot(op.in_slot, (long long)r.elem() * T * op.heads * op.k, &in, "a per-head product's operand")) return rc;
@@ -613,6 +661,7 @@ int latent_splits(int T, int heads, int context, int sms, int least = 256) {
 
 int run_latent_attention(Run &r, const RunnerOp &op) {
     if (int rc = need_blocks("a latent attention")) return rc;
+    if (latent_over_heads(r, op)) return run_latent_over_heads(r, op);
     const int T = r.st.ntok, H = op.heads, D = op.rank + op.rot_width;
     void *q, *o;
     if (int rc = r.slot(op.in_slot, (long long)r.elem() * T * H * D, &q, "the queries")) return rc;
@@ -1029,6 +1078,8 @@ JK_EXPORT int jk_runner_slot_bytes(const RunnerEnv *env, const RunnerOp *ops, in
                 break;
             case OP_LATENT_ATTENTION: {
                 need(op.in_slot, e * rows * op.heads * (op.rank + op.rot_width)); need(op.out_slot, e * rows * op.heads * op.rank);
+                // four times as many positions as the step may have rows: prompts, and portions of longer ones up to there
+                if (op.fold != 0 && env->dtype == JK_BF16 && rows >= 32) need(SLOT_HEADS, HeadsLayout(op, 4 * rows, rows, rows / 16).total);
                 long long worst = 0;
                 for (int n = 1; n <= 16 && n <= max_rows; ++n)
                     worst = std::max(worst, (long long)n * op.heads * latent_splits(n, op.heads, op.max_positions, env->routing.sms, 128) * (op.rank + 2));
@@ -1091,6 +1142,9 @@ JK_EXPORT int jk_runner_needs_gemm_tcgen05(const RunnerEnv *env, const RunnerOp 
             case OP_QKV: case OP_LINEAR: case OP_REINJECT: kind = jk::PRODUCT_F32; break;
             case OP_RESIDUAL: kind = jk::PRODUCT_RESIDUAL; break;
             case OP_GATE_UP: kind = jk::PRODUCT_SWIGLU; break;
+            case OP_LATENT_ATTENTION:
+                if (op.fold != 0 && max_rows >= 32) return 1;
+                continue;
             default: continue;
         }
         for (int rows : {1, 16, 17, 128, 129, max_rows})

@@ -103,6 +103,11 @@ typedef int (*GatedRecurrenceFn)(const float *, const void *, const void *, cons
                                  const int *, int, const int *, int, float *, long long, cudaStream_t);
 typedef long long (*GatedScratchFn)(int, int, int);
 typedef int (*GatedLaunchesFn)(int, int, int, int);
+typedef int (*LatentGatherFn)(const void *, const int *, int, int, const int *, const int *, int, int, int, void *, void *, int, int *, int, int,
+                              cudaStream_t);
+// csrc/attention_tcgen05.cu
+typedef int (*AttentionLaidFn)(const void *, const void *, int, int, const void *, const void *, long long, void *, const int *, int, int,
+                               const int *, const int *, int, int, float, int, int *, const float *, const float *, int, int, cudaStream_t);
 typedef int (*ArgmaxFn)(const float *, long long, int, int, int *, void *, cudaStream_t);
 typedef int (*SampleFn)(const float *, long long, int, int, const float *, const int *, const float *, const float *, int *,
                         cudaStream_t);
@@ -180,6 +185,9 @@ struct RunnerFns {
     GatedScratchFn gated_recurrence_scratch;
     GatedLaunchesFn gated_recurrence_launches;
     RotateRowsFn rotate_rows;
+    // a latent attention's heads made for a step of many rows: csrc/blocks.cu and csrc/attention_tcgen05.cu, bound with them
+    LatentGatherFn latent_gather;
+    AttentionLaidFn attention_laid;
 };
 
 // ---- records ---------------------------------------------------------------------------------------------------
@@ -205,6 +213,7 @@ enum RunnerSlot {
     SLOT_H2,            // activations [T, hidden]: a second norm's output, for a sublayer beside the one that reads SLOT_H
     SLOT_PART1,         // float32 [T, hidden]: the outputs of mixers side by side, which a norm of their own or another sublayer's
     SLOT_PART2,         // output still has to meet before they join the stream
+    SLOT_HEADS,         // a latent attention's positions laid one after the other, the heads made from them and its query tiles
     RUNNER_SLOTS
 };
 
@@ -364,6 +373,11 @@ struct RunnerOp {
     const float *b1;            // GATED_RECURRENCE: [n] bias of the first gate
     // ACTIVATE: w (null: none) [tokens, k]: times w[token, g_off + c].  GATED_RECURRENCE: decay = [n] log a per unit of the first gate.
     // EMBED_PAIR: state = int32 [slots, 2, 2].  LINEAR_ATTENTION: vec may be null (no weight).
+    // ---- what a latent attention over heads made for the step adds ---------------------------------------------------------------------
+    int fold;                   // HEAD_LINEAR 1, 3 and LATENT_ATTENTION 2: parts of a latent attention that may run over heads made from the
+                                // latent rows (head_dim, v_head_dim, rot_width, rank say which sizes): 1 and 3 are then not needed, and 2
+                                // reads the plain query parts in in2_slot and the gate, and writes value heads to out2_slot
+    const void *w_heads;        // LATENT_ATTENTION: [heads head_dim | heads v_head_dim, rank] the key and the value maps, or null
     // ATTENTION: gated 2: a gate per output element, sigmoid(SLOT_TMP[t, g_off + h dv + e]).  HEAD_LINEAR: gated 2: a gate per head.
     // LATENT_QKV: k_off < 0 makes the heads' queries only, from rows [heads, head_dim + rot_width] at q_off (no cache row, no latent).
     // EXPERTS: score_form 2: softmax over all router outputs, the chosen scores as they are, multiplying the units' outputs;
@@ -390,6 +404,7 @@ struct RunnerStep {
     const int *block_tables[jk::MAX_CACHE_GROUPS];
     const int *lists[jk::MAX_STEP_LISTS];     // work lists that mixers asked for; null with n == ntok means "rows 0..ntok-1"
     int list_n[jk::MAX_STEP_LISTS];
+    int tile_keys;              // positions of all requests, this step's rows among them, if each brings more than jk::SHORT_ROWS rows; else 0
 };
 
 struct RunnerBuffers {

@@ -129,6 +129,11 @@ def context_bucket(longest: int, max_positions: int) -> int:
     return lib().jk_context_bucket(longest, max_positions)
 
 
+def latent_heads_fit(dn: int, dr: int, dv: int, rank: int) -> bool:
+    """Whether a latent attention of these sizes can run over heads made for the step."""
+    return bool(lib().jk_latent_heads_fit(dn, dr, dv, rank))
+
+
 def attention_tcgen05_takes(dh: int, page_size: int, dv: int = 0) -> bool:
     return bool(lib().jk_attention_tcgen05_takes(dh, page_size, dv))
 

@@ -12,6 +12,11 @@ queries, norms the latent vector, rotates (float32 angles) and writes the cache 
 query parts into the latent space; the attention over the paged rows (float32 scores and weights); a product per head
 back to value heads, times the sigmoid of the gate; the output product.  Kernels: csrc/blocks.cu.
 
+Steps whose requests bring many rows (heads of 64 or 128 for keys and values alike, a rotated part of 64 or none, bfloat16) run the
+three records in the middle another way: one product makes the heads' keys and values of all positions from the latent rows, and
+the tensor-core attention of plain heads runs over them, which is a third of the multiply-adds a (row, key) pair costs over
+the latent rows (``fold``; rule: jk::latent_takes_heads).
+
 Options of the same records: queries through a latent of their own (``q_rank``: the fused product is [query latent | key
 and value latent (| gate)], ``latent_qkv`` norms both, a product makes the heads' queries from the normed one and a cast
 hands them to the per-head product; where queries have a rotated part, ``latent_qkv`` over that product's rows splits and
@@ -25,6 +30,7 @@ from typing import Dict
 import torch
 
 from ..cache import PagedKV
+from ..kernels.host import latent_heads_fit
 from ..weights import MATRIX, VECTOR, TensorDecl
 from .base import register
 from .program import record
@@ -70,9 +76,12 @@ class LatentAttention:
             self.q_norm = weights.get(prefix + spec.q_down_name + spec.norm_suffix, VECTOR)
             self.w_q_up = weights.get(prefix + spec.q_up_name, MATRIX)
         self.norm = weights.get(prefix + spec.kv_down_name + spec.norm_suffix, VECTOR)
+        # the key and value maps as stored, one below the other: what makes heads from latent rows
+        self.w_heads = weights.get_rows([prefix + spec.k_up_name, prefix + spec.v_up_name], MATRIX)
         # head h's key map [dn, R], transposed: the matrix that takes the head's plain query part into the latent space
-        self.w_q_latent = weights.get(prefix + spec.k_up_name, MATRIX).view(H, dn, R).transpose(1, 2).contiguous()
-        self.w_v = weights.get(prefix + spec.v_up_name, MATRIX)         # [H, dv, R] as stored
+        self.w_q_latent = self.w_heads[:H * dn].view(H, dn, R).transpose(1, 2).contiguous()
+        self.w_v = self.w_heads[H * dn:]                                # [H, dv, R] as stored
+        self.fold = runtime.dtype == torch.bfloat16 and latent_heads_fit(dn, spec.rot_dim, spec.v_head_dim, R)
         self.w_o = weights.get(prefix + spec.o_name, MATRIX)
         self.freq, self.magnitude, self.rot_dims = None, 1.0, 0
         if spec.position is not None and spec.position.dims:
@@ -104,6 +113,8 @@ class LatentAttention:
         g_off = kv_off + R + dr
         rotation = dict(rot_dims=self.rot_dims, freq=self.freq, rot_mag=self.magnitude,
                         rot_half=self.freq is not None and s.position.layout == "halves")
+        gate = dict(gated=2 if s.output_gate == "head" else int(s.output_gate), g_off=g_off, ld=ld)
+        fold = lambda part: dict(fold=part, head_dim=dn, v_head_dim=dv, rot_width=dr, rank=R, window=s.window or 0) if self.fold else {}
         if s.q_rank and dr:
             # the queries' latent, normed, into "o"; the heads' queries as float32 rows into "mix" ("tmp" keeps the gate), split
             # into the plain parts ("act") and the rotated ones ("q", behind the part that the per-head product fills)
@@ -113,7 +124,7 @@ class LatentAttention:
                     record("linear", "o", "mix", n=H * (dn + dr), k=s.q_rank, w=self.w_q_up),
                     record("latent_qkv", "mix", "q", out2_slot="act", heads=H, head_dim=dn, rot_width=dr, rank=R, ld=H * (dn + dr),
                            q_off=0, k_off=-1, **rotation),
-                    record("head_linear", "act", "q", heads=H, n=R, k=dn, out_hs=R + dr, w=self.w_q_latent)]
+                    record("head_linear", "act", "q", heads=H, n=R, k=dn, out_hs=R + dr, w=self.w_q_latent, **fold(1))]
         elif s.q_rank:
             # the queries' latent, normed, into "o"; the heads' queries by a product of it (float32 rows in "tmp", which the
             # norms have read by then), cast into "act" as the per-head product's operand
@@ -122,20 +133,22 @@ class LatentAttention:
                            cache_group=view.group_index, k_pages=view.k_pages, num_pages=view.k_pages.shape[0]),
                     record("linear", "o", "tmp", n=H * dn, k=s.q_rank, w=self.w_q_up),
                     record("activate", "tmp", "act", n=H * dn, ld=H * dn, act=0),
-                    record("head_linear", "act", "q", heads=H, n=R, k=dn, out_hs=R, w=self.w_q_latent)]
+                    record("head_linear", "act", "q", heads=H, n=R, k=dn, out_hs=R, w=self.w_q_latent, **fold(1))]
         else:
             head = [record("latent_qkv", "tmp", "q", out2_slot="o", heads=H, head_dim=dn, rot_width=dr, rank=R, **rotation, norm_k=self.norm, eps=s.norm_eps, ld=ld, q_off=0, k_off=kv_off,
                            cache_group=view.group_index, k_pages=view.k_pages, num_pages=view.k_pages.shape[0]),
-                    record("head_linear", "o", "q", heads=H, n=R, k=dn, out_hs=R + dr, w=self.w_q_latent)]
+                    record("head_linear", "o", "q", heads=H, n=R, k=dn, out_hs=R + dr, w=self.w_q_latent, **fold(1))]
         program.emit_records([
             record("linear", "h", "tmp", n=ld, k=s.hidden_size, w=self.w_in)] + head + [
             record("latent_attention", "q", "o", heads=H, rank=R, rot_width=dr, softmax_scale=s.softmax_scale, window=s.window or 0,
                    sink_w=self.sink_w, cache_group=view.group_index, k_pages=view.k_pages, num_pages=view.k_pages.shape[0],
-                   max_positions=program.max_blocks * program.page_size),
-            record("head_linear", "o", "act", heads=H, n=dv, k=R, out_hs=dv, w=self.w_v, gated=2 if s.output_gate == "head" else int(s.output_gate), g_off=g_off, ld=ld),
+                   max_positions=program.max_blocks * program.page_size,
+                   **(dict(fold=2, head_dim=dn, v_head_dim=dv, w_heads=self.w_heads, in2_slot="act" if s.q_rank else "o", out2_slot="act", **gate)
+                      if self.fold else {})),
+            record("head_linear", "o", "act", heads=H, n=dv, k=R, out_hs=dv, w=self.w_v, **gate, **fold(3)),
             record("linear", "act", "delta", n=s.hidden_size, k=H * dv, w=self.w_o) if into_stream is None else
             record("residual", "act", "x", n=s.hidden_size, k=H * dv, w=self.w_o, scale=float(into_stream)),
-        ], keep=(self.sink_w, self.w_in, self.norm, self.w_q_latent, self.w_v, self.w_o, self.freq, view.k_pages, self.q_norm, self.w_q_up))
+        ], keep=(self.sink_w, self.w_in, self.norm, self.w_q_latent, self.w_v, self.w_o, self.freq, view.k_pages, self.q_norm, self.w_q_up, self.w_heads))
 
     def forward(self, h: torch.Tensor, ctx, view, writes_cache: bool = True, state_view=None) -> torch.Tensor:
         """The part alone: its own records over ``h``; float32 ``[T, hidden]``."""

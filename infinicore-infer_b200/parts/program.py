@@ -24,7 +24,7 @@ from ..kernels import host as _host
 
 _i, _f, _p, _ll = ctypes.c_int, ctypes.c_float, ctypes.c_void_p, ctypes.c_longlong
 
-SLOTS = ("x", "delta", "h", "q", "o", "act", "hw", "logits", "tmp", "decode", "mix", "scan", "x0", "route", "shift", "h2", "part1", "part2")       # RunnerSlot of csrc/runner.h
+SLOTS = ("x", "delta", "h", "q", "o", "act", "hw", "logits", "tmp", "decode", "mix", "scan", "x0", "route", "shift", "h2", "part1", "part2", "heads")       # RunnerSlot of csrc/runner.h
 SLOT = {name: i for i, name in enumerate(SLOTS)}
 OP_NAMES = {1: "embed", 2: "norm", 3: "qkv", 4: "attention", 5: "residual", 6: "gate_up", 7: "linear", 8: "cast",
             9: "layernorm", 10: "conv_qkv", 11: "linear_attention", 12: "norm_add", 13: "reinject", 14: "latent_qkv",
@@ -37,6 +37,7 @@ _MIXERS_OPS = (OP["cast"], OP["layernorm"], OP["conv_qkv"], OP["linear_attention
                OP["rotate"])
 _BLOCKS_OPS = tuple(OP[n] for n in ("norm_add", "reinject", "latent_qkv", "head_linear", "latent_attention", "causal_conv",
                                     "selective_scan", "experts", "softcap", "add_rows", "norm_pair", "embed_pair", "join", "gated_recurrence"))
+SHORT_ROWS = 8                  # jk::SHORT_ROWS of csrc/host_rules.h
 MAX_GROUPS = 8
 MAX_LISTS = 8
 
@@ -71,7 +72,9 @@ class RunnerOp(ctypes.Structure):
                 # what pairs of tokens, joined parts, real-gated recurrences and a token's own vectors add
                 + [(n, _i) for n in ("buckets", "mul_prev", "mul_cur", "blocks")]
                 + [("score_scale", _f)]
-                + [(n, _p) for n in ("vec3", "in_bias", "b1")])
+                + [(n, _p) for n in ("vec3", "in_bias", "b1")]
+                # what a latent attention over heads made for the step adds
+                + [("fold", _i), ("w_heads", _p)])
 
 
 class Routing(ctypes.Structure):
@@ -87,7 +90,7 @@ class RunnerEnv(ctypes.Structure):
 class RunnerStep(ctypes.Structure):
     _fields_ = ([(n, _i) for n in ("ntok", "nreq", "n_want", "context")]
                 + [(n, _p) for n in ("tokens", "positions", "row_req", "req_start", "req_pos", "want_rows", "slot_ids")]
-                + [("block_tables", _p * MAX_GROUPS), ("lists", _p * MAX_LISTS), ("list_n", _i * MAX_LISTS)])
+                + [("block_tables", _p * MAX_GROUPS), ("lists", _p * MAX_LISTS), ("list_n", _i * MAX_LISTS), ("tile_keys", _i)])
 
 
 class RunnerBuffers(ctypes.Structure):
@@ -105,7 +108,8 @@ class _Fns(ctypes.Structure):
         "norm_gate", "token_shift", "act_rows", "err_mixers", "norm_add", "concat_cast", "add_bias_rows", "latent_qkv", "head_linear", "latent_attention",
         "latent_attention_scratch", "causal_conv", "selective_scan", "routed_experts", "routed_experts_workspace",
         "routed_experts_launches", "softcap", "err_blocks", "linear_small_parts", "linear_small_parts_supports", "add_rows", "delta_rule", "delta_rule_scratch",
-        "norm_pair", "embed_pair", "join_parts", "gated_recurrence", "gated_recurrence_scratch", "gated_recurrence_launches", "rotate_rows")]
+        "norm_pair", "embed_pair", "join_parts", "gated_recurrence", "gated_recurrence_scratch", "gated_recurrence_launches", "rotate_rows", "latent_gather",
+        "attention_laid")]
 
 
 def _addr(lib, name: str) -> int:
@@ -168,7 +172,8 @@ def runner_lib(gemm_tcgen05: bool = False, attention_tcgen05: bool = False, mixe
         add_rows=get("blocks", "jk_add_rows"), delta_rule=get("mixers", "jk_delta_rule"), delta_rule_scratch=get("mixers", "jk_delta_rule_scratch_floats"),
         norm_pair=get("blocks", "jk_norm_pair"), embed_pair=get("blocks", "jk_embed_pair"), join_parts=get("blocks", "jk_join_parts"),
         gated_recurrence=get("blocks", "jk_gated_recurrence"), gated_recurrence_scratch=get("blocks", "jk_gated_recurrence_scratch_floats"),
-        gated_recurrence_launches=get("blocks", "jk_gated_recurrence_launches"), rotate_rows=get("mixers", "jk_rotate_rows"))
+        gated_recurrence_launches=get("blocks", "jk_gated_recurrence_launches"), rotate_rows=get("mixers", "jk_rotate_rows"),
+        latent_gather=get("blocks", "jk_latent_gather"), attention_laid=get("attention_tcgen05", "jk_attention_laid_tcgen05"))
     if lib.jk_runner_bind(ctypes.byref(fns)):
         from ..kernels import KernelError
         raise KernelError(lib.jk_runner_last_error().decode(errors="replace"))
@@ -349,8 +354,8 @@ class ProgramRunner:
         self.env = rt.env(program.page_size, program.max_blocks)
         need_gemm = bool(program.lib.jk_runner_needs_gemm_tcgen05(ctypes.byref(self.env), program.ops, program.count, max_rows))
         need_attn = rt.dtype == torch.bfloat16 and not rt.legacy_tensor_cores and any(
-            program.ops[i].kind == 4 and _host.attention_tcgen05_takes(program.ops[i].head_dim, program.page_size, program.ops[i].v_head_dim)
-            for i in range(program.count))
+            (program.ops[i].kind == OP["attention"] and _host.attention_tcgen05_takes(program.ops[i].head_dim, program.page_size, program.ops[i].v_head_dim))
+            or (program.ops[i].kind == OP["latent_attention"] and program.ops[i].fold and max_rows >= 64) for i in range(program.count))
         need_mixers = any(program.ops[i].kind in _MIXERS_OPS or (program.ops[i].kind == OP["gate_up"] and program.ops[i].act > ACT["silu"])
                           for i in range(program.count))
         need_blocks = any(program.ops[i].kind in _BLOCKS_OPS for i in range(program.count))
@@ -400,6 +405,7 @@ class ProgramRunner:
                           tokens=ctx.tokens.data_ptr(), positions=ctx.positions.data_ptr(), row_req=ctx.row_req.data_ptr(),
                           req_start=ctx.req_start.data_ptr(), req_pos=ctx.req_pos.data_ptr(), want_rows=ctx.want_rows.data_ptr(),
                           slot_ids=ctx.slot_ids.data_ptr())
+        step.tile_keys = tile_keys(ctx)
         for g, table in enumerate(ctx.block_tables):
             step.block_tables[g] = table.data_ptr()
         for name, index in prog.lists.items():
@@ -429,6 +435,16 @@ class ProgramRunner:
                                                    ctypes.byref(self.buffers), flush, stream))
                 self.launches += self.lib.jk_runner_launches()
         return logits
+
+
+def tile_keys(ctx) -> int:
+    """Positions of all requests of a step, its own rows among them, if each request brings more rows than a decode kernel
+    takes one by one; else 0."""
+    starts, pos = ctx.host_req_start, ctx.host_req_pos
+    if len(starts) <= ctx.nreq or len(pos) < ctx.nreq:
+        return 0
+    lens = [starts[i + 1] - starts[i] for i in range(ctx.nreq)]
+    return sum(lens) + sum(pos[:ctx.nreq]) if lens and min(lens) > SHORT_ROWS else 0
 
 
 def step_lists_for(owners, ctx, device) -> Dict[str, tuple]:
@@ -471,7 +487,7 @@ def run_part_alone(runtime, plan, ctx, h: torch.Tensor, hidden_size: int, page_s
     from .. import kernels
     step = RunnerStep(ntok=T, nreq=ctx.nreq, n_want=0, context=ctx.context, tokens=ctx.tokens.data_ptr(),
                       positions=ctx.positions.data_ptr(), row_req=ctx.row_req.data_ptr(), req_start=ctx.req_start.data_ptr(),
-                      req_pos=ctx.req_pos.data_ptr(), want_rows=None, slot_ids=ctx.slot_ids.data_ptr())
+                      req_pos=ctx.req_pos.data_ptr(), want_rows=None, slot_ids=ctx.slot_ids.data_ptr(), tile_keys=tile_keys(ctx))
     for g, table in enumerate(ctx.block_tables):
         step.block_tables[g] = table.data_ptr()
     for name, index in program.lists.items():

@@ -1,0 +1,52 @@
+"""Steps of many rows through the kernels that only they reach: latent attention over heads made for the step.  At the edges of
+tiles, against the plain implementation (tests/plain_vunelix.py)."""
+import json
+import os
+
+import pytest
+import torch
+
+from conftest import random_tokens
+import plain_vunelix as plain
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("heads,dim,rank", [(3, 64, 72), (2, 128, 64), (16, 128, 512)])
+def test_latent_attention_over_heads_made_for_the_step(tmp_path, heads, dim, rank):
+    """Prompts and portions of one and several requests, tiles of 128 rows and keys at their edges.  The other way of running the
+    same records, over the latent rows, has the same operands and one rounding to bfloat16 more or less at each of its
+    products: both lie within a few units of 2^-8 of the float64 model, and of each other."""
+    from infinicore_infer_b200.config import config_class_for
+    from infinicore_infer_b200.engine import Engine, StepEntry
+    from infinicore_infer_b200.weights import index_directory, read_tensor, write_model_folder
+    cfg = {"architecture": "Vunelix", "norm": {"eps": 1e-5}, "vocab": 97, "width": 64, "logit_softcap": None, "layers": [
+        {"type": "latent_attention", "mlp": None, "mixer": {"heads": heads, "dim": dim, "rot_dim": 64, "vdim": dim, "kv_rank": rank,
+                                                            "scale": (dim + 64) ** -0.5, "rot": {"base": 1e3, "dims": 32}}}]}
+    write_model_folder(config_class_for(cfg).from_dict(cfg), str(tmp_path), seed=5, std=0.16, norm_std=0.2)
+    with open(os.path.join(tmp_path, "config.json")) as f:
+        disk = json.load(f)
+    weights = {n: read_tensor(i).float() for n, i in index_directory(str(tmp_path)).items()}
+    engine = Engine.from_folder(str(tmp_path), max_tokens=640, cache_tokens=1280, page_size=16, max_requests=3, max_step_tokens=512)
+    toks = [random_tokens(s, 400, 97) for s in range(3)]
+    want = [plain.forward(t, disk, weights) for t in toks]
+    scale = want[0].std()
+    # (request, from, to) of every step's entries; the last step decodes
+    steps = [[(0, 0, 128)], [(0, 128, 148), (1, 0, 129)], [(0, 148, 400)], [(1, 129, 385), (2, 0, 64)], [(2, 64, 200)], [(1, 385, 386), (2, 200, 201)]]
+    logits = {}
+    for other_way in (False, True):
+        engine.runtime.plain_attention = other_way
+        rows = []
+        for step in steps:
+            out = engine.step([StepEntry((other_way, r), toks[r][a:b], list(range(b - a))) for r, a, b in step])
+            rows.append(out.double().cpu())
+            ref = torch.cat([want[r][a:b] for r, a, b in step])
+            err = (rows[-1] - ref).square().mean().sqrt() / scale
+            assert err <= 0.03, f"{step}, over the latent rows: {other_way}: {err:.4f} of the logits' spread"
+        logits[other_way] = torch.cat(rows)
+        for r in range(3):
+            engine.end((other_way, r))
+    engine.check()
+    engine.runtime.plain_attention = False
+    assert (logits[False] - logits[True]).square().mean().sqrt() <= 0.03 * scale
+    assert not torch.equal(logits[False], logits[True])         # both ways ran
