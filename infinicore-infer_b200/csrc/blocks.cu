@@ -57,6 +57,8 @@ __device__ __forceinline__ float expert_inner(int act, float s, float g, float u
     return block_act(act, s * g) * (s * u);
 }
 
+#include "experts_tcgen05.cuh"
+
 #define BLOCKS_BY_DTYPE(dtype, name, LAUNCH)                                      \
     do {                                                                          \
         if ((dtype) == JK_F32) { LAUNCH(float); }                                 \
@@ -2099,6 +2101,8 @@ __global__ void expert_combine_kernel(CombineArgs a, size_t total) {
     }
 }
 
+static thread_local int g_expert_launches = 0;      // launches of this thread's last call beyond the six that every call has
+
 // ints of workspace (`route`) that T rows need: counts [N], starts [N + 1], ids, entry_row, pair_entry [T top] and, as
 // floats, scores and entry_score [T top] and the rows' gates [T]; N counts the router's outputs
 JK_EXPORT long long jk_routed_experts_workspace(int T, int N, int top) { return 2LL * N + 1 + 5LL * T * top + T + 16; }
@@ -2110,7 +2114,7 @@ JK_EXPORT int jk_routed_experts(const void *h, const float *router, const void *
                                 int dtype, int T, int D, int ff, int E, int top, int actf, int *route, void *act, float *y,
                                 int score_form, float limit, const float *router_bias, const float *gate_w, int identity, int group_count,
                                 int group_keep, const float *correction, float *x, float x_scale, const float *pend, float pend_scale,
-                                float score_scale, cudaStream_t stream) {
+                                float score_scale, int *status, cudaStream_t stream) {
     if (T == 0) return JK_OK;
     const int N = E + identity;
     JK_REQUIRE(gate_w == nullptr || add, "routed_experts: a gate on a shared unit's output that is not there");
@@ -2146,7 +2150,26 @@ JK_EXPORT int jk_routed_experts(const void *h, const float *router, const void *
     const int per16 = dtype == JK_F32 ? 4 : 8;
     const bool stream_rows = pairs <= 64 && D % per16 == 0 && ff % per16 == 0 && (uintptr_t)w_gate_up % 16 == 0 && (uintptr_t)w_down % 16 == 0 &&
                              (size_t)ER_ROWS * std::max(D, ff) * 4 <= 160 * 1024;
-    if (stream_rows) {
+    // Many rows an expert: tiles of 128 entries on tcgen05 (bfloat16, whole vectors, a status word for their waits).  The
+    // weights' bytes bound both kinds of tiles at few entries an expert (8 experts of 1,408, width 2,048, two a row; tiles of 64 on
+    // mma.sync -> of 128 here): 128 rows 118 -> 74 us, 512 169 -> 84, 2,048 405 -> 135; with fewer than eight entries an expert
+    // most of a tile's rows are padding.
+    g_expert_launches = 0;
+    const bool tc = dtype == JK_BF16 && !stream_rows && status != nullptr && E <= ET_MAX_EXPERTS && D % 8 == 0 && ff % 8 == 0 && pairs >= 8LL * E &&
+                    (((uintptr_t)h | (uintptr_t)w_gate_up | (uintptr_t)w_down | (uintptr_t)act | (uintptr_t)y) & 15) == 0;
+    if (tc) {
+        // the entries' rows lie in y's place until the second product writes there
+        static const int sms = [] { int n = 148, dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); return n; }();
+        __nv_bfloat16 *rows = (__nv_bfloat16 *)y;
+        jk_launch(expert_gather_kernel, dim3(std::min(pairs, sms * 8)), dim3(256), 0, stream, (const uint4 *)h, (const int *)entry_row, (const int *)starts, E,
+                  (uint4 *)rows, D / 8);
+        JK_CHECK_LAUNCH("expert_gather");
+        const int down = pairs / TG_BM + E;
+        const ExpertTcArgs up{act, starts, in_score, E, pairs, ff, D, actf, limit, status}, dn{y, starts, nullptr, E, pairs, D, ff, 0, 0.f, status};
+        if (int rc = launch_expert_tc<true>(rows, (const __nv_bfloat16 *)w_gate_up, up, down * ((ff + ET_BN / 2 - 1) / (ET_BN / 2)), sms, stream)) return rc;
+        if (int rc = launch_expert_tc<false>((const __nv_bfloat16 *)act, (const __nv_bfloat16 *)w_down, dn, down * ((D + ET_BN - 1) / ET_BN), sms, stream)) return rc;
+        g_expert_launches = 1;
+    } else if (stream_rows) {
         const size_t elem = dtype == JK_F32 ? 4 : 2, smem_up = (size_t)ER_ROWS * D * elem, smem_down = (size_t)ER_ROWS * ff * elem;
 #define LAUNCH(TT)                                                                                                                           \
     if (smem_up > 46 * 1024) cudaFuncSetAttribute(expert_rows_kernel<TT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_up);  \
@@ -2182,8 +2205,8 @@ JK_EXPORT int jk_routed_experts(const void *h, const float *router, const void *
     JK_CHECK_LAUNCH("expert_combine");
     return JK_OK;
 }
-// kernels that one call of jk_routed_experts launches (the clearing of the counts included)
-JK_EXPORT int jk_routed_experts_launches() { return 6; }
+// kernels that this thread's last call of jk_routed_experts launched (the clearing of the counts included)
+JK_EXPORT int jk_routed_experts_launches() { return 6 + g_expert_launches; }
 
 // ---------------------------------------------------------------------------------------------------------------
 // x[t] += table[index[t]] (index null: row `fixed` for every t): learned position vectors picked by the rows' positions,

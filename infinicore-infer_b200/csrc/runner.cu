@@ -726,7 +726,7 @@ int run_experts(Run &r, const RunnerOp &op) {
     RUN(blocks, g_fns.routed_experts(h, op.vec, op.w, op.w3, (float *)delta, op.add, r.env.dtype, T, op.n, op.ff, op.experts, op.top, op.act,
                                      (int *)route, act, (float *)y, op.score_form, op.limit, op.router_bias, op.gate_w, op.identity, op.group_count, op.group_keep,
                                    op.correction, adds ? r.x() : nullptr, op.scale, r.pending ? (const float *)delta : nullptr, r.pending_scale,
-                                   op.score_scale > 0.f ? op.score_scale : 1.f, r.stream));
+                                   op.score_scale > 0.f ? op.score_scale : 1.f, r.env.status, r.stream));
     g_launches += g_fns.routed_experts_launches() - 1;
     if (adds) {
         r.pending = false;

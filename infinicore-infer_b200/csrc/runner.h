@@ -82,7 +82,7 @@ typedef int (*SelectiveScanFn)(const float *, const float *, int, int, int, int,
                                cudaStream_t);
 typedef int (*RoutedExpertsFn)(const void *, const float *, const void *, const void *, float *, int, int, int, int, int, int, int, int,
                                int *, void *, float *, int, float, const float *, const float *, int, int, int, const float *, float *, float,
-                               const float *, float, float, cudaStream_t);
+                               const float *, float, float, int *, cudaStream_t);
 typedef long long (*RoutedWorkspaceFn)(int, int, int);
 typedef int (*CountFn)();
 typedef int (*SoftcapFn)(float *, float, long long, cudaStream_t);

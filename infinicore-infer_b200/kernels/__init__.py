@@ -860,7 +860,7 @@ def routed_experts(h: torch.Tensor, router: torch.Tensor, w_gate_up: torch.Tenso
                                            _c_int(dtype_code(h.dtype)), _c_int(T), _c_int(d), _c_int(ff), _c_int(experts), _c_int(top),
                                            _c_int(act), _ptr(route), _ptr(act_buf), _ptr(y), _c_int(score_form), _c_float(limit), _ptr(router_bias), _ptr(gate_w),
                                            _c_int(identity), _c_int(groups[0]), _c_int(groups[1]), _ptr(correction), _ptr(x), _c_float(x_scale),
-                                           _ptr(pending), _c_float(pending_scale), _c_float(score_scale), _stream()))
+                                           _ptr(pending), _c_float(pending_scale), _c_float(score_scale), _ptr(gemm_status(h.device)), _stream()))
     return delta
 
 

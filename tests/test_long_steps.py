@@ -1,5 +1,5 @@
-"""Steps of many rows through the kernels that only they reach: latent attention over heads made for the step.  At the edges of
-tiles, against the plain implementation (tests/plain_vunelix.py)."""
+"""Steps of many rows through the kernels that only they reach: latent attention over heads made for the step, experts'
+products in tiles of 128 entries.  At the edges of tiles, against the plain implementation (tests/plain_vunelix.py)."""
 import json
 import os
 
@@ -10,6 +10,13 @@ from conftest import random_tokens
 import plain_vunelix as plain
 
 pytestmark = pytest.mark.gpu
+F = torch.float64
+
+
+@pytest.fixture(scope="module")
+def K():
+    from infinicore_infer_b200 import kernels
+    return kernels
 
 
 @pytest.mark.parametrize("heads,dim,rank", [(3, 64, 72), (2, 128, 64), (16, 128, 512)])
@@ -50,3 +57,40 @@ def test_latent_attention_over_heads_made_for_the_step(tmp_path, heads, dim, ran
     engine.runtime.plain_attention = False
     assert (logits[False] - logits[True]).square().mean().sqrt() <= 0.03 * scale
     assert not torch.equal(logits[False], logits[True])         # both ways ran
+
+
+@pytest.mark.parametrize("T,d,ff,experts,top,act", [(128, 64, 128, 1, 1, "silu"), (129, 72, 136, 2, 2, "swish_clamp"), (300, 512, 264, 5, 2, "silu"),
+                                                    (600, 264, 8, 3, 1, "silu")])
+def test_expert_products_in_tiles_of_entries(K, T, d, ff, experts, top, act):
+    """Entries that fill tiles of 128 exactly, by one more and by part, an expert without rows (the router's bias shuns it), widths
+    that end inside a tile and inside a step of K.  A product's operands are exact, its sums float32, the inner activations
+    rounded to bfloat16: 2^-9 of each, averaged over ff of them."""
+    dev, g = torch.device("cuda:0"), torch.Generator().manual_seed(T + d)
+    h = torch.randn(T, d, generator=g).to(torch.bfloat16)
+    w_gu, w_dn = (torch.randn(experts * n, k, generator=g).div(k ** 0.5).to(torch.bfloat16) for n, k in ((2 * ff, d), (d, ff)))
+    router = torch.randn(experts, d, generator=g)
+    bias = torch.zeros(experts)
+    if experts > 2:
+        bias[1] = -1e3
+    code = {"silu": K.ACT_SILU, "swish_clamp": 6}[act]
+    delta = torch.full((T, d), 9.0, device=dev)
+    K.routed_experts(h.to(dev), router.to(dev), w_gu.to(dev), w_dn.to(dev), delta, False, experts, top, code, score_form=1, limit=1.5,
+                     router_bias=bias.to(dev))
+    K.check_gemm_status(dev)
+    z = h.double() @ router.double().T + bias.double()
+    score = torch.softmax(z, -1)
+    chosen = z.topk(top, -1).indices
+    want = torch.zeros(T, d, dtype=F)
+    for e in range(experts):
+        rows = (chosen == e).any(-1)
+        gu = h[rows].double() @ w_gu[e * 2 * ff: (e + 1) * 2 * ff].double().T
+        a, u = gu[:, :ff], gu[:, ff:]
+        if act == "silu":
+            inner = plain.silu(a) * u
+        else:
+            a, u = a.clamp(max=1.5), u.clamp(-1.5, 1.5)
+            inner = a * torch.sigmoid(1.702 * a) * (u + 1)
+        share = score[rows, e] / (score[rows].gather(1, chosen[rows]).sum(-1) + 1e-20)
+        want[rows] += share.unsqueeze(-1) * (inner @ w_dn[e * d: (e + 1) * d].double().T)
+    err = (delta.double().cpu() - want).abs().max()
+    assert err <= 2.0 ** -8 * want.abs().max(), float(err)
