@@ -1640,12 +1640,150 @@ __global__ void __launch_bounds__(SS_THREADS) selective_scan_kernel(ScanArgs a) 
     }
 }
 
+// Long steps: a request's rows are cut into pieces of SP_ROWS that run side by side, a thread a channel with all of its states.
+// The first launch (OUT false) takes every piece but a request's last from a state of zeros, the first piece from the
+// request's state, and leaves its end state and the sum of its step sizes; the second starts each piece from
+// S <- exp(A sum dt) S + end over the pieces before it, makes the outputs, and its last piece leaves the request's state.  No
+// decay is divided by; where a piece starts moves the rounding of a row's sums only.  Requests of one piece skip the
+// first launch.  The request's state as the step found it lies where its last piece's end state would (which nobody asks
+// for), since the last piece overwrites it while the first is still at work.
+//
+// What bounds it: instructions (sixteen states: about 170 a row and channel, the exponentials half of them).  Eight lanes a
+// channel walking a prompt from end to end waited 600 cycles a row for one another and for the next rows.  B200, 2,048 rows,
+// 4,096 channels, 16 states, with the product of the step sizes: 589 -> 360 us.
+constexpr int SP_THREADS = 128, SP_ROWS = 128, SP_AHEAD = 4;
+struct PieceArgs {
+    float *ends, *sums;         // [pieces, N, E] end states, [pieces, E] sums of step sizes
+    int nreq;
+};
+template <typename T, int NS, bool OUT>
+__global__ void __launch_bounds__(SP_THREADS) selective_pieces_kernel(ScanArgs a, PieceArgs p) {
+    pdl_trigger();
+    pdl_wait();
+    __shared__ __align__(16) float s_bc[SP_AHEAD * 8][2 * NS];       // B and C of a chunk's rows
+    constexpr int CHUNK = SP_AHEAD * 8;
+    // the block's request and piece; `at`: the place of the request's first piece among all that leave something
+    int req = -1, piece = 0, count = 0, at = 0;
+    for (int r = 0, blocks = 0; r < p.nreq; ++r) {
+        const int n = (a.req_start[r + 1] - a.req_start[r] + SP_ROWS - 1) / SP_ROWS;
+        if ((int)blockIdx.y < blocks + n) { req = r; piece = blockIdx.y - blocks; count = n; break; }
+        blocks += n;
+        if (n > 1) at += n;
+    }
+    if (req < 0 || (!OUT && piece == count - 1)) return;
+    const int c = blockIdx.x * SP_THREADS + threadIdx.x;
+    const bool live = c < a.E;
+    const int cc = live ? c : a.E - 1;
+    const int first = a.req_start[req] + piece * SP_ROWS, last = min(first + SP_ROWS, a.req_start[req + 1]);
+    float *state = a.state + ((size_t)a.slot_ids[req] * a.E + cc) * a.N;
+    auto end_of = [&](int q, int n) -> float & { return p.ends[((size_t)(at + q) * a.N + n) * a.E + cc]; };
+    float s[NS], An[NS];
+#pragma unroll
+    for (int n = 0; n < NS; ++n) {
+        An[n] = n < a.N ? a.A[(size_t)cc * a.N + n] : 0.f;
+        s[n] = 0.f;
+    }
+    if (!OUT) {
+        if (piece == 0)
+#pragma unroll
+            for (int n = 0; n < NS; ++n)
+                if (n < a.N) {
+                    s[n] = state[n];
+                    if (live) end_of(count - 1, n) = s[n];
+                }
+    } else if (count == 1) {
+#pragma unroll
+        for (int n = 0; n < NS; ++n)
+            if (n < a.N) s[n] = state[n];
+    } else if (piece == 0) {
+#pragma unroll
+        for (int n = 0; n < NS; ++n)
+            if (n < a.N) s[n] = end_of(count - 1, n);
+    } else {
+#pragma unroll
+        for (int n = 0; n < NS; ++n)
+            if (n < a.N) s[n] = end_of(0, n);
+        for (int q = 1; q < piece; ++q) {
+            const float sum = p.sums[(size_t)(at + q) * a.E + cc];
+#pragma unroll
+            for (int n = 0; n < NS; ++n)
+                if (n < a.N) s[n] = fmaf(expf(sum * An[n]), s[n], end_of(q, n));
+        }
+    }
+    const float skip = OUT ? a.Dskip[cc] : 0.f;
+    float total = 0.f;
+    for (int t0 = first; t0 < last; t0 += CHUNK) {
+        const int rows = min(CHUNK, last - t0);
+        __syncthreads();
+        for (int i = threadIdx.x; i < CHUNK * 2 * NS; i += SP_THREADS) {
+            const int r = i / (2 * NS), n = i % NS, which = i / NS & 1;
+            s_bc[r][i % (2 * NS)] = r < rows && n < a.N ? a.low[(size_t)(t0 + r) * a.ld_low + a.K + which * a.N + n] : 0.f;
+        }
+        __syncthreads();
+        float dt[SP_AHEAD], x[SP_AHEAD], z[SP_AHEAD];
+        auto fetch = [&](int r0) {          // the next rows' inputs, asked for together
+#pragma unroll
+            for (int j = 0; j < SP_AHEAD; ++j) {
+                const size_t t = (size_t)min(t0 + r0 + j, last - 1);
+                dt[j] = a.dt[t * a.ld_dt + cc];
+                x[j] = a.x[t * a.E + cc];
+                if (OUT) z[j] = a.z[t * a.ld_z + cc];
+            }
+        };
+        fetch(0);
+        for (int r0 = 0; r0 < rows; r0 += SP_AHEAD) {
+            float d[SP_AHEAD], u[SP_AHEAD], g[SP_AHEAD];
+#pragma unroll
+            for (int j = 0; j < SP_AHEAD; ++j) { d[j] = dt[j]; u[j] = x[j]; g[j] = OUT ? z[j] : 0.f; }
+            if (r0 + SP_AHEAD < rows) fetch(r0 + SP_AHEAD);
+#pragma unroll
+            for (int j = 0; j < SP_AHEAD; ++j) {
+                if (r0 + j >= rows) break;
+                const float *bc = s_bc[r0 + j], dx = d[j] * u[j];
+                float y = 0.f;
+#pragma unroll
+                for (int n = 0; n < NS; n += 4) {
+                    const float4 B = *reinterpret_cast<const float4 *>(bc + n);
+                    const float b[4] = {B.x, B.y, B.z, B.w};
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) s[n + k] = fmaf(expf(d[j] * An[n + k]), s[n + k], dx * b[k]);
+                    if (OUT) {
+                        const float4 C = *reinterpret_cast<const float4 *>(bc + NS + n);
+                        y = fmaf(s[n + 3], C.w, fmaf(s[n + 2], C.z, fmaf(s[n + 1], C.y, fmaf(s[n], C.x, y))));
+                    }
+                }
+                total += d[j];
+                if (OUT && live) {
+                    y = fmaf(skip, u[j], y);
+                    ((T *)a.out)[(size_t)(t0 + r0 + j) * a.E + c] = from_f32<T>(y * silu_f(g[j]));
+                }
+            }
+        }
+    }
+    if (!live) return;
+    if (!OUT) {
+        p.sums[(size_t)(at + piece) * a.E + c] = total;
+#pragma unroll
+        for (int n = 0; n < NS; ++n)
+            if (n < a.N) end_of(piece, n) = s[n];
+    } else if (piece == count - 1) {
+#pragma unroll
+        for (int n = 0; n < NS; ++n)
+            if (n < a.N) state[n] = s[n];
+    }
+}
+
+// Floats of scratch that a scan of `rows` rows over pieces needs (0: it runs without).
+JK_EXPORT long long jk_selective_scan_scratch_floats(int rows, int E, int N) {
+    return N <= 32 && rows > SP_ROWS ? 2LL * rows / SP_ROWS * (N + 1) * E : 0;
+}
+
 // `dt_buf` (may be null): room for step sizes [T, ld_dt], made ahead with one product; without it they are formed while
 // the rows are staged.  `Wdt` is of the type `dtype` names.
 JK_EXPORT int jk_selective_scan(const float *x, const float *low, int ld_low, int K, int N, int E, const float *z, int ld_z,
                                 const void *Wdt, const float *bdt, const float *A, const float *Dskip, float *state,
                                 const int *req_start, const int *slot_ids, int nreq, void *out, int dtype, float *dt_buf, int ld_dt,
-                                int T, cudaStream_t stream) {
+                                int T, float *scratch, long long scratch_floats, cudaStream_t stream) {
     if (nreq == 0) return JK_OK;
     JK_REQUIRE(x && low && z && Wdt && bdt && A && Dskip && state && req_start && slot_ids && out, "selective_scan: an argument is missing");
     JK_REQUIRE(K > 0 && N > 0 && E > 0 && ld_low >= K + 2 * N, "selective_scan: rank %d, states %d, channels %d, rows of %d", K, N, E, ld_low);
@@ -1660,6 +1798,27 @@ JK_EXPORT int jk_selective_scan(const float *x, const float *low, int ld_low, in
         JK_CHECK_LAUNCH("scan_steps");
     }
     ScanArgs a{x, low, ld_low, K, N, E, z, ld_z, Wdt, bdt, A, Dskip, state, req_start, slot_ids, out, ahead ? dt_buf : nullptr, ld_dt};
+    // The line: the pieces walk every row twice but side by side.  One request, 4,096 channels, 16 states (step sizes included; a walk from end
+    // to end -> pieces): 128 rows 50 -> 69 us, 256 81 -> 114, 512 148 -> 148, 2,048 589 -> 360.
+    const long long need = jk_selective_scan_scratch_floats(T, E, N);
+    if (ahead && N <= 32 && T >= 768LL * nreq && (need == 0 || (scratch != nullptr && scratch_floats >= need)) && T / SP_ROWS + nreq <= 65535) {
+        const PieceArgs p{scratch, scratch + need / (N + 1) * N, nreq};
+        const dim3 pieces((E + SP_THREADS - 1) / SP_THREADS, T / SP_ROWS + nreq);
+#define LAUNCH_S(TT, NS)                                                                                              \
+    do {                                                                                                              \
+        if (need > 0) jk_launch(selective_pieces_kernel<TT, NS, false>, pieces, dim3(SP_THREADS), 0, stream, a, p);   \
+        jk_launch(selective_pieces_kernel<TT, NS, true>, pieces, dim3(SP_THREADS), 0, stream, a, p);                  \
+    } while (0)
+#define LAUNCH(TT)                    \
+    if (N <= 8) LAUNCH_S(TT, 8);      \
+    else if (N <= 16) LAUNCH_S(TT, 16); \
+    else LAUNCH_S(TT, 32)
+        BLOCKS_BY_DTYPE(dtype, "selective_scan", LAUNCH);
+#undef LAUNCH
+#undef LAUNCH_S
+        JK_CHECK_LAUNCH("selective_scan");
+        return JK_OK;
+    }
     dim3 grid((E + SS_CHANNELS - 1) / SS_CHANNELS, nreq);
     const int per = (N + SS_LANES - 1) / SS_LANES;
     const size_t smem = (size_t)SS_CHUNK * (2 * SS_CHANNELS + SS_THREADS + 2 * N) * sizeof(float);

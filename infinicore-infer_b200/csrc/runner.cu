@@ -705,9 +705,14 @@ int run_selective_scan(Run &r, const RunnerOp &op) {
     if (int rc = r.slot(SLOT_TMP, 4LL * T * op.ld, &u, "the projection that holds a scan's gate")) return rc;
     if (int rc = r.slot(op.out_slot, (long long)r.elem() * T * op.n, &out, "a scan's output")) return rc;
     JK_REQUIRE(r.st.slot_ids != nullptr && op.state != nullptr, "runner: a scan without its state slots");
+    const long long floats = g_fns.selective_scan_scratch != nullptr ? g_fns.selective_scan_scratch(T, op.n, op.k) : 0;
+    void *scratch = nullptr;
+    if (floats > 0)
+        if (int rc = r.slot(SLOT_DECODE, 4 * floats, &scratch, "a scan's pieces")) return rc;       // (SLOT_SCAN holds the scan's maps)
     RUN(blocks, g_fns.selective_scan((const float *)x, (const float *)low, ld_low, op.rank, op.k, op.n, (const float *)u + op.g_off, op.ld,
                                      op.w2, op.b2, op.decay, op.vec, op.state, r.st.req_start, r.st.slot_ids, r.st.nreq, out,
-                                     r.env.dtype, (float *)u + op.q_off, op.ld, T, r.stream));
+                                     r.env.dtype, (float *)u + op.q_off, op.ld, T, (float *)scratch, floats, r.stream));
+    if (floats > 0 && T >= 768LL * r.st.nreq) ++g_launches;
     ++g_launches;       // the step sizes' product
     return JK_OK;
 }
@@ -1094,6 +1099,7 @@ JK_EXPORT int jk_runner_slot_bytes(const RunnerEnv *env, const RunnerOp *ops, in
             case OP_SELECTIVE_SCAN:
                 need(op.in_slot, 4 * rows * op.n); need(op.in2_slot, 4 * rows * (op.rank + 2 * op.k)); need(SLOT_TMP, 4 * rows * op.ld);
                 need(op.out_slot, e * rows * op.n);
+                if (g_fns.selective_scan_scratch != nullptr) need(SLOT_DECODE, 4 * g_fns.selective_scan_scratch((int)rows, op.n, op.k));
                 break;
             case OP_EXPERTS:
                 need(op.in_slot, e * rows * op.n); need(SLOT_DELTA, 4 * rows * op.n);

@@ -79,7 +79,8 @@ typedef int (*CausalConvFn)(const float *, int, int, int, const float *, const f
                             const int *, float *, void *, int, int, int, const float *, cudaStream_t);
 typedef int (*SelectiveScanFn)(const float *, const float *, int, int, int, int, const float *, int, const void *, const float *,
                                const float *, const float *, float *, const int *, const int *, int, void *, int, float *, int, int,
-                               cudaStream_t);
+                               float *, long long, cudaStream_t);
+typedef long long (*SelectiveScratchFn)(int, int, int);
 typedef int (*RoutedExpertsFn)(const void *, const float *, const void *, const void *, float *, int, int, int, int, int, int, int, int,
                                int *, void *, float *, int, float, const float *, const float *, int, int, int, const float *, float *, float,
                                const float *, float, float, int *, cudaStream_t);
@@ -187,6 +188,7 @@ struct RunnerFns {
     RotateRowsFn rotate_rows;
     // a latent attention's heads made for a step of many rows: csrc/blocks.cu and csrc/attention_tcgen05.cu, bound with them
     LatentGatherFn latent_gather;
+    SelectiveScratchFn selective_scan_scratch;
     AttentionLaidFn attention_laid;
 };
 

@@ -832,10 +832,13 @@ def selective_scan(x: torch.Tensor, low: torch.Tensor, dt_rank: int, states: int
     _need(w_dt, "w_dt", out.dtype)
     _need(z, "z", torch.float32, contiguous=False)
     lib = _build.load("blocks")
+    lib.jk_selective_scan_scratch_floats.restype = ctypes.c_longlong
+    floats = int(lib.jk_selective_scan_scratch_floats(_c_int(x.shape[0]), _c_int(x.shape[1]), _c_int(states))) if dt_buf is not None else 0
+    scratch = torch.empty(floats, dtype=torch.float32, device=x.device) if floats else None
     _check("blocks", lib.jk_selective_scan(_ptr(x), _ptr(low), _c_int(low.shape[1]), _c_int(dt_rank), _c_int(states), _c_int(x.shape[1]),
                                            _ptr(z), _c_int(z_ld), _ptr(w_dt), _ptr(dt_bias), _ptr(A), _ptr(skip), _ptr(state), _ptr(req_start),
                                            _ptr(slot_ids), _c_int(req_start.numel() - 1), _ptr(out), _c_int(dtype_code(out.dtype)), _ptr(dt_buf),
-                                           _c_int(dt_buf.shape[1] if dt_buf is not None else 0), _c_int(x.shape[0]), _stream()))
+                                           _c_int(dt_buf.shape[1] if dt_buf is not None else 0), _c_int(x.shape[0]), _ptr(scratch), _c_ll(floats), _stream()))
     return out
 
 

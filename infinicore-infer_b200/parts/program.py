@@ -108,7 +108,7 @@ class _Fns(ctypes.Structure):
         "norm_gate", "token_shift", "act_rows", "err_mixers", "norm_add", "concat_cast", "add_bias_rows", "latent_qkv", "head_linear", "latent_attention",
         "latent_attention_scratch", "causal_conv", "selective_scan", "routed_experts", "routed_experts_workspace",
         "routed_experts_launches", "softcap", "err_blocks", "linear_small_parts", "linear_small_parts_supports", "add_rows", "delta_rule", "delta_rule_scratch",
-        "norm_pair", "embed_pair", "join_parts", "gated_recurrence", "gated_recurrence_scratch", "gated_recurrence_launches", "rotate_rows", "latent_gather",
+        "norm_pair", "embed_pair", "join_parts", "gated_recurrence", "gated_recurrence_scratch", "gated_recurrence_launches", "rotate_rows", "latent_gather", "selective_scan_scratch",
         "attention_laid")]
 
 
@@ -173,7 +173,7 @@ def runner_lib(gemm_tcgen05: bool = False, attention_tcgen05: bool = False, mixe
         norm_pair=get("blocks", "jk_norm_pair"), embed_pair=get("blocks", "jk_embed_pair"), join_parts=get("blocks", "jk_join_parts"),
         gated_recurrence=get("blocks", "jk_gated_recurrence"), gated_recurrence_scratch=get("blocks", "jk_gated_recurrence_scratch_floats"),
         gated_recurrence_launches=get("blocks", "jk_gated_recurrence_launches"), rotate_rows=get("mixers", "jk_rotate_rows"),
-        latent_gather=get("blocks", "jk_latent_gather"), attention_laid=get("attention_tcgen05", "jk_attention_laid_tcgen05"))
+        latent_gather=get("blocks", "jk_latent_gather"), selective_scan_scratch=get("blocks", "jk_selective_scan_scratch_floats"), attention_laid=get("attention_tcgen05", "jk_attention_laid_tcgen05"))
     if lib.jk_runner_bind(ctypes.byref(fns)):
         from ..kernels import KernelError
         raise KernelError(lib.jk_runner_last_error().decode(errors="replace"))

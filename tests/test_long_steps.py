@@ -1,5 +1,6 @@
 """Steps of many rows through the kernels that only they reach: latent attention over heads made for the step, experts'
-products in tiles of 128 entries.  At the edges of tiles, against the plain implementation (tests/plain_vunelix.py)."""
+products in tiles of 128 entries, selective scans over pieces.  At the edges of tiles and pieces, against the plain
+implementation (tests/plain_vunelix.py)."""
 import json
 import os
 
@@ -94,3 +95,33 @@ def test_expert_products_in_tiles_of_entries(K, T, d, ff, experts, top, act):
         want[rows] += share.unsqueeze(-1) * (inner @ w_dn[e * d: (e + 1) * d].double().T)
     err = (delta.double().cpu() - want).abs().max()
     assert err <= 2.0 ** -8 * want.abs().max(), float(err)
+
+
+@pytest.mark.parametrize("states", [5, 16, 20])
+@pytest.mark.parametrize("lens", [(768,), (1793, 1, 513), (1475, 64), (900, 640)])
+def test_selective_scan_over_pieces(K, states, lens):
+    """Requests of exactly one piece, of one row more, and of several, from states that are not zero; 130 channels.  Float32
+    throughout: rounding of 2^-24 a step over a chain whose decays are below 1."""
+    dev, g, E, rank = torch.device("cuda:0"), torch.Generator().manual_seed(states), 130, 3
+    T = sum(lens)
+    x, z = torch.randn(T, E, generator=g), torch.randn(T, E, generator=g)
+    low = torch.randn(T, rank + 2 * states, generator=g)
+    w_dt, b_dt = torch.randn(E, rank, generator=g) * 0.3, torch.randn(E, generator=g) - 3.0
+    A, skip = -torch.exp(torch.randn(E, states, generator=g)), torch.randn(E, generator=g)
+    first = torch.randn(len(lens) + 1, E, states, generator=g)
+    state, slots = first.clone().to(dev), torch.arange(len(lens), 0, -1, dtype=torch.int32)
+    starts = torch.tensor([0] + list(lens)).cumsum(0).to(torch.int32)
+    out = torch.empty(T, E, device=dev)
+    K.selective_scan(x.to(dev), low.to(dev), rank, states, z.to(dev), E, w_dt.to(dev), b_dt.to(dev), A.to(dev), skip.to(dev), state, starts.to(dev),
+                     slots.to(dev), out, dt_buf=torch.empty(T, E, device=dev))
+    dt = torch.nn.functional.softplus(low[:, :rank].double() @ w_dt.double().T + b_dt.double())
+    for i, s in enumerate(slots.tolist()):
+        a, b = int(starts[i]), int(starts[i + 1])
+        S = first[s].double()
+        want = torch.empty(b - a, E, dtype=F)
+        for t in range(a, b):
+            S = torch.exp(dt[t].unsqueeze(1) * A.double()) * S + (dt[t] * x[t].double()).unsqueeze(1) * low[t, rank: rank + states].double()
+            want[t - a] = (S @ low[t, rank + states:].double() + skip.double() * x[t].double()) * plain.silu(z[t].double())
+        assert (out[a:b].double().cpu() - want).abs().max() <= 2e-5 * want.abs().max()
+        assert (state[s].double().cpu() - S).abs().max() <= 2e-5 * S.abs().max()
+    assert torch.equal(state[0].cpu(), first[0])
