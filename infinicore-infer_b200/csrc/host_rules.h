@@ -177,13 +177,15 @@ inline AttentionLists attention_work_lists(int B, int pad_B, const int *lens, co
 // `rows` rows has at most scan_max_pieces(rows) pieces.
 constexpr int SCAN_PIECE = 64;
 inline long long scan_max_pieces(long long rows) { return 2 * rows / SCAN_PIECE + 1; }
-// Whether the pieces of a recurrence run as tiled products within the piece (csrc/mixers.cu: piece_state, piece_rows): a constant decay per
-// head, rows that read the state after their own write, and sizes of whole vectors of four floats.
-inline bool scan_runs_tiled(int dk, int dv, int ld, int q_off, int k_off, int v_off, bool projected, bool bonus) {
-    return !projected && !bonus && dk <= 256 && ((dk | dv | ld | q_off | k_off | v_off) & 3) == 0;
+// Whether the pieces of a recurrence run as tiled products within the piece (csrc/mixers.cu: piece_state, piece_rows): rows that read the
+// state after their own write, sizes of whole vectors of four floats, and a constant decay per head; or a projected one (`rank` > 0) for
+// heads of at most 128 key channels (a warp's four channels a lane), while its weights and a piece's columns fit shared memory.
+inline bool scan_runs_tiled(int dk, int dv, int ld, int q_off, int k_off, int v_off, int rank, bool bonus) {
+    const bool decay = rank == 0 ? dk <= 256 : dk <= 128 && (long long)rank * (SCAN_PIECE + dk + 1) <= 24 * 1024;
+    return decay && !bonus && ((dk | dv | ld | q_off | k_off | v_off) & 3) == 0;
 }
 inline long long scan_scratch_floats(long long rows, int heads, int dk, int dv, bool projected) {
-    return scan_max_pieces(rows) * heads * dk * dv + (projected ? rows * heads * dk : 0);
+    return scan_max_pieces(rows) * heads * dk * dv + (projected ? (rows + scan_max_pieces(rows)) * heads * dk : 0);
 }
 
 // ---- how many ways the decode attention cuts each row's key range ------------------------------------------------

@@ -480,9 +480,9 @@ JK_EXPORT int jk_conv_qkv(const float *u, int ld, int q_off, int k_off, int v_of
 // zeros: a piece leaves its rows' outputs without what came before the piece, its own end state in `piece_state`, and (for
 // a projected decay) the running product of the decays since the piece's start, b_t, in `cum`.  `scan_carry_kernel` then
 // walks each such request's pieces in order, S <- diag(b_end) S + S_piece, leaving in `piece_state` the state at each piece's
-// START and in the slot the state after the last; `scan_prefix_kernel` adds (q_t * b_t)^T S_start to the piece's rows.  Where the decay is
-// a constant, the pieces do not walk their rows at all: their end states and rows are tiled products (`piece_state_kernel` ahead of the
-// carry, `piece_rows_kernel` behind it).
+// START and in the slot the state after the last; `scan_prefix_kernel` adds (q_t * b_t)^T S_start to the piece's rows.  Where
+// jk::scan_runs_tiled says so, the pieces do not walk their rows at all: their end states and rows are tiled products
+// (`piece_state_kernel` ahead of the carry, `piece_rows_kernel` behind it).
 // Nothing is ever divided by a decay.  The order of the sums of a row depends on where its piece starts (every SCAN_PIECE
 // rows from the start of its portion) and on nothing else of the batch.
 // ---------------------------------------------------------------------------------------------------------------
@@ -509,7 +509,8 @@ struct ScanArgs {
     int n_pieces;
     const int *piece_reqs;      // [n_piece_reqs, 3] (request, its first piece, its pieces)
     float *piece_state;         // [n_pieces, heads, dk, dv]
-    float *cum;                 // [T, heads, dk] running products of a projected decay inside each piece
+    float *cum;                 // [T, heads, dk] running products of a projected decay inside each piece (pieces that run as products: the decays)
+    float *ends;                // [n_pieces, heads, dk] pieces that run as products: the product of a piece's projected decays; else null
     int vec4;                   // 1: rows, offsets and sizes are multiples of four floats: staging moves 16 bytes at a time
     int dkp;                    // channels of a staged row: dk rounded up to kq * KS; the padding stays zero, so the scan's
                                 // inner loop needs no bounds
@@ -772,7 +773,9 @@ __global__ void scan_carry_kernel(ScanArgs a) {
             if (p < np) {
                 mine[j] = ps[(size_t)p * stride];
                 const int first = a.pieces[2 * (p0 + p)], n = a.pieces[2 * (p0 + p) + 1];
-                if (a.w2 != nullptr) {
+                if (a.ends != nullptr) {
+                    d[j] = a.ends[((size_t)(p0 + p) * a.heads + head) * a.dk + kk];
+                } else if (a.w2 != nullptr) {
                     d[j] = a.cum[((size_t)(first + n - 1) * a.heads + head) * a.dk + kk];
                 } else if (n == SCAN_PIECE) {
                     d[j] = d_whole;
@@ -892,12 +895,23 @@ scan_prefix_kernel(ScanArgs a) {
     }
 }
 
-// ---- pieces of a recurrence with a constant decay d, as products within the piece ---------------------------------------------------------
+// ---- pieces of a recurrence as products within the piece: a constant decay d -------------------------------------------------------------
 // With t, s the rows of a piece of n rows, the recurrence from zeros written out:
 //     end state   S_piece = sum_s d^(n-1-s) k_s v_s^T                               piece_state_kernel, ahead of the carry
 //     rows        o_t = d^(t+1) S_start^T q_t + sum_(s <= t) d^(t-s) (q_t . k_s) v_s    piece_rows_kernel, behind it
 // Everything is float32 on the CUDA cores, operands through shared memory by asynchronous copies, a register tile a thread; no power of the
 // decay is ever divided by, and those of a piece are made by repeated products.
+// ---- and a projected one, a_t[k] a channel and row (heads of at most 128 key channels) -----------------------------------------------------
+// With D(s, t)[k] the product of a[k] over the rows s + 1 .. t, the factor d^(t-s) moves inside the sum over the channels:
+//     end state   S_piece = sum_s (D(s, n-1) k_s) v_s^T
+//     rows        o_t = S_start^T (D(-1, t) q_t) + sum_(s <= t) (sum_k q_t[k] D(s, t)[k] k_s[k]) v_s
+// piece_decays_kernel leaves the decays in `cum` and their product over each piece in `ends`.  D(s, t) is never a quotient: the piece's rows
+// are cut in four quarters of 16; with e the last row of s's quarter (half) and t in a later one, D(s, t) = D(s, e) D(e, t), a factor for
+// the key and one for the query, so quarters (1 on 0, 3 on 2) and halves (1 on 0) are plain products of scaled rows; within a quarter
+// a warp walks the running products, four channels a lane, its 16 rows' decays in registers.
+// What bounded it: walking the rows, every row reads its decay, key and query from shared memory for every four columns and waits on
+// the row before (16 heads of 128 x 128, 2,048 rows: the scan 332 us, the carry 42, the prefix product 150; now decays 30, end states 42, carry 40, rows 90.
+// All of it: 65 rows 153 -> 82 us, 512 rows 183 -> 91, 2,048 rows 501 -> 190).
 // ------------------------------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void piece_copy16(float *dst, const float *src, bool valid) {
     const int bytes = valid ? 16 : 0;           // 0 bytes read: the 16 bytes are filled with zeros
@@ -920,17 +934,73 @@ __device__ __forceinline__ float4 piece_act(int act, float4 v, float f) {
 
 // A block makes KB x CB of a piece's end state; thread (ty, tx) of 16 x 16 keeps key channels ty * 4 + {0..3} (and 64 on), columns
 // tx * 4 + {0..3} (and 64 on).
-template <int KB, int CB>
+// A block = (piece, head): z = W2 act(r_t) + b2 and the decay of it, the chain of sums of the scan kernel, four rows a thread; the product of
+// the piece's decays.  Heads of at most 128 key channels, the head's rows of W2 and the piece's rows of r in shared memory.
+template <typename TW>
+__global__ void __launch_bounds__(256) piece_decays_kernel(ScanArgs a) {
+    pdl_trigger();
+    extern __shared__ __align__(16) float pd_sm[];
+    __shared__ float part[256];
+    float *sr = pd_sm, *sw = pd_sm + SCAN_PIECE * a.rank;       // [64][rank], [rank][dk + 1]
+    const int p = blockIdx.x, head = blockIdx.y, dk = a.dk;
+    const int first = a.pieces[2 * p], n = a.pieces[2 * p + 1];
+    pdl_wait();
+    for (int i = threadIdx.x; i < dk * a.rank; i += 256) {
+        const int kk = i / a.rank, r = i - kk * a.rank;
+        sw[r * (dk + 1) + kk] = to_f32(((const TW *)a.w2)[(size_t)head * dk * a.rank + i]);
+    }
+    for (int i = threadIdx.x; i < n * a.rank; i += 256) {
+        const int tt = i / a.rank;
+        sr[i] = apply_act(a.rank_act, a.u[(size_t)(first + tt) * a.ld + a.r_off + (i - tt * a.rank)]);
+    }
+    __syncthreads();
+    const int groups = 256 / dk, kk = threadIdx.x % dk, g = threadIdx.x / dk;
+    if (g < groups) {
+        const float bias = a.b2 ? a.b2[head * dk + kk] : 0.f;
+        float prod = 1.f;
+        for (int t0 = 4 * g; t0 < n; t0 += 4 * groups) {
+            float z[4] = {bias, bias, bias, bias};
+            const float *r0 = sr + (size_t)t0 * a.rank, *r1 = sr + (size_t)min(t0 + 1, n - 1) * a.rank;
+            const float *r2 = sr + (size_t)min(t0 + 2, n - 1) * a.rank, *r3 = sr + (size_t)min(t0 + 3, n - 1) * a.rank;
+            const float *w = sw + kk;
+#pragma unroll 4
+            for (int r = 0; r < a.rank; ++r) {
+                const float wv = w[r * (dk + 1)];
+                z[0] = fmaf(wv, r0[r], z[0]);
+                z[1] = fmaf(wv, r1[r], z[1]);
+                z[2] = fmaf(wv, r2[r], z[2]);
+                z[3] = fmaf(wv, r3[r], z[3]);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (t0 + j < n) {
+                    const float d = a.decay_form == 1 ? expf(-expf(z[j])) : expf(log_sigmoid_f(z[j]) * a.inv_tau);
+                    a.cum[((size_t)(first + t0 + j) * a.heads + head) * dk + kk] = d;
+                    prod *= d;
+                }
+        }
+        part[threadIdx.x] = prod;
+    }
+    __syncthreads();
+    if (threadIdx.x < dk) {
+        float b = part[threadIdx.x];
+        for (int j = 1; j < groups; ++j) b *= part[j * dk + threadIdx.x];
+        a.ends[((size_t)p * a.heads + head) * dk + threadIdx.x] = b;
+    }
+}
+
+// PROJ: the decays are those in `cum` (one block of key channels then, dk <= KB)
+template <int KB, int CB, bool PROJ>
 __global__ void __launch_bounds__(256) piece_state_kernel(ScanArgs a) {
     pdl_trigger();
     constexpr int KH = KB / 64, CH = CB / 64;
     extern __shared__ __align__(16) float ps_sm[];      // [64][KB] keys, [64][CB] values
-    __shared__ float pw[SCAN_PIECE + 1];
+    __shared__ __align__(16) float pw[PROJ ? 8 * KB : SCAN_PIECE + 1];        // the constant's powers; PROJ: [8][KB] the decays' products over eight rows each
     float *Ks = ps_sm, *Vs = ps_sm + SCAN_PIECE * KB;
     const int p = blockIdx.x, head = blockIdx.y, nkb = (a.dk + KB - 1) / KB;
     const int k0 = (blockIdx.z % nkb) * KB, c0 = (blockIdx.z / nkb) * CB;
     const int first = a.pieces[2 * p], n = a.pieces[2 * p + 1];
-    piece_powers(a.decay[head], pw);
+    if (!PROJ) piece_powers(a.decay[head], pw);
     pdl_wait();
     const float *u = a.u + (size_t)first * a.ld;
     for (int i = threadIdx.x; i < SCAN_PIECE * (KB / 4); i += 256) {
@@ -943,12 +1013,39 @@ __global__ void __launch_bounds__(256) piece_state_kernel(ScanArgs a) {
         const bool valid = t < n && c < a.dv;
         piece_copy16(Vs + 4 * i, valid ? u + (size_t)t * a.ld + a.v_off + head * a.dv + c : u, valid);
     }
-    piece_copies_done();
-    __syncthreads();            // the powers
-    for (int i = threadIdx.x; i < SCAN_PIECE * (KB / 4); i += 256) {        // what this thread brought itself
-        const int t = i / (KB / 4);
-        float4 *v = reinterpret_cast<float4 *>(Ks) + i;
-        *v = piece_act(a.qkv_act, *v, t < n ? pw[n - 1 - t] : 0.f);
+    if (PROJ) {     // warp w: rows 8 w .. 8 w + 7, four channels a lane; a key times the decays of the rows behind it
+        const int warp = threadIdx.x >> 5, kk = (threadIdx.x & 31) * 4;
+        float4 d[8], c = make_float4(1.f, 1.f, 1.f, 1.f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            d[j] = kk < a.dk && warp * 8 + j < n ? *reinterpret_cast<const float4 *>(a.cum + ((size_t)(first + warp * 8 + j) * a.heads + head) * a.dk + kk) : c;
+        float4 all = d[7];
+#pragma unroll
+        for (int j = 6; j >= 0; --j) { all.x *= d[j].x; all.y *= d[j].y; all.z *= d[j].z; all.w *= d[j].w; }
+        if (kk < KB) *reinterpret_cast<float4 *>(pw + warp * KB + kk) = all;
+        piece_copies_done();
+        __syncthreads();
+        if (kk < KB) {
+            for (int w = 7; w > warp; --w) {
+                const float4 f = *reinterpret_cast<const float4 *>(pw + w * KB + kk);
+                c.x *= f.x; c.y *= f.y; c.z *= f.z; c.w *= f.w;
+            }
+#pragma unroll
+            for (int j = 7; j >= 0; --j) {
+                float4 *v = reinterpret_cast<float4 *>(Ks + (warp * 8 + j) * KB + kk);
+                const float4 k = piece_act(a.qkv_act, *v, 1.f);
+                *v = make_float4(k.x * c.x, k.y * c.y, k.z * c.z, k.w * c.w);
+                c.x *= d[j].x; c.y *= d[j].y; c.z *= d[j].z; c.w *= d[j].w;
+            }
+        }
+    } else {
+        piece_copies_done();
+        __syncthreads();            // the powers
+        for (int i = threadIdx.x; i < SCAN_PIECE * (KB / 4); i += 256) {        // what this thread brought itself
+            const int t = i / (KB / 4);
+            float4 *v = reinterpret_cast<float4 *>(Ks) + i;
+            *v = piece_act(a.qkv_act, *v, t < n ? pw[n - 1 - t] : 0.f);
+        }
     }
     if (a.qkv_act != ACT_NONE)
         for (int i = threadIdx.x; i < SCAN_PIECE * (CB / 4); i += 256) {
@@ -989,17 +1086,18 @@ __global__ void __launch_bounds__(256) piece_state_kernel(ScanArgs a) {
 
 // A block makes the 64 rows x COLS columns of a piece and head.  First the weights A[t, s] = d^(t-s) (q_t . k_s) for s <= t (thread (ty, tx)
 // of 16 x 16: rows ty * 4 + {0..3}, columns tx + 16 {0..3}); then warp w has rows 8 w .. 8 w + 7, a lane four neighbouring columns.
-template <int COLS>
+// PROJ: with the decays in `cum` (at most 128 key channels), the weights by quarters and halves, as above.
+template <int COLS, bool PROJ>
 __global__ void __launch_bounds__(256, 2) piece_rows_kernel(ScanArgs a) {
     pdl_trigger();
     constexpr int L = COLS / 4, GROUPS = 32 / L, ROWS = 8 / GROUPS, AL = SCAN_PIECE + 4;      // lanes a row; rows a thread
     extern __shared__ __align__(16) float pr_sm[];
-    __shared__ float pw[SCAN_PIECE + 1];
+    __shared__ __align__(16) float pw[PROJ ? 4 * 128 : SCAN_PIECE + 1];         // the constant's powers; PROJ: [4][128] the decays' products over a quarter
     const int dkp = a.dk + 4;           // rows of q and k four floats apart in their banks
     float *Qs = pr_sm, *As = Qs + SCAN_PIECE * dkp, *B = As + SCAN_PIECE * AL;      // B: keys, then pieces of the state, then values
     const int p = blockIdx.x, head = blockIdx.y, c0 = blockIdx.z * COLS;
     const int first = a.pieces[2 * p], n = a.pieces[2 * p + 1];
-    piece_powers(a.decay[head], pw);
+    if (!PROJ) piece_powers(a.decay[head], pw);
     pdl_wait();
     const float *u = a.u + (size_t)first * a.ld;
     const int quads = a.dk / 4;
@@ -1009,6 +1107,17 @@ __global__ void __launch_bounds__(256, 2) piece_rows_kernel(ScanArgs a) {
         piece_copy16(Qs + t * dkp + kk, t < n ? row + a.q_off : u, t < n);
         piece_copy16(B + t * dkp + kk, t < n ? row + a.k_off : u, t < n);
     }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    [[maybe_unused]] float4 d16[PROJ ? 16 : 1];          // the decays of the warp's quarter
+    if constexpr (PROJ) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const int t = (warp >> 1) * 16 + j;
+            d16[j] = lane < quads && t < n ? *reinterpret_cast<const float4 *>(a.cum + ((size_t)(first + t) * a.heads + head) * a.dk + 4 * lane)
+                                           : make_float4(1.f, 1.f, 1.f, 1.f);
+        }
+        for (int i = threadIdx.x; i < SCAN_PIECE * AL; i += 256) As[i] = 0.f;
+    }
     piece_copies_done();
     for (int i = threadIdx.x; i < SCAN_PIECE * quads; i += 256) {
         const int t = i / quads, kk = (i - t * quads) * 4;
@@ -1017,7 +1126,102 @@ __global__ void __launch_bounds__(256, 2) piece_rows_kernel(ScanArgs a) {
         if (a.qkv_act != ACT_NONE) *k = piece_act(a.qkv_act, *k, 1.f);
     }
     __syncthreads();
-    {
+    if constexpr (PROJ) {
+        const int quarter = warp >> 1, odd = warp & 1, tq = quarter * 16, kl = 4 * lane;
+        const bool live = lane < quads;
+        // within a quarter, the even or the odd s: w = D(s, t) k_s walks down t; 16 sums over the warp's channels at a time
+        for (int s = odd; s < 16; s += 2) {
+            float4 w = live ? *reinterpret_cast<const float4 *>(B + (tq + s) * dkp + kl) : make_float4(0.f, 0.f, 0.f, 0.f);
+            float v[16];
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                v[t] = 0.f;
+                if (t >= s) {
+                    if (t > s) { w.x *= d16[t].x; w.y *= d16[t].y; w.z *= d16[t].z; w.w *= d16[t].w; }
+                    const float4 q = live ? *reinterpret_cast<const float4 *>(Qs + (tq + t) * dkp + kl) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    v[t] = fmaf(q.w, w.w, fmaf(q.z, w.z, fmaf(q.y, w.y, q.x * w.x)));
+                }
+            }
+            // lanes halve the sums they keep: lane l ends with t = l / 2
+#pragma unroll
+            for (int half = 8; half >= 1; half >>= 1) {
+                const bool up = lane & (2 * half);
+#pragma unroll
+                for (int i = 0; i < half; ++i) {
+                    const float give = up ? v[i] : v[i + half], keep = up ? v[i + half] : v[i];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * half);
+                }
+            }
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+            if (!(lane & 1) && (lane >> 1) >= s) As[(tq + (lane >> 1)) * AL + tq + s] = v[0];
+        }
+        __syncthreads();
+        // queries times the decays from their quarter's start, keys times those to its end
+        if (live) {
+            float4 c = make_float4(1.f, 1.f, 1.f, 1.f);
+            if (odd) {
+#pragma unroll
+                for (int s = 15; s >= 0; --s) {
+                    float4 *k = reinterpret_cast<float4 *>(B + (tq + s) * dkp + kl);
+                    *k = make_float4(k->x * c.x, k->y * c.y, k->z * c.z, k->w * c.w);
+                    c.x *= d16[s].x; c.y *= d16[s].y; c.z *= d16[s].z; c.w *= d16[s].w;
+                }
+                *reinterpret_cast<float4 *>(pw + quarter * 128 + kl) = c;
+            } else {
+#pragma unroll
+                for (int t = 0; t < 16; ++t) {
+                    float4 *q = reinterpret_cast<float4 *>(Qs + (tq + t) * dkp + kl);
+                    c.x *= d16[t].x; c.y *= d16[t].y; c.z *= d16[t].z; c.w *= d16[t].w;
+                    *q = make_float4(q->x * c.x, q->y * c.y, q->z * c.z, q->w * c.w);
+                }
+            }
+        }
+        __syncthreads();
+        auto dot4 = [](float4 q, float4 k, float s) { return fmaf(q.w, k.w, fmaf(q.z, k.z, fmaf(q.y, k.y, fmaf(q.x, k.x, s)))); };
+        {       // quarters 1 on 0 and 3 on 2: two columns a thread
+            const int pair = threadIdx.x >> 7, t = 32 * pair + 16 + ((threadIdx.x >> 3) & 15), s = 32 * pair + (threadIdx.x & 7);
+            float s0 = 0.f, s1 = 0.f;
+            for (int kk = 0; kk < a.dk; kk += 4) {
+                const float4 q = *reinterpret_cast<const float4 *>(Qs + t * dkp + kk);
+                s0 = dot4(q, *reinterpret_cast<const float4 *>(B + s * dkp + kk), s0);
+                s1 = dot4(q, *reinterpret_cast<const float4 *>(B + (s + 8) * dkp + kk), s1);
+            }
+            As[t * AL + s] = s0;
+            As[t * AL + s + 8] = s1;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < 16 * quads; i += 256) {       // from the half's start, to the half's end
+            const int r = i / quads, kk = (i - r * quads) * 4;
+            float4 *q = reinterpret_cast<float4 *>(Qs + (48 + r) * dkp + kk), *k = reinterpret_cast<float4 *>(B + r * dkp + kk);
+            const float4 f2 = *reinterpret_cast<const float4 *>(pw + 2 * 128 + kk), f1 = *reinterpret_cast<const float4 *>(pw + 128 + kk);
+            *q = make_float4(q->x * f2.x, q->y * f2.y, q->z * f2.z, q->w * f2.w);
+            *k = make_float4(k->x * f1.x, k->y * f1.y, k->z * f1.z, k->w * f1.w);
+        }
+        __syncthreads();
+        {       // the second half's rows on the first half's: two rows and two columns a thread
+            const int t = 32 + (threadIdx.x >> 4), s = threadIdx.x & 15;
+            float s00 = 0.f, s01 = 0.f, s10 = 0.f, s11 = 0.f;
+            for (int kk = 0; kk < a.dk; kk += 4) {
+                const float4 q0 = *reinterpret_cast<const float4 *>(Qs + t * dkp + kk), q1 = *reinterpret_cast<const float4 *>(Qs + (t + 16) * dkp + kk);
+                const float4 k0 = *reinterpret_cast<const float4 *>(B + s * dkp + kk), k1 = *reinterpret_cast<const float4 *>(B + (s + 16) * dkp + kk);
+                s00 = dot4(q0, k0, s00); s01 = dot4(q0, k1, s01);
+                s10 = dot4(q1, k0, s10); s11 = dot4(q1, k1, s11);
+            }
+            As[t * AL + s] = s00; As[t * AL + s + 16] = s01;
+            As[(t + 16) * AL + s] = s10; As[(t + 16) * AL + s + 16] = s11;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < 48 * quads; i += 256) {       // queries times the decays from the piece's start
+            const int r = i / quads, kk = (i - r * quads) * 4;
+            float4 *q = reinterpret_cast<float4 *>(Qs + (16 + r) * dkp + kk);
+            float4 f = *reinterpret_cast<const float4 *>(pw + kk);
+            if (r >= 16) {
+                const float4 f1 = *reinterpret_cast<const float4 *>(pw + 128 + kk);
+                f.x *= f1.x; f.y *= f1.y; f.z *= f1.z; f.w *= f1.w;
+            }
+            *q = make_float4(q->x * f.x, q->y * f.y, q->z * f.z, q->w * f.w);
+        }
+    } else {
         const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
         float acc[4][4];
 #pragma unroll
@@ -1046,7 +1250,6 @@ __global__ void __launch_bounds__(256, 2) piece_rows_kernel(ScanArgs a) {
                 As[t * AL + s] = s <= t ? acc[r][c] * pw[t - s] : 0.f;
             }
     }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = warp * 8 + (lane / L) * ROWS, cl = (lane % L) * 4;
     float acc[ROWS][4];
 #pragma unroll
@@ -1083,10 +1286,12 @@ __global__ void __launch_bounds__(256, 2) piece_rows_kernel(ScanArgs a) {
         __syncthreads();
         rows_product(Qs + kb, dkp, nk);
     }
+    if constexpr (!PROJ) {
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r)
+        for (int r = 0; r < ROWS; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] *= pw[t0 + r + 1];
+            for (int c = 0; c < 4; ++c) acc[r][c] *= pw[t0 + r + 1];
+    }
     // the piece's own rows
     __syncthreads();
     for (int i = threadIdx.x; i < SCAN_PIECE * L; i += 256) {
@@ -1101,7 +1306,17 @@ __global__ void __launch_bounds__(256, 2) piece_rows_kernel(ScanArgs a) {
             *v = piece_act(a.qkv_act, *v, 1.f);
         }
     __syncthreads();
-    rows_product(As, AL, warp * 8 + 8);        // no row of the warp sees a later one
+    rows_product(As, AL, warp * 8);
+    for (int s = warp * 8; s < warp * 8 + 8; ++s) {         // no row sees a later one, not even times zero
+        const float4 b = *reinterpret_cast<const float4 *>(B + s * COLS + cl);
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r)
+            if (t0 + r >= s) {
+                const float x = As[(t0 + r) * AL + s];
+                acc[r][0] = fmaf(x, b.x, acc[r][0]); acc[r][1] = fmaf(x, b.y, acc[r][1]);
+                acc[r][2] = fmaf(x, b.z, acc[r][2]); acc[r][3] = fmaf(x, b.w, acc[r][3]);
+            }
+    }
     if (c0 + cl < a.dv) {
 #pragma unroll
         for (int r = 0; r < ROWS; ++r)
@@ -1113,14 +1328,17 @@ __global__ void __launch_bounds__(256, 2) piece_rows_kernel(ScanArgs a) {
 template <int KB, int CB>
 static void launch_piece_state(const ScanArgs &a, cudaStream_t stream) {
     const size_t smem = sizeof(float) * SCAN_PIECE * (KB + CB);
-    cudaFuncSetAttribute(piece_state_kernel<KB, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    jk_launch(piece_state_kernel<KB, CB>, dim3(a.n_pieces, a.heads, ((a.dk + KB - 1) / KB) * ((a.dv + CB - 1) / CB)), dim3(256), smem, stream, a);
+    const dim3 grid(a.n_pieces, a.heads, ((a.dk + KB - 1) / KB) * ((a.dv + CB - 1) / CB));
+    auto *kernel = a.ends != nullptr ? piece_state_kernel<KB, CB, true> : piece_state_kernel<KB, CB, false>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    jk_launch(kernel, grid, dim3(256), smem, stream, a);
 }
 template <int COLS>
 static void launch_piece_rows(const ScanArgs &a, cudaStream_t stream) {
     const size_t smem = sizeof(float) * SCAN_PIECE * ((a.dk + 4) + (SCAN_PIECE + 4) + std::max(a.dk + 4, COLS));
-    cudaFuncSetAttribute(piece_rows_kernel<COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    jk_launch(piece_rows_kernel<COLS>, dim3(a.n_pieces, a.heads, (a.dv + COLS - 1) / COLS), dim3(256), smem, stream, a);
+    auto *kernel = a.ends != nullptr ? piece_rows_kernel<COLS, true> : piece_rows_kernel<COLS, false>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    jk_launch(kernel, dim3(a.n_pieces, a.heads, (a.dv + COLS - 1) / COLS), dim3(256), smem, stream, a);
 }
 
 // Rows of scratch the pieces of a step of `rows` rows need at most: piece_state floats, cum floats.
@@ -1149,8 +1367,9 @@ JK_EXPORT int jk_linear_scan(const float *u, int ld, int q_off, int k_off, int v
     // lanes per column: as few as keep a thread's state at 64 values (more beyond 1024 and 512 channels); more of them,
     // and so fewer columns a block and more blocks, while the blocks do not fill the SMs
     const int sm_count = sms > 0 ? sms : 148;
-    const bool tiled = n_pieces > 0 && jk::scan_runs_tiled(dk, dv, ld, q_off, k_off, v_off, w2 != nullptr, bonus != nullptr) &&
-                       ((uintptr_t)u | (uintptr_t)scratch | (uintptr_t)out) % 16 == 0;
+    const bool tiled = n_pieces > 0 && jk::scan_runs_tiled(dk, dv, ld, q_off, k_off, v_off, w2 ? rank : 0, bonus != nullptr) &&
+                       ((uintptr_t)u | (uintptr_t)scratch | (uintptr_t)out) % 16 == 0 &&
+                       (w2 == nullptr || state_floats + (long long)T * heads * dk + (long long)n_pieces * heads * dk <= scratch_floats);
     const int items = n_direct + (tiled ? 0 : n_pieces);        // of the scan kernel
     auto lanes_for = [&](int c) {
         int q = 1;
@@ -1180,7 +1399,7 @@ JK_EXPORT int jk_linear_scan(const float *u, int ld, int q_off, int k_off, int v
     const int stage_w2 = w2 != nullptr && w2_bytes <= 64 * 1024 ? 1 : 0;
     ScanArgs a{u, ld, q_off, k_off, v_off, r_off, heads, dk, dv, qkv_act, q_scale, decay, w2, b2, rank, tau > 0.f ? 1.f / tau : 0.f,
                state, req_start, slot_ids, out, kq, chunk, direct, n_direct, pieces, n_pieces, piece_reqs, scratch,
-               scratch ? scratch + state_floats : nullptr,
+               scratch ? scratch + state_floats : nullptr, tiled && w2 ? scratch + state_floats + (long long)T * heads * dk : nullptr,
                (dk % 4 == 0 && dv % 4 == 0 && ld % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && (uintptr_t)u % 16 == 0 &&
                 (scratch == nullptr || (uintptr_t)scratch % 16 == 0)) ? 1 : 0,
                dkp, bonus, decay_form, rank_act, stage_w2};
@@ -1228,6 +1447,13 @@ JK_EXPORT int jk_linear_scan(const float *u, int ld, int q_off, int k_off, int v
     JK_CHECK_LAUNCH("linear_scan");
     if (n_pieces > 0) {
         if (tiled) {
+            if (w2 != nullptr) {
+                const size_t bytes = sizeof(float) * (size_t)rank * (SCAN_PIECE + dk + 1);
+                auto *kernel = w2_dtype == JK_BF16 ? piece_decays_kernel<__nv_bfloat16> : piece_decays_kernel<float>;
+                if (bytes > 46 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+                jk_launch(kernel, dim3(n_pieces, heads), dim3(256), bytes, stream, a);
+                JK_CHECK_LAUNCH("piece_decays");
+            }
             if (dk <= 64) { if (dv <= 64) launch_piece_state<64, 64>(a, stream); else launch_piece_state<64, 128>(a, stream); }
             else { if (dv <= 64) launch_piece_state<128, 64>(a, stream); else launch_piece_state<128, 128>(a, stream); }
             JK_CHECK_LAUNCH("piece_state");

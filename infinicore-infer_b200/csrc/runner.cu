@@ -510,7 +510,7 @@ int run_linear_attention(Run &r, const RunnerOp &op) {
     void *scratch = nullptr;
     long long scratch_floats = 0;
     if (n_pieces > 0) {
-        scratch_floats = (long long)n_pieces * op.heads * op.head_dim * dv + (op.rank ? (long long)T * op.heads * op.head_dim : 0);
+        scratch_floats = (long long)n_pieces * op.heads * op.head_dim * dv + (op.rank ? (long long)(T + n_pieces) * op.heads * op.head_dim : 0);
         if (int rc = r.slot(SLOT_SCAN, 4 * scratch_floats, &scratch, "the pieces of a recurrence")) return rc;
     }
     RUN(mixers, g_fns.linear_scan((const float *)u, op.ld, op.q_off, op.k_off, op.v_off, op.heads, op.head_dim, dv, op.act, op.q_scale,
@@ -518,9 +518,13 @@ int run_linear_attention(Run &r, const RunnerOp &op) {
                                   r.st.nreq, T, (float *)mix, r.st.lists[op.list_short], r.st.list_n[op.list_short],
                                   r.st.lists[op.list_tiles], n_pieces, r.st.lists[op.list_aux], r.st.list_n[op.list_aux],
                                   (float *)scratch, scratch_floats, r.env.routing.sms, op.bonus, op.decay_form, op.rank_act, r.stream));
-    // the carry and the prefix kernels; pieces that run as tiled products have a kernel beside the one of the requests that run in one go
-    if (n_pieces > 0)
-        g_launches += 2 + (r.st.list_n[op.list_short] > 0 && jk::scan_runs_tiled(op.head_dim, dv, op.ld, op.q_off, op.k_off, op.v_off, op.w2 != nullptr, op.bonus != nullptr) ? 1 : 0);
+    // the carry and the prefix kernels; pieces that run as tiled products have a kernel beside the one of the requests that run in one go,
+    // and one for a projected decay
+    if (n_pieces > 0) {
+        g_launches += 2;
+        if (jk::scan_runs_tiled(op.head_dim, dv, op.ld, op.q_off, op.k_off, op.v_off, op.rank, op.bonus != nullptr))
+            g_launches += (r.st.list_n[op.list_short] > 0 ? 1 : 0) + (op.rank > 0 ? 1 : 0);
+    }
     RUN(mixers, g_fns.norm_gate((const float *)mix, (const float *)u, op.ld, op.g_off, op.vec, op.eps, op.heads, dv, op.per_head_norm,
                                 op.gate_act, out, r.env.dtype, T, r.stream));
     return JK_OK;

@@ -666,7 +666,7 @@ def linear_scan(u: torch.Tensor, offsets, heads: int, dk: int, dv: int, qkv_act:
     scratch, floats = None, 0
     if n_pieces:
         _need(pieces, "pieces", torch.int32); _need(piece_reqs, "piece_reqs", torch.int32)
-        floats = n_pieces * heads * dk * dv + (T * heads * dk if w2 is not None else 0)
+        floats = n_pieces * heads * dk * dv + ((T + n_pieces) * heads * dk if w2 is not None else 0)
         scratch = torch.empty(floats, dtype=torch.float32, device=u.device)
     if direct is not None:
         _need(direct, "direct", torch.int32)

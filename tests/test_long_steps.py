@@ -1,9 +1,10 @@
 """Steps of many rows through the kernels that only they reach: latent attention over heads made for the step, experts'
-products in tiles of 128 entries, selective scans over pieces.  At the edges of tiles and pieces, against the plain
-implementation (tests/plain_vunelix.py)."""
+products in tiles of 128 entries, selective scans and recurrences over pieces.  At the edges of tiles and pieces, against the
+plain implementation (tests/plain_vunelix.py) or the sums written out."""
 import json
 import os
 
+import numpy as np
 import pytest
 import torch
 
@@ -125,3 +126,47 @@ def test_selective_scan_over_pieces(K, states, lens):
         assert (out[a:b].double().cpu() - want).abs().max() <= 2e-5 * want.abs().max()
         assert (state[s].double().cpu() - S).abs().max() <= 2e-5 * S.abs().max()
     assert torch.equal(state[0].cpu(), first[0])
+
+
+@pytest.mark.parametrize("dk,dv,rank,form,act,w2_type", [(128, 128, 16, 0, 0, torch.bfloat16), (64, 160, 5, 1, 1, torch.float32), (4, 12, 3, 0, 0, torch.float32),
+                                                         (100, 36, 24, 0, 1, torch.bfloat16), (68, 64, 1, 1, 0, torch.float32)])
+def test_projected_decay_recurrence_as_products_within_pieces(K, dk, dv, rank, form, act, w2_type):
+    """Portions that end at the edges of quarters and halves of a piece, beside one that runs in one go, from states that are not
+    zero; the same rows laid so that vectors of four do not fit walk the pieces row by row.  Float32 sums of at most dk + 64 terms
+    whose decays are below 1: rounding of 2^-24 a step."""
+    from infinicore_infer_b200.parts import LinearAttention
+    dev, g, H = torch.device("cuda:0"), torch.Generator().manual_seed(dk + dv), 2
+    lens = [65, 80, 3, 97, 160, 127]
+    T, n = sum(lens), len(lens)
+    u = torch.randn(T, 2 * H * dk + H * dv + rank, generator=g)
+    w2 = (torch.randn(H * dk, rank, generator=g) * 0.7).to(w2_type)
+    b2 = torch.randn(H * dk, generator=g) - (2.0 if form else -2.0)
+    first = torch.randn(n + 1, H, dk, dv, generator=g)
+    starts, slots = torch.tensor([0] + lens).cumsum(0).to(torch.int32), torch.arange(n, 0, -1, dtype=torch.int32)
+    caps = LinearAttention.step_list_capacity(T, n)
+    arrays = {name: np.zeros(max(1, c), dtype=np.int32) for name, c in caps.items()}
+    counts = LinearAttention.fill_step_lists(n, n, lens, [0] * n, arrays)
+    lists = {name: torch.from_numpy(arrays[name][:max(1, counts[name][0] * w)]).to(dev) for name, w in (("direct", 1), ("pieces", 2), ("piece_reqs", 3))}
+    got = []
+    for shift in (0, 1):        # 1: offsets that are no multiples of four
+        rows = torch.cat([torch.zeros(T, shift), u, torch.zeros(T, -(u.shape[1] + shift) % 4)], 1).contiguous().to(dev)
+        state, out = first.clone().to(dev), torch.empty(T, H * dv, device=dev)
+        K.linear_scan(rows, (shift, shift + H * dk, shift + 2 * H * dk), H, dk, dv, act, 0.5, None, w2.to(dev), b2.to(dev), shift + 2 * H * dk + H * dv,
+                      6.0, state, starts.to(dev), slots.to(dev), out, decay_form=form, **lists)
+        got.append((out.double().cpu(), state.double().cpu()))
+    f = plain.silu if act else (lambda x: x)
+    U = u.double()
+    q, k = f(U[:, :H * dk]).view(T, H, dk) * 0.5, f(U[:, H * dk: 2 * H * dk]).view(T, H, dk)
+    v = f(U[:, 2 * H * dk: 2 * H * dk + H * dv]).view(T, H, dv)
+    z = (U[:, 2 * H * dk + H * dv:] @ w2.double().T + b2.double()).view(T, H, dk)
+    a = torch.exp(-torch.exp(z)) if form else torch.exp(torch.nn.functional.logsigmoid(z) / 6.0)
+    for i, s in enumerate(slots.tolist()):
+        S, want = first[s].double(), []
+        for t in range(int(starts[i]), int(starts[i + 1])):
+            S = a[t].unsqueeze(-1) * S + k[t].unsqueeze(-1) * v[t].unsqueeze(1)
+            want.append(torch.einsum("hkv,hk->hv", S, q[t]).reshape(-1))
+        want = torch.stack(want)
+        for out, state in got:
+            assert (out[int(starts[i]): int(starts[i + 1])] - want).abs().max() <= 2e-5 * want.abs().max(), f"request {i}"
+            assert (state[s] - S).abs().max() <= 2e-5 * S.abs().max(), f"state of request {i}"
+    assert torch.equal(got[0][1][0], first[0].double()) and not torch.equal(got[0][0], got[1][0])
