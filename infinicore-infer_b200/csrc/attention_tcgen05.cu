@@ -43,7 +43,7 @@
 
 JK_DEFINE_ERROR_BUFFER(jk_attention_tcgen05)
 
-constexpr int AT_BM = 128, AT_BN = 128, AT_HALF = 64, AT_THREADS = 320;
+constexpr int AT_BM = 128, AT_HALF = 64;
 constexpr unsigned AT_SPIN_LIMIT = 1u << 20;
 constexpr float AT_RESCALE_THRESHOLD = 8.f;      // in log2 units
 // Of every 8 pairs of probabilities, this many are computed by a polynomial on the FMA pipes and the
@@ -227,32 +227,39 @@ __host__ __device__ constexpr unsigned instr_desc(int n, bool b_mn) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn ? 1u : 0u) << 16) | ((unsigned)(n >> 3) << 17) | ((unsigned)(AT_BM >> 4) << 24);
 }
 
-template <int DK, int DV> struct AtSmem {
+template <int DK, int DV, int HALVES> struct AtSmem {
+    static constexpr int BN = HALVES * AT_HALF;               // keys a tile
     static constexpr int SUB_K = DK / 64, SUB_V = DV / 64;    // 64-wide sub-tiles along the head
     static constexpr int STAGES_V = DK > 128 ? 1 : 2;         // keys of 192 leave room for one tile of values of 128
     __nv_bfloat16 q[SUB_K][AT_BM * 64];                       // K-major, per sub-tile [128 rows][64]
-    __nv_bfloat16 k[2][SUB_K][AT_BN * 64];                    // two stages
-    __nv_bfloat16 v[STAGES_V][SUB_V][AT_BN * 64];
-    __nv_bfloat16 p[2][AT_BM * 64];                           // [128 rows][128 keys] as two sub-tiles of 64 keys
+    __nv_bfloat16 k[2][SUB_K][BN * 64];                       // two stages
+    __nv_bfloat16 v[STAGES_V][SUB_V][BN * 64];
+    __nv_bfloat16 p[HALVES][AT_BM * 64];                      // [128 rows][BN keys] as sub-tiles of 64 keys
     unsigned long long q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full, s_free, p_ready, pv_done, met[4];
     unsigned tmem_base;
 };
 
+// HALVES: 2 as described above.  1: tiles of 64 keys and four softmax warps, a thread a row, one reference, sum and accumulator; half
+// the threads, shared and tensor memory, so that two blocks fit an SM where heads are 128 wide and one's waits lie under the other's
+// work.  B200, 128 keys a tile and one block an SM -> 64 and two: 32 heads of 128 over prompts of 833, 1,667 and 2,503 tokens 207 -> 152 us,
+// 16 heads, 2,048 tokens, window 1,024 40 -> 33.  Keys of 192 would have room for one stage of each operand only: 74 -> 105 us, so they
+// stay at 128 keys a tile.
 // ELEM: the gate, if there is one, has a column per output element (an instance of its own, so that the others carry neither
 // its code nor its registers)
 // Keys and values may differ in size.  Heads of dk or dv elements that are no multiple of 64 run as ones of DK or DV: TMA fills what
 // lies beyond a cached row with zeros (of a query row it brings the next head's elements, which meet the keys' zeros), and columns
 // of the output beyond dv are not written.
-template <int DK, int DV, bool ELEM, int FROM = AT_PAGED>
-__global__ void __launch_bounds__(AT_THREADS, DK <= 64 && DV <= 64 ? 2 : 1)
+template <int DK, int DV, bool ELEM, int FROM, int HALVES>
+__global__ void __launch_bounds__(64 + HALVES * 128, HALVES == 1 || (DK <= 64 && DV <= 64) ? 2 : 1)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                          const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_q_rot,
                          const __grid_constant__ CUtensorMap map_k_rot, AtArgs a) {
     constexpr int SUB_K = DK / 64, SUB_V = DV / 64, SUB_PLAIN = FROM == AT_LAID_ROT ? SUB_K - 1 : SUB_K;
-    constexpr int STAGES_V = AtSmem<DK, DV>::STAGES_V;
-    constexpr unsigned TMEM_COLS = DV <= 64 ? 256 : 512;      // S: 128 columns; two accumulators of DV columns
+    using Smem = AtSmem<DK, DV, HALVES>;
+    constexpr int BN = Smem::BN, STAGES_V = Smem::STAGES_V;
+    constexpr unsigned TMEM_COLS = HALVES * DV <= 128 ? 256 : 512;      // S: up to 128 columns; HALVES accumulators of DV columns
     extern __shared__ __align__(1024) unsigned char at_raw[];      // swizzled tiles need 1024-byte alignment
-    AtSmem<DK, DV> &s = *reinterpret_cast<AtSmem<DK, DV> *>(at_raw);
+    Smem &s = *reinterpret_cast<Smem *>(at_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (smem_u32(at_raw) & 1023u) {                            // never seen; a wrong result is not an option
         if (threadIdx.x == 0) atomicExch(a.status, 14);
@@ -267,7 +274,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     if (threadIdx.x == 0) {
         mbar_init(&s.q_full, 1);
         for (int i = 0; i < 2; ++i) { mbar_init(&s.k_full[i], 1); mbar_init(&s.k_empty[i], 1); mbar_init(&s.v_full[i], 1); mbar_init(&s.v_empty[i], 1); }
-        mbar_init(&s.s_full, 1); mbar_init(&s.s_free, 8); mbar_init(&s.p_ready, 8); mbar_init(&s.pv_done, 1);
+        mbar_init(&s.s_full, 1); mbar_init(&s.s_free, 4 * HALVES); mbar_init(&s.p_ready, 4 * HALVES); mbar_init(&s.pv_done, 1);
         for (int i = 0; i < 4; ++i) mbar_init(&s.met[i], 2);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -275,7 +282,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem_s = s.tmem_base, tmem_o = s.tmem_base + AT_BN;
+    const unsigned tmem_s = s.tmem_base, tmem_o = s.tmem_base + 128;
     // Only now may the next kernel be scheduled: a later kernel that took tensor memory on this SM and
     // then waited for this grid, while a block of this grid still waited for tensor memory, would never end.
     pdl_trigger();
@@ -295,12 +302,12 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     const int lo = jk_mask_lo(p0, a.window);
     // key tiles this query tile sees: those that hold kept first keys and lie before the window's first tile, then the
     // window's
-    const int kv_first = lo / AT_BN * AT_BN;
-    const int n_kept = a.keep_first > 0 ? (min(a.keep_first, kv_first) + AT_BN - 1) / AT_BN : 0;
-    const int n_kv = n_kept + (p_last - kv_first) / AT_BN + 1;
-    auto tile_at = [&](int i) { return i < n_kept ? i * AT_BN : kv_first + (i - n_kept) * AT_BN; };
+    const int kv_first = lo / BN * BN;
+    const int n_kept = a.keep_first > 0 ? (min(a.keep_first, kv_first) + BN - 1) / BN : 0;
+    const int n_kv = n_kept + (p_last - kv_first) / BN + 1;
+    auto tile_at = [&](int i) { return i < n_kept ? i * BN : kv_first + (i - n_kept) * BN; };
     const int *bt = FROM == AT_PAGED ? a.block_table + (size_t)r * a.max_blocks : nullptr;
-    const int pages_per_tile = FROM == AT_PAGED ? AT_BN / a.page_size : 1;
+    const int pages_per_tile = FROM == AT_PAGED ? BN / a.page_size : 1;
     int failed = 0;
 
     if (warp == 0) {
@@ -311,7 +318,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             if (FROM == AT_LAID_ROT) tma_load_2d(s.q[SUB_K - 1], &map_q_rot, &s.q_full, h * a.rot_ld + a.rot_off, row0);
         }
         for (int i = 0; i < n_kv && !failed; ++i) {
-            const int st = i & 1, kv0 = tile_at(i);
+            const int kv0 = tile_at(i);
             // this lane's page of the tile, read from the block table once for keys and values of one size;
             // a page beyond what the request holds is never looked at: its keys are masked
             int pg = lane / SUB_K, u = lane % SUB_K;
@@ -324,7 +331,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             int grow = first_row();
             for (int kind = 0; kind < 2; ++kind) {               // 0: keys, 1: values
                 if (SUB_K != SUB_V && kind == 1) { pg = lane / SUB_V; u = lane % SUB_V; grow = first_row(); }
-                const int stages = kind ? STAGES_V : 2, sk = kind ? i % STAGES_V : st;
+                const int stages = kind ? STAGES_V : 2, sk = i % stages;
                 unsigned long long *empty = kind ? &s.v_empty[sk] : &s.k_empty[sk];
                 unsigned long long *full = kind ? &s.v_full[sk] : &s.k_full[sk];
                 int ok = 1;
@@ -333,7 +340,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     ok = __shfl_sync(0xffffffffu, ok, 0);
                 }
                 if (!ok) { failed = 1; break; }
-                if (lane == 0) mbar_expect_tx(full, AT_BN * (kind ? DV : DK) * 2);
+                if (lane == 0) mbar_expect_tx(full, BN * (kind ? DV : DK) * 2);
                 __syncwarp();
                 if (pg < pages_per_tile) {                       // at most 16 pages x 2 parts
                     if (FROM == AT_PAGED) {
@@ -353,16 +360,16 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     } else if (warp == 1) {
         // ---- product issuer ----
         if (lane == 0) {
-            constexpr unsigned idesc_qk = instr_desc(AT_BN, false), idesc_pv = instr_desc(DV, true);
+            constexpr unsigned idesc_qk = instr_desc(BN, false), idesc_pv = instr_desc(DV, true);
             // descriptor words, built once: low = start address and leading offset, high = stride
             // offset 1024, version 1, 128-byte swizzle
             constexpr unsigned desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
             auto lo_k = [](const void *tile) { return ((smem_u32(tile) & 0x3FFFFu) >> 4) | (1u << 16); };
-            auto lo_mn = [](const void *tile) { return ((smem_u32(tile) & 0x3FFFFu) >> 4) | ((unsigned)((AT_BN * 64 * 2) >> 4) << 16); };
-            unsigned q_lo[SUB_K], k_lo[2][SUB_K], p_lo[2], v_lo[2];       // one stage of values: both the same
+            auto lo_mn = [](const void *tile) { return ((smem_u32(tile) & 0x3FFFFu) >> 4) | ((unsigned)((BN * 64 * 2) >> 4) << 16); };
+            unsigned q_lo[SUB_K], k_lo[2][SUB_K], p_lo[2], v_lo[2];       // one stage, one half: both the same
 #pragma unroll
             for (int u = 0; u < SUB_K; ++u) { q_lo[u] = lo_k(s.q[u]); k_lo[0][u] = lo_k(s.k[0][u]); k_lo[1][u] = lo_k(s.k[1][u]); }
-            p_lo[0] = lo_k(s.p[0]); p_lo[1] = lo_k(s.p[1]);
+            p_lo[0] = lo_k(s.p[0]); p_lo[1] = lo_k(s.p[HALVES - 1]);
             v_lo[0] = lo_mn(s.v[0][0]); v_lo[1] = lo_mn(s.v[STAGES_V - 1][0]);
             auto issue_qk = [&](int st) {
 #pragma unroll
@@ -395,7 +402,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 if (!mbar_wait(&s.v_full[i % STAGES_V], (i / STAGES_V) & 1)) { failed = 2; break; }
                 tc_fence_after();
 #pragma unroll
-                for (int k = 0; k < AT_BN / 16; ++k) {   // 16 keys per instruction
+                for (int k = 0; k < BN / 16; ++k) {   // 16 keys per instruction
                     // P: 32 bytes further in the row of sub-tile k / 4; V: 16 rows of 128 bytes further.
                     // Keys 0..63 of the tile add to the first accumulator, keys 64..127 to the second.
                     umma_bf16_words(tmem_o + (k / 4) * DV, p_lo[k / 4] + 2 * (k % 4), desc_hi,
@@ -411,7 +418,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         // Warps w and w + 4 share the 32 rows of tensor-memory lane quarter w % 4; one takes keys 0..63 of
         // every tile, the other keys 64..127.  Each half has a reference maximum, a sum and an output
         // accumulator of its own, so the two never talk until the end.
-        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        const int quarter = warp & 3, half = HALVES == 2 ? (warp - 2) >> 2 : 0;
         const int row = quarter * 32 + lane;                   // row of the tile
         const int pos = p0 + min(row, nrows - 1);              // rows beyond the request repeat its last row
         const int lo_row = jk_mask_lo(pos, a.window);
@@ -511,9 +518,9 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             // 0 x NaN is NaN: slots of the request's last page that lie beyond its end hold whatever an earlier
             // holder of the page left there.  Those rows become zeros before the product reads them (only the last
             // tile of keys has any; the first half's threads take one key row each).
-            if (i == n_kv - 1 && half == 0 && tile_at(i) + AT_BN - 1 > p_last) {
+            if (i == n_kv - 1 && half == 0 && tile_at(i) + BN - 1 > p_last) {
                 if (!__all_sync(0xffffffffu, mbar_wait(&s.v_full[i % STAGES_V], (i / STAGES_V) & 1))) { alive = false; break; }
-                if (tile_at(i) + row > p_last) {
+                if (row < BN && tile_at(i) + row > p_last) {
 #pragma unroll
                     for (int u = 0; u < SUB_V; ++u) {
                         uint4 *vrow = reinterpret_cast<uint4 *>(s.v[i % STAGES_V][u] + row * 64);      // 128 bytes; the swizzle stays inside
@@ -531,7 +538,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         tc_fence_after();
         // the halves meet: P's place in shared memory is free now and carries (reference, sum) across
         float2 *meet = reinterpret_cast<float2 *>(s.p[0]);      // [half][row]
-        if (alive) {
+        if (HALVES == 2 && alive) {
             meet[half * AT_BM + row] = make_float2(m_ref, l);
             __syncwarp();
             if (lane == 0) mbar_arrive(&s.met[quarter]);
@@ -539,23 +546,23 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         }
         if (!alive) { failed = 3; if (lane == 0) atomicExch(a.status, 13); }
         if (alive) {
-            const float2 other = meet[(half ^ 1) * AT_BM + row];
+            const float2 other = HALVES == 2 ? meet[(half ^ 1) * AT_BM + row] : make_float2(-INFINITY, 0.f);
             // a half that saw no key has reference -inf, sum 0 and an accumulator of zeros
             const float m_all = fmaxf(m_ref, other.x);
             const float w_mine = ex2(m_ref - m_all), w_other = ex2(other.x - m_all);
             // a sink adds its term 2^(sink - m_all); a gate multiplies the row's output
             float inv = 1.f / (l * w_mine + other.y * w_other + (a.sink ? exp2f(jk_sink_log2(a.sink_w, h) - m_all) : 0.f));
             if (!ELEM && a.gate != nullptr && row < nrows) inv *= jk_sigmoid(a.gate[(size_t)(row0 + row) * a.gate_ld + h]);
-            const float *gate = ELEM && row < nrows ? a.gate + (size_t)(row0 + row) * a.gate_ld + (size_t)h * a.dv + half * (DV / 2) : nullptr;   // of this thread's columns
+            const float *gate = ELEM && row < nrows ? a.gate + (size_t)(row0 + row) * a.gate_ld + (size_t)h * a.dv + half * (DV / HALVES) : nullptr;   // of this thread's columns
             const float w0 = (half ? w_other : w_mine) * inv, w1 = (half ? w_mine : w_other) * inv;
-            // this thread writes columns [half * DV / 2, + DV / 2) of its row, as far as the head has them
-            __nv_bfloat16 *dst = a.out + ((size_t)(row0 + row) * a.nh + h) * a.dv + half * (DV / 2);
-            const int mine = a.dv - half * (DV / 2);
+            // this thread writes columns [half * DV / HALVES, + DV / HALVES) of its row, as far as the head has them
+            __nv_bfloat16 *dst = a.out + ((size_t)(row0 + row) * a.nh + h) * a.dv + half * (DV / HALVES);
+            const int mine = a.dv - half * (DV / HALVES);
 #pragma unroll 1
-            for (int c = 0; c < DV / 64; ++c) {
+            for (int c = 0; c < DV / HALVES / 32; ++c) {
                 unsigned o0[32], o1[32];
-                tmem_ld32_issue(tmem_o + lane_addr + half * (DV / 2) + c * 32, o0);
-                tmem_ld32_issue(tmem_o + lane_addr + DV + half * (DV / 2) + c * 32, o1);
+                tmem_ld32_issue(tmem_o + lane_addr + half * (DV / HALVES) + c * 32, o0);
+                if (HALVES == 2) tmem_ld32_issue(tmem_o + lane_addr + DV + half * (DV / HALVES) + c * 32, o1);
                 tmem_wait_ld();
                 if (row < nrows) {
 #pragma unroll
@@ -575,8 +582,11 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                         }
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
-                            float lo = __uint_as_float(o0[j + 2 * q]) * w0 + __uint_as_float(o1[j + 2 * q]) * w1;
-                            float hi = __uint_as_float(o0[j + 2 * q + 1]) * w0 + __uint_as_float(o1[j + 2 * q + 1]) * w1;
+                            float lo = __uint_as_float(o0[j + 2 * q]) * w0, hi = __uint_as_float(o0[j + 2 * q + 1]) * w0;
+                            if (HALVES == 2) {
+                                lo += __uint_as_float(o1[j + 2 * q]) * w1;
+                                hi += __uint_as_float(o1[j + 2 * q + 1]) * w1;
+                            }
                             if constexpr (ELEM) { lo *= jk_sigmoid(z[2 * q]); hi *= jk_sigmoid(z[2 * q + 1]); }
                             const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
                             w[q] = *reinterpret_cast<const unsigned *>(&b);
@@ -648,15 +658,15 @@ JK_EXPORT int jk_attention_tcgen05_supports(int dh, int page_size) {
     return (dh == 64 || dh == 128) && (page_size == 8 || page_size == 16 || page_size == 32 || page_size == 64 || page_size == 128);
 }
 
-template <int DK, int DV, bool ELEM, int FROM = AT_PAGED>
+template <int DK, int DV, bool ELEM, int FROM, int HALVES>
 static int launch_at(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const CUtensorMap &mqr, const CUtensorMap &mkr,
                      const AtArgs &a, cudaStream_t stream) {
-    const size_t smem = sizeof(AtSmem<DK, DV>);
-    static_assert(sizeof(AtSmem<DK, DV>) <= 227 * 1024, "shared memory");
-    auto kernel = attention_tcgen05_kernel<DK, DV, ELEM, FROM>;
+    const size_t smem = sizeof(AtSmem<DK, DV, HALVES>);
+    static_assert(sizeof(AtSmem<DK, DV, HALVES>) <= (HALVES == 1 ? 113 : 227) * 1024, "shared memory");
+    auto kernel = attention_tcgen05_kernel<DK, DV, ELEM, FROM, HALVES>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) JK_FAIL(JK_CUDA_ERROR, "attention_tcgen05: %s", cudaGetErrorString(e));
-    jk_launch(kernel, dim3(a.nh, a.ntiles), dim3(AT_THREADS), smem, stream, mq, mk, mv, mqr, mkr, a);
+    jk_launch(kernel, dim3(a.nh, a.ntiles), dim3(64 + HALVES * 128), smem, stream, mq, mk, mv, mqr, mkr, a);
     JK_CHECK_LAUNCH("attention_tcgen05");
     return JK_OK;
 }
@@ -681,13 +691,14 @@ JK_EXPORT int jk_attention_tcgen05(const void *q, const void *k_pages, const voi
              cap > 0.f ? cap / scale : 0.f, window > 0 ? keep_first : 0, sink_w, dh, dv, 0, 0};
     JK_REQUIRE(cap >= 0.f && keep_first >= 0 && scale > 0.f, "attention_tcgen05: cap %g, %d kept keys, scale %g", cap, keep_first, scale);
     const bool elem = gate != nullptr && gate_elem;
-#define LAUNCH_AT(DK, DV) return elem ? launch_at<DK, DV, true>(mq, mk, mv, mq, mk, a, stream) : launch_at<DK, DV, false>(mq, mk, mv, mq, mk, a, stream)
+#define LAUNCH_AT(DK, DV, H) return elem ? launch_at<DK, DV, true, AT_PAGED, H>(mq, mk, mv, mq, mk, a, stream) : launch_at<DK, DV, false, AT_PAGED, H>(mq, mk, mv, mq, mk, a, stream)
     if (dh <= 64) {
-        if (dv <= 64) LAUNCH_AT(64, 64);
-        LAUNCH_AT(64, 128);
+        if (dv <= 64) LAUNCH_AT(64, 64, 2);
+        LAUNCH_AT(64, 128, 2);
     }
-    if (dv <= 64) LAUNCH_AT(128, 64);
-    LAUNCH_AT(128, 128);
+    if (dv <= 64) LAUNCH_AT(128, 64, 2);
+    if (page_size <= AT_HALF) LAUNCH_AT(128, 128, 1);
+    LAUNCH_AT(128, 128, 2);
 #undef LAUNCH_AT
 }
 
@@ -707,22 +718,23 @@ JK_EXPORT int jk_attention_laid_tcgen05(const void *q, const void *q_rot, int ro
     JK_REQUIRE(gate == nullptr || gate_ld >= nh * (gate_elem ? dh : 1), "attention_laid: a gate row of %d holds no %d heads", gate_ld, nh);
     CUtensorMap mq, mk, mv, mqr, mkr;
     if (int rc = tensor_map(q, ntok, nh * dh, AT_BM, &mq)) return rc;
-    if (int rc = tensor_map(kv, rows, nh * dh, AT_BN, &mk, 2 * nh * dh)) return rc;
-    if (int rc = tensor_map((const __nv_bfloat16 *)kv + nh * dh, rows, nh * dh, AT_BN, &mv, 2 * nh * dh)) return rc;
+    const int keys = dh == 128 && k_rot == nullptr ? AT_HALF : 2 * AT_HALF;         // a tile of the instances below
+    if (int rc = tensor_map(kv, rows, nh * dh, keys, &mk, 2 * nh * dh)) return rc;
+    if (int rc = tensor_map((const __nv_bfloat16 *)kv + nh * dh, rows, nh * dh, keys, &mv, 2 * nh * dh)) return rc;
     mqr = mq, mkr = mk;
     if (k_rot != nullptr) {
         if (int rc = tensor_map(q_rot, ntok, nh * rot_ld, AT_BM, &mqr)) return rc;
-        if (int rc = tensor_map(k_rot, rows, 64, AT_BN, &mkr)) return rc;
+        if (int rc = tensor_map(k_rot, rows, 64, keys, &mkr)) return rc;
     }
     AtArgs a{(__nv_bfloat16 *)out, tiles, req_start, req_pos, nullptr, status, ntiles, nh, nh, 1, 1, window, scale * 1.4426950408889634f,
              sink_w != nullptr, gate, gate_ld, 0.f, 0, sink_w, dh, dh, rot_ld, rot_off};
     const bool elem = gate != nullptr && gate_elem;
-#define LAUNCH_LAID(DK, DV, FROM) return elem ? launch_at<DK, DV, true, FROM>(mq, mk, mv, mqr, mkr, a, stream) : launch_at<DK, DV, false, FROM>(mq, mk, mv, mqr, mkr, a, stream)
+#define LAUNCH_LAID(DK, DV, FROM, H) return elem ? launch_at<DK, DV, true, FROM, H>(mq, mk, mv, mqr, mkr, a, stream) : launch_at<DK, DV, false, FROM, H>(mq, mk, mv, mqr, mkr, a, stream)
     if (dh == 64) {
-        if (k_rot != nullptr) LAUNCH_LAID(128, 64, AT_LAID_ROT);
-        LAUNCH_LAID(64, 64, AT_LAID);
+        if (k_rot != nullptr) LAUNCH_LAID(128, 64, AT_LAID_ROT, 2);
+        LAUNCH_LAID(64, 64, AT_LAID, 2);
     }
-    if (k_rot != nullptr) LAUNCH_LAID(192, 128, AT_LAID_ROT);
-    LAUNCH_LAID(128, 128, AT_LAID);
+    if (k_rot != nullptr) LAUNCH_LAID(192, 128, AT_LAID_ROT, 2);
+    LAUNCH_LAID(128, 128, AT_LAID, 1);
 #undef LAUNCH_LAID
 }
