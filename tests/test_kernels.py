@@ -526,6 +526,16 @@ def test_attention_prefill_kernel_on_tcgen05(K, nh, nkvh, dh, page, window):
     _close(got, want, torch.bfloat16, scale=2.0)
 
 
+@pytest.mark.parametrize("page,window", [(8, None), (64, None), (128, None), (16, 70), (32, 64)])
+def test_attention_tcgen05_tiles_of_64_keys(K, page, window):
+    """Heads of 128 walk 64 keys at a time where a page fits into that (pages of 128: 128 keys): prompts and portions that end at, one
+    before and one past the edges of key tiles and of query tiles; the operands and the bound of the cases above."""
+    lens = [64, 65, 127, 193, 321]
+    queries = [list(range(0, 64)), list(range(0, 65)), list(range(62, 127)), list(range(0, 193)), list(range(192, 321))]
+    got, want, _ = _attention_case(K, torch.bfloat16, 6, 2, 128, page, window, lens, queries, seed=page, impl="tcgen05")
+    _close(got, want, torch.bfloat16, scale=2.0)
+
+
 @pytest.mark.parametrize("impl,dtype", [("rows", torch.float32), ("rows", torch.bfloat16), ("decode", torch.bfloat16),
                                          ("decode grouped", torch.bfloat16), ("prefill", torch.bfloat16),
                                          ("tcgen05", torch.bfloat16)])
