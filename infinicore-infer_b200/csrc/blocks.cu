@@ -1440,6 +1440,71 @@ __global__ void causal_conv_kernel(ConvArgs a, int rows) {
     }
 }
 
+// The same for steps of many rows and whole vectors: a thread owns four channels of CV_ROWS rows, its taps and the J - 1 inputs before
+// the row in registers, so that a row is read once instead of J times and no division is left in the loop.  Sums in the same
+// order.  What bounds it: the bytes (read and written once).
+constexpr int CV_ROWS = 8, CV_THREADS = 128;
+
+template <typename T, int J>
+__global__ void __launch_bounds__(CV_THREADS) causal_conv_rows_kernel(ConvArgs a, int rows) {
+    pdl_trigger();
+    pdl_wait();
+    const int c = (blockIdx.x * CV_THREADS + threadIdx.x) * 4;
+    if (c >= a.C) return;
+    auto at = [](const float *p) { return *reinterpret_cast<const float4 *>(p); };
+    auto plus = [](float4 x, float4 y) { return make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w); };
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), bias = a.bias ? at(a.bias + c) : zero, in_bias = a.in_bias ? at(a.in_bias + c) : zero;
+    float w[4][J];
+#pragma unroll
+    for (int i = 0; i < 4 * J; ++i) w[i / J][i % J] = a.taps[(size_t)c * J + i];
+    const float *u = a.u + a.off + c;
+    const int t0 = blockIdx.y * CV_ROWS, n = min(CV_ROWS, rows - t0);
+    float4 in[CV_ROWS];
+#pragma unroll
+    for (int r = 0; r < CV_ROWS; ++r) in[r] = r < n ? plus(at(u + (size_t)(t0 + r) * a.ld), in_bias) : zero;
+    float4 before[J];            // the J - 1 inputs before the row, the oldest first (before[J - 1] is the row's own)
+    int req = -1;
+#pragma unroll
+    for (int r = 0; r < CV_ROWS; ++r) {
+        if (r >= n) break;
+        const int t = t0 + r, own = a.row_req[t];
+        if (own != req) {       // the rows before it: this request's, else its tail
+            req = own;
+            const int back = t - a.req_start[req];
+            const float *tail = J > 1 ? a.tail + (size_t)a.slot_ids[req] * (J - 1) * a.C + c : nullptr;
+#pragma unroll
+            for (int j = 0; j < J - 1; ++j) {
+                const int d = J - 1 - j;
+                before[j] = d <= back ? plus(at(u + (size_t)(t - d) * a.ld), in_bias) : at(tail + (size_t)(J - 1 + back - d) * a.C);
+            }
+        }
+        before[J - 1] = in[r];
+        float acc[4] = {bias.x, bias.y, bias.z, bias.w};
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            acc[0] = fmaf(w[0][j], before[j].x, acc[0]); acc[1] = fmaf(w[1][j], before[j].y, acc[1]);
+            acc[2] = fmaf(w[2][j], before[j].z, acc[2]); acc[3] = fmaf(w[3][j], before[j].w, acc[3]);
+        }
+        if (J > 1 && a.req_start[req + 1] - a.req_start[req] == 1) {        // a request with one row: its tail moves forward here
+            float *tail = a.tail + (size_t)a.slot_ids[req] * (J - 1) * a.C + c;
+#pragma unroll
+            for (int s = 0; s < J - 1; ++s) *reinterpret_cast<float4 *>(tail + (size_t)s * a.C) = before[s + 1];
+        }
+#pragma unroll
+        for (int j = 0; j < J - 1; ++j) before[j] = before[j + 1];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[e] = block_act(a.act, acc[e]);
+        const size_t o = (size_t)t * a.C + c;
+        if (a.y32) *reinterpret_cast<float4 *>(a.y32 + o) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        if (a.yT) {
+            struct __align__(sizeof(T) * 4) Four { T f[4]; } four;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) four.f[e] = from_f32<T>(acc[e]);
+            *reinterpret_cast<Four *>((T *)a.yT + o) = four;
+        }
+    }
+}
+
 // tail[slot, s, c] <- the input J - 1 - s rows before the end of the request's sequence after this step; a thread owns
 // (request, channel) and reads every old entry before it overwrites it
 __global__ void conv_tails_kernel(ConvArgs a, int nreq) {
@@ -1466,11 +1531,21 @@ JK_EXPORT int jk_causal_conv(const float *u, int ld, int off, int C, const float
     JK_REQUIRE(u && taps && row_req && req_start && C > 0 && J >= 1 && (y32 || yT), "causal_conv: an argument is missing");
     JK_REQUIRE(J == 1 || (tail && slot_ids), "causal_conv: %d taps without the tails' state", J);
     ConvArgs a{u, ld, off, C, J, act, taps, bias, tail, row_req, req_start, slot_ids, y32, yT, in_bias};
+    const uintptr_t vectors = (uintptr_t)u | (uintptr_t)bias | (uintptr_t)in_bias | (uintptr_t)tail | (uintptr_t)y32 | (uintptr_t)yT;
     const size_t total = (size_t)T * C;
     const int blocks = (int)std::min<size_t>((total + 255) / 256, 148 * 16);
-#define LAUNCH(TT) jk_launch(causal_conv_kernel<TT>, dim3(blocks), dim3(256), 0, stream, a, T)
+    // The line: eight rows one after the other are a chain that few rows do not hide (4,096 channels, four taps, an element a thread -> rows):
+    // 32 rows 11 -> 15 us, 64 13 -> 15, 256 21 -> 15, 2,048 97 -> 42.
+    const bool by_rows = T >= 128 && J >= 2 && J <= 4 && ((C | ld | off) & 3) == 0 && (vectors & 15) == 0 && (T + CV_ROWS - 1) / CV_ROWS <= 65535;
+#define LAUNCH_J(TT, JJ) jk_launch(causal_conv_rows_kernel<TT, JJ>, dim3((C / 4 + CV_THREADS - 1) / CV_THREADS, (T + CV_ROWS - 1) / CV_ROWS), dim3(CV_THREADS), 0, stream, a, T)
+#define LAUNCH(TT)                                                                                 \
+    if (!by_rows) jk_launch(causal_conv_kernel<TT>, dim3(blocks), dim3(256), 0, stream, a, T);     \
+    else if (J == 2) LAUNCH_J(TT, 2);                                                              \
+    else if (J == 3) LAUNCH_J(TT, 3);                                                              \
+    else LAUNCH_J(TT, 4)
     BLOCKS_BY_DTYPE(dtype, "causal_conv", LAUNCH);
 #undef LAUNCH
+#undef LAUNCH_J
     JK_CHECK_LAUNCH("causal_conv");
     if (J > 1 && T > nreq) {
         jk_launch(conv_tails_kernel, dim3((nreq * C + 127) / 128), dim3(128), 0, stream, a, nreq);

@@ -170,3 +170,28 @@ def test_projected_decay_recurrence_as_products_within_pieces(K, dk, dv, rank, f
             assert (out[int(starts[i]): int(starts[i + 1])] - want).abs().max() <= 2e-5 * want.abs().max(), f"request {i}"
             assert (state[s] - S).abs().max() <= 2e-5 * S.abs().max(), f"state of request {i}"
     assert torch.equal(got[0][1][0], first[0].double()) and not torch.equal(got[0][0], got[1][0])
+
+
+@pytest.mark.parametrize("taps,C,lens", [(4, 516, [128]), (3, 64, [7, 1, 2, 1, 140]), (2, 128, [1, 129]), (4, 520, [9, 3, 1, 1, 130])])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_causal_convolution_of_many_rows(K, taps, C, lens, dtype):
+    """Requests shorter than the taps, of one row and across the blocks' eight rows; the same rows laid so that vectors of four do not
+    fit take a thread an element.  Both add the taps in the same order: the same bits."""
+    dev, g, T, n = torch.device("cuda:0"), torch.Generator().manual_seed(C), sum(lens), len(lens)
+    u, w, b, ib = (torch.randn(*s, generator=g) for s in ((T, C), (C, taps), (C,), (C,)))
+    tail = torch.randn(n + 1, taps - 1, C, generator=g)
+    starts, slots = torch.tensor([0] + lens).cumsum(0).to(torch.int32), torch.arange(n, 0, -1, dtype=torch.int32)
+    row_req = torch.repeat_interleave(torch.arange(n, dtype=torch.int32), torch.tensor(lens))
+    got = []
+    for shift in (0, 1):
+        rows = torch.cat([torch.zeros(T, shift), u, torch.zeros(T, 4 - shift)], 1).contiguous().to(dev)
+        state, y32, yT = tail.clone().to(dev), torch.empty(T, C, device=dev), torch.empty(T, C, dtype=dtype, device=dev)
+        K.causal_conv(rows, shift, C, w.to(dev), b.to(dev), K.ACT_SILU, state, row_req.to(dev), starts.to(dev), slots.to(dev), y32, yT, in_bias=ib.to(dev))
+        got.append((y32.cpu(), yT.cpu(), state.cpu()))
+    assert all(torch.equal(x, y) for x, y in zip(*got))
+    for r, s in enumerate(slots.tolist()):
+        a, e = int(starts[r]), int(starts[r + 1])
+        x = torch.cat([tail[s].double(), u[a:e].double() + ib.double()])
+        want = plain.silu(b.double() + sum(w[:, j].double() * x[j: j + e - a] for j in range(taps)))
+        assert (got[0][0][a:e].double() - want).abs().max() <= 2.0 ** -20 * want.abs().max()
+        assert (got[0][2][s].double() - x[-(taps - 1):]).abs().max() <= 2.0 ** -22 * x.abs().max()
