@@ -594,6 +594,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                         *reinterpret_cast<uint4 *>(dst + c * 32 + j) = make_uint4(w[0], w[1], w[2], w[3]);
                     }
                 }
+                __syncwarp();           // the next reads of tensor memory take the warp as a whole
             }
         }
     }

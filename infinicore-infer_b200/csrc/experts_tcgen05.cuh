@@ -145,7 +145,7 @@ expert_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             int e, m0, n0;
             locate(tile, e, m0, n0);
             const int buf = j & 1;
-            if (!mbar_wait(&s.acc_full[buf], (j >> 1) & 1)) { failed = 3; if (lane == 0) atomicExch(a.status, 23); break; }
+            if (!__all_sync(0xffffffffu, mbar_wait(&s.acc_full[buf], (j >> 1) & 1))) { failed = 3; if (lane == 0) atomicExch(a.status, 23); break; }
             tc_fence_after();
             const unsigned acc = tmem + buf * ET_BN + ((unsigned)(quarter * 32) << 16);
             const int entry = m0 + quarter * 32 + lane;
@@ -159,20 +159,21 @@ expert_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                 if (GLU) {
                     unsigned u[32];
                     tmem_ld32(acc + ET_BN / 2 + c0, u);
-                    if (!mine) continue;
-                    __nv_bfloat16 *dst = (__nv_bfloat16 *)a.out + (size_t)entry * a.N + n0 + c0;
+                    if (mine) {
+                        __nv_bfloat16 *dst = (__nv_bfloat16 *)a.out + (size_t)entry * a.N + n0 + c0;
 #pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
-                        if (n0 + c0 + i >= a.N) break;
-                        unsigned w[4];
+                        for (int i = 0; i < 32; i += 8) {
+                            if (n0 + c0 + i >= a.N) break;
+                            unsigned w[4];
 #pragma unroll
-                        for (int p = 0; p < 4; ++p) {
-                            const __nv_bfloat162 b = __floats2bfloat162_rn(
-                                expert_inner_short(a.act, score, __uint_as_float(v[i + 2 * p]), __uint_as_float(u[i + 2 * p]), a.limit),
-                                expert_inner_short(a.act, score, __uint_as_float(v[i + 2 * p + 1]), __uint_as_float(u[i + 2 * p + 1]), a.limit));
-                            w[p] = *reinterpret_cast<const unsigned *>(&b);
+                            for (int p = 0; p < 4; ++p) {
+                                const __nv_bfloat162 b = __floats2bfloat162_rn(
+                                    expert_inner_short(a.act, score, __uint_as_float(v[i + 2 * p]), __uint_as_float(u[i + 2 * p]), a.limit),
+                                    expert_inner_short(a.act, score, __uint_as_float(v[i + 2 * p + 1]), __uint_as_float(u[i + 2 * p + 1]), a.limit));
+                                w[p] = *reinterpret_cast<const unsigned *>(&b);
+                            }
+                            *reinterpret_cast<uint4 *>(dst + i) = make_uint4(w[0], w[1], w[2], w[3]);
                         }
-                        *reinterpret_cast<uint4 *>(dst + i) = make_uint4(w[0], w[1], w[2], w[3]);
                     }
                 } else if (mine) {
                     float *dst = (float *)a.out + (size_t)entry * a.N + n0 + c0;
@@ -180,6 +181,7 @@ expert_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                     for (int i = 0; i < 32; i += 4)
                         if (n0 + c0 + i < a.N) *reinterpret_cast<uint4 *>(dst + i) = make_uint4(v[i], v[i + 1], v[i + 2], v[i + 3]);
                 }
+                __syncwarp();           // the next pass reads tensor memory, which takes the warp as a whole
             }
             tc_fence_before();
             __syncwarp();

@@ -106,7 +106,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     } else {
         const int quarter = warp & 3;                                      // lanes (features) quarter * 32 ... of the accumulator
         pdl_wait();                                                        // before this block's first global write
-        if (!mbar_wait(&b.acc_full, 0)) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&b.acc_full, 0))) {
             failed = 3;
             if (lane == 0) atomicExch(a.status, 3);
         }
@@ -137,6 +137,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                         const float g = __uint_as_float(v[i]), u = xch[m * 64 + quarter * 32 + lane];
                         if (m < a.M && n < a.N) out[(size_t)m * a.ldo + n] = __float2bfloat16_rn(gated_unit(a.gate_act, g, u));
                     }
+                    __syncwarp();           // the next read of tensor memory takes the warp as a whole
                 }
             }
         } else if (!failed) {
@@ -153,6 +154,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                         else out[(size_t)m * a.ldo + n] = __uint_as_float(v[i]);
                     }
                 }
+                __syncwarp();           // as above
             }
         }
     }

@@ -242,7 +242,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             tile_coords(tile / ksplit, tiles_m, tiles_n, tm, tn);
             const int m0 = tm * TILE_M + rank * TG_BM, n0 = tn * OUT_COLS;
             const int buf = j & 1;
-            if (!mbar_wait(&s.acc_full[buf], (j >> 1) & 1)) { failed = 3; if (lane == 0) atomicExch(a.status, 3); break; }
+            if (!__all_sync(0xffffffffu, mbar_wait(&s.acc_full[buf], (j >> 1) & 1))) { failed = 3; if (lane == 0) atomicExch(a.status, 3); break; }
             tc_fence_after();
             const unsigned acc = tmem + buf * BN + ((unsigned)(quarter * 32) << 16);
             const int row0 = m0 + quarter * 32, row = row0 + lane;
@@ -309,6 +309,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                 *reinterpret_cast<uint4 *>(dst + half + part + i) = make_uint4(w1[0], w1[1], w1[2], w1[3]);
                             }
                         }
+                        __syncwarp();           // the next reads of tensor memory take the warp as a whole
                     }
                 }
                 release_accumulator(buf);
@@ -352,6 +353,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                 else reinterpret_cast<__nv_bfloat16 *>(a.out)[(size_t)row * a.ldo + c] = __float2bfloat16_rn(f[i]);
                             }
                         }
+                        __syncwarp();           // as above
                     } else if (PASS == 32) {
 #pragma unroll
                         for (int i = 0; i < 8; ++i)

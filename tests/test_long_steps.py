@@ -98,6 +98,44 @@ def test_expert_products_in_tiles_of_entries(K, T, d, ff, experts, top, act):
     assert err <= 2.0 ** -8 * want.abs().max(), float(err)
 
 
+@pytest.mark.parametrize("act", ["none", "silu", "gelu_tanh", "sigmoid", "relu", "swish_clamp"])
+def test_expert_products_of_groups_of_rows_that_are_part_full(K, act):
+    """Experts with 1, 31, 33, 63 and 142 entries: the groups of 32 rows that a warp of the products finishes are full, part full and
+    empty, over 200 and 264 features, so that a warp comes back for more columns after a pass in which some of its rows had nothing
+    to store.  Every activation; scores that multiply the units' inputs.  The bound of the test above."""
+    dev, g = torch.device("cuda:0"), torch.Generator().manual_seed(len(act))
+    counts, d, ff, limit = [1, 31, 33, 63, 142], 264, 200, 1.5
+    T, E = sum(counts), len(counts)
+    owner = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(T, generator=g)]
+    h = torch.randn(T, d, generator=g)
+    h[:, :E] = 20.0 * torch.nn.functional.one_hot(owner, E)         # the router reads the owner
+    h = h.to(torch.bfloat16)
+    router = torch.zeros(E, d)
+    router[:, :E] = torch.eye(E)
+    w_gu, w_dn = (torch.randn(E * n, k, generator=g).div(k ** 0.5).to(torch.bfloat16) for n, k in ((2 * ff, d), (d, ff)))
+    w_gu[:, :E] = 0.0
+    delta = torch.full((T, d), 9.0, device=dev)
+    code = {"none": 0, "silu": 1, "gelu_tanh": 2, "sigmoid": 3, "relu": 4, "swish_clamp": 6}[act]
+    K.routed_experts(h.to(dev), router.to(dev), w_gu.to(dev), w_dn.to(dev), delta, False, E, 1, code, limit=limit)
+    K.check_gemm_status(dev)
+    score = 1.0 / (1.0 + np.exp(-20.0))                             # the default form: sigmoid of the router's output, times the inputs
+    want = torch.zeros(T, d, dtype=F)
+    for e in range(E):
+        rows = owner == e
+        gu = score * (h[rows].double() @ w_gu[e * 2 * ff: (e + 1) * 2 * ff].double().T)
+        a, u = gu[:, :ff], gu[:, ff:]
+        if act == "swish_clamp":
+            a, u = a.clamp(max=limit), u.clamp(-limit, limit)
+            inner = a * torch.sigmoid(1.702 * a) * (u + 1)
+        else:
+            f = {"none": lambda x: x, "silu": plain.silu, "sigmoid": torch.sigmoid, "relu": torch.relu,
+                 "gelu_tanh": lambda x: torch.nn.functional.gelu(x, approximate="tanh")}[act]
+            inner = f(a) * u
+        want[rows] = inner @ w_dn[e * d: (e + 1) * d].double().T
+    err = (delta.double().cpu() - want).abs().max()
+    assert err <= 2.0 ** -8 * want.abs().max(), float(err)
+
+
 @pytest.mark.parametrize("states", [5, 16, 20])
 @pytest.mark.parametrize("lens", [(768,), (1793, 1, 513), (1475, 64), (900, 640)])
 def test_selective_scan_over_pieces(K, states, lens):
