@@ -128,15 +128,15 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(flo
 // act(gate) * up with act = silu (GATE_SILU), the tanh form of gelu (GATE_GELU_TANH) or relu (GATE_RELU).  The products
 // whose epilogue is a gated unit take the activation in the bits above the epilogue's own code: `epilogue | (gate_act << 8)`.
 enum JkGateAct : int { GATE_SILU = 0, GATE_GELU_TANH = 2, GATE_RELU = 4 };
-// Both smooth activations are gate * sigmoid(s): s = gate for silu, and for gelu 0.5 (1 + tanh(t)) = sigmoid(2 t), which does not
-// cancel for negative gates as the sum does.  One exponential and one quotient of the special-function unit (2 units in the
-// last place of float32 each, and of the exponent's rounding: |s| 2^-24): the results are rounded to bfloat16.  With expf, a
-// full division and tanhf an unrolled epilogue was thousands of instructions long and ran at the speed of their fetches:
-// 20 us a tile of 128 x 128 outputs, where a tile's products of K 2,304 take 12.
+// Both smooth activations are gate / (1 + e^-s): s = gate for silu, and for gelu 0.5 (1 + tanh(t)) = 1 / (1 + e^(-2 t)), which
+// does not cancel for negative gates as the sum does (largest relative error for gates in [-4, -1]: 1.5e-3 -> 1.5e-6; above
+// zero both are within 2 units in the last place).  expf and a true division, not the special-function unit's quotient: that one
+// is 0 where its divisor passes 2^126 (gates below -87.3), and __expf errs by |s| 2^-24 more.  Without tanhf behind a switch
+// the unrolled epilogue stays short enough for this: 2,048 x 5,760 x 2,304 82 us, 78 with the short forms.
 __device__ __forceinline__ float gated_unit(int act, float gate, float up) {
     if (act == GATE_RELU) return fmaxf(gate, 0.f) * up;
     const float s = act == GATE_GELU_TANH ? 1.5957691216057308f * (gate + 0.044715f * gate * gate * gate) : gate;
-    return __fdividef(gate, 1.f + __expf(-s)) * up;
+    return gate / (1.f + expf(-s)) * up;
 }
 static inline int jk_epilogue_code(int epilogue) { return epilogue & 0xff; }
 static inline int jk_epilogue_gate(int epilogue) {

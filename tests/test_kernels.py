@@ -827,6 +827,36 @@ def test_gemm_tcgen05_with_swiglu_epilogue(K, pairs, M, N, K_):
     _close(out, gu[:, :N] * torch.sigmoid(gu[:, :N]) * gu[:, N:], torch.bfloat16, scale=2.0)
 
 
+@pytest.mark.parametrize("gate", ["silu", "gelu_tanh"])
+@pytest.mark.parametrize("impl,M", [("small", 7), ("small", 16), ("skinny", 100), ("tiled", 300)])
+def test_gated_units_are_float32_accurate_over_the_gates_range(K, impl, M, gate):
+    """Gates and ups that arrive exactly (rows of W pick one element each), from where the unit vanishes on: what is stored is the unit
+    rounded to bfloat16.  A rounding is 2^-8 at most, and what float32 adds before it (e^-s to one unit in the last place, a sum,
+    a quotient, a product: 2.5 x 2^-23; for gelu three roundings of s as well) seldom moves one: by at most twice that over the
+    spacing 2^-8, 2^-12 for silu."""
+    g, N = torch.Generator().manual_seed(M), 2048
+    least = -88.5 if gate == "silu" else -9.9          # beyond, e^-s is no float32 any more and the unit is 0
+    z = (least + (8.0 - least) * torch.rand(M, N, generator=g)).to(torch.bfloat16)
+    z[:, :3] = torch.tensor([-88.5, -88.0, -87.5] if gate == "silu" else [-9.875, -9.75, -9.5])
+    up = torch.randn(M, N, generator=g).abs().add(1.0).to(torch.bfloat16)
+    act, w = torch.cat([z, up], 1).to(DEV), torch.eye(2 * N, dtype=torch.bfloat16, device=DEV)
+    out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    module, entry = {"small": ("linear_small", "jk_linear_small"), "skinny": ("gemm_tcgen05", "jk_gemm_skinny"),
+                     "tiled": ("gemm_tcgen05", "jk_gemm_tcgen05")}[impl]
+    code = (K.EPI_SWIGLU if impl == "small" else K.TG_SWIGLU) | ({"silu": 0, "gelu_tanh": 2}[gate] << 8)
+    extra = () if impl == "small" else (K._c_float(1.0), K._ptr(K.gemm_status(act.device)))
+    K._check(module, getattr(K._build.load(module), entry)(K._ptr(act), K._ptr(w), K._ptr(out), *map(K._c_int, (M, N, 2 * N, N, code)), *extra,
+                                                            K._c_int(148), K._stream()))
+    K.check_gemm_status(DEV)
+    z, up, got = z.double(), up.double(), out.double().cpu()
+    s = z if gate == "silu" else 2 * math.sqrt(2 / math.pi) * (z + 0.044715 * z ** 3)
+    want = z * torch.sigmoid(s) * up
+    before = 2.5 * 2.0 ** -23 + (0 if gate == "silu" else 3 * 2.0 ** -24 * s.abs())
+    assert ((got - want).abs() <= (2.0 ** -8 + before) * want.abs() + 2.0 ** -133).all()
+    if gate == "silu":
+        assert (got != want.to(torch.bfloat16).double()).double().mean() <= 2.0 ** -12
+
+
 @pytest.mark.parametrize("M,N,K_", [(32, 128, 64), (17, 256, 512), (64, 520, 200), (1, 100, 72), (100, 333, 4096), (128, 1200, 2304),
                                     (9, 77, 16384)])
 @pytest.mark.parametrize("epi", ["f32", "residual", "swiglu"])
