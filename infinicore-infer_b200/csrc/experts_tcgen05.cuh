@@ -14,14 +14,15 @@
 
 constexpr int ET_BN = 256, ET_MAX_EXPERTS = 256, ET_EPI_WARPS = 8, ET_THREADS = 64 + 32 * ET_EPI_WARPS;
 
-// expert_inner through one exponential and one quotient of the special-function unit (2 units in the last place of float32
-// each), for results that are rounded to bfloat16.
-__device__ __forceinline__ float expert_inner_short(int act, float s, float g, float u, float limit) {
+// expert_inner with its smooth activations in one form, c / (1 + e^-at) (gelu's as in gated_unit, common.cuh), so that 32 of them
+// unrolled carry one exponential and one division each and no tanhf.
+__device__ __forceinline__ float expert_inner_unrolled(int act, float s, float g, float u, float limit) {
     const float z = s * g, v = s * u, c = act == BACT_SWISH_CLAMP ? fminf(z, limit) : z;
     const float at = act == BACT_GELU_TANH ? 1.5957691216057308f * (z + 0.044715f * z * z * z) : act == BACT_SWISH_CLAMP ? 1.702f * c : z;
-    const float share = __fdividef(act == BACT_SIGMOID ? 1.f : c, 1.f + __expf(-at));        // c sigmoid(at), or sigmoid(z) itself
-    if (act == BACT_SWISH_CLAMP) return share * (fminf(fmaxf(v, -limit), limit) + 1.f);
-    return (act == BACT_RELU ? fmaxf(z, 0.f) : act == BACT_NONE ? z : share) * v;
+    const float smooth = (act == BACT_SIGMOID ? 1.f : c) / (1.f + expf(-at));
+    if (act == BACT_SWISH_CLAMP) return smooth * (fminf(fmaxf(v, -limit), limit) + 1.f);
+    if (act == BACT_SILU || act == BACT_GELU_TANH || act == BACT_SIGMOID) return smooth * v;
+    return (act == BACT_RELU ? fmaxf(z, 0.f) : z) * v;
 }
 
 struct ExpertTcArgs {
@@ -168,8 +169,8 @@ expert_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
 #pragma unroll
                             for (int p = 0; p < 4; ++p) {
                                 const __nv_bfloat162 b = __floats2bfloat162_rn(
-                                    expert_inner_short(a.act, score, __uint_as_float(v[i + 2 * p]), __uint_as_float(u[i + 2 * p]), a.limit),
-                                    expert_inner_short(a.act, score, __uint_as_float(v[i + 2 * p + 1]), __uint_as_float(u[i + 2 * p + 1]), a.limit));
+                                    expert_inner_unrolled(a.act, score, __uint_as_float(v[i + 2 * p]), __uint_as_float(u[i + 2 * p]), a.limit),
+                                    expert_inner_unrolled(a.act, score, __uint_as_float(v[i + 2 * p + 1]), __uint_as_float(u[i + 2 * p + 1]), a.limit));
                                 w[p] = *reinterpret_cast<const unsigned *>(&b);
                             }
                             *reinterpret_cast<uint4 *>(dst + i) = make_uint4(w[0], w[1], w[2], w[3]);

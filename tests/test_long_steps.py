@@ -136,6 +136,34 @@ def test_expert_products_of_groups_of_rows_that_are_part_full(K, act):
     assert err <= 2.0 ** -8 * want.abs().max(), float(err)
 
 
+@pytest.mark.parametrize("act,code,least", [("silu", 1, -88.5), ("sigmoid", 3, -80.0), ("gelu_tanh", 2, -9.9), ("swish_clamp", 6, -52.0),
+                                            ("none", 5, -88.5), ("none", 7, -88.5)])
+def test_experts_units_are_float32_accurate_over_the_gates_range(K, act, code, least):
+    """One expert whose rows of W pick single elements of a row: gates and ups arrive exactly, from where the unit vanishes on, and what
+    leaves is the unit rounded to bfloat16.  A rounding is 2^-8 at most; what float32 adds before it (e^-s to one unit in the last place, a
+    sum, a quotient, a product: 2.5 x 2^-23; three roundings of s where it is not the gate) seldom moves one: by at most twice that
+    over the spacing 2^-8, 2^-12 where s is the gate.  Codes that name no unit of an expert leave the gate as it is."""
+    dev, g, T, ff, limit = torch.device("cuda:0"), torch.Generator().manual_seed(code), 300, 1024, 4.0
+    z = (least + (8.0 - least) * torch.rand(T, ff, generator=g)).to(torch.bfloat16)
+    z[:, :3] = torch.tensor([-88.5, -88.0, -87.5]).clamp(min=least)
+    up = torch.randn(T, ff, generator=g).abs().add(1.0).to(torch.bfloat16)
+    h, w_gu, w_dn = torch.cat([z, up], 1).to(dev), torch.eye(2 * ff, dtype=torch.bfloat16, device=dev), torch.zeros(2 * ff, ff, dtype=torch.bfloat16, device=dev)
+    w_dn[:ff] = torch.eye(ff)
+    delta = torch.empty(T, 2 * ff, device=dev)
+    K.routed_experts(h, torch.zeros(1, 2 * ff, device=dev), w_gu, w_dn, delta, False, 1, 1, code, score_form=1, limit=limit)        # a score of 1
+    K.check_gemm_status(dev)
+    z, up, got = z.double(), up.double(), delta[:, :ff].double().cpu()
+    if act == "swish_clamp":
+        z, up = z.clamp(max=limit), up.clamp(-limit, limit) + 1
+    s = {"gelu_tanh": 2 * (2 / np.pi) ** 0.5 * (z + 0.044715 * z ** 3), "swish_clamp": 1.702 * z}.get(act, z)
+    want = {"sigmoid": torch.sigmoid(s), "none": z}.get(act, z * torch.sigmoid(s)) * up
+    exact = act in ("silu", "sigmoid", "none")
+    before = 2.5 * 2.0 ** -23 + (0 if exact else 3 * 2.0 ** -24 * s.abs())
+    assert ((got - want).abs() <= (2.0 ** -8 + before) * want.abs()).all()
+    if exact:
+        assert (got != want.to(torch.bfloat16).double()).double().mean() <= 2.0 ** -12
+
+
 @pytest.mark.parametrize("states", [5, 16, 20])
 @pytest.mark.parametrize("lens", [(768,), (1793, 1, 513), (1475, 64), (900, 640)])
 def test_selective_scan_over_pieces(K, states, lens):
