@@ -61,6 +61,39 @@ def test_latent_attention_over_heads_made_for_the_step(tmp_path, heads, dim, ran
     assert not torch.equal(logits[False], logits[True])         # both ways ran
 
 
+@pytest.mark.parametrize("dh,rotated", [(64, False), (64, True), (128, False), (128, True)])
+def test_weights_of_an_attention_over_laid_heads_are_float32_accurate(K, dh, rotated):
+    """Each instance, with values that pick single weights: row t has scores -a_t b_j (exact in float32) over 64 keys and far lower ones
+    over the rest, and column j of its output is key j's weight, rounded to bfloat16 as an operand, over the float32 sum of the weights,
+    rounded once more.  Scores in [-8, 0]: the exponent's factor and product err by 8 x 1.5 x 2^-24, the special-function unit by 2^-22, the sum
+    and the quotient by another 2^-22; each of the two roundings moves by at most twice that over the spacing 2^-8: 2^-10 of them
+    in all."""
+    dev, g, T, before = torch.device("cuda:0"), torch.Generator().manual_seed(dh), 1000, 200
+    C = T + before
+    a = (torch.rand(T, generator=g) * 1.5 + 0.5).to(torch.bfloat16)
+    b = (torch.rand(64, generator=g) * 4).to(torch.bfloat16)
+    b[0] = 0
+    q, kv, out = torch.zeros(T, dh), torch.zeros(C, 2 * dh), torch.empty(T, dh, dtype=torch.bfloat16, device=dev)
+    q[:, 3] = a.float()
+    kv[:64, 3], kv[64:, 3] = -b.float(), -256.0
+    kv[:64, dh:dh + 64] = torch.eye(64)
+    q, kv = q.to(torch.bfloat16).to(dev), kv.to(torch.bfloat16).to(dev)
+    q_rot, k_rot = torch.zeros(T, 72, dtype=torch.bfloat16, device=dev), torch.zeros(C, 64, dtype=torch.bfloat16, device=dev)
+    n = (T + 127) // 128
+    ints = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+    tiles, start, pos, status = ints([[0, 128 * i, 0] for i in reversed(range(n))]), ints([0, T]), ints([before]), K.gemm_status(dev)
+    i, p = K._c_int, K._ptr
+    K._check("attention_tcgen05", K._build.load("attention_tcgen05").jk_attention_laid_tcgen05(
+        p(q), p(q_rot if rotated else None), i(72), i(8), p(kv), p(k_rot if rotated else None), K._c_ll(C), p(out), p(tiles), i(n), i(T), p(start), p(pos),
+        i(1), i(dh), K._c_float(1.0), i(0), p(status), p(None), p(None), i(0), i(0), K._stream()))
+    K.check_gemm_status(dev)
+    e = torch.exp(-a.double()[:, None] * b.double())
+    want = e.to(torch.bfloat16).double() / e.sum(1, keepdim=True)
+    got = out[:, :64].double().cpu()
+    assert ((got - want).abs() <= 2.0 ** -6 * want).all()
+    assert (got != want.to(torch.bfloat16).double()).double().mean() <= 2.0 ** -10
+
+
 @pytest.mark.parametrize("T,d,ff,experts,top,act", [(128, 64, 128, 1, 1, "silu"), (129, 72, 136, 2, 2, "swish_clamp"), (300, 512, 264, 5, 2, "silu"),
                                                     (600, 264, 8, 3, 1, "silu")])
 def test_expert_products_in_tiles_of_entries(K, T, d, ff, experts, top, act):
