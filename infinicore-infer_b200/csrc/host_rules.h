@@ -267,6 +267,14 @@ inline bool latent_takes_heads(int rows, int nreq, long long keys, int window, i
     const long long reach = window > 0 ? std::min<long long>(window, keys / nreq) : keys / nreq;
     return rows * reach >= 16LL * keys;
 }
+// The positions that room is kept for in an engine of steps of up to `rows` rows: four times as many as a step may have rows (prompts, and
+// portions of longer ones up to there; steps that see more run over the latent rows), but no more than its requests can have: the
+// rule above takes at most rows / 16 of them, of at most `max_positions` each, and without a window all their positions lie in the
+// cache's `cached`.
+inline long long latent_heads_positions(long long rows, long long max_positions, long long cached, int window) {
+    const long long most = std::min(4 * rows, std::max(1LL, rows / 16) * max_positions);
+    return window > 0 ? most : std::min(most, cached);
+}
 
 // ---- which kernel takes a bfloat16 product ------------------------------------------------------------------------
 struct Routing {

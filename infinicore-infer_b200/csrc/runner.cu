@@ -1087,8 +1087,10 @@ JK_EXPORT int jk_runner_slot_bytes(const RunnerEnv *env, const RunnerOp *ops, in
                 break;
             case OP_LATENT_ATTENTION: {
                 need(op.in_slot, e * rows * op.heads * (op.rank + op.rot_width)); need(op.out_slot, e * rows * op.heads * op.rank);
-                // four times as many positions as the step may have rows: prompts, and portions of longer ones up to there
-                if (op.fold != 0 && env->dtype == JK_BF16 && rows >= 32) need(SLOT_HEADS, HeadsLayout(op, 4 * rows, rows, rows / 16).total);
+                if (op.fold != 0 && env->dtype == JK_BF16 && rows >= 32) {       // page 0 holds no positions
+                    const long long cached = (long long)std::max(1, op.num_pages - 1) * env->page_size;
+                    need(SLOT_HEADS, HeadsLayout(op, jk::latent_heads_positions(rows, op.max_positions, cached, op.window), rows, rows / 16).total);
+                }
                 long long worst = 0;
                 for (int n = 1; n <= 16 && n <= max_rows; ++n)
                     worst = std::max(worst, (long long)n * op.heads * latent_splits(n, op.heads, op.max_positions, env->routing.sms, 128) * (op.rank + 2));

@@ -37,6 +37,8 @@ _MIXERS_OPS = (OP["cast"], OP["layernorm"], OP["conv_qkv"], OP["linear_attention
                OP["rotate"])
 _BLOCKS_OPS = tuple(OP[n] for n in ("norm_add", "reinject", "latent_qkv", "head_linear", "latent_attention", "causal_conv",
                                     "selective_scan", "experts", "softcap", "add_rows", "norm_pair", "embed_pair", "join", "gated_recurrence"))
+OPTIONAL_SLOTS = ("heads",)     # a step finds another way where these are too small,
+LEAVE_FREE = 4 << 30            # so they are made only where this much stays free after them (logits of 8,192 rows over 122,753 tokens)
 SHORT_ROWS = 8                  # jk::SHORT_ROWS of csrc/host_rules.h
 MAX_GROUPS = 8
 MAX_LISTS = 8
@@ -340,6 +342,22 @@ def _dtype_code(dtype: torch.dtype) -> int:
     return kernels.dtype_code(dtype)
 
 
+def free_bytes(device) -> int:
+    return torch.cuda.mem_get_info(device)[0] if device.type == "cuda" else 1 << 62
+
+
+def allocate_slots(sizes, device):
+    """The slots' buffers, of the bytes in ``sizes`` (``SLOTS``' order) and 16 at the least.  The optional ones come last, and stay at
+    16 bytes where memory is short: an engine fits where it did without them."""
+    room = lambda b: torch.empty(max(int(b), 16), dtype=torch.uint8, device=device)
+    slots = [room(0 if name in OPTIONAL_SLOTS else b) for name, b in zip(SLOTS, sizes)]
+    for name in OPTIONAL_SLOTS:
+        i = SLOT[name]
+        if 16 < sizes[i] <= free_bytes(device) - LEAVE_FREE:
+            slots[i] = room(sizes[i])
+    return slots
+
+
 class ProgramRunner:
     """Buffers for steps of up to ``max_rows`` rows, and the call that replays a program over them."""
 
@@ -366,9 +384,9 @@ class ProgramRunner:
         sizes[SLOT["x"]] = max(sizes[SLOT["x"]], 4 * max_rows * program.hidden_size)         # host steps see the stream too
         sizes[SLOT["h"]] = max(sizes[SLOT["h"]], 4 * max_rows * program.hidden_size)
         sizes[SLOT["logits"]] = 0                                                           # made per step: the caller keeps them
-        self._slots = [torch.empty(max(int(b), 16), dtype=torch.uint8, device=rt.device) for b in sizes]
         self._workspace = torch.empty(self.WORKSPACE_BYTES, dtype=torch.uint8, device=rt.device)
         self._sumsq = torch.zeros(max(1, program.count), 16, dtype=torch.int64, device=rt.device)
+        self._slots = allocate_slots(sizes, rt.device)
         self.buffers = RunnerBuffers(workspace=self._workspace.data_ptr(), workspace_bytes=self.WORKSPACE_BYTES,
                                      sumsq=self._sumsq.data_ptr(), sumsq_rows=max(1, program.count))
         for s, t in enumerate(self._slots):

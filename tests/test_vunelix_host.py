@@ -1,10 +1,13 @@
 """Vunelix without a GPU: the configuration, the run order of a looped span, the manifest, the rotation's frequencies."""
+import ctypes
 import math
 
 import pytest
+import torch
 
 import plain_vunelix as plain
 from infinicore_infer_b200.config import ConfigError, FrequencyRampSpec, PairRotarySpec, VunelixConfig, config_class_for
+from infinicore_infer_b200.kernels import _build
 from infinicore_infer_b200.parts import cache_needs, model_manifest, state_needs
 
 
@@ -83,3 +86,45 @@ def test_what_the_configuration_refuses(change, what):
     change(c)
     with pytest.raises(ConfigError, match=what):
         VunelixConfig.from_dict(c)
+
+
+def latent_program(heads=16, dim=128, rot=64, rank=512, window=0, num_pages=65, page_size=16, max_positions=640):
+    """The record of a latent attention that may run over heads made for the step, and the environment of an engine that holds
+    ``num_pages`` pages (the null page among them)."""
+    from infinicore_infer_b200.kernels import dtype_code
+    from infinicore_infer_b200.parts import program
+    op = program.record("latent_attention", "q", "o", heads=heads, rank=rank, rot_width=rot, softmax_scale=0.1, window=window, num_pages=num_pages,
+                        max_positions=max_positions, fold=2, head_dim=dim, v_head_dim=dim, in2_slot="o", out2_slot="act")
+    env = program.RunnerEnv(dtype=dtype_code(torch.bfloat16), page_size=page_size, max_blocks=max_positions // page_size)
+    env.routing.sms = 148
+    return program, (program.RunnerOp * 1)(op), env
+
+
+def slot_bytes(program, ops, env, rows):
+    sizes = (ctypes.c_longlong * len(program.SLOTS))()
+    assert _build.load("runner").jk_runner_slot_bytes(ctypes.byref(env), ops, len(ops), rows, rows, sizes) == 0
+    return dict(zip(program.SLOTS, sizes))
+
+
+def test_room_for_heads_is_bounded_by_the_positions_a_step_can_see():
+    """16 heads of 128 + 64 over a latent of 512 take 2 (512 + 64 + 4,096) bytes a position."""
+    per = 2 * (512 + 64 + 16 * 256)
+    for rows, pages, window, max_positions, positions in ((2048, 65, 0, 640, 64 * 16),             # the cache holds fewer positions
+                                                         (2048, 100000, 0, 100000, 4 * 2048),      # four times the step's rows
+                                                         (2048, 65, 100, 100000, 4 * 2048),        # a window: pages come and go
+                                                         (64, 100000, 0, 48, 4 * 48),              # four requests at most, of 48 positions
+                                                         (40, 65, 0, 112, 112 + 48)):              # two requests would not meet the rule with more
+        program, ops, env = latent_program(num_pages=pages, window=window, max_positions=max_positions)
+        got = slot_bytes(program, ops, env, rows)["heads"]
+        assert got <= per * positions + 4096 + 12 * (rows // 128 + rows // 16), (rows, pages, window, got)
+        assert got >= per * min(positions, 2 * max_positions if rows == 40 else positions) - per * 48, (rows, pages, window, got)
+
+
+@pytest.mark.parametrize("left", [0, -1])
+def test_an_engine_leaves_the_room_for_heads_out_where_memory_is_short(monkeypatch, left):
+    """The buffer is optional: it is made where enough stays free after it, and is else too small for any step."""
+    module, ops, env = latent_program()
+    sizes = slot_bytes(module, ops, env, 64)
+    monkeypatch.setattr(module, "free_bytes", lambda device: module.LEAVE_FREE + sizes["heads"] + left)
+    slots = module.allocate_slots(list(sizes.values()), torch.device("cpu"))
+    assert [t.numel() for t in slots] == [16 if n == "heads" and left < 0 else max(16, b) for n, b in sizes.items()]
