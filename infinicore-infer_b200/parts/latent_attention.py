@@ -76,12 +76,16 @@ class LatentAttention:
             self.q_norm = weights.get(prefix + spec.q_down_name + spec.norm_suffix, VECTOR)
             self.w_q_up = weights.get(prefix + spec.q_up_name, MATRIX)
         self.norm = weights.get(prefix + spec.kv_down_name + spec.norm_suffix, VECTOR)
-        # the key and value maps as stored, one below the other: what makes heads from latent rows
-        self.w_heads = weights.get_rows([prefix + spec.k_up_name, prefix + spec.v_up_name], MATRIX)
-        # head h's key map [dn, R], transposed: the matrix that takes the head's plain query part into the latent space
-        self.w_q_latent = self.w_heads[:H * dn].view(H, dn, R).transpose(1, 2).contiguous()
-        self.w_v = self.w_heads[H * dn:]                                # [H, dv, R] as stored
         self.fold = runtime.dtype == torch.bfloat16 and latent_heads_fit(dn, spec.rot_dim, spec.v_head_dim, R)
+        self.w_heads = None
+        if self.fold:
+            # the key and value maps as stored, one below the other: what makes heads from latent rows
+            self.w_heads = weights.get_rows([prefix + spec.k_up_name, prefix + spec.v_up_name], MATRIX)
+            key_map, self.w_v = self.w_heads[:H * dn], self.w_heads[H * dn:]
+        else:
+            key_map, self.w_v = weights.get(prefix + spec.k_up_name, MATRIX), weights.get(prefix + spec.v_up_name, MATRIX)   # [H, dv, R] as stored
+        # head h's key map [dn, R], transposed: the matrix that takes the head's plain query part into the latent space
+        self.w_q_latent = key_map.view(H, dn, R).transpose(1, 2).contiguous()
         self.w_o = weights.get(prefix + spec.o_name, MATRIX)
         self.freq, self.magnitude, self.rot_dims = None, 1.0, 0
         if spec.position is not None and spec.position.dims:

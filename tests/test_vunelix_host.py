@@ -128,3 +128,26 @@ def test_an_engine_leaves_the_room_for_heads_out_where_memory_is_short(monkeypat
     monkeypatch.setattr(module, "free_bytes", lambda device: module.LEAVE_FREE + sizes["heads"] + left)
     slots = module.allocate_slots(list(sizes.values()), torch.device("cpu"))
     assert [t.numel() for t in slots] == [16 if n == "heads" and left < 0 else max(16, b) for n, b in sizes.items()]
+
+
+@pytest.mark.parametrize("dtype,dim,twice", [(torch.float32, 64, False), (torch.bfloat16, 48, False), (torch.bfloat16, 64, True)])
+def test_the_key_map_is_kept_as_stored_only_where_heads_can_be_made_from_it(dtype, dim, twice):
+    """Beside its transpose; elsewhere (float32, sizes outside the rule) the layer holds one copy of each map and no more."""
+    from infinicore_infer_b200.parts import LatentAttention
+    from infinicore_infer_b200.parts.base import Runtime
+    layer = dict(type="latent_attention", mlp=None, mixer=dict(heads=2, dim=dim, rot_dim=64, vdim=dim, kv_rank=72, scale=0.1, rot=dict(base=1e3, dims=32)))
+    c = dict(architecture="Vunelix", norm=dict(eps=1e-5), vocab=40, width=16, logit_softcap=None, layers=[layer])
+    spec = VunelixConfig.from_dict(c).model_spec()
+    names = model_manifest(spec)
+
+    class Weights:
+        def get(self, name, role):
+            return torch.zeros(names[name].shape, dtype=dtype)
+
+        def get_rows(self, wanted, role):
+            return torch.cat([self.get(n, role) for n in wanted])
+
+    part = LatentAttention(spec.layers[0].mixer, Weights(), "l0.mix.", Runtime(dtype, "cpu"))
+    held = {t.untyped_storage().data_ptr(): t.untyped_storage().nbytes() for t in (part.w_heads, part.w_q_latent, part.w_v) if t is not None}
+    one = 2 * dim * 72 * dtype.itemsize
+    assert sum(held.values()) == (3 if twice else 2) * one
