@@ -262,8 +262,9 @@ inline bool attention_tcgen05_takes(int dh, int page_size, int dv = 0) {
 // 102 -> 41; 64 rows after 2,048 297 -> 64; 2,048 rows after 0 887 -> 74.  Below it the way over heads costs 24 us at the least, while
 // 8 requests of one row over the latent rows take 17.
 inline bool latent_heads_fit(int dn, int dr, int dv, int R) { return dn == dv && (dn == 64 || dn == 128) && (dr == 0 || dr == 64) && R % 8 == 0 && R >= 64; }
+constexpr int LATENT_HEADS_ROWS = 32;       // the fewest rows of a step that goes this way; an engine of smaller steps has neither the room nor the modules
 inline bool latent_takes_heads(int rows, int nreq, long long keys, int window, int dn, int dr, int dv, int R) {
-    if (keys <= 0 || rows < 32 || nreq <= 0 || !latent_heads_fit(dn, dr, dv, R)) return false;
+    if (keys <= 0 || rows < LATENT_HEADS_ROWS || nreq <= 0 || !latent_heads_fit(dn, dr, dv, R)) return false;
     const long long reach = window > 0 ? std::min<long long>(window, keys / nreq) : keys / nreq;
     return rows * reach >= 16LL * keys;
 }

@@ -1087,7 +1087,8 @@ JK_EXPORT int jk_runner_slot_bytes(const RunnerEnv *env, const RunnerOp *ops, in
                 break;
             case OP_LATENT_ATTENTION: {
                 need(op.in_slot, e * rows * op.heads * (op.rank + op.rot_width)); need(op.out_slot, e * rows * op.heads * op.rank);
-                if (op.fold != 0 && env->dtype == JK_BF16 && rows >= 32) {       // page 0 holds no positions
+                if (op.fold != 0 && env->dtype == JK_BF16 && rows >= jk::LATENT_HEADS_ROWS && !env->legacy_tensor_cores && !env->routing.library_only) {
+                    // (page 0 holds no positions)
                     const long long cached = (long long)std::max(1, op.num_pages - 1) * env->page_size;
                     need(SLOT_HEADS, HeadsLayout(op, jk::latent_heads_positions(rows, op.max_positions, cached, op.window), rows, rows / 16).total);
                 }
@@ -1155,7 +1156,7 @@ JK_EXPORT int jk_runner_needs_gemm_tcgen05(const RunnerEnv *env, const RunnerOp 
             case OP_RESIDUAL: kind = jk::PRODUCT_RESIDUAL; break;
             case OP_GATE_UP: kind = jk::PRODUCT_SWIGLU; break;
             case OP_LATENT_ATTENTION:
-                if (op.fold != 0 && max_rows >= 32) return 1;
+                if (op.fold != 0 && max_rows >= jk::LATENT_HEADS_ROWS && !env->legacy_tensor_cores) return 1;
                 continue;
             default: continue;
         }

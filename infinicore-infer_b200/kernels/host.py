@@ -134,6 +134,11 @@ def latent_heads_fit(dn: int, dr: int, dv: int, rank: int) -> bool:
     return bool(lib().jk_latent_heads_fit(dn, dr, dv, rank))
 
 
+def latent_heads_rows() -> int:
+    """The fewest rows of a step whose latent attentions can run over heads made for it."""
+    return lib().jk_latent_heads_rows()
+
+
 def attention_tcgen05_takes(dh: int, page_size: int, dv: int = 0) -> bool:
     return bool(lib().jk_attention_tcgen05_takes(dh, page_size, dv))
 

@@ -342,6 +342,18 @@ def _dtype_code(dtype: torch.dtype) -> int:
     return kernels.dtype_code(dtype)
 
 
+def modules_needed(env: RunnerEnv, ops, count: int, max_rows: int) -> Dict[str, bool]:
+    """Which of ``runner_lib``'s modules the first ``count`` records can reach in steps of up to ``max_rows`` rows."""
+    records = [ops[i] for i in range(count)]
+    # heads made for a step: where jk_runner_slot_bytes keeps room for them, so that a step's way depends on its own engine only
+    heads = max_rows >= _host.latent_heads_rows() and not env.routing.library_only and any(op.kind == OP["latent_attention"] and op.fold for op in records)
+    return {"gemm_tcgen05": bool(_build.load("runner").jk_runner_needs_gemm_tcgen05(ctypes.byref(env), ops, count, max_rows)),
+            "attention_tcgen05": env.dtype == _dtype_code(torch.bfloat16) and not env.legacy_tensor_cores and (heads or any(
+                op.kind == OP["attention"] and _host.attention_tcgen05_takes(op.head_dim, env.page_size, op.v_head_dim) for op in records)),
+            "mixers": any(op.kind in _MIXERS_OPS or (op.kind == OP["gate_up"] and op.act > ACT["silu"]) for op in records),
+            "blocks": any(op.kind in _BLOCKS_OPS for op in records)}
+
+
 def free_bytes(device) -> int:
     return torch.cuda.mem_get_info(device)[0] if device.type == "cuda" else 1 << 62
 
@@ -370,14 +382,7 @@ class ProgramRunner:
         self.max_rows, self.max_want = max_rows, max_want or max_rows
         self.one_by_one = one_by_one
         self.env = rt.env(program.page_size, program.max_blocks)
-        need_gemm = bool(program.lib.jk_runner_needs_gemm_tcgen05(ctypes.byref(self.env), program.ops, program.count, max_rows))
-        need_attn = rt.dtype == torch.bfloat16 and not rt.legacy_tensor_cores and any(
-            (program.ops[i].kind == OP["attention"] and _host.attention_tcgen05_takes(program.ops[i].head_dim, program.page_size, program.ops[i].v_head_dim))
-            or (program.ops[i].kind == OP["latent_attention"] and program.ops[i].fold and max_rows >= 64) for i in range(program.count))
-        need_mixers = any(program.ops[i].kind in _MIXERS_OPS or (program.ops[i].kind == OP["gate_up"] and program.ops[i].act > ACT["silu"])
-                          for i in range(program.count))
-        need_blocks = any(program.ops[i].kind in _BLOCKS_OPS for i in range(program.count))
-        self.lib = runner_lib(need_gemm, need_attn, need_mixers, need_blocks)
+        self.lib = runner_lib(**modules_needed(self.env, program.ops, program.count, max_rows))
         self.lib.jk_runner_last_error.restype = ctypes.c_char_p
         sizes = (_ll * len(SLOTS))()
         self._check(self.lib.jk_runner_slot_bytes(ctypes.byref(self.env), program.ops, program.count, max_rows, self.max_want, sizes))

@@ -120,6 +120,20 @@ def test_room_for_heads_is_bounded_by_the_positions_a_step_can_see():
         assert got >= per * min(positions, 2 * max_positions if rows == 40 else positions) - per * 48, (rows, pages, window, got)
 
 
+@pytest.mark.parametrize("switch", ["", "legacy_tensor_cores", "library_only"])
+@pytest.mark.parametrize("rows", [1, 31, 32, 63, 64, 4096])
+def test_an_engine_has_room_for_heads_exactly_where_it_binds_the_kernels(rows, switch):
+    """The table of entry points is shared by all engines of a process: an engine that keeps room without binding both modules would go
+    over heads or not by what another engine has bound."""
+    program, ops, env = latent_program()
+    if switch:
+        setattr(env if switch in dict(env._fields_) else env.routing, switch, 1)
+    needed = program.modules_needed(env, ops, len(ops), rows)
+    room = slot_bytes(program, ops, env, rows)["heads"] > 0
+    assert needed["attention_tcgen05"] == needed["gemm_tcgen05"] == room == (rows >= 32 and not switch)
+    assert needed["blocks"] and not needed["mixers"]
+
+
 @pytest.mark.parametrize("left", [0, -1])
 def test_an_engine_leaves_the_room_for_heads_out_where_memory_is_short(monkeypatch, left):
     """The buffer is optional: it is made where enough stays free after it, and is else too small for any step."""
