@@ -61,6 +61,61 @@ def test_latent_attention_over_heads_made_for_the_step(tmp_path, heads, dim, ran
     assert not torch.equal(logits[False], logits[True])         # both ways ran
 
 
+def _one_layer(family, mixer):
+    extra = {"vunelix": dict(logit_softcap=None), "fupapel": dict(residual_mult=1.0),
+             "fapenex": dict(max_positions=640, logit_scale=1.0, logit_softcap=None)}[family]
+    return dict(architecture=family.capitalize(), norm=dict(eps=1e-5), vocab=97, width=64, layers=[dict(type="latent_attention", mlp=None, mixer=mixer)], **extra)
+
+
+@pytest.mark.parametrize("family,heads,dim,rot,rank,q_rank,window", [
+    ("fapenex", 2, 128, 0, 64, 40, 100), ("fapenex", 3, 64, 0, 72, 40, 70), ("fapenex", 2, 128, 0, 64, 40, 600),       # queries through a latent, a window
+    ("fupapel", 2, 128, 64, 72, 48, 0), ("fupapel", 3, 64, 64, 64, 40, 0),      # and rotated parts, learned sinks, a gate per head
+    ("vunelix", 2, 128, 64, 64, 0, 0)])                                         # neither; a gate per element
+def test_every_form_of_latent_attention_over_heads_and_who_goes_which_way(tmp_path, family, heads, dim, rot, rank, q_rank, window):
+    """Every instance and option, prompts and portions whose tiles end inside other requests' rows (with a query latent the output lies
+    where the plain queries lay), windows that cross key tiles.  A step goes over heads as a whole: one request of eight rows or fewer
+    keeps all of it on the latent rows, where the bits are those of an engine that knows no other way.  Both ways round operands and
+    results to bfloat16 (2^-9 each, about ten on the way to a logit): within 0.03 of the logits' spread of float64."""
+    import importlib
+    from infinicore_infer_b200.config import config_class_for
+    from infinicore_infer_b200.engine import Engine, StepEntry
+    from infinicore_infer_b200.weights import index_directory, read_tensor, write_model_folder
+    mixer = dict(heads=heads, dim=dim, vdim=dim, kv_rank=rank, scale=(dim + rot) ** -0.5)
+    mixer.update(dict(rot_dim=rot, rot=dict(base=1e3, dims=64 if q_rank else 32)) if rot else {}, **(dict(q_rank=q_rank) if q_rank else {}),
+                 **(dict(mask=dict(size=window)) if window else {}))
+    cfg = _one_layer(family, mixer)
+    write_model_folder(config_class_for(cfg).from_dict(cfg), str(tmp_path), seed=heads + dim, std=0.16, norm_std=0.2)
+    with open(os.path.join(tmp_path, "config.json")) as f:
+        disk = json.load(f)
+    index = index_directory(str(tmp_path))
+    toks = [random_tokens(s, 400, 97) for s in range(3)]
+    reference = importlib.import_module("plain_" + family)
+    if family == "vunelix":
+        weights = {n: read_tensor(i).float() for n, i in index.items()}
+        want = [reference.forward(t, disk, weights) for t in toks]
+    else:
+        weights = {n: read_tensor(i).double().numpy() for n, i in index.items()}
+        want = [torch.from_numpy(np.asarray(reference.forward(disk, weights, t))) for t in toks]
+    engine = Engine.from_folder(str(tmp_path), max_tokens=640, cache_tokens=1280, page_size=16, max_requests=3, max_step_tokens=512)
+    # (over heads, (request, from, to) of every entry); a step that has a request of at most eight rows is not
+    steps = [(True, [(0, 0, 150)]), (True, [(0, 150, 190), (1, 0, 129)]), (False, [(1, 129, 321), (0, 190, 191)]), (False, [(2, 0, 8), (1, 321, 395)]),
+             (True, [(2, 8, 200), (0, 191, 400)]), (False, [(1, 395, 396), (2, 200, 201)])]
+    got = {}
+    for other_way in (False, True):
+        engine.runtime.plain_attention = other_way
+        got[other_way] = [engine.step([StepEntry((other_way, r), toks[r][a:b], list(range(b - a))) for r, a, b in step]).double().cpu() for _, step in steps]
+        for r in range(3):
+            engine.end((other_way, r))
+    engine.check()
+    engine.runtime.plain_attention = False
+    for (over_heads, step), one, other in zip(steps, got[False], got[True]):
+        ref = torch.cat([want[r][a:b] for r, a, b in step])
+        for out in (one, other):
+            err = (out - ref).square().mean().sqrt() / want[0].std()
+            assert err <= 0.03, f"{step}: {err:.4f} of the logits' spread"
+        assert torch.equal(one, other) == (not over_heads), step
+
+
 @pytest.mark.parametrize("dh,rotated", [(64, False), (64, True), (128, False), (128, True)])
 def test_weights_of_an_attention_over_laid_heads_are_float32_accurate(K, dh, rotated):
     """Each instance, with values that pick single weights: row t has scores -a_t b_j (exact in float32) over 64 keys and far lower ones
