@@ -192,7 +192,7 @@ def time_records(engine, ctx, which, repeats=3):
     import ctypes
     import torch
     from infinicore_infer_b200 import kernels
-    from infinicore_infer_b200.parts.program import SLOT, RunnerStep, tile_keys
+    from infinicore_infer_b200.parts.program import SLOT, RunnerStep, set_host_lengths
     runner, prog = engine.runner, engine.program
     T = ctx.ntok
     logits = torch.empty(max(1, ctx.want_rows.numel()), engine.spec.vocab_size, dtype=torch.float32, device=engine.device)
@@ -200,8 +200,8 @@ def time_records(engine, ctx, which, repeats=3):
     runner.buffers.bytes[SLOT["logits"]] = logits.numel() * 4
     step = RunnerStep(ntok=T, nreq=ctx.nreq, n_want=ctx.want_rows.numel(), context=ctx.context, tokens=ctx.tokens.data_ptr(),
                       positions=ctx.positions.data_ptr(), row_req=ctx.row_req.data_ptr(), req_start=ctx.req_start.data_ptr(),
-                      req_pos=ctx.req_pos.data_ptr(), want_rows=ctx.want_rows.data_ptr(), slot_ids=ctx.slot_ids.data_ptr(),
-                      tile_keys=tile_keys(ctx))
+                      req_pos=ctx.req_pos.data_ptr(), want_rows=ctx.want_rows.data_ptr(), slot_ids=ctx.slot_ids.data_ptr())
+    host = set_host_lengths(step, ctx)      # noqa: F841 (alive while the records run)
     for g, table in enumerate(ctx.block_tables):
         step.block_tables[g] = table.data_ptr()
     for name, index in prog.lists.items():

@@ -244,8 +244,8 @@ template <int DK, int DV, int HALVES> struct AtSmem {
 
 // HALVES: 2 as described above.  1: tiles of 64 keys and four softmax warps, a thread a row, one reference, sum and accumulator; half
 // the threads, shared and tensor memory, so that two blocks fit an SM where heads are 128 wide and one's waits lie under the other's
-// work.  B200, 128 keys a tile and one block an SM -> 64 and two: 32 heads of 128 over prompts of 833, 1,667 and 2,503 tokens 207 -> 152 us,
-// 16 heads, 2,048 tokens, window 1,024 40 -> 33.  Keys of 192 would have room for one stage of each operand only: 74 -> 105 us, so they
+// work (where a launch has that many: jk::attention_tile_keys).  B200, 128 keys a tile and one block an SM -> 64 and two: 32 heads of 128 over
+// prompts of 833, 1,667 and 2,503 tokens 207 -> 152 us, 16 heads, 2,048 tokens, window 1,024 40 -> 33.  Keys of 192 would have room for one stage of each operand only: 74 -> 105 us, so they
 // stay at 128 keys a tile.
 // ELEM: the gate, if there is one, has a column per output element (an instance of its own, so that the others carry neither
 // its code nor its registers)
@@ -663,6 +663,10 @@ JK_EXPORT int jk_attention_tcgen05_supports(int dh, int page_size) {
     return (dh == 64 || dh == 128) && (page_size == 8 || page_size == 16 || page_size == 32 || page_size == 64 || page_size == 128);
 }
 
+// Whether heads of 128 walk tiles of 64 keys: the caller's 64 or 128 (jk::attention_tile_keys, which knows the requests); 0: as it would say of
+// tiles whose keys grow evenly from none, half the longest one's on average.
+static bool tiles_of_64(int tile_keys, int heads, int ntiles) { return (tile_keys > 0 ? tile_keys : jk::attention_tile_keys(heads, 0.5 * ntiles, 148)) == 64; }
+
 template <int DK, int DV, bool ELEM, int FROM, int HALVES>
 static int launch_at(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const CUtensorMap &mqr, const CUtensorMap &mkr,
                      const AtArgs &a, cudaStream_t stream) {
@@ -680,7 +684,7 @@ JK_EXPORT int jk_attention_tcgen05(const void *q, const void *k_pages, const voi
                                    int ntiles, int ntok, const int *req_start, const int *req_pos, const int *block_table,
                                    int max_blocks, int num_pages, int page_size, int nh, int nkvh, int dh, float scale,
                                    int window, int *status, int sink, const float *gate, int gate_ld, float cap, int keep_first,
-                                   const float *sink_w, int gate_elem, int dv, cudaStream_t stream) {
+                                   const float *sink_w, int gate_elem, int dv, int tile_keys, cudaStream_t stream) {
     if (ntiles == 0) return JK_OK;
     if (dv <= 0) dv = dh;
     JK_REQUIRE(gate == nullptr || gate_ld >= nh * (gate_elem ? dv : 1), "attention_tcgen05: a gate row of %d holds no %d heads", gate_ld, nh);
@@ -702,7 +706,7 @@ JK_EXPORT int jk_attention_tcgen05(const void *q, const void *k_pages, const voi
         LAUNCH_AT(64, 128, 2);
     }
     if (dv <= 64) LAUNCH_AT(128, 64, 2);
-    if (page_size <= AT_HALF) LAUNCH_AT(128, 128, 1);
+    if (page_size <= AT_HALF && tiles_of_64(tile_keys, nh, ntiles)) LAUNCH_AT(128, 128, 1);
     LAUNCH_AT(128, 128, 2);
 #undef LAUNCH_AT
 }
@@ -714,7 +718,7 @@ JK_EXPORT int jk_attention_tcgen05(const void *q, const void *k_pages, const voi
 JK_EXPORT int jk_attention_laid_tcgen05(const void *q, const void *q_rot, int rot_ld, int rot_off, const void *kv, const void *k_rot, long long rows,
                                         void *out, const int *tiles, int ntiles, int ntok, const int *req_start, const int *req_pos, int nh,
                                         int dh, float scale, int window, int *status, const float *sink_w, const float *gate, int gate_ld,
-                                        int gate_elem, cudaStream_t stream) {
+                                        int gate_elem, int tile_keys, cudaStream_t stream) {
     if (ntiles == 0 || ntok == 0) return JK_OK;
     JK_REQUIRE(dh == 64 || dh == 128, "attention_laid: heads of %d are not built", dh);
     JK_REQUIRE(q && kv && out && tiles && req_start && req_pos && status && (k_rot == nullptr || q_rot != nullptr), "attention_laid: an argument is missing");
@@ -723,7 +727,8 @@ JK_EXPORT int jk_attention_laid_tcgen05(const void *q, const void *q_rot, int ro
     JK_REQUIRE(gate == nullptr || gate_ld >= nh * (gate_elem ? dh : 1), "attention_laid: a gate row of %d holds no %d heads", gate_ld, nh);
     CUtensorMap mq, mk, mv, mqr, mkr;
     if (int rc = tensor_map(q, ntok, nh * dh, AT_BM, &mq)) return rc;
-    const int keys = dh == 128 && k_rot == nullptr ? AT_HALF : 2 * AT_HALF;         // a tile of the instances below
+    const bool of_64 = dh == 128 && k_rot == nullptr && tiles_of_64(tile_keys, nh, ntiles);
+    const int keys = of_64 ? AT_HALF : 2 * AT_HALF;         // a tile of the instances below
     if (int rc = tensor_map(kv, rows, nh * dh, keys, &mk, 2 * nh * dh)) return rc;
     if (int rc = tensor_map((const __nv_bfloat16 *)kv + nh * dh, rows, nh * dh, keys, &mv, 2 * nh * dh)) return rc;
     mqr = mq, mkr = mk;
@@ -740,6 +745,7 @@ JK_EXPORT int jk_attention_laid_tcgen05(const void *q, const void *q_rot, int ro
         LAUNCH_LAID(64, 64, AT_LAID, 2);
     }
     if (k_rot != nullptr) LAUNCH_LAID(192, 128, AT_LAID_ROT, 2);
-    LAUNCH_LAID(128, 128, AT_LAID, 1);
+    if (of_64) LAUNCH_LAID(128, 128, AT_LAID, 1);
+    LAUNCH_LAID(128, 128, AT_LAID, 2);
 #undef LAUNCH_LAID
 }

@@ -416,6 +416,7 @@ int run_batch(JkModel *m, const uint32_t *tokens, uint32_t ntok, const uint32_t 
     const int *dv = m->meta_dev;
     st.tokens = dv + lay.tokens; st.positions = dv + lay.positions; st.row_req = dv + lay.row_req;
     st.req_start = dv + lay.req_start; st.req_pos = dv + lay.req_pos; st.want_rows = dv + lay.want_rows;
+    st.host_req_start = h + lay.req_start; st.host_req_pos = h + lay.req_pos;
     st.block_tables[0] = dv + lay.tables[0];
     st.lists[0] = lists.n_short == T ? nullptr : dv + lay.extra;       // every row is a short row: no list is needed
     st.list_n[0] = lists.n_short;

@@ -54,6 +54,10 @@ JK_HOST_EXPORT void jk_attention_work_lists(int B, int pad_B, const int *lens, c
     counts[0] = c.n_short; counts[1] = c.n_tiles;
 }
 
+JK_HOST_EXPORT int jk_attention_tile_keys(int heads, int nreq, const int *req_start, const int *req_pos, int window, int sms) {
+    return jk::attention_tile_keys(heads, jk::attention_tile_load(nreq, req_start, req_pos, window), sms);
+}
+
 // ---- attention cuts, product routes, tables, uniforms -----------------------------------------------------------
 JK_HOST_EXPORT int jk_decode_splits(int nrows, int nkvh, int group, int keys, int sms, int dh) {
     return jk::decode_splits(nrows, nkvh, group, keys, sms, dh);

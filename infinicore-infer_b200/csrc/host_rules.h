@@ -171,6 +171,28 @@ inline AttentionLists attention_work_lists(int B, int pad_B, const int *lens, co
     return c;
 }
 
+// The first key that a query at `pos` sees (jk_mask_lo of csrc/common.cuh).
+inline int mask_lo(int pos, int window) { return window > 0 ? std::max(pos - window + 1, 0) : window < 0 ? pos / -window * -window : 0; }
+// The keys that a step's query tiles walk, counted in the longest one's: req_start [nreq + 1], req_pos [nreq].
+inline double attention_tile_load(int nreq, const int *req_start, const int *req_pos, int window) {
+    long long sum = 0, most = 0;
+    for (int r = 0; r < nreq; ++r) {
+        const int n = req_start[r + 1] - req_start[r];
+        for (int t0 = 0; t0 < n && n > SHORT_ROWS; t0 += TILE_ROWS) {
+            const long long keys = req_pos[r] + std::min(t0 + TILE_ROWS, n) - mask_lo(req_pos[r] + t0, window);
+            sum += keys;
+            most = std::max(most, keys);
+        }
+    }
+    return most > 0 ? (double)sum / (double)most : 0.0;
+}
+// Keys a tile of the tcgen05 prefill attention, heads of 128.  Tiles of 64 let two blocks share an SM: more keys an SM and microsecond, but
+// a block alone walks its own at 0.82 of the rate of tiles of 128.  So they pay where the blocks' work makes more than one wave of the
+// longest block (B200, tiles of 128 -> 64; work in longest blocks over 148 SMs): 16 heads, 2,048 rows 45 -> 52 us (0.9); after 1,000 positions
+// 76 -> 75 (1.2), after 4,000 164 -> 138 (1.4); 1,024 rows after 4,000 87 -> 106 (0.8); 32 heads, 1,536 rows 55 -> 48 (1.4), 1,024 rows 32 -> 34
+// (1.0), 128 rows after 4,000 72 -> 88 (0.2); 1,000 rows beside 64 after 3,000 56 -> 72 (0.5), beside 200 39 -> 34 (1.1).
+inline int attention_tile_keys(int heads, double load, int sms) { return heads * load > sms ? 64 : 128; }
+
 // ---- the pieces of a linear-attention recurrence -------------------------------------------------------------------
 // A request that brings more than SCAN_PIECE rows to a step has its recurrence cut into pieces of that many rows, which
 // run side by side and are then joined (csrc/mixers.cu); the others run from their state slot in one go.  A step of

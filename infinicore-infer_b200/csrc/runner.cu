@@ -110,6 +110,15 @@ struct Run {
     cudaStream_t stream;
     bool pending = false;         // SLOT_DELTA holds a product that has not been added to the stream yet
     float pending_scale = 1.f;
+    // keys a tile of a prefill attention (0: the kernel's own guess); layers of one window have the same tiles
+    int load_window = 0;
+    double load = -1.0;
+    int tile_keys(int heads, int window) {
+        if (st.host_req_start == nullptr || st.host_req_pos == nullptr) return 0;
+        if (load < 0.0 || window != load_window) load = jk::attention_tile_load(st.nreq, st.host_req_start, st.host_req_pos, window);
+        load_window = window;
+        return jk::attention_tile_keys(heads, load, env.routing.sms);
+    }
 
     int elem() const { return env.dtype == JK_F32 ? 4 : 2; }
     bool tcgen05_bound() const { return g_fns.gemm_tcgen05 != nullptr; }
@@ -279,7 +288,7 @@ int run_attention(Run &r, const RunnerOp &op) {
             RUN(attention_tcgen05, g_fns.attention_tcgen05(q, op.k_pages, op.v_pages, o, tiles, n_tiles, T, r.st.req_start, r.st.req_pos,
                                                            table, r.env.max_blocks, op.num_pages, page, nh, nkvh, dh, op.softmax_scale,
                                                            op.window, r.env.status, op.sink, gate, op.ld, op.cap, op.keep_first, op.sink_w,
-                                                           op.gated == 2, dv, r.stream));
+                                                           op.gated == 2, dv, r.tile_keys(nh, op.window), r.stream));
         else
             RUN(attention, g_fns.attention_prefill(q, op.k_pages, op.v_pages, o, tiles, n_tiles, jk::TILE_ROWS, r.st.req_start,
                                                    r.st.req_pos, table, r.env.max_blocks, page, nh, nkvh, dh, op.softmax_scale,
@@ -633,7 +642,7 @@ int run_latent_over_heads(Run &r, const RunnerOp &op) {
     RUN(gemm_tcgen05, g_fns.gemm_tcgen05(base, op.w_heads, base + at.kv, C, 2 * H * dh, op.rank, 2 * H * dh, 1, 1.f, r.env.status, r.env.routing.sms, r.stream));
     RUN(attention_tcgen05, g_fns.attention_laid(plain, q, D, op.rank, base + at.kv, rot, C, out, (const int *)(base + at.tiles), at.ntiles, T, r.st.req_start,
                                                 r.st.req_pos, H, dh, op.softmax_scale, op.window, r.env.status, op.sink_w, gate, op.ld, op.gated == 1,
-                                                r.stream));
+                                                r.tile_keys(H, op.window), r.stream));
     return JK_OK;
 }
 

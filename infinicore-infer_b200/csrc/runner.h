@@ -40,7 +40,7 @@ typedef int (*AttentionPrefillFn)(const void *, const void *, const void *, void
                                   const float *, int, cudaStream_t);
 typedef int (*AttentionTcgen05Fn)(const void *, const void *, const void *, void *, const int *, int, int, const int *,
                                   const int *, const int *, int, int, int, int, int, int, float, int, int *, int, const float *, int,
-                                  float, int, const float *, int, int, cudaStream_t);
+                                  float, int, const float *, int, int, int, cudaStream_t);
 typedef int (*SupportsFn)(int, int, int);
 typedef int (*LinearSmallPartsFn)(const void *, long long, const int *, int, const void *, void *, int, int, int, int, int, cudaStream_t);
 typedef int (*Supports1Fn)(int);
@@ -108,7 +108,7 @@ typedef int (*LatentGatherFn)(const void *, const int *, int, int, const int *, 
                               cudaStream_t);
 // csrc/attention_tcgen05.cu
 typedef int (*AttentionLaidFn)(const void *, const void *, int, int, const void *, const void *, long long, void *, const int *, int, int,
-                               const int *, const int *, int, int, float, int, int *, const float *, const float *, int, int, cudaStream_t);
+                               const int *, const int *, int, int, float, int, int *, const float *, const float *, int, int, int, cudaStream_t);
 typedef int (*ArgmaxFn)(const float *, long long, int, int, int *, void *, cudaStream_t);
 typedef int (*SampleFn)(const float *, long long, int, int, const float *, const int *, const float *, const float *, int *,
                         cudaStream_t);
@@ -407,6 +407,7 @@ struct RunnerStep {
     const int *lists[jk::MAX_STEP_LISTS];     // work lists that mixers asked for; null with n == ntok means "rows 0..ntok-1"
     int list_n[jk::MAX_STEP_LISTS];
     int tile_keys;              // positions of all requests, this step's rows among them, if each brings more than jk::SHORT_ROWS rows; else 0
+    const int *host_req_start, *host_req_pos;       // the host's copies of req_start and req_pos, or null
 };
 
 struct RunnerBuffers {

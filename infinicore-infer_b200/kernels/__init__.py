@@ -566,10 +566,10 @@ def attention_tcgen05(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
                       tiles: torch.Tensor, ntiles: int, ntok: int, req_start: torch.Tensor, req_pos: torch.Tensor,
                       block_table: torch.Tensor, nh: int, scale: float, window: int = 0, sink: bool = False,
                       gate: Optional[torch.Tensor] = None, cap: float = 0.0, keep_first: int = 0,
-                      sink_w: Optional[torch.Tensor] = None, gate_elem: bool = False) -> torch.Tensor:
+                      sink_w: Optional[torch.Tensor] = None, gate_elem: bool = False, tile_keys: int = 0) -> torch.Tensor:
     """The same attention of TILE_ROWS-row query tiles on the tcgen05 tensor cores (TMA operands, both
     products with accumulators in tensor memory); head sizes 64 and 128, or keys and values of unlike sizes (multiples of 8 up to
-    128), pages that divide 128."""
+    128), pages that divide 128.  ``tile_keys``: 64 or 128 keys at a time for heads of 128 (0: by the number of tiles)."""
     for name, t in (("q", q), ("k_pages", k_pages), ("v_pages", v_pages), ("out", out)):
         _need(t, name, torch.bfloat16)
     for name, t in (("tiles", tiles), ("req_start", req_start), ("req_pos", req_pos), ("block_table", block_table)):
@@ -584,7 +584,7 @@ def attention_tcgen05(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
         _ptr(req_pos), _ptr(block_table), _c_int(block_table.shape[1]), _c_int(num_pages), _c_int(page_size), _c_int(nh),
         _c_int(nkvh), _c_int(dh), _c_float(scale), _c_int(window or 0), _ptr(gemm_status(q.device)), _c_int(1 if sink else 0),
         *_gate_args(gate, ntok, nh * (dv if gate_elem else 1)), _c_float(cap), _c_int(keep_first), _ptr(sink_w), _c_int(1 if gate_elem else 0), _c_int(dv),
-        _stream()))
+        _c_int(tile_keys), _stream()))
     return out
 
 

@@ -106,6 +106,12 @@ def attention_list_capacity(T: int, B: int) -> (int, int):
     return h.jk_attention_short_rows_capacity(T), h.jk_attention_tiles_capacity(T, B)
 
 
+def attention_tile_keys(heads: int, req_start, req_pos, window: int = 0, sms: int = 148) -> int:
+    """Keys a tile (64 or 128) of a step's prefill attention with heads of 128."""
+    start, pos = _i32(req_start), _i32(req_pos)
+    return lib().jk_attention_tile_keys(heads, len(pos), _c_p(_ptr(start)), _c_p(_ptr(pos)), window, sms)
+
+
 def attention_work_lists(B: int, pad_B: int, lens, starts, short_rows: np.ndarray, tiles: np.ndarray) -> (int, int):
     """Fill the attention's work lists for a batch (``jk::attention_work_lists``); returns (short rows, tiles)."""
     lens, starts = _i32(lens), _i32(starts)

@@ -92,7 +92,8 @@ class RunnerEnv(ctypes.Structure):
 class RunnerStep(ctypes.Structure):
     _fields_ = ([(n, _i) for n in ("ntok", "nreq", "n_want", "context")]
                 + [(n, _p) for n in ("tokens", "positions", "row_req", "req_start", "req_pos", "want_rows", "slot_ids")]
-                + [("block_tables", _p * MAX_GROUPS), ("lists", _p * MAX_LISTS), ("list_n", _i * MAX_LISTS), ("tile_keys", _i)])
+                + [("block_tables", _p * MAX_GROUPS), ("lists", _p * MAX_LISTS), ("list_n", _i * MAX_LISTS), ("tile_keys", _i)]
+                + [(n, _p) for n in ("host_req_start", "host_req_pos")])
 
 
 class RunnerBuffers(ctypes.Structure):
@@ -428,7 +429,7 @@ class ProgramRunner:
                           tokens=ctx.tokens.data_ptr(), positions=ctx.positions.data_ptr(), row_req=ctx.row_req.data_ptr(),
                           req_start=ctx.req_start.data_ptr(), req_pos=ctx.req_pos.data_ptr(), want_rows=ctx.want_rows.data_ptr(),
                           slot_ids=ctx.slot_ids.data_ptr())
-        step.tile_keys = tile_keys(ctx)
+        host = set_host_lengths(step, ctx)      # noqa: F841 (alive until the step is launched)
         for g, table in enumerate(ctx.block_tables):
             step.block_tables[g] = table.data_ptr()
         for name, index in prog.lists.items():
@@ -458,6 +459,16 @@ class ProgramRunner:
                                                    ctypes.byref(self.buffers), flush, stream))
                 self.launches += self.lib.jk_runner_launches()
         return logits
+
+
+def set_host_lengths(step: RunnerStep, ctx):
+    """What the native step's rules read of the requests' lengths on the host; returns the arrays, to be kept until the call is over."""
+    step.tile_keys = tile_keys(ctx)
+    if len(ctx.host_req_start) <= ctx.nreq or len(ctx.host_req_pos) < ctx.nreq or ctx.ntok <= ctx.nreq:
+        return None                             # not known, or no request has more than one row
+    start, pos = (_i * (ctx.nreq + 1))(*ctx.host_req_start[:ctx.nreq + 1]), (_i * ctx.nreq)(*ctx.host_req_pos[:ctx.nreq])
+    step.host_req_start, step.host_req_pos = ctypes.addressof(start), ctypes.addressof(pos)
+    return start, pos
 
 
 def tile_keys(ctx) -> int:
@@ -510,7 +521,8 @@ def run_part_alone(runtime, plan, ctx, h: torch.Tensor, hidden_size: int, page_s
     from .. import kernels
     step = RunnerStep(ntok=T, nreq=ctx.nreq, n_want=0, context=ctx.context, tokens=ctx.tokens.data_ptr(),
                       positions=ctx.positions.data_ptr(), row_req=ctx.row_req.data_ptr(), req_start=ctx.req_start.data_ptr(),
-                      req_pos=ctx.req_pos.data_ptr(), want_rows=None, slot_ids=ctx.slot_ids.data_ptr(), tile_keys=tile_keys(ctx))
+                      req_pos=ctx.req_pos.data_ptr(), want_rows=None, slot_ids=ctx.slot_ids.data_ptr())
+    host = set_host_lengths(step, ctx)          # noqa: F841 (alive until the step is launched)
     for g, table in enumerate(ctx.block_tables):
         step.block_tables[g] = table.data_ptr()
     for name, index in program.lists.items():

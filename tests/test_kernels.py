@@ -387,7 +387,7 @@ def test_rope_and_cache_write(K, dtype, nh, nkvh, dh, page, interleaved):
     assert float(kp[0].abs().max()) == 0.0              # the null page was not written
 
 
-def _attention_case(K, dtype, nh, nkvh, dh, page, window, lens, queries, plant=None, seed=0, impl="rows", splits=1, junk=7.0):
+def _attention_case(K, dtype, nh, nkvh, dh, page, window, lens, queries, plant=None, seed=0, impl="rows", splits=1, junk=7.0, tile_keys=0):
     """lens: cached length of each request; queries: per request the positions that are rows.
     impl: "rows" (one warp per row and head), "decode" (split keys), "prefill" (tensor cores; the
     positions of a request must be consecutive)."""
@@ -432,7 +432,7 @@ def _attention_case(K, dtype, nh, nkvh, dh, page, window, lens, queries, plant=N
         i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
         if impl == "tcgen05":
             K.attention_tcgen05(qd, kd, vd, out, i32(tiles).flatten(), len(tiles), T, i32(starts), i32(req_pos), bt, nh,
-                                scale, window or 0)
+                                scale, window or 0, tile_keys=tile_keys)
             K.check_gemm_status(DEV)
         else:
             K.attention_prefill(qd, kd, vd, out, i32(tiles).flatten(), len(tiles), i32(starts), i32(req_pos), bt, nh,
@@ -526,13 +526,14 @@ def test_attention_prefill_kernel_on_tcgen05(K, nh, nkvh, dh, page, window):
     _close(got, want, torch.bfloat16, scale=2.0)
 
 
+@pytest.mark.parametrize("tile_keys", [64, 128])
 @pytest.mark.parametrize("page,window", [(8, None), (64, None), (128, None), (16, 70), (32, 64)])
-def test_attention_tcgen05_tiles_of_64_keys(K, page, window):
-    """Heads of 128 walk 64 keys at a time where a page fits into that (pages of 128: 128 keys): prompts and portions that end at, one
-    before and one past the edges of key tiles and of query tiles; the operands and the bound of the cases above."""
+def test_attention_tcgen05_tiles_of_64_keys(K, page, window, tile_keys):
+    """Heads of 128 walk 128 keys at a time, or 64 where a page fits into that (pages of 128: always 128): prompts and portions that end
+    at, one before and one past the edges of key tiles and of query tiles; the operands and the bound of the cases above."""
     lens = [64, 65, 127, 193, 321]
     queries = [list(range(0, 64)), list(range(0, 65)), list(range(62, 127)), list(range(0, 193)), list(range(192, 321))]
-    got, want, _ = _attention_case(K, torch.bfloat16, 6, 2, 128, page, window, lens, queries, seed=page, impl="tcgen05")
+    got, want, _ = _attention_case(K, torch.bfloat16, 6, 2, 128, page, window, lens, queries, seed=page, impl="tcgen05", tile_keys=tile_keys)
     _close(got, want, torch.bfloat16, scale=2.0)
 
 

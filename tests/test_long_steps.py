@@ -116,8 +116,8 @@ def test_every_form_of_latent_attention_over_heads_and_who_goes_which_way(tmp_pa
         assert torch.equal(one, other) == (not over_heads), step
 
 
-@pytest.mark.parametrize("dh,rotated", [(64, False), (64, True), (128, False), (128, True)])
-def test_weights_of_an_attention_over_laid_heads_are_float32_accurate(K, dh, rotated):
+@pytest.mark.parametrize("dh,rotated,tile_keys", [(64, False, 128), (64, True, 128), (128, False, 64), (128, False, 128), (128, True, 128)])
+def test_weights_of_an_attention_over_laid_heads_are_float32_accurate(K, dh, rotated, tile_keys):
     """Each instance, with values that pick single weights: row t has scores -a_t b_j (exact in float32) over 64 keys and far lower ones
     over the rest, and column j of its output is key j's weight, rounded to bfloat16 as an operand, over the float32 sum of the weights,
     rounded once more.  Scores in [-8, 0]: the exponent's factor and product err by 8 x 1.5 x 2^-24, the special-function unit by 2^-22, the sum
@@ -140,7 +140,7 @@ def test_weights_of_an_attention_over_laid_heads_are_float32_accurate(K, dh, rot
     i, p = K._c_int, K._ptr
     K._check("attention_tcgen05", K._build.load("attention_tcgen05").jk_attention_laid_tcgen05(
         p(q), p(q_rot if rotated else None), i(72), i(8), p(kv), p(k_rot if rotated else None), K._c_ll(C), p(out), p(tiles), i(n), i(T), p(start), p(pos),
-        i(1), i(dh), K._c_float(1.0), i(0), p(status), p(None), p(None), i(0), i(0), K._stream()))
+        i(1), i(dh), K._c_float(1.0), i(0), p(status), p(None), p(None), i(0), i(0), i(tile_keys), K._stream()))
     K.check_gemm_status(dev)
     e = torch.exp(-a.double()[:, None] * b.double())
     want = e.to(torch.bfloat16).double() / e.sum(1, keepdim=True)
