@@ -24,6 +24,7 @@
 // accumulate in float32.  A step's rows are laid out request after request (req_start), continue at req_pos, and keep
 // their state in slot slot_ids[request]; a whole prompt, a portion and a single token are one case.
 #include "common.cuh"
+#include "host_rules.h"
 
 #include <algorithm>
 #include <cstdlib>
@@ -1534,9 +1535,7 @@ JK_EXPORT int jk_causal_conv(const float *u, int ld, int off, int C, const float
     const uintptr_t vectors = (uintptr_t)u | (uintptr_t)bias | (uintptr_t)in_bias | (uintptr_t)tail | (uintptr_t)y32 | (uintptr_t)yT;
     const size_t total = (size_t)T * C;
     const int blocks = (int)std::min<size_t>((total + 255) / 256, 148 * 16);
-    // The line: eight rows one after the other are a chain that few rows do not hide (4,096 channels, four taps, an element a thread -> rows):
-    // 32 rows 11 -> 15 us, 64 13 -> 15, 256 21 -> 15, 2,048 97 -> 42.
-    const bool by_rows = T >= 128 && J >= 2 && J <= 4 && ((C | ld | off) & 3) == 0 && (vectors & 15) == 0 && (T + CV_ROWS - 1) / CV_ROWS <= 65535;
+    const bool by_rows = jk::conv_walks_rows(T, nreq, C) && J >= 2 && J <= 4 && ((C | ld | off) & 3) == 0 && (vectors & 15) == 0 && (T + CV_ROWS - 1) / CV_ROWS <= 65535;
 #define LAUNCH_J(TT, JJ) jk_launch(causal_conv_rows_kernel<TT, JJ>, dim3((C / 4 + CV_THREADS - 1) / CV_THREADS, (T + CV_ROWS - 1) / CV_ROWS), dim3(CV_THREADS), 0, stream, a, T)
 #define LAUNCH(TT)                                                                                 \
     if (!by_rows) jk_launch(causal_conv_kernel<TT>, dim3(blocks), dim3(256), 0, stream, a, T);     \

@@ -276,6 +276,15 @@ inline bool attention_tcgen05_takes(int dh, int page_size, int dv = 0) {
     return size && (page_size == 8 || page_size == 16 || page_size == 32 || page_size == 64 || page_size == 128);
 }
 
+// Whether a causal convolution over `rows` rows of `nreq` requests walks eight rows a thread (csrc/blocks.cu) instead of making an element
+// a thread: a walk is a chain that takes a large launch to hide, the more so where every row is a request of its own and reads and
+// moves its own tail.  B200, element a thread -> rows (us): 64 channels, 128 to 2,048 rows 9 -> 13; 512 channels, 512 rows 11 to 13 -> 13,
+// 2,048 17 to 20 -> 15; 4,096 channels, 128 rows 13 to 15 -> 13 to 15, 256 17 to 20 -> 15, 2,048 75 to 95 -> 36 to 42; requests of one row: 4,096
+// channels, 128 of them 12 to 15 -> 16 to 19, 256 18 to 21 -> 19 to 23, 8,192 channels, 256 of them 27 to 36 -> 21 to 26.
+inline bool conv_walks_rows(long long rows, long long nreq, long long channels) {
+    return rows >= 128 && rows * channels >= (rows < 2 * nreq ? 1LL << 21 : 1LL << 20);
+}
+
 // Whether a latent attention over `rows` query rows of `nreq` requests makes the heads' keys and values from the latent rows
 // (one product per cached position) instead of running over the latent rows: heads of 64 or 128 for keys and values alike, a
 // rotated part of 64 or none, whole vectors; `keys`: positions of all requests, or 0 when a request brings few rows.  The line, 16

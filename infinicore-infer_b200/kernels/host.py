@@ -135,6 +135,12 @@ def context_bucket(longest: int, max_positions: int) -> int:
     return lib().jk_context_bucket(longest, max_positions)
 
 
+def conv_walks_rows(rows: int, nreq: int, channels: int) -> bool:
+    """Whether a causal convolution (two to four taps, whole vectors) walks eight rows a thread."""
+    c = ctypes.c_longlong
+    return bool(lib().jk_conv_walks_rows(c(rows), c(nreq), c(channels)))
+
+
 def latent_heads_fit(dn: int, dr: int, dv: int, rank: int) -> bool:
     """Whether a latent attention of these sizes can run over heads made for the step."""
     return bool(lib().jk_latent_heads_fit(dn, dr, dv, rank))

@@ -30,3 +30,16 @@ def test_keys_a_tile_of_the_prefill_attention(heads, requests, window, keys):
     for n, _ in requests:
         start.append(start[-1] + n)
     assert host.attention_tile_keys(heads, start, [p for _, p in requests], window) == keys
+
+
+@pytest.mark.parametrize("rows,requests,channels,walks", [
+    # microseconds, two and four taps: an element a thread, eight rows a thread
+    (128, 1, 64, False), (2048, 1, 64, False),          # 9 and 11, 13
+    (128, 128, 64, False), (256, 256, 512, False),      # 8, 16 and 17
+    (512, 1, 512, False), (640, 16, 512, False),        # 11 and 13, 13; 13, 13 and 15
+    (256, 1, 2048, False), (128, 128, 4096, False), (256, 256, 4096, False),    # 13 and 15, 15; 12 and 15, 16 and 19; 18 and 21, 19 and 23
+    (2048, 1, 512, True), (512, 1, 2048, True),         # 17 and 20, 15 both
+    (640, 16, 2048, True), (256, 1, 4096, True),        # 20 and 24, 15 and 17; 17 and 20, 15
+    (256, 256, 8192, True), (2048, 1, 4096, True)])     # 27 and 36, 21 and 26; 75 and 95, 36 and 42
+def test_rows_a_thread_of_the_causal_convolution(rows, requests, channels, walks):
+    assert host.conv_walks_rows(rows, requests, channels) == walks

@@ -9,6 +9,7 @@ import pytest
 import torch
 
 from conftest import random_tokens
+from infinicore_infer_b200.kernels.host import conv_walks_rows
 import plain_vunelix as plain
 
 pytestmark = pytest.mark.gpu
@@ -326,12 +327,13 @@ def test_projected_decay_recurrence_as_products_within_pieces(K, dk, dv, rank, f
     assert torch.equal(got[0][1][0], first[0].double()) and not torch.equal(got[0][0], got[1][0])
 
 
-@pytest.mark.parametrize("taps,C,lens", [(4, 516, [128]), (3, 64, [7, 1, 2, 1, 140]), (2, 128, [1, 129]), (4, 520, [9, 3, 1, 1, 130])])
+@pytest.mark.parametrize("taps,C,lens", [(4, 8196, [128]), (3, 7044, [7, 1, 2, 1, 140]), (2, 8192, [1, 129]), (4, 7304, [9, 3, 1, 1, 130]), (4, 8196, [1] * 257)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_causal_convolution_of_many_rows(K, taps, C, lens, dtype):
     """Requests shorter than the taps, of one row and across the blocks' eight rows; the same rows laid so that vectors of four do not
     fit take a thread an element.  Both add the taps in the same order: the same bits."""
     dev, g, T, n = torch.device("cuda:0"), torch.Generator().manual_seed(C), sum(lens), len(lens)
+    assert conv_walks_rows(T, n, C)
     u, w, b, ib = (torch.randn(*s, generator=g) for s in ((T, C), (C, taps), (C,), (C,)))
     tail = torch.randn(n + 1, taps - 1, C, generator=g)
     starts, slots = torch.tensor([0] + lens).cumsum(0).to(torch.int32), torch.arange(n, 0, -1, dtype=torch.int32)
