@@ -2383,13 +2383,9 @@ JK_EXPORT int jk_routed_experts(const void *h, const float *router, const void *
     const int per16 = dtype == JK_F32 ? 4 : 8;
     const bool stream_rows = pairs <= 64 && D % per16 == 0 && ff % per16 == 0 && (uintptr_t)w_gate_up % 16 == 0 && (uintptr_t)w_down % 16 == 0 &&
                              (size_t)ER_ROWS * std::max(D, ff) * 4 <= 160 * 1024;
-    // Many rows an expert: tiles of 128 entries on tcgen05 (bfloat16, whole vectors, a status word for their waits).  The
-    // weights' bytes bound both kinds of tiles at few entries an expert (8 experts of 1,408, width 2,048, two a row; tiles of 64 on
-    // mma.sync -> of 128 here): 48 rows 102 -> 72 us, 128 119 -> 74, 512 172 -> 84, 2,048 408 -> 136; 32 experts, 64 rows 218 -> 137;
-    // 64 experts, 128 rows 367 -> 218.  A tile that holds few entries costs its weights' bytes in either form.  Below two entries an expert
-    // nothing is measured.
+    // Many rows an expert: tiles of 128 entries on tcgen05 (bfloat16, whole vectors, a status word for their waits).
     g_expert_launches = 0;
-    const bool tc = dtype == JK_BF16 && !stream_rows && status != nullptr && E <= ET_MAX_EXPERTS && D % 8 == 0 && ff % 8 == 0 && pairs >= 2LL * E &&
+    const bool tc = dtype == JK_BF16 && !stream_rows && status != nullptr && E <= ET_MAX_EXPERTS && D % 8 == 0 && ff % 8 == 0 && jk::experts_take_tiles(pairs, E, D, ff) &&
                     (((uintptr_t)h | (uintptr_t)w_gate_up | (uintptr_t)w_down | (uintptr_t)act | (uintptr_t)y) & 15) == 0;
     if (tc) {
         // the entries' rows lie in y's place until the second product writes there

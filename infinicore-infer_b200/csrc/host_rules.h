@@ -285,6 +285,17 @@ inline bool conv_walks_rows(long long rows, long long nreq, long long channels) 
     return rows >= 128 && rows * channels >= (rows < 2 * nreq ? 1LL << 21 : 1LL << 20);
 }
 
+// Whether the routed experts' products run in tiles of 128 entries on tcgen05 (csrc/experts_tcgen05.cuh) rather than of 64 on mma.sync:
+// from two entries an expert on, and for products large enough to pay for the gather and the tensor memory's setup, about 5 us a layer:
+// by themselves, by all experts' weights or by the multiply-adds of many entries.  B200, whole layers, tiles of 64 -> of 128 (us):
+// 64 x 64 to 512 x 128, up to 32 experts, 64 to 512 rows 26 to 48 -> 31 to 49; 512 x 512, 4 experts, 512 rows 48 -> 49 to 52, 16 experts, 64 rows 48 -> 43,
+// 8 experts, 2,048 rows 87 -> 61; 1,024 x 256, 1 to 8 experts 44 to 53 -> 43 to 51; 512 x 128, 64 experts, 64 rows 54 -> 46; 2,048 x 1,408, 8 experts: 48
+// rows 102 -> 72, 128 119 -> 77, 512 172 -> 88, 2,048 408 -> 141, 64 experts, 128 rows 367 -> 223.  Below two entries an expert nothing is measured.
+inline bool experts_take_tiles(long long entries, long long experts, long long width, long long ff) {
+    const long long one = width * ff;
+    return entries >= 2 * experts && ((width >= 1024 && one >= 1LL << 18) || experts * one >= 1LL << 22 || (entries >= 2048 && entries * one >= 1LL << 28));
+}
+
 // Whether a latent attention over `rows` query rows of `nreq` requests makes the heads' keys and values from the latent rows
 // (one product per cached position) instead of running over the latent rows: heads of 64 or 128 for keys and values alike, a
 // rotated part of 64 or none, whole vectors; `keys`: positions of all requests, or 0 when a request brings few rows.  The line, 16

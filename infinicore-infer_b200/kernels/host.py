@@ -141,6 +141,12 @@ def conv_walks_rows(rows: int, nreq: int, channels: int) -> bool:
     return bool(lib().jk_conv_walks_rows(c(rows), c(nreq), c(channels)))
 
 
+def experts_take_tiles(entries: int, experts: int, width: int, ff: int) -> bool:
+    """Whether routed experts' products (bfloat16, more than 64 entries) run in tiles of 128 entries."""
+    c = ctypes.c_longlong
+    return bool(lib().jk_experts_take_tiles(c(entries), c(experts), c(width), c(ff)))
+
+
 def latent_heads_fit(dn: int, dr: int, dv: int, rank: int) -> bool:
     """Whether a latent attention of these sizes can run over heads made for the step."""
     return bool(lib().jk_latent_heads_fit(dn, dr, dv, rank))

@@ -43,3 +43,18 @@ def test_keys_a_tile_of_the_prefill_attention(heads, requests, window, keys):
     (256, 256, 8192, True), (2048, 1, 4096, True)])     # 27 and 36, 21 and 26; 75 and 95, 36 and 42
 def test_rows_a_thread_of_the_causal_convolution(rows, requests, channels, walks):
     assert host.conv_walks_rows(rows, requests, channels) == walks
+
+
+@pytest.mark.parametrize("rows,experts,top,width,ff,tiles", [
+    # microseconds of a layer in tiles of 64 entries and of 128
+    (65, 1, 1, 64, 64, False), (512, 4, 2, 64, 64, False), (64, 32, 2, 64, 64, False),      # 26, 31; 30, 37; 30, 33
+    (33, 2, 2, 256, 64, False), (512, 4, 2, 256, 256, False), (2048, 8, 2, 256, 64, False),     # 30, 33; 36, 49; 42, 47
+    (512, 4, 2, 128, 512, False), (64, 4, 2, 512, 128, False), (65, 1, 1, 512, 512, False),     # 38, 43; 34, 39; 38, 41
+    (512, 4, 2, 512, 512, False),           # 48, 49 to 52
+    (128, 128, 1, 2048, 1408, False),       # one entry an expert: not measured
+    (2048, 8, 2, 512, 512, True), (64, 32, 2, 512, 512, True), (64, 16, 2, 512, 512, True),     # 87, 61; 60, 49; 48, 43
+    (2048, 8, 2, 128, 512, True), (64, 64, 2, 512, 128, True),      # 59, 49; 54, 46
+    (65, 1, 1, 1024, 256, True), (33, 2, 2, 1024, 1024, True), (64, 4, 2, 2048, 512, True),     # 44, 43; 56, 47; 69, 54
+    (48, 8, 2, 2048, 1408, True), (128, 64, 2, 2048, 1408, True)])      # 102, 72; 367, 223
+def test_tiles_of_the_routed_experts(rows, experts, top, width, ff, tiles):
+    assert host.experts_take_tiles(rows * top, experts, width, ff) == tiles

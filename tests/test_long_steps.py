@@ -9,7 +9,7 @@ import pytest
 import torch
 
 from conftest import random_tokens
-from infinicore_infer_b200.kernels.host import conv_walks_rows
+from infinicore_infer_b200.kernels.host import conv_walks_rows, experts_take_tiles
 import plain_vunelix as plain
 
 pytestmark = pytest.mark.gpu
@@ -150,13 +150,14 @@ def test_weights_of_an_attention_over_laid_heads_are_float32_accurate(K, dh, rot
     assert (got != want.to(torch.bfloat16).double()).double().mean() <= 2.0 ** -10
 
 
-@pytest.mark.parametrize("T,d,ff,experts,top,act", [(128, 64, 128, 1, 1, "silu"), (129, 72, 136, 2, 2, "swish_clamp"), (300, 512, 264, 5, 2, "silu"),
-                                                    (600, 264, 8, 3, 1, "silu")])
+@pytest.mark.parametrize("T,d,ff,experts,top,act", [(128, 1024, 256, 1, 1, "silu"), (129, 1032, 264, 2, 2, "swish_clamp"), (300, 1096, 264, 5, 2, "silu"),
+                                                    (600, 32776, 8, 3, 1, "silu")])
 def test_expert_products_in_tiles_of_entries(K, T, d, ff, experts, top, act):
     """Entries that fill tiles of 128 exactly, by one more and by part, an expert without rows (the router's bias shuns it), widths
     that end inside a tile and inside a step of K.  A product's operands are exact, its sums float32, the inner activations
     rounded to bfloat16: 2^-9 of each, averaged over ff of them."""
     dev, g = torch.device("cuda:0"), torch.Generator().manual_seed(T + d)
+    assert experts_take_tiles(T * top, experts, d, ff)
     h = torch.randn(T, d, generator=g).to(torch.bfloat16)
     w_gu, w_dn = (torch.randn(experts * n, k, generator=g).div(k ** 0.5).to(torch.bfloat16) for n, k in ((2 * ff, d), (d, ff)))
     router = torch.randn(experts, d, generator=g)
@@ -190,11 +191,12 @@ def test_expert_products_in_tiles_of_entries(K, T, d, ff, experts, top, act):
 @pytest.mark.parametrize("act", ["none", "silu", "gelu_tanh", "sigmoid", "relu", "swish_clamp"])
 def test_expert_products_of_groups_of_rows_that_are_part_full(K, act):
     """Experts with 1, 31, 33, 63 and 142 entries: the groups of 32 rows that a warp of the products finishes are full, part full and
-    empty, over 200 and 264 features, so that a warp comes back for more columns after a pass in which some of its rows had nothing
+    empty, over 208 and 1,288 features, so that a warp comes back for more columns after a pass in which some of its rows had nothing
     to store.  Every activation; scores that multiply the units' inputs.  The bound of the test above."""
     dev, g = torch.device("cuda:0"), torch.Generator().manual_seed(len(act))
-    counts, d, ff, limit = [1, 31, 33, 63, 142], 264, 200, 1.5
+    counts, d, ff, limit = [1, 31, 33, 63, 142], 1288, 208, 1.5
     T, E = sum(counts), len(counts)
+    assert experts_take_tiles(T, E, d, ff)
     owner = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(T, generator=g)]
     h = torch.randn(T, d, generator=g)
     h[:, :E] = 20.0 * torch.nn.functional.one_hot(owner, E)         # the router reads the owner
