@@ -71,6 +71,9 @@ JK_HOST_EXPORT int jk_experts_take_tiles(long long entries, long long experts, l
     return jk::experts_take_tiles(entries, experts, width, ff) ? 1 : 0;
 }
 JK_HOST_EXPORT int jk_latent_heads_fit(int dn, int dr, int dv, int R) { return jk::latent_heads_fit(dn, dr, dv, R) ? 1 : 0; }
+JK_HOST_EXPORT int jk_latent_takes_heads(int rows, int nreq, long long keys, int window, int dn, int dr, int dv, int R) {
+    return jk::latent_takes_heads(rows, nreq, keys, window, dn, dr, dv, R) ? 1 : 0;
+}
 JK_HOST_EXPORT int jk_latent_heads_rows() { return jk::LATENT_HEADS_ROWS; }
 JK_HOST_EXPORT int jk_attention_tcgen05_takes(int dh, int page_size, int dv) { return jk::attention_tcgen05_takes(dh, page_size, dv) ? 1 : 0; }
 JK_HOST_EXPORT int jk_context_bucket(int longest, int max_positions) { return jk::context_bucket(longest, max_positions); }

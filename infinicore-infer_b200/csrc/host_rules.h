@@ -298,17 +298,21 @@ inline bool experts_take_tiles(long long entries, long long experts, long long w
 
 // Whether a latent attention over `rows` query rows of `nreq` requests makes the heads' keys and values from the latent rows
 // (one product per cached position) instead of running over the latent rows: heads of 64 or 128 for keys and values alike, a
-// rotated part of 64 or none, whole vectors; `keys`: positions of all requests, or 0 when a request brings few rows.  The line, 16
-// rows for each position within reach, lies where the product per position is shared by enough rows (B200, 16 heads of 128 + 64 and 128
-// over a latent of 512; over the latent rows -> over heads): 4 requests of 17 rows after 0 positions 37 -> 25 us, after 512
-// 102 -> 41; 64 rows after 2,048 297 -> 64; 2,048 rows after 0 887 -> 74.  Below it the way over heads costs 24 us at the least, while
-// 8 requests of one row over the latent rows take 17.
+// rotated part of 64 or none, whole vectors; `keys`: positions of all requests, or 0 when one of them brings few rows (a step goes one way
+// as a whole).  With `reach` the positions that a row sees of a request's on average, two lines:
+//   rows x reach >= 16 keys (without a window: 16 rows a request on average), so that enough rows share the product per position;
+//   a latent of 256 or reach x (latent + rotated part) >= 12,288: the way over heads costs 24 us at the least, over short contexts of
+//   small latents the other one less.
+// B200, over the latent rows -> over heads (us): 16 heads of 128 + 64, latent 512: 4 requests of 17 rows after 500 101 -> 42, one of 48 rows
+// after 2,000 288 -> 60, 256 rows after 0 73 -> 30, 2,048 after 0 887 -> 75; 2 of 16 rows after 0 36 -> 28; 2 heads of 64, latent 64: 32 rows after 0
+// 17 -> 24, 16 requests of 20 after 100 26 -> 30, 256 rows after 0 34 -> 24, 32 after 500 52 -> 28; 4 heads of 64 + 64, latent 160: 32 rows after 0 22 -> 24,
+// 16 requests of 20 after 100 34 -> 30; 16 heads of 64, latent 256: 32 rows after 0 24 -> 24.  8 requests of one row over latents of 512 take 17.
 inline bool latent_heads_fit(int dn, int dr, int dv, int R) { return dn == dv && (dn == 64 || dn == 128) && (dr == 0 || dr == 64) && R % 8 == 0 && R >= 64; }
 constexpr int LATENT_HEADS_ROWS = 32;       // the fewest rows of a step that goes this way; an engine of smaller steps has neither the room nor the modules
 inline bool latent_takes_heads(int rows, int nreq, long long keys, int window, int dn, int dr, int dv, int R) {
     if (keys <= 0 || rows < LATENT_HEADS_ROWS || nreq <= 0 || !latent_heads_fit(dn, dr, dv, R)) return false;
     const long long reach = window > 0 ? std::min<long long>(window, keys / nreq) : keys / nreq;
-    return rows * reach >= 16LL * keys;
+    return rows * reach >= 16LL * keys && (R >= 256 || reach * (R + dr) >= 12288);
 }
 // The positions that room is kept for in an engine of steps of up to `rows` rows: four times as many as a step may have rows (prompts, and
 // portions of longer ones up to there; steps that see more run over the latent rows), but no more than its requests can have: the

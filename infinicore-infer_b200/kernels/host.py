@@ -152,6 +152,11 @@ def latent_heads_fit(dn: int, dr: int, dv: int, rank: int) -> bool:
     return bool(lib().jk_latent_heads_fit(dn, dr, dv, rank))
 
 
+def latent_takes_heads(rows: int, nreq: int, keys: int, window: int, dn: int, dr: int, dv: int, rank: int) -> bool:
+    """Whether a step's latent attention of these sizes runs over heads made for it; ``keys``: positions of all requests."""
+    return bool(lib().jk_latent_takes_heads(rows, nreq, ctypes.c_longlong(keys), window, dn, dr, dv, rank))
+
+
 def latent_heads_rows() -> int:
     """The fewest rows of a step whose latent attentions can run over heads made for it."""
     return lib().jk_latent_heads_rows()

@@ -58,3 +58,15 @@ def test_rows_a_thread_of_the_causal_convolution(rows, requests, channels, walks
     (48, 8, 2, 2048, 1408, True), (128, 64, 2, 2048, 1408, True)])      # 102, 72; 367, 223
 def test_tiles_of_the_routed_experts(rows, experts, top, width, ff, tiles):
     assert host.experts_take_tiles(rows * top, experts, width, ff) == tiles
+
+
+@pytest.mark.parametrize("dim,rot,rank,requests,window,heads", [
+    # (rows, position of the first) of every request; microseconds over the latent rows and over heads made for the step
+    (64, 0, 64, [(32, 0)], 0, False), (64, 0, 64, [(16, 0)] * 2, 0, False), (64, 0, 64, [(20, 100)] * 16, 0, False),    # 17, 24 twice; 26, 30
+    (64, 0, 64, [(100, 100)] * 4, 64, False), (64, 64, 160, [(32, 0)], 0, False), (64, 64, 160, [(16, 0)] * 2, 0, False),   # 24, 28; 22, 24 twice
+    (128, 64, 512, [(1, 500)] * 8, 0, False), (128, 64, 512, [(31, 0)], 0, False),
+    (64, 0, 64, [(32, 500)], 0, True), (64, 0, 64, [(256, 0)], 0, True), (64, 64, 160, [(20, 100)] * 16, 0, True),      # 52, 28; 34, 24; 34, 30
+    (64, 64, 160, [(100, 100)] * 4, 64, True), (128, 64, 512, [(16, 0)] * 2, 0, True), (128, 64, 512, [(2048, 0)], 0, True)])   # 30, 28; 36, 28; 887, 75
+def test_way_of_a_latent_attention(dim, rot, rank, requests, window, heads):
+    rows, keys = sum(n for n, _ in requests), sum(n + p for n, p in requests)
+    assert host.latent_takes_heads(rows, len(requests), keys, window, dim, rot, dim, rank) == heads

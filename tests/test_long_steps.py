@@ -69,7 +69,7 @@ def _one_layer(family, mixer):
 
 
 @pytest.mark.parametrize("family,heads,dim,rot,rank,q_rank,window", [
-    ("fapenex", 2, 128, 0, 64, 40, 100), ("fapenex", 3, 64, 0, 72, 40, 70), ("fapenex", 2, 128, 0, 64, 40, 600),       # queries through a latent, a window
+    ("fapenex", 2, 128, 0, 128, 40, 100), ("fapenex", 3, 64, 0, 136, 40, 100), ("fapenex", 2, 128, 0, 128, 40, 600),       # queries through a latent, a window
     ("fupapel", 2, 128, 64, 72, 48, 0), ("fupapel", 3, 64, 64, 64, 40, 0),      # and rotated parts, learned sinks, a gate per head
     ("vunelix", 2, 128, 64, 64, 0, 0)])                                         # neither; a gate per element
 def test_every_form_of_latent_attention_over_heads_and_who_goes_which_way(tmp_path, family, heads, dim, rot, rank, q_rank, window):
