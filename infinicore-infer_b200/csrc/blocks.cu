@@ -1725,7 +1725,7 @@ __global__ void __launch_bounds__(SS_THREADS) selective_scan_kernel(ScanArgs a) 
 // What bounds it: instructions (sixteen states: about 170 a row and channel, the exponentials half of them).  Eight lanes a
 // channel walking a prompt from end to end waited 600 cycles a row for one another and for the next rows.  B200, 2,048 rows,
 // 4,096 channels, 16 states, with the product of the step sizes: 589 -> 360 us.
-constexpr int SP_THREADS = 128, SP_ROWS = 128, SP_AHEAD = 4;
+constexpr int SP_THREADS = 128, SP_ROWS = jk::SELECTIVE_PIECE, SP_AHEAD = 4;
 struct PieceArgs {
     float *ends, *sums;         // [pieces, N, E] end states, [pieces, E] sums of step sizes
     int nreq;
@@ -1872,10 +1872,8 @@ JK_EXPORT int jk_selective_scan(const float *x, const float *low, int ld_low, in
         JK_CHECK_LAUNCH("scan_steps");
     }
     ScanArgs a{x, low, ld_low, K, N, E, z, ld_z, Wdt, bdt, A, Dskip, state, req_start, slot_ids, out, ahead ? dt_buf : nullptr, ld_dt};
-    // The line: the pieces walk every row twice but side by side.  One request, 4,096 channels, 16 states (step sizes included; a walk from end
-    // to end -> pieces): 128 rows 50 -> 69 us, 256 81 -> 114, 512 148 -> 148, 2,048 589 -> 360.
     const long long need = jk_selective_scan_scratch_floats(T, E, N);
-    if (ahead && N <= 32 && T >= 768LL * nreq && (need == 0 || (scratch != nullptr && scratch_floats >= need)) && T / SP_ROWS + nreq <= 65535) {
+    if (ahead && jk::selective_scan_cuts(T, nreq, E, N) && (need == 0 || (scratch != nullptr && scratch_floats >= need)) && T / SP_ROWS + nreq <= 65535) {
         const PieceArgs p{scratch, scratch + need / (N + 1) * N, nreq};
         const dim3 pieces((E + SP_THREADS - 1) / SP_THREADS, T / SP_ROWS + nreq);
 #define LAUNCH_S(TT, NS)                                                                                              \

@@ -67,6 +67,9 @@ JK_HOST_EXPORT long long jk_decode_scratch_floats(int nrows, int nh, int dh, int
 }
 JK_HOST_EXPORT int jk_decode_keys_hint(int context, int window) { return jk::decode_keys_hint(context, window); }
 JK_HOST_EXPORT int jk_conv_walks_rows(long long rows, long long nreq, long long channels) { return jk::conv_walks_rows(rows, nreq, channels) ? 1 : 0; }
+JK_HOST_EXPORT int jk_selective_scan_cuts(long long rows, long long nreq, long long channels, long long states) {
+    return jk::selective_scan_cuts(rows, nreq, channels, states) ? 1 : 0;
+}
 JK_HOST_EXPORT int jk_experts_take_tiles(long long entries, long long experts, long long width, long long ff) {
     return jk::experts_take_tiles(entries, experts, width, ff) ? 1 : 0;
 }

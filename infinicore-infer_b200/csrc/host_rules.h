@@ -285,6 +285,19 @@ inline bool conv_walks_rows(long long rows, long long nreq, long long channels) 
     return rows >= 128 && rows * channels >= (rows < 2 * nreq ? 1LL << 21 : 1LL << 20);
 }
 
+// Whether a selective scan over `rows` rows of `nreq` requests runs over pieces of SELECTIVE_PIECE rows side by side (csrc/blocks.cu) rather
+// than from end to end.  The pieces make every row twice, so they pay where the walks leave the chip idle: long requests, and with more than
+// 16 states, whose pieces keep too much to hide anything, few channels of them all.  The rule knows the mean length only: a long prompt beside
+// many decoding rows walks.  B200, step sizes included, walk -> pieces (us): 16 states, 4,096 channels, one request: 512 rows 148 -> 148,
+// 2,048 589 -> 360; 64 channels, 8 requests of 768 104 -> 113, 4 of 1,024 132 -> 113; 512 channels, 2 of 768 127 -> 133, one of 1,000 149 -> 111.  32
+// states, 512 channels: one of 768 135 -> 178, 4 of 1,024 279 -> 302, one of 2,048 548 -> 276, 4 of 2,048 647 -> 374; 4,096 channels: 2 of 2,048
+// 989 -> 768, 4 of 2,048 1,161 -> 1,357.
+constexpr int SELECTIVE_PIECE = 128;
+inline bool selective_scan_cuts(long long rows, long long nreq, long long channels, long long states) {
+    if (states > 16) return states <= 32 && rows >= 1280 * nreq && nreq * channels <= 8192;
+    return rows >= (channels < 1024 ? 896 : 768) * nreq;
+}
+
 // Whether the routed experts' products run in tiles of 128 entries on tcgen05 (csrc/experts_tcgen05.cuh) rather than of 64 on mma.sync:
 // from two entries an expert on, and for products large enough to pay for the gather and the tensor memory's setup, about 5 us a layer:
 // by themselves, by all experts' weights or by the multiply-adds of many entries.  B200, whole layers, tiles of 64 -> of 128 (us):

@@ -725,7 +725,7 @@ int run_selective_scan(Run &r, const RunnerOp &op) {
     RUN(blocks, g_fns.selective_scan((const float *)x, (const float *)low, ld_low, op.rank, op.k, op.n, (const float *)u + op.g_off, op.ld,
                                      op.w2, op.b2, op.decay, op.vec, op.state, r.st.req_start, r.st.slot_ids, r.st.nreq, out,
                                      r.env.dtype, (float *)u + op.q_off, op.ld, T, (float *)scratch, floats, r.stream));
-    if (floats > 0 && T >= 768LL * r.st.nreq) ++g_launches;
+    if (floats > 0 && jk::selective_scan_cuts(T, r.st.nreq, op.n, op.k)) ++g_launches;      // the pieces' end states
     ++g_launches;       // the step sizes' product
     return JK_OK;
 }

@@ -135,6 +135,12 @@ def context_bucket(longest: int, max_positions: int) -> int:
     return lib().jk_context_bucket(longest, max_positions)
 
 
+def selective_scan_cuts(rows: int, nreq: int, channels: int, states: int) -> bool:
+    """Whether a selective scan runs over pieces of its requests side by side."""
+    c = ctypes.c_longlong
+    return bool(lib().jk_selective_scan_cuts(c(rows), c(nreq), c(channels), c(states)))
+
+
 def conv_walks_rows(rows: int, nreq: int, channels: int) -> bool:
     """Whether a causal convolution (two to four taps, whole vectors) walks eight rows a thread."""
     c = ctypes.c_longlong

@@ -45,6 +45,17 @@ def test_rows_a_thread_of_the_causal_convolution(rows, requests, channels, walks
     assert host.conv_walks_rows(rows, requests, channels) == walks
 
 
+@pytest.mark.parametrize("lens,channels,states,cuts", [
+    # microseconds end to end and over pieces
+    ([512], 4096, 16, False), ([768], 4096, 16, True), ([2048], 4096, 16, True),        # 148 twice; 589, 360
+    ([768] * 8, 64, 16, False), ([768] * 2, 512, 16, False), ([1000], 512, 16, True), ([1024] * 4, 64, 16, True),      # 104, 113; 127, 133; 149, 111; 132, 113
+    ([896], 130, 5, True), ([1921, 1, 769], 130, 16, True), ([895], 130, 16, False), ([2500, 65], 130, 20, True),
+    ([768], 512, 32, False), ([1024] * 4, 512, 32, False), ([2048], 512, 32, True), ([2048] * 4, 512, 32, True),     # 135, 178; 279, 302; 548, 276; 647, 374
+    ([2048] * 2, 4096, 32, True), ([2048] * 4, 4096, 32, False), ([4096], 64, 33, False)])      # 989, 768; 1,161, 1,357; more states than a thread keeps
+def test_pieces_of_the_selective_scan(lens, channels, states, cuts):
+    assert host.selective_scan_cuts(sum(lens), len(lens), channels, states) == cuts
+
+
 @pytest.mark.parametrize("rows,experts,top,width,ff,tiles", [
     # microseconds of a layer in tiles of 64 entries and of 128
     (65, 1, 1, 64, 64, False), (512, 4, 2, 64, 64, False), (64, 32, 2, 64, 64, False),      # 26, 31; 30, 37; 30, 33

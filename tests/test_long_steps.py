@@ -256,7 +256,7 @@ def test_experts_units_are_float32_accurate_over_the_gates_range(K, act, code, l
 
 
 @pytest.mark.parametrize("states", [5, 16, 20])
-@pytest.mark.parametrize("lens", [(768,), (1793, 1, 513), (1475, 64), (900, 640)])
+@pytest.mark.parametrize("lens", [(768,), (1793, 1, 513), (1475, 64), (900, 640), (896,), (1921, 1, 769), (2500, 65)])
 def test_selective_scan_over_pieces(K, states, lens):
     """Requests of exactly one piece, of one row more, and of several, from states that are not zero; 130 channels.  Float32
     throughout: rounding of 2^-24 a step over a chain whose decays are below 1."""
