@@ -6,8 +6,9 @@
 // accumulators that take turns, eight epilogue warps (two a lane quarter, every second 32 columns each).  A tile's rows behind the expert's last entry are other experts' and are
 // not stored.  With GLU a tile's B rows are 128 gate rows and the 128 up rows that belong to them.
 //
-// What bounds it: the tensor cores.  Measured on a B200 at 2,048 rows, eight experts of 1,408 of which a row takes two, width
-// 2,048, all six launches: 405 us in tiles of 64 on mma.sync -> 135.
+// What bounds it: neither the tensor cores (2,048 rows, eight experts of 1,408 of which a row takes two, width 2,048: 71 GFLOP in 141 us,
+// a third of the burst rate) nor memory (138 MB of weights, 21 us), but part-filled last waves (352 and 256 tiles over 148 blocks) and
+// the five launches around the two products.  All seven launches of that layer on a B200: 405 us in tiles of 64 on mma.sync -> 141.
 #pragma once
 
 #include "tcgen05.cuh"

@@ -39,7 +39,6 @@ _BLOCKS_OPS = tuple(OP[n] for n in ("norm_add", "reinject", "latent_qkv", "head_
                                     "selective_scan", "experts", "softcap", "add_rows", "norm_pair", "embed_pair", "join", "gated_recurrence"))
 OPTIONAL_SLOTS = ("heads",)     # a step finds another way where these are too small,
 LEAVE_FREE = 4 << 30            # so they are made only where this much stays free after them (logits of 8,192 rows over 122,753 tokens)
-SHORT_ROWS = 8                  # jk::SHORT_ROWS of csrc/host_rules.h
 MAX_GROUPS = 8
 MAX_LISTS = 8
 
@@ -478,7 +477,7 @@ def tile_keys(ctx) -> int:
     if len(starts) <= ctx.nreq or len(pos) < ctx.nreq:
         return 0
     lens = [starts[i + 1] - starts[i] for i in range(ctx.nreq)]
-    return sum(lens) + sum(pos[:ctx.nreq]) if lens and min(lens) > SHORT_ROWS else 0
+    return sum(lens) + sum(pos[:ctx.nreq]) if lens and min(lens) > _host.attention_short_rows() else 0
 
 
 def step_lists_for(owners, ctx, device) -> Dict[str, tuple]:
