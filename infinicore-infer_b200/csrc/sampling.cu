@@ -149,7 +149,11 @@ template <typename T> __device__ __forceinline__ T warp_prefix(T v) {
     return v;
 }
 
-__global__ void __launch_bounds__(SAMPLE_THREADS)
+// OCC: blocks an SM that the registers must allow.  Two for more rows than there are SMs, whose second wave would otherwise run alone: 200
+// rows of 122,753, greedy ones 97 -> 59 us, 200 of 384 with topp 64 -> 54; one for fewer, whose passes have more loads in flight (one row of
+// 122,753, topk 50: 45 -> 43).
+template <int OCC>
+__global__ void __launch_bounds__(SAMPLE_THREADS, OCC)
 sample_kernel(const float *__restrict__ logits, long long ld, int V,
               const float *__restrict__ temperature, const int *__restrict__ topk,
               const float *__restrict__ topp, const float *__restrict__ uniform,
@@ -349,7 +353,7 @@ JK_EXPORT int jk_sample(const float *logits, long long ld, int nrows, int V, con
                         cudaStream_t stream) {
     if (nrows == 0) return JK_OK;
     JK_REQUIRE(nrows > 0 && V > 0 && ld >= V, "sample: rows %d, vocabulary %d, stride %lld", nrows, V, ld);
-    jk_launch(sample_kernel, dim3(nrows), dim3(SAMPLE_THREADS), 0, stream, logits, ld, V, temperature, topk, topp, uniform, out);
+    jk_launch(nrows > 148 ? sample_kernel<2> : sample_kernel<1>, dim3(nrows), dim3(SAMPLE_THREADS), 0, stream, logits, ld, V, temperature, topk, topp, uniform, out);
     JK_CHECK_LAUNCH("sample");
     return JK_OK;
 }
