@@ -937,8 +937,6 @@ __device__ __forceinline__ float4 piece_act(int act, float4 v, float f) {
     return make_float4(apply_act(act, v.x) * f, apply_act(act, v.y) * f, apply_act(act, v.z) * f, apply_act(act, v.w) * f);
 }
 
-// A block makes KB x CB of a piece's end state; thread (ty, tx) of 16 x 16 keeps key channels ty * 4 + {0..3} (and 64 on), columns
-// tx * 4 + {0..3} (and 64 on).
 // A block = (piece, head): z = W2 act(r_t) + b2 and the decay of it, the chain of sums of the scan kernel, four rows a thread; the product of
 // the piece's decays.  Heads of at most 128 key channels, the head's rows of W2 and the piece's rows of r in shared memory.
 template <typename TW>
@@ -994,6 +992,8 @@ __global__ void __launch_bounds__(256) piece_decays_kernel(ScanArgs a) {
     }
 }
 
+// A block makes KB x CB of a piece's end state; thread (ty, tx) of 16 x 16 keeps key channels ty * 4 + {0..3} (and 64 on), columns
+// tx * 4 + {0..3} (and 64 on).
 // PROJ: the decays are those in `cum` (one block of key channels then, dk <= KB)
 template <int KB, int CB, bool PROJ>
 __global__ void __launch_bounds__(256) piece_state_kernel(ScanArgs a) {
