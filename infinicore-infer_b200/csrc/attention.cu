@@ -65,7 +65,7 @@ struct AttnArgs {
 // over 8, a prompt of 301 rows 375 -> 62, one row over 1,000 keys 293 -> 72, 8 rows over 4,000 keys each 2,072 -> 279; 36
 // heads, a prompt of 512 rows 1,554 -> 168; bfloat16, 16 heads of 256, a prompt of 1,024 rows 9,515 -> 1,369.
 // ---------------------------------------------------------------------------------------
-constexpr int ROW_WARPS = 8, ROW_SLOTS = 4, ROW_PAIRS = ROW_WARPS * ROW_SLOTS, ROW_KEYS = 32;
+constexpr int ROW_WARPS = 8, ROW_PAIRS = jk::ROW_PAIRS, ROW_SLOTS = ROW_PAIRS / ROW_WARPS, ROW_KEYS = 32;
 constexpr int ROW_MAX_DH = 512;
 
 // 32 rows of `size` elements as floats into rows of `ld`, four rows a warp, 2^`lanes` lanes a row.  `row`: the number of this
@@ -170,6 +170,29 @@ __device__ __forceinline__ void row_chunk(const AttnArgs &a, const float *ks, co
     __syncwarp();
 }
 
+// The end of a pair: the sink, the sum, the gate, and the row's head goes out.
+template <typename T, int NS>
+__device__ __forceinline__ void row_store(const AttnArgs &a, int t, int h, float m, float l, float (&acc)[NS]) {
+    const int lane = threadIdx.x & 31;
+    if (a.sink) {       // one more key that brings no value
+        const float sink = a.sink_w != nullptr ? a.sink_w[h] : 0.f;
+        const float m_new = fmaxf(m, sink);
+        const float corr = expf(m - m_new);
+        l = l * corr + expf(sink - m_new);
+#pragma unroll
+        for (int n = 0; n < NS; ++n) acc[n] *= corr;
+    }
+    T *orow = (T *)a.out + ((size_t)t * a.nh + h) * a.dv;
+    float inv = 1.f / l;
+    const float *gate = a.gate != nullptr ? a.gate + (size_t)t * a.gate_ld + (size_t)h * (a.gate_elem ? a.dv : 1) : nullptr;
+    if (gate != nullptr && !a.gate_elem) inv *= jk_sigmoid(gate[0]);
+#pragma unroll
+    for (int n = 0; n < NS; ++n) {
+        const int e = lane + 32 * n;
+        if (e < a.dv) orow[e] = from_f32<T>(acc[n] * inv * (a.gate_elem && gate != nullptr ? jk_sigmoid(gate[e]) : 1.f));
+    }
+}
+
 template <typename T, int NS>     // NS: slices of 32 elements that cover one head's values
 __global__ void __launch_bounds__(ROW_WARPS * 32)
 attention_row_kernel(AttnArgs a) {
@@ -259,25 +282,73 @@ attention_row_kernel(AttnArgs a) {
     for (int i = 0; i < ROW_SLOTS; ++i) {
         const int pair = warp + i * ROW_WARPS;
         if (pair >= pairs) continue;
-        const int t = t0 + pair / heads, h = h0 + pair % heads;
-        if (a.sink) {       // one more key that brings no value
-            const float sink = a.sink_w != nullptr ? a.sink_w[h] : 0.f;
-            const float m_new = fmaxf(m[i], sink);
-            const float corr = expf(m[i] - m_new);
-            l[i] = l[i] * corr + expf(sink - m_new);
+        row_store<T, NS>(a, t0 + pair / heads, h0 + pair % heads, m[i], l[i], acc[i]);
+    }
+}
+
+// Walk kernel: the same sums in the same order, a warp a (row, query head), lanes with a key row of their own in memory.  Nothing is staged
+// and no barrier waited for, so it is the better one where a block of the row kernel would have few pairs for its warps or few
+// keys to walk (jk::attention_rows_walk, where both sides' times stand).  What bounds it: a cache line a lane and load.  Chunks of
+// keys start at multiples of 32 positions as they do above: a row's result is the same, bit for bit, in either kernel.
+constexpr int WALK_WARPS = 4;
+
+template <typename T, int NS>
+__global__ void __launch_bounds__(WALK_WARPS * 32)
+attention_walk_kernel(AttnArgs a) {
+    pdl_trigger();
+    pdl_wait();
+    extern __shared__ __align__(16) float row_smem[];          // [WALK_WARPS][dh]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = blockIdx.y, h = blockIdx.x * WALK_WARPS + warp;
+    if (h >= a.nh) return;
+    const int dh = a.dh, dv = a.dv, hk = h / (a.nh / a.nkvh), pos = a.positions[t];
+    const int *bt = a.block_table + (size_t)a.row_req[t] * a.max_blocks;
+    const int lo = jk_mask_lo(pos, a.window), kept = min(a.keep_first, pos + 1);
+    float *qs = row_smem + warp * dh;
+    const T *qrow = (const T *)a.q + ((size_t)t * a.nh + h) * dh;
+    for (int e = lane; e < dh; e += 32) qs[e] = to_f32(qrow[e]);
+    __syncwarp();
+    const T *kp = (const T *)a.k_pages, *vp = (const T *)a.v_pages;
+    float m = -INFINITY, l = 0.f, acc[NS];
 #pragma unroll
-            for (int n = 0; n < NS; ++n) acc[i][n] *= corr;
+    for (int n = 0; n < NS; ++n) acc[n] = 0.f;
+    // every chunk visited holds a seen key: kept ones first, then those from the window's first on
+    auto after = [&](int j) { return j + ROW_KEYS < kept ? j + ROW_KEYS : max(j + ROW_KEYS, lo / ROW_KEYS * ROW_KEYS); };
+    for (int j0 = kept > 0 ? 0 : lo / ROW_KEYS * ROW_KEYS; j0 <= pos; j0 = after(j0)) {
+        const int j = j0 + lane;
+        const bool seen = j <= pos && (j >= lo || j < kept);
+        long long row = 0;
+        float s = -INFINITY;
+        if (seen) {
+            const int block = a.page_shift >= 0 ? j >> a.page_shift : j / a.page_size;
+            row = ((long long)bt[block] * a.nkvh + hk) * a.page_size + (j - block * a.page_size);
+            const T *kr = kp + (size_t)row * dh;
+            float dot = 0.f;
+            for (int e = 0; e < dh; ++e) dot = fmaf(qs[e], to_f32(kr[e]), dot);
+            s = dot * a.scale;
+            if (a.cap > 0.f) s = a.cap * tanhf(s / a.cap);
         }
-        T *orow = (T *)a.out + ((size_t)t * a.nh + h) * a.dv;
-        float inv = 1.f / l[i];
-        const float *gate = a.gate != nullptr ? a.gate + (size_t)t * a.gate_ld + (size_t)h * (a.gate_elem ? a.dv : 1) : nullptr;
-        if (gate != nullptr && !a.gate_elem) inv *= jk_sigmoid(gate[0]);
+        const float m_new = fmaxf(m, warp_max(s)), p = seen ? expf(s - m_new) : 0.f, corr = expf(m - m_new);
+        l = l * corr + warp_sum(p);
+        m = m_new;
 #pragma unroll
-        for (int n = 0; n < NS; ++n) {
-            const int e = lane + 32 * n;
-            if (e < a.dv) orow[e] = from_f32<T>(acc[i][n] * inv * (a.gate_elem && gate != nullptr ? jk_sigmoid(gate[e]) : 1.f));
+        for (int n = 0; n < NS; ++n) acc[n] *= corr;
+        // the seen keys, run by run (one run but where a window has passed kept keys of the same chunk)
+        for (unsigned mask = __ballot_sync(0xffffffffu, seen); mask != 0;) {
+            const int first = __ffs(mask) - 1, end = first + __clz(~__brev(mask >> first));
+#pragma unroll 4
+            for (int jj = first; jj < end; ++jj) {
+                const float w = __shfl_sync(0xffffffffu, p, jj);
+                const T *vr = vp + (size_t)__shfl_sync(0xffffffffu, row, jj) * dv;
+#pragma unroll
+                for (int n = 0; n < NS; ++n) {
+                    const int e = lane + 32 * n;
+                    if (e < dv) acc[n] = fmaf(w, to_f32(vr[e]), acc[n]);
+                }
+            }
+            mask = end < 32 ? mask >> end << end : 0u;
         }
     }
+    row_store<T, NS>(a, t, h, m, l, acc);
 }
 
 static int check_args(const AttnArgs &a) {
@@ -292,7 +363,7 @@ JK_EXPORT int jk_attention_rows(const void *q, const void *k_pages, const void *
                                 int dtype, const int *positions, const int *row_req,
                                 const int *block_table, int max_blocks, int page_size, int T, int nh,
                                 int nkvh, int dh, float scale, int window, int dv, int sink, const float *gate, int gate_ld,
-                                float cap, int keep_first, const float *sink_w, int gate_elem, cudaStream_t stream) {
+                                float cap, int keep_first, const float *sink_w, int gate_elem, int nreq, int context, cudaStream_t stream) {
     if (T == 0) return JK_OK;
     if (dv <= 0) dv = dh;
     AttnArgs a{q, k_pages, v_pages, out, positions, row_req, block_table,
@@ -301,22 +372,41 @@ JK_EXPORT int jk_attention_rows(const void *q, const void *k_pages, const void *
     JK_REQUIRE(dh <= ROW_MAX_DH && dv <= ROW_MAX_DH, "attention: head size %d / %d exceeds %d", dh, dv, ROW_MAX_DH);
     JK_REQUIRE(gate == nullptr || gate_ld >= nh * (gate_elem ? dv : 1), "attention: a gate row of %d holds no %d heads", gate_ld, nh);
     JK_REQUIRE(T <= 65535, "attention: %d rows exceed one launch (65535)", T);
-    // A block's pairs: as many heads of one key/value head as there are, then rows until the pairs are full (every row alike: the
-    // cut does not change a row's result)
-    const int group = nh / nkvh, elem = dtype == JK_F32 ? 4 : 2;
-    a.tile_heads = group < ROW_PAIRS ? group : ROW_PAIRS;
-    a.tile_rows = ROW_PAIRS / a.tile_heads;
+    const int elem = dtype == JK_F32 ? 4 : 2;
     a.page_shift = -1;
     for (int i = 0; i < 31; ++i)
         if (page_size == 1 << i) a.page_shift = i;
+#define BY_SLICES(LAUNCH, T)                      \
+    do {                                          \
+        if (dv <= 32) LAUNCH(T, 1);               \
+        else if (dv <= 64) LAUNCH(T, 2);          \
+        else if (dv <= 128) LAUNCH(T, 4);         \
+        else if (dv <= 256) LAUNCH(T, 8);         \
+        else LAUNCH(T, 16);                       \
+    } while (0)
+#define BY_TYPE(LAUNCH)                                                        \
+    do {                                                                       \
+        if (dtype == JK_F32) BY_SLICES(LAUNCH, float);                         \
+        else if (dtype == JK_BF16) BY_SLICES(LAUNCH, __nv_bfloat16);           \
+        else JK_FAIL(JK_UNSUPPORTED, "attention: dtype %d", dtype);            \
+    } while (0)
+    if (jk::attention_rows_walk(T, nreq, window > 0 ? std::min(context, window + keep_first) : context, nh, nkvh, std::max(dh, dv), elem)) {
+        const dim3 grid((nh + WALK_WARPS - 1) / WALK_WARPS, T);
+        const size_t smem = (size_t)WALK_WARPS * dh * sizeof(float);
+#define LAUNCH_WALK(T, NS) jk_launch(attention_walk_kernel<T, NS>, grid, dim3(WALK_WARPS * 32), smem, stream, a)
+        BY_TYPE(LAUNCH_WALK);
+#undef LAUNCH_WALK
+        JK_CHECK_LAUNCH("attention_walk");
+        return JK_OK;
+    }
+    const jk::RowCut cut = jk::attention_rows_cut(T, nh, nkvh);         // (every row alike: the cut does not change a row's result)
+    a.tile_heads = cut.heads;
+    a.tile_rows = cut.rows;
     a.vec = dh * elem % 16 == 0 && dv * elem % 16 == 0 && (((uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0;
     const int vectors = std::max(dh, dv) * elem / (a.vec ? 16 : elem);
     for (a.lanes = 2; a.lanes < 5 && (1 << a.lanes) < vectors;) ++a.lanes;
-    const long long parts = (group + a.tile_heads - 1) / a.tile_heads;
-    JK_REQUIRE(parts * nkvh <= 65535, "attention: %d heads exceed one launch", nh);
-    // fewer rows a block until there are three blocks for every SM: a block alone there waits for its chunks and its barriers
-    while (a.tile_rows > 1 && (T + a.tile_rows - 1) / a.tile_rows * parts * nkvh < 3 * 148) a.tile_rows = (a.tile_rows + 1) / 2;
-    dim3 grid(T, (unsigned)(parts * nkvh));
+    JK_REQUIRE(cut.parts * nkvh <= 65535, "attention: %d heads exceed one launch", nh);
+    dim3 grid(T, (unsigned)(cut.parts * nkvh));
     const int width = (dh + 3) / 4 * 4;
     // two chunks of keys as long as two blocks fit an SM with them
     const size_t tile = (size_t)ROW_KEYS * (width + 4 + (dv + 3) / 4 * 4), fixed = (size_t)ROW_PAIRS * (width + ROW_KEYS);
@@ -327,20 +417,10 @@ JK_EXPORT int jk_attention_rows(const void *q, const void *k_pages, const void *
         if (smem > 46 * 1024) cudaFuncSetAttribute(attention_row_kernel<T, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
         jk_launch(attention_row_kernel<T, NS>, grid, dim3(ROW_WARPS * 32), smem, stream, a);                                            \
     } while (0)
-#define LAUNCH_ROWS_T(T)                                \
-    do {                                                \
-        if (dv <= 32) LAUNCH_ROWS(T, 1);                \
-        else if (dv <= 64) LAUNCH_ROWS(T, 2);           \
-        else if (dv <= 128) LAUNCH_ROWS(T, 4);          \
-        else if (dv <= 256) LAUNCH_ROWS(T, 8);          \
-        else LAUNCH_ROWS(T, 16);                        \
-    } while (0)
-    if (dtype == JK_F32)
-        LAUNCH_ROWS_T(float);
-    else if (dtype == JK_BF16)
-        LAUNCH_ROWS_T(__nv_bfloat16);
-    else
-        JK_FAIL(JK_UNSUPPORTED, "attention: dtype %d", dtype);
+    BY_TYPE(LAUNCH_ROWS);
+#undef LAUNCH_ROWS
+#undef BY_TYPE
+#undef BY_SLICES
     JK_CHECK_LAUNCH("attention_rows");
     return JK_OK;
 }

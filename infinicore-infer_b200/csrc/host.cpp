@@ -66,6 +66,9 @@ JK_HOST_EXPORT long long jk_decode_scratch_floats(int nrows, int nh, int dh, int
     return jk::decode_scratch_floats(nrows, nh, dh, splits);
 }
 JK_HOST_EXPORT int jk_decode_keys_hint(int context, int window) { return jk::decode_keys_hint(context, window); }
+JK_HOST_EXPORT int jk_attention_rows_walk(int T, int nreq, int context, int nh, int nkvh, int size, int elem) {
+    return jk::attention_rows_walk(T, nreq, context, nh, nkvh, size, elem) ? 1 : 0;
+}
 JK_HOST_EXPORT int jk_conv_walks_rows(long long rows, long long nreq, long long channels) { return jk::conv_walks_rows(rows, nreq, channels) ? 1 : 0; }
 JK_HOST_EXPORT int jk_selective_scan_cuts(long long rows, long long nreq, long long channels, long long states) {
     return jk::selective_scan_cuts(rows, nreq, channels, states) ? 1 : 0;

@@ -276,6 +276,49 @@ inline bool attention_tcgen05_takes(int dh, int page_size, int dv = 0) {
     return size && (page_size == 8 || page_size == 16 || page_size == 32 || page_size == 64 || page_size == 128);
 }
 
+// ---- the float32 row attention's two kernels (csrc/attention.cu) -------------------------------------------------------------------
+constexpr int ROW_PAIRS = 32;       // (row, head) pairs of a block at most
+// Rows and heads of a block: as many heads of one key/value head as there are, then rows until the pairs are full, but fewer rows until there
+// are three blocks for every SM (a block alone there waits for its chunks and its barriers).  `parts`: blocks a key/value head.
+struct RowCut { int heads, rows; long long parts; };
+inline RowCut attention_rows_cut(int T, int nh, int nkvh) {
+    RowCut c;
+    c.heads = std::min(nh / nkvh, ROW_PAIRS);
+    c.rows = ROW_PAIRS / c.heads;
+    c.parts = (nh / nkvh + c.heads - 1) / c.heads;
+    while (c.rows > 1 && (T + c.rows - 1) / c.rows * c.parts * nkvh < 3 * 148) c.rows = (c.rows + 1) / 2;
+    return c;
+}
+// Whether a warp a pair walks its keys in memory instead (attention_walk_kernel): where a block would have few pairs for its eight warps and
+// there are more blocks than run at once, or where there are too few keys to make up for staging them.  `context`: the longest
+// history that is known of (a bound); `size`: the larger of a key's and a value's; T rows of `nreq` requests.  Results are the same bits.
+// B200, warps -> blocks (us), single rows after n keys where nothing else is said:
+//   bfloat16, heads of 16 to 32, whose rows a lane reads with few lines: 512 requests, 4 heads of 16, n = 100 18 -> 70; one of them 13 -> 14, n = 1,000
+//     96 -> 70; 512, 7 of 30, n = 100 38 -> 194, a prompt of 300 40 -> 66, of 2,048 744 -> 567; 1,024, 4 heads of 32 over one, n = 400 216 -> 116.
+//   bfloat16, 512 requests, n = 100: 36 heads of 64 666 -> 701, 8 of 96 284 -> 310, 16 of 256 1,034 -> 2,129; 64, 16 of 256, n = 300 585 -> 676.
+//   float32, 512 requests, n = 100: 4 heads of 16 37 -> 61, 7 of 30 151 -> 225, 16 of 256 1,134 -> 1,603, but 36 of 64 713 -> 556.
+//   short histories, float32: a prompt of 17 rows, 16 heads of 256 18 -> 26, 36 of 64 9 -> 12, but 24 of 64 over 8 8 -> 7; 4 rows, 64 requests, 36 heads of
+//     128 27 -> 78; 16 rows, 256 requests, 16 of 80 172 -> 266.
+// Decode steps know their histories to the next power of two from 256 on only: below 40 keys some of them would be faster the other way.
+inline bool attention_rows_walk(int T, int nreq, int context, int nh, int nkvh, int size, int elem) {
+    if (nreq <= 0 || context <= 0) return false;
+    const RowCut c = attention_rows_cut(T, nh, nkvh);
+    const long long n = (T + nreq - 1) / nreq, pairs = c.heads * std::min<long long>(c.rows, n), blocks = nreq * ((n + c.rows - 1) / c.rows) * c.parts * nkvh;
+    const bool single = pairs == 1 && blocks >= 3 * 148;
+    if (context <= 8) return true;
+    if (context <= 24 && (size < 32 || (size > 128 && size <= 256) || single || (elem == 2 && size == 32))) return true;
+    if (context <= 24 && blocks >= 1500 && size > 64 && size < 128) return true;
+    if (context <= 16 && pairs <= 4 && blocks >= 3 * 148 && size <= 96) return true;
+    if (elem == 4) {
+        if (size < 32) return (pairs == 1 && (blocks >= 5000 || (blocks >= 1500 && context <= 512))) || (pairs <= 4 && blocks >= 3 * 148 && context <= 64);
+        return size > 128 && size <= 256 && single && context <= 256;
+    }
+    if (size % 8 != 0 && size < 32) return context <= 512 || pairs <= 8;            // nor can a block copy 16 bytes at a time
+    if (size <= 32) return single || (pairs <= 4 && context <= 256) || (size < 32 && context <= 64);
+    if (size <= 128) return pairs == 1 && blocks >= 4096 && context <= 256;
+    return single && n <= 8 && context <= 512;
+}
+
 // Whether a causal convolution over `rows` rows of `nreq` requests walks eight rows a thread (csrc/blocks.cu) instead of making an element
 // a thread: a walk is a chain that takes a large launch to hide, the more so where every row is a request of its own and reads and
 // moves its own tail.  B200, element a thread -> rows (us): 64 channels, 128 to 2,048 rows 9 -> 13; 512 channels, 512 rows 11 to 13 -> 13,

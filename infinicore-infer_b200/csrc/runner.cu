@@ -120,6 +120,14 @@ struct Run {
         return jk::attention_tile_keys(heads, load, env.routing.sms);
     }
 
+    // the longest history of the step's requests: known, or (decode steps, which graphs replay) the length that the step is planned for
+    int longest(int max_positions) const {
+        if (st.host_req_start == nullptr || st.host_req_pos == nullptr || st.ntok <= st.nreq) return st.context > 0 ? st.context : max_positions;
+        int most = 0;
+        for (int i = 0; i < st.nreq; ++i) most = std::max(most, st.host_req_pos[i] + st.host_req_start[i + 1] - st.host_req_start[i]);
+        return most;
+    }
+
     int elem() const { return env.dtype == JK_F32 ? 4 : 2; }
     bool tcgen05_bound() const { return g_fns.gemm_tcgen05 != nullptr; }
     jk::Route route(int rows, int n, int k, int kind) const {
@@ -280,7 +288,8 @@ int run_attention(Run &r, const RunnerOp &op) {
         // float32 arithmetic throughout: float32 mode, and every shape the tensor-core kernels are not built for
         RUN(attention, g_fns.attention_rows(q, op.k_pages, op.v_pages, o, r.env.dtype, r.st.positions, r.st.row_req, table,
                                             r.env.max_blocks, page, T, nh, nkvh, dh, op.softmax_scale, op.window, dv, op.sink, gate, op.ld,
-                                            op.cap, op.keep_first, op.sink_w, op.gated == 2, r.stream));
+                                            op.cap, op.keep_first, op.sink_w, op.gated == 2, r.st.nreq, r.longest(op.max_positions),
+                                            r.stream));
         return JK_OK;
     }
     if (n_tiles > 0) {

@@ -31,7 +31,7 @@ typedef int (*GemmTcgen05QkvFn)(const void *, const void *, int, int, void *, vo
                                 const int *, const int *, const int *, int, int, int, int, int, int *, int, cudaStream_t);
 typedef int (*AttentionRowsFn)(const void *, const void *, const void *, void *, int, const int *, const int *, const int *, int,
                                int, int, int, int, int, float, int, int, int, const float *, int, float, int, const float *, int,
-                               cudaStream_t);
+                               int, int, cudaStream_t);
 typedef int (*AttentionDecodeFn)(const void *, const void *, const void *, void *, float *, const int *, int, const int *,
                                  const int *, const int *, int, int, int, int, int, float, int, int, int, const float *, int, float, int,
                                  const float *, int, int, cudaStream_t);

@@ -455,13 +455,14 @@ def attention_rows(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor
                    positions: torch.Tensor, row_req: torch.Tensor, block_table: torch.Tensor, ntok: int,
                    nh: int, scale: float, window: int = 0, sink: bool = False,
                    gate: Optional[torch.Tensor] = None, cap: float = 0.0, keep_first: int = 0,
-                   sink_w: Optional[torch.Tensor] = None, gate_elem: bool = False) -> torch.Tensor:
+                   sink_w: Optional[torch.Tensor] = None, gate_elem: bool = False, context: int = -1) -> torch.Tensor:
     """Causal attention of ``ntok`` query rows over the paged cache, float32 arithmetic.  Values may have
     another size than keys (``v_pages [..., dv]``, ``out [ntok, nh, dv]``); ``sink`` adds a key of score 0 without a
     value; ``gate`` (float32 ``[ntok, >= nh]``, a view of wider rows is fine) multiplies head h's output by
     sigmoid(gate[t, h]); ``cap`` > 0 caps the scores by cap tanh(s / cap); keys at positions below ``keep_first`` stay
     visible when the window has passed them; ``sink_w`` (float32 [nh]): the sinks' scores instead of 0; ``gate_elem``: the gate
-    has a column for every output element (``[ntok, >= nh dv]``)."""
+    has a column for every output element (``[ntok, >= nh dv]``).  ``context``: a bound on the histories, by which the kernel is
+    chosen (0: not known; -1: what a request's blocks hold); the results are the same."""
     _need(q, "q"); _need(k_pages, "k_pages"); _need(v_pages, "v_pages"); _need(out, "out")
     _need(positions, "positions", torch.int32); _need(row_req, "row_req", torch.int32)
     _need(block_table, "block_table", torch.int32)
@@ -482,7 +483,8 @@ def attention_rows(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor
         _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _c_int(dtype_code(q.dtype)), _ptr(positions),
         _ptr(row_req), _ptr(block_table), _c_int(block_table.shape[1]), _c_int(page_size), _c_int(ntok),
         _c_int(nh), _c_int(nkvh), _c_int(dh), _c_float(scale), _c_int(window or 0), _c_int(dv), _c_int(1 if sink else 0),
-        _ptr(gate), _c_int(gate_ld), _c_float(cap), _c_int(keep_first), _ptr(sink_w), _c_int(1 if gate_elem else 0), _stream()))
+        _ptr(gate), _c_int(gate_ld), _c_float(cap), _c_int(keep_first), _ptr(sink_w), _c_int(1 if gate_elem else 0), _c_int(block_table.shape[0]),
+        _c_int(context if context >= 0 else block_table.shape[1] * page_size), _stream()))
     return out
 
 

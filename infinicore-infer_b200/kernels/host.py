@@ -135,6 +135,11 @@ def context_bucket(longest: int, max_positions: int) -> int:
     return lib().jk_context_bucket(longest, max_positions)
 
 
+def attention_rows_walk(rows: int, nreq: int, context: int, heads: int, kv_heads: int, size: int, elem: int) -> bool:
+    """Whether the float32 row attention runs a warp a (row, head) instead of blocks that share keys."""
+    return bool(lib().jk_attention_rows_walk(rows, nreq, context, heads, kv_heads, size, elem))
+
+
 def selective_scan_cuts(rows: int, nreq: int, channels: int, states: int) -> bool:
     """Whether a selective scan runs over pieces of its requests side by side."""
     c = ctypes.c_longlong

@@ -45,6 +45,18 @@ def test_rows_a_thread_of_the_causal_convolution(rows, requests, channels, walks
     assert host.conv_walks_rows(rows, requests, channels) == walks
 
 
+@pytest.mark.parametrize("elem,heads,kv_heads,size,requests,rows,context,walks", [
+    # (rows of each request, bound on the histories); microseconds by warps and by blocks
+    (2, 4, 4, 16, 512, 1, 256, True), (2, 4, 4, 16, 1, 1, 1001, False), (2, 7, 7, 30, 512, 1, 256, True), (2, 7, 7, 30, 1, 300, 300, True),     # 18, 70; 96, 70; 38, 194; 40, 66
+    (2, 7, 7, 30, 1, 2048, 2048, False), (2, 4, 1, 32, 1024, 1, 512, False),        # 744, 567; 216, 116
+    (2, 8, 8, 96, 512, 1, 256, True), (2, 36, 36, 64, 64, 1, 512, False), (2, 16, 16, 256, 64, 1, 512, True), (2, 1, 1, 512, 1, 500, 500, False),     # 284, 310; -; 585, 676; 699, 406
+    (4, 4, 4, 16, 512, 1, 256, True), (4, 16, 16, 256, 512, 1, 256, True), (4, 36, 36, 64, 512, 1, 256, False),      # 37, 61; 1,134, 1,603; 713, 556
+    (4, 36, 36, 64, 1, 17, 17, True), (4, 24, 8, 64, 1, 17, 17, False), (4, 16, 16, 256, 1, 17, 17, True),        # 9, 12; 8, 7; 18, 26
+    (4, 24, 8, 64, 1, 301, 301, False), (4, 24, 8, 64, 8, 1, 4096, False), (4, 36, 36, 128, 64, 4, 4, True), (4, 4, 4, 16, 8, 1, 0, False)])     # -; -; 27, 78; not known
+def test_kernel_of_the_float32_row_attention(elem, heads, kv_heads, size, requests, rows, context, walks):
+    assert host.attention_rows_walk(rows * requests, requests, context, heads, kv_heads, size, elem) == walks
+
+
 @pytest.mark.parametrize("lens,channels,states,cuts", [
     # microseconds end to end and over pieces
     ([512], 4096, 16, False), ([768], 4096, 16, True), ([2048], 4096, 16, True),        # 148 twice; 589, 360

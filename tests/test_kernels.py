@@ -470,6 +470,37 @@ def test_attention_rows_tiles(K, dtype, nh, nkvh, dh, page, window):
     assert torch.equal(torch.cat([got[2:67], got[68:]]), less)
 
 
+@pytest.mark.parametrize("dtype,nh,nkvh,dh,dv,page,window,lens,rows", [
+    # (dtype, heads, sizes, page, window (< 0: chunks), histories, rows of each request)
+    (torch.float32, 4, 4, 16, 16, 8, 0, [1, 24, 17, 9], [1, 1, 2, 1]), (torch.float32, 2, 1, 256, 256, 8, 7, [24, 1, 23], [1, 1, 1]),
+    (torch.bfloat16, 2, 2, 192, 160, 6, -10, [24, 11, 10, 1], [1, 1, 1, 1]), (torch.float32, 3, 3, 7, 30, 8, 9, [24, 24], [1, 1]),
+    (torch.float32, 20, 20, 64, 48, 8, 5, [24, 19], [24, 1]), (torch.bfloat16, 40, 40, 40, 40, 8, 0, [24], [14]),
+    (torch.bfloat16, 4, 2, 32, 32, 16, 50, [256, 100, 31, 33], [1, 1, 1, 1]), (torch.bfloat16, 4, 4, 16, 16, 16, -32, [256, 65, 64, 1], [1, 1, 1, 1])])
+@pytest.mark.parametrize("extra", ["none", "sink and gate", "element gate, cap and kept keys"])
+def test_attention_rows_by_warps_and_by_blocks(K, dtype, nh, nkvh, dh, dv, page, window, lens, rows, extra):
+    """Not to know a bound on the histories moves a call from one kernel to the other: the same bits, whatever lies behind the histories."""
+    from infinicore_infer_b200.kernels.host import attention_rows_walk
+    g, R, T = torch.Generator().manual_seed(dh), len(lens), sum(rows)
+    r = lambda *s: torch.randn(*s, generator=g)
+    few = -(-max(lens) // page)
+    kp, vp = r(R * few + 1, nkvh, page, dh), r(R * few + 1, nkvh, page, dv)
+    table = (torch.randperm(R * few, generator=g) + 1).view(R, few)
+    for i, n in enumerate(lens):
+        if n % page:
+            kp[table[i, n // page], :, n % page:], vp[table[i, n // page], :, n % page:] = float("nan"), float("nan")
+    positions = torch.tensor([n - m + i for n, m in zip(lens, rows) for i in range(m)], dtype=torch.int32, device=DEV)
+    row_req = torch.tensor([i for i, m in enumerate(rows) for _ in range(m)], dtype=torch.int32, device=DEV)
+    q, kp, vp = (t.to(dtype).to(DEV) for t in (r(T, nh * dh), kp, vp))
+    keep = 4 if window > 0 else 0
+    options = {"none": {}, "sink and gate": dict(sink=True, sink_w=r(nh).to(DEV), gate=r(T, nh).to(DEV)),
+               "element gate, cap and kept keys": dict(gate=r(T, nh * dv).to(DEV), gate_elem=True, cap=3.0, keep_first=keep)}[extra]
+    for context, walks in ((max(lens), True), (0, False)):
+        assert attention_rows_walk(T, R, min(context, window + keep) if window > 0 else context, nh, nkvh, max(dh, dv), 4 if dtype == torch.float32 else 2) == walks
+    got = [K.attention_rows(q, kp, vp, torch.full((T, nh * dv), 55.0, dtype=dtype, device=DEV), positions, row_req, table.to(torch.int32).to(DEV), T, nh,
+                            dh ** -0.5, window, context=context, **options) for context in (max(lens), 0)]
+    assert torch.isfinite(got[0].float()).all() and torch.equal(*got)
+
+
 # grouped heads of 64 or 128: the decode kernel that puts the group on the tensor cores (16 heads fill a tile;
 # 20 need a second one; 2 to 7 leave most of it empty)
 GROUPED = [(32, 2, 128, 16, None), (10, 2, 64, 16, 70), (40, 2, 128, 8, None), (6, 1, 64, 32, 33), (7, 1, 128, 5, None),
