@@ -1,4 +1,5 @@
-// The float32 matrix product on the CUDA cores:  C[M, N] = A[M, K] * W[N, K]^T (+ bias[N]).
+// The float32 matrix product on the CUDA cores:  C[M, N] = A[M, K] * W[N, K]^T (+ bias[N]).  Steps of few rows and short sums take it;
+// the others go to gemm_f32_tcgen05.cu (jk::f32_plan).
 //
 // Fused multiply-adds in float32: no tensor cores, hence no TF32 rounding of the operands.
 // (reference: the products at jiuge.cpp:200, :236, :247, :249, :264 go to a library.)
@@ -19,6 +20,7 @@
 // 1,536 393 -> 72, 301 x 1,536 x 1,536 262 -> 44, 301 x 7,680 x 1,536 551 -> 195, 301 x 1,536 x 3,840 656 -> 101,
 // 2,048 x 7,680 x 1,536 2,202 -> 1,065 (0.61 of the pipes' 74 TFLOP/s), 8 x 2,560 x 1,536 264 -> 15.
 #include "common.cuh"
+#include "host_rules.h"
 
 #include <cmath>
 
@@ -156,16 +158,8 @@ template <int MW, int TM, int TN, int STAGES> int gf_run(const GfCall &c) {
     return JK_OK;
 }
 
-// The tile by what a launch of it takes, from measurements at K 1,536 (us): `first` for a block on every SM, `each` for every
-// further one, where blocks of one SM run side by side.  Outputs of few tiles take small ones until they fill the SMs
-// (24 x 2,560: 27 us with 16 x 32 against 37 with 32 x 64; 60 x 7,680: 45 with 64 x 64 against 51 with 16 x 32).
-struct GfTile {
-    int rows, cols;
-    float first, each;
-    int (*run)(const GfCall &);
-};
-constexpr GfTile GF_TILES[] = {{8, 64, 14.f, 14.f, gf_run<1, 2, 8, 3>}, {16, 32, 21.f, 7.f, gf_run<1, 4, 4, 4>},
-                               {32, 64, 33.f, 22.f, gf_run<1, 8, 8, 3>}, {64, 64, 42.f, 42.f, gf_run<2, 8, 8, 2>}};
+// by jk::F32_TILES
+constexpr int (*GF_RUN[])(const GfCall &) = {gf_run<1, 2, 8, 3>, gf_run<1, 4, 4, 4>, gf_run<1, 8, 8, 3>, gf_run<2, 8, 8, 2>};
 
 }  // namespace
 
@@ -173,13 +167,8 @@ JK_EXPORT int jk_gemm_f32(const float *A, int lda, const float *W, int ldw, cons
                           float *C, int ldc, int M, int N, int K, cudaStream_t stream) {
     if (M == 0 || N == 0) return JK_OK;
     JK_REQUIRE(M > 0 && N > 0 && K > 0, "gemm_f32: M %d N %d K %d", M, N, K);
-    const GfTile *best = nullptr;
-    float least = 0.f;
-    for (const GfTile &t : GF_TILES) {
-        const long long down = ((long long)M + t.rows - 1) / t.rows, blocks = down * ((N + t.cols - 1) / t.cols);
-        const float cost = fmaxf(t.first, t.each * (float)((blocks + 147) / 148));
-        if (down <= 65535 && (best == nullptr || cost < least)) { best = &t; least = cost; }
-    }
-    JK_REQUIRE(best != nullptr, "gemm_f32: M %d is too large for one launch", M);
-    return best->run(GfCall{A, W, bias, C, M, N, K, lda, ldw, ldc, stream});
+    double us = 0.;
+    const int tile = jk::f32_tile(M, N, 148, &us);
+    JK_REQUIRE(tile >= 0, "gemm_f32: M %d is too large for one launch", M);
+    return GF_RUN[tile](GfCall{A, W, bias, C, M, N, K, lda, ldw, ldc, stream});
 }

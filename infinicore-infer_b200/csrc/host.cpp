@@ -96,6 +96,11 @@ JK_HOST_EXPORT int jk_product_route(const int *routing, int rows, int n, int k, 
 JK_HOST_EXPORT int jk_takes_tcgen05(const int *routing, int rows, int n, int k) {
     return jk::takes_tcgen05(routing_of(routing), rows, n, k) ? 1 : 0;
 }
+JK_HOST_EXPORT int jk_f32_plan(long long rows, long long n, long long k, int sms) {      // tokens a tile << 8 | cuts of K
+    const jk::F32Plan p = jk::f32_plan(rows, n, k, sms);
+    return p.tile << 8 | p.cuts;
+}
+JK_HOST_EXPORT int jk_f32_tensor_rows() { return jk::F32_TENSOR_ROWS; }
 JK_HOST_EXPORT void jk_rotary_tables(double theta, int half, int positions, double angle_scale, float *cos_out, float *sin_out) {
     jk::rotary_tables(theta, half, positions, angle_scale, cos_out, sin_out);
 }

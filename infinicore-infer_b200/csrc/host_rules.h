@@ -6,7 +6,7 @@
 //   - the layout of a step's metadata buffer and the packing of a batch into it;
 //   - the attention mixer's work lists (rows of requests that bring few rows, tiles of the others);
 //   - how many ways the decode attention cuts a row's keys;
-//   - which kernel takes a bfloat16 product of a given shape;
+//   - which kernel takes a product of a given shape;
 //   - the rotary tables;
 //   - the uniform number for the token at a position of a request.
 #pragma once
@@ -437,6 +437,53 @@ inline Route product_route(const Routing &r, int rows, int n, int k, int kind, b
     }
     if (tcgen05_ok && takes_tcgen05(r, rows, n, k)) return ROUTE_TCGEN05;
     return ROUTE_LIBRARY;
+}
+
+// ---- which kernel takes a float32 product ---------------------------------------------------------------------------
+// On the CUDA cores (csrc/gemm_f32.cu), the tile by what a launch of it takes, from measurements at K 1,536 (us): `first` for a
+// block on every SM, `each` for every further one, where blocks of one SM run side by side.  Outputs of few tiles take small ones
+// until they fill the SMs (24 x 2,560: 27 us with 16 x 32 against 37 with 32 x 64; 60 x 7,680: 45 with 64 x 64 against 51 with 16 x 32).
+struct F32Tile { int rows, cols; double first, each; };
+constexpr F32Tile F32_TILES[] = {{8, 64, 14., 14.}, {16, 32, 21., 7.}, {32, 64, 33., 22.}, {64, 64, 42., 42.}};
+// the tile's place in that list, or -1 where no launch holds them; `us`: what it takes at K 1,536
+inline int f32_tile(long long M, long long N, int sms, double *us) {
+    int best = -1;
+    for (int i = 0; i < 4; ++i) {
+        const F32Tile &t = F32_TILES[i];
+        const long long down = (M + t.rows - 1) / t.rows, blocks = down * ((N + t.cols - 1) / t.cols);
+        const double cost = std::max(t.first, t.each * (double)((blocks + sms - 1) / sms));
+        if (down <= 65535 && (best < 0 || cost < *us)) { best = i; *us = cost; }
+    }
+    return best;
+}
+// On the tensor cores (csrc/gemm_f32_tcgen05.cu) with the operands split: tokens a tile and cuts of K, or a tile of 0 where the
+// product stays on the CUDA cores.  A wave takes 0.8 us, 2.8 more with cuts, 0.036 a token of the tile, and a chunk of 64 columns of K its
+// tile's time; fitted to 1,700 launches of 18 shapes with 16 to 2,048 rows, nine of ten within 8 %, and what the fit chooses is within
+// 12 % of the fastest form everywhere.  A block fills an SM, and clusters of four or eight leave some SMs of a chip of 148 without a block:
+// 33 and 14 of them run at once (three tiles of 96 x 12 of 128, four cuts, 36 clusters: 29 us where 24 clusters take 20).
+// From F32_TENSOR_ROWS rows on, so that steps of few rows (decoding) add in an order that does not depend on the batch, and from K 512:
+// below, a launch costs what it saves.  CUDA cores -> tensor cores (us): 301 rows, 7,680 x 1,536 199 -> 45, 2,560 x 1,536 73 -> 27, 1,536 x 1,536
+// 46 -> 20, 1,536 x 3,840 108 -> 33; 24 rows, 1,536 x 1,536 20 -> 10; 48 rows, 2,560 x 1,536 23 -> 14; 2,048 rows, 4,608 x 4,096 1,768 -> 397.
+struct F32Plan { int tile, cuts; };
+constexpr int F32_TENSOR_ROWS = 24, F32_TENSOR_K = 512;
+inline F32Plan f32_plan(long long M, long long N, long long K, int sms) {
+    F32Plan best = {0, 1};
+    if (M < F32_TENSOR_ROWS || K < F32_TENSOR_K || sms <= 0) return best;
+    constexpr int TILES[5] = {32, 64, 96, 128, 160};
+    constexpr double CHUNK[5] = {1.25, 1.30, 1.30, 1.42, 1.57};
+    double least = 0.;
+    if (f32_tile(M, N, sms, &least) < 0) least = 1e30;
+    least = least * (double)K / 1536. + 2.;
+    const long long chunks = (K + 63) / 64;
+    for (int i = 0; i < 5; ++i)
+        for (int cuts = 1; cuts <= 8; cuts *= 2) {
+            const long long blocks = (M + TILES[i] - 1) / TILES[i] * ((N + 127) / 128) * cuts;
+            if (blocks > (1LL << 30) || (cuts > 1 && (chunks < 2 * cuts || blocks > (cuts == 8 ? sms * 112 / 148 : cuts == 4 ? sms * 132 / 148 : sms)))) continue;
+            const double cost = (double)((blocks + sms - 1) / sms) *
+                                (0.8 + (cuts > 1 ? 2.8 : 0.) + 0.036 * TILES[i] + CHUNK[i] * (double)((chunks + cuts - 1) / cuts));
+            if (cost < least) { least = cost; best = {TILES[i], cuts}; }
+        }
+    return best;
 }
 
 // ---- rotary tables --------------------------------------------------------------------------------------------

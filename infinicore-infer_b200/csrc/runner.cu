@@ -3,7 +3,8 @@
 // One call launches every kernel of a run of records (for the standard stack: the whole step, embedding to logits)
 // where Python would make a dozen calls a layer.  Which kernel runs a record is decided here and nowhere else:
 //
-//   float32       every product on the CUDA cores (gemm_f32, no tensor cores), attention by the row kernel
+//   float32       products of few rows on the CUDA cores (gemm_f32), of many rows on the tensor cores with every operand split into
+//                 three bfloat16 parts (gemm_f32_tcgen05), by jk::f32_plan; attention by the row kernel
 //   bfloat16      products by the rules of host_rules.h (jk::product_route):
 //                   rows <= 16          the weight-streaming kernels of linear_small.cu (q/k/v with rotation and cache
 //                                       write in the epilogue, gate/up with SwiGLU in the epilogue)
@@ -56,6 +57,8 @@ JK_EXPORT int jk_runner_bind(const RunnerFns *fns) {
                (f.layernorm != nullptr) == (f.conv_qkv != nullptr) && (f.layernorm != nullptr) == (f.linear_scan != nullptr) &&
                (f.layernorm != nullptr) == (f.norm_gate != nullptr) && (f.layernorm != nullptr) == (f.err_mixers != nullptr) &&
                (f.layernorm != nullptr) == (f.token_shift != nullptr) && (f.layernorm != nullptr) == (f.act_rows != nullptr),
+               "runner_bind: a module's entries come together");
+    JK_REQUIRE((f.gemm_f32_tcgen05 != nullptr) == (f.gemm_f32_tcgen05_supports != nullptr) && (f.gemm_f32_tcgen05 != nullptr) == (f.err_gemm_f32_tcgen05 != nullptr),
                "runner_bind: a module's entries come together");
     {
         void *const *first = (void *const *)&f.norm_add, *const *last = (void *const *)&f.err_blocks;
@@ -144,14 +147,25 @@ struct Run {
     float *delta() const { return (float *)buf.slot[SLOT_DELTA]; }
 };
 
+// out [rows, n] = act * w^T (+ bias), all float32: on the tensor cores by jk::f32_plan, else (and where rows do not start on 16 bytes) on
+// the CUDA cores
+int float32_product(Run &r, const float *act, const float *w, const float *bias, float *out, int rows, int n, int k, int ldc) {
+    if (g_fns.gemm_f32_tcgen05 != nullptr && !r.env.routing.library_only && r.env.status != nullptr) {
+        const jk::F32Plan plan = jk::f32_plan(rows, n, k, r.env.routing.sms);
+        if (plan.tile > 0 && g_fns.gemm_f32_tcgen05_supports(act, k, w, k, rows, n, k)) {
+            RUN(gemm_f32_tcgen05, g_fns.gemm_f32_tcgen05(act, k, w, k, bias, out, ldc, rows, n, k, plan.tile, plan.cuts, r.env.status, r.stream));
+            return JK_OK;
+        }
+    }
+    RUN(elementwise, g_fns.gemm_f32(act, k, w, k, bias, out, ldc, rows, n, k, r.stream));
+    return JK_OK;
+}
+
 // out (float32 [rows, n]) = act * w^T (+ bias) by whichever kernel takes `rows`
 // (`ldc` > 0: rows of out are that many floats apart)
 int product_f32(Run &r, const void *act, const void *w, const float *bias, float *out, int rows, int n, int k, int ldc = 0) {
     if (ldc <= 0) ldc = n;
-    if (r.env.dtype == JK_F32) {
-        RUN(elementwise, g_fns.gemm_f32((const float *)act, k, (const float *)w, k, bias, out, ldc, rows, n, k, r.stream));
-        return JK_OK;
-    }
+    if (r.env.dtype == JK_F32) return float32_product(r, (const float *)act, (const float *)w, bias, out, rows, n, k, ldc);
     // a bias outside q/k/v (whose bias the rotary kernel adds) does not occur in this architecture; no kernel adds one
     JK_REQUIRE(bias == nullptr, "runner: a bfloat16 product with a bias outside q/k/v is not built");
     const jk::Routing &ro = r.env.routing;
@@ -394,7 +408,7 @@ int run_gate_up(Run &r, const RunnerOp &op, const FusedNorm &fused) {
     void *tmp;
     if (int rc = r.slot(SLOT_TMP, 4LL * T * 2 * di, &tmp, "the gate/up product")) return rc;
     if (r.env.dtype == JK_F32) {
-        RUN(elementwise, g_fns.gemm_f32((const float *)h, d, (const float *)op.w, d, nullptr, (float *)tmp, 2 * di, T, 2 * di, d, r.stream));
+        if (int rc = float32_product(r, (const float *)h, (const float *)op.w, nullptr, (float *)tmp, T, 2 * di, d, 2 * di)) return rc;
     } else if (clamped) {
         if (int rc = product_f32(r, h, op.w, nullptr, (float *)tmp, T, 2 * di, d)) return rc;       // by the rows' route, float32 sums
     } else {
@@ -579,7 +593,7 @@ int run_reinject(Run &r, const RunnerOp &op) {
     if (int rc = flush_pending(r, T, op.n)) return rc;
     RUN(blocks, g_fns.concat_cast(r.x(), (const float *)x0, both, r.env.dtype, T, op.n, r.stream));
     if (r.env.dtype == JK_F32) {
-        RUN(elementwise, g_fns.gemm_f32((const float *)both, op.k, (const float *)op.w, op.k, op.vec, r.x(), op.n, T, op.n, op.k, r.stream));
+        if (int rc = float32_product(r, (const float *)both, (const float *)op.w, op.vec, r.x(), T, op.n, op.k, op.n)) return rc;
         return JK_OK;
     }
     if (int rc = product_f32(r, both, op.w, nullptr, r.x(), T, op.n, op.k)) return rc;

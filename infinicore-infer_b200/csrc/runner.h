@@ -23,6 +23,8 @@ typedef int (*RopeKvFn)(const void *, int, int, const float *, const int *, cons
                         const float *, const float *, int, void *, void *, void *, int, int, int, int, int, int,
                         cudaStream_t);
 typedef int (*GemmF32Fn)(const float *, int, const float *, int, const float *, float *, int, int, int, int, cudaStream_t);
+typedef int (*GemmF32SplitFn)(const float *, int, const float *, int, const float *, float *, int, int, int, int, int, int, int *, cudaStream_t);
+typedef int (*GemmF32SupportsFn)(const float *, int, const float *, int, int, int, int);
 typedef int (*LinearSmallFn)(const void *, const void *, void *, int, int, int, int, int, int, cudaStream_t);
 typedef int (*LinearSmallQkvFn)(const void *, const void *, int, int, void *, void *, void *, const float *, const float *,
                                 const int *, const int *, const int *, int, int, int, int, int, int, cudaStream_t);
@@ -190,6 +192,10 @@ struct RunnerFns {
     LatentGatherFn latent_gather;
     SelectiveScratchFn selective_scan_scratch;
     AttentionLaidFn attention_laid;
+    // float32 products of many rows on the tensor cores (csrc/gemm_f32_tcgen05.cu): bound together, or not at all
+    GemmF32SplitFn gemm_f32_tcgen05;
+    GemmF32SupportsFn gemm_f32_tcgen05_supports;
+    LastErrorFn err_gemm_f32_tcgen05;
 };
 
 // ---- records ---------------------------------------------------------------------------------------------------

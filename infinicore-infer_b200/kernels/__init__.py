@@ -177,6 +177,25 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional
     return out
 
 
+def gemm_f32_tcgen05(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None, tile: int = 0, cuts: int = 1) -> torch.Tensor:
+    """The same product with the operands split into three bfloat16 parts on the tensor cores: errors as ``gemm_f32``'s or smaller, sums
+    in an order that depends on ``tile`` (tokens: 32, 64, 96, 128 or 160; 0: by the rule, or 96) and ``cuts`` of K (1, 2, 4 or 8)."""
+    _need(a, "a", torch.float32); _need(w, "w", torch.float32); _need(out, "out", torch.float32)
+    m, k = a.shape
+    n = w.shape[0]
+    if w.shape[1] != k or tuple(out.shape) != (m, n):
+        raise KernelError(f"gemm_f32_tcgen05: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+    if bias is not None:
+        _need(bias, "bias", torch.float32)
+    if tile == 0:
+        tile, cuts = _host.f32_plan(m, n, k, _sm_count(a.device))
+        tile = tile or 96
+    _check("gemm_f32_tcgen05", _build.load("gemm_f32_tcgen05").jk_gemm_f32_tcgen05(
+        _ptr(a), _c_int(k), _ptr(w), _c_int(k), _ptr(bias), _ptr(out), _c_int(n), _c_int(m), _c_int(n), _c_int(k), _c_int(tile), _c_int(cuts),
+        _ptr(gemm_status(a.device)), _stream()))
+    return out
+
+
 EPI_F32, EPI_SWIGLU, EPI_RESIDUAL = 0, 1, 3
 
 
@@ -370,6 +389,9 @@ def check_gemm_status(device) -> None:
                 raise KernelError("linear_small: a row's sum of squares is beyond the range of the fixed-point counters "
                                   "(activations of several thousand on average); the step's results are not valid; "
                                   "JK_NO_FUSED_NORM=1 keeps the norm kernels, which have no such limit")
+            if 31 <= code <= 33:
+                raise KernelError(f"gemm_f32_tcgen05: a bounded wait ran out (role {code - 30}: 1 MMA, 2 tokens, 3 weights and sums); "
+                                  "the step's results are not valid")
             raise KernelError(f"gemm_tcgen05: a bounded wait ran out (role {code}: 1 TMA, 2 MMA, 3 epilogue); "
                               "the step's results are not valid")
 

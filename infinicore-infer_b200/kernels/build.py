@@ -28,6 +28,7 @@ MODULES: Dict[str, List[str]] = {
     "sampling": ["sampling.cu"],
     "linear_small": ["linear_small.cu"],
     "gemm_tcgen05": ["gemm_tcgen05.cu", "gemm_skinny.cu"],
+    "gemm_f32_tcgen05": ["gemm_f32_tcgen05.cu"],
     "attention_tcgen05": ["attention_tcgen05.cu"],
     "mixers": ["mixers.cu"],
     "blocks": ["blocks.cu"],

@@ -187,6 +187,17 @@ def product_route(routing: Sequence[int], rows: int, n: int, k: int, kind: int, 
     return lib().jk_product_route(arr, rows, n, k, kind, int(small_ok), int(tcgen05_ok))
 
 
+def f32_plan(rows: int, n: int, k: int, sms: int = 148):
+    """(tokens a tile, cuts of K) of a float32 product that goes to the tensor cores; (0, 1) where it stays on the CUDA cores."""
+    plan = lib().jk_f32_plan(rows, n, k, sms)
+    return plan >> 8, plan & 255
+
+
+def f32_tensor_rows() -> int:
+    """Fewest rows of a float32 product on the tensor cores."""
+    return lib().jk_f32_tensor_rows()
+
+
 # ---- tables and uniforms -----------------------------------------------------------------------------------------------
 def rotary_tables(theta: float, half: int, positions: int, angle_scale: float = 1.0):
     """(cos, sin) float32 ``[positions, half]``: angle of pair j at position p = angle_scale * p / theta^(j / half),

@@ -111,27 +111,31 @@ class _Fns(ctypes.Structure):
         "latent_attention_scratch", "causal_conv", "selective_scan", "routed_experts", "routed_experts_workspace",
         "routed_experts_launches", "softcap", "err_blocks", "linear_small_parts", "linear_small_parts_supports", "add_rows", "delta_rule", "delta_rule_scratch",
         "norm_pair", "embed_pair", "join_parts", "gated_recurrence", "gated_recurrence_scratch", "gated_recurrence_launches", "rotate_rows", "latent_gather", "selective_scan_scratch",
-        "attention_laid")]
+        "attention_laid", "gemm_f32_tcgen05", "gemm_f32_tcgen05_supports", "err_gemm_f32_tcgen05")]
 
 
 def _addr(lib, name: str) -> int:
     return ctypes.cast(getattr(lib, name), ctypes.c_void_p).value
 
 
-_bound: Dict[str, bool] = {"base": False, "gemm_tcgen05": False, "attention_tcgen05": False, "mixers": False, "blocks": False}
+_bound: Dict[str, bool] = {"base": False, "gemm_tcgen05": False, "attention_tcgen05": False, "mixers": False, "blocks": False,
+                           "gemm_f32_tcgen05": False}
 
 
-def runner_lib(gemm_tcgen05: bool = False, attention_tcgen05: bool = False, mixers: bool = False, blocks: bool = False) -> ctypes.CDLL:
+def runner_lib(gemm_tcgen05: bool = False, attention_tcgen05: bool = False, mixers: bool = False, blocks: bool = False,
+               gemm_f32_tcgen05: bool = False) -> ctypes.CDLL:
     """The native step's library with the kernel modules' entry points handed over.  The tcgen05 modules and the module of
     the mixers beyond softmax attention are bound (and so compiled) only when asked for: a model whose steps never reach
     them never builds them."""
     lib = _build.load("runner")
-    want = {"base": True, "gemm_tcgen05": gemm_tcgen05, "attention_tcgen05": attention_tcgen05, "mixers": mixers, "blocks": blocks}
+    want = {"base": True, "gemm_tcgen05": gemm_tcgen05, "attention_tcgen05": attention_tcgen05, "mixers": mixers, "blocks": blocks,
+            "gemm_f32_tcgen05": gemm_f32_tcgen05}
     if all(_bound[k] or not want[k] for k in want):
         return lib
     lib.jk_runner_last_error.restype = ctypes.c_char_p
     names = ["elementwise", "linear_small", "attention", "sampling"] + (["gemm_tcgen05"] if gemm_tcgen05 else []) \
-        + (["attention_tcgen05"] if attention_tcgen05 else []) + (["mixers"] if mixers else []) + (["blocks"] if blocks else [])
+        + (["attention_tcgen05"] if attention_tcgen05 else []) + (["mixers"] if mixers else []) + (["blocks"] if blocks else []) \
+        + (["gemm_f32_tcgen05"] if gemm_f32_tcgen05 else [])
     mods = {m: _build.load(m) for m in names}
     get = lambda module, name: _addr(mods[module], name) if module in mods else None
     fns = _Fns(
@@ -175,7 +179,9 @@ def runner_lib(gemm_tcgen05: bool = False, attention_tcgen05: bool = False, mixe
         norm_pair=get("blocks", "jk_norm_pair"), embed_pair=get("blocks", "jk_embed_pair"), join_parts=get("blocks", "jk_join_parts"),
         gated_recurrence=get("blocks", "jk_gated_recurrence"), gated_recurrence_scratch=get("blocks", "jk_gated_recurrence_scratch_floats"),
         gated_recurrence_launches=get("blocks", "jk_gated_recurrence_launches"), rotate_rows=get("mixers", "jk_rotate_rows"),
-        latent_gather=get("blocks", "jk_latent_gather"), selective_scan_scratch=get("blocks", "jk_selective_scan_scratch_floats"), attention_laid=get("attention_tcgen05", "jk_attention_laid_tcgen05"))
+        latent_gather=get("blocks", "jk_latent_gather"), selective_scan_scratch=get("blocks", "jk_selective_scan_scratch_floats"), attention_laid=get("attention_tcgen05", "jk_attention_laid_tcgen05"),
+        gemm_f32_tcgen05=get("gemm_f32_tcgen05", "jk_gemm_f32_tcgen05"), gemm_f32_tcgen05_supports=get("gemm_f32_tcgen05", "jk_gemm_f32_tcgen05_supports"),
+        err_gemm_f32_tcgen05=get("gemm_f32_tcgen05", "jk_gemm_f32_tcgen05_last_error"))
     if lib.jk_runner_bind(ctypes.byref(fns)):
         from ..kernels import KernelError
         raise KernelError(lib.jk_runner_last_error().decode(errors="replace"))
@@ -351,7 +357,8 @@ def modules_needed(env: RunnerEnv, ops, count: int, max_rows: int) -> Dict[str, 
             "attention_tcgen05": env.dtype == _dtype_code(torch.bfloat16) and not env.legacy_tensor_cores and (heads or any(
                 op.kind == OP["attention"] and _host.attention_tcgen05_takes(op.head_dim, env.page_size, op.v_head_dim) for op in records)),
             "mixers": any(op.kind in _MIXERS_OPS or (op.kind == OP["gate_up"] and op.act > ACT["silu"]) for op in records),
-            "blocks": any(op.kind in _BLOCKS_OPS for op in records)}
+            "blocks": any(op.kind in _BLOCKS_OPS for op in records),
+            "gemm_f32_tcgen05": env.dtype == _dtype_code(torch.float32) and not env.routing.library_only and max_rows >= _host.f32_tensor_rows()}
 
 
 def free_bytes(device) -> int:

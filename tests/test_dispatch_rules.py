@@ -93,3 +93,19 @@ def test_tiles_of_the_routed_experts(rows, experts, top, width, ff, tiles):
 def test_way_of_a_latent_attention(dim, rot, rank, requests, window, heads):
     rows, keys = sum(n for n, _ in requests), sum(n + p for n, p in requests)
     assert host.latent_takes_heads(rows, len(requests), keys, window, dim, rot, dim, rank) == heads
+
+
+@pytest.mark.parametrize("rows,n,k,tensor", [
+    # microseconds: on the CUDA cores, on the tensor cores
+    (16, 2560, 1536, False), (23, 7680, 1536, False),               # few rows keep the order of sums that single rows have
+    (24, 1536, 1536, True), (32, 11264, 2048, True),                # 20, 10; 52, 45
+    (301, 7680, 1536, True), (301, 1536, 3840, True),               # 199, 45; 108, 33
+    (64, 64, 2048, True), (2048, 512, 512, True),                   # 19, 9; 35, 14
+    (32, 512, 512, False), (64, 512, 512, False),                   # 7, 7; 7, 7
+    (301, 288, 96, False), (640, 1024, 256, False)])                # 3, 5; 15, 9: short sums stay
+def test_float32_products_on_the_tensor_cores(rows, n, k, tensor):
+    tile, cuts = host.f32_plan(rows, n, k)
+    assert (tile != 0) == tensor
+    # the blocks of clusters that run at once on 148 SMs, one a block: 33 of four, 14 of eight
+    blocks = -(-rows // tile) * -(-n // 128) * cuts if tile else 0
+    assert cuts in (1, 2, 4, 8) and (cuts == 1 or blocks <= {2: 148, 4: 132, 8: 112}[cuts])

@@ -127,6 +127,40 @@ def test_gemm_f32_tiles_agree_bit_for_bit(K, M, N, K_):
         assert torch.equal(part, out[rows, cols])
 
 
+@pytest.mark.parametrize("M,N,K_", [(1, 1, 4), (33, 130, 68), (97, 127, 1024), (161, 257, 640), (301, 129, 3840)])
+@pytest.mark.parametrize("tile,cuts", [(32, 1), (32, 8), (64, 4), (96, 2), (128, 1), (160, 1), (160, 4)])
+def test_gemm_f32_tcgen05_keeps_float32(K, M, N, K_, tile, cuts):
+    """Tokens, features and K at the edges of their tiles, cuts of K with and without chunks of their own."""
+    g = torch.Generator().manual_seed(M + N + K_)
+    a, w, bias = torch.randn(M, K_, generator=g).to(DEV), torch.randn(N, K_, generator=g).to(DEV), torch.randn(N, generator=g).to(DEV)
+    out, plain = torch.full((M, N), 7.0, device=DEV), torch.empty(M, N, device=DEV)
+    K.gemm_f32_tcgen05(a, w, out, bias, tile=tile, cuts=cuts)
+    K.check_gemm_status(DEV)
+    want = a.double() @ w.double().T + bias.double()
+    # a chunk's sum is cut off at most 24 times (a unit in the last place, 2^-23 of what is summed: below 25 x 64), then ceil(K / 64) sums round
+    size = (a.double().abs() @ w.double().abs().T + bias.double().abs()).max().item()
+    assert (out.double() - want).abs().max().item() <= 2.0 ** -23 * size
+    K.gemm_f32(a, w, plain, bias)
+    # no further off than the multiply-adds in float32, but for what three units in the last place of the few outputs' sizes make
+    assert (out.double() - want).norm() <= (plain.double() - want).norm() + 3 * 2.0 ** -24 * want.norm()
+
+
+@pytest.mark.parametrize("cuts", [1, 4])
+def test_gemm_f32_tcgen05_what_the_split_does_not_carry(K, cuts):
+    """Infinities, NaN and magnitudes that bfloat16 rounds to infinity: what float32 multiply-adds give."""
+    g = torch.Generator().manual_seed(5)
+    a, w = torch.randn(40, 512, generator=g), torch.randn(200, 512, generator=g)
+    a[3, 5], a[7, 9], a[9, 1], w[11, 0], w[12, 4] = math.inf, math.nan, -math.inf, 3.4e38, 1e-42
+    a, w = a.to(DEV), w.to(DEV)
+    out, plain = torch.empty(40, 200, device=DEV), torch.empty(40, 200, device=DEV)
+    K.gemm_f32_tcgen05(a, w, out, tile=32, cuts=cuts)
+    K.gemm_f32(a, w, plain)
+    assert torch.equal(out.isnan(), plain.isnan()) and torch.equal(out.isinf(), plain.isinf())
+    assert torch.equal(out[out.isinf()], plain[plain.isinf()])
+    ok = plain.isfinite()
+    assert ((out - plain).abs()[ok] <= 1e-6 * plain.abs()[ok] + 2e-4).all()
+
+
 def _scatter_pages(k, v, tables, page, num_pages, dtype, junk=7.0):
     """Dense per-request keys/values [len, nkvh, dh] -> pages [num_pages, nkvh, page, dh]."""
     nkvh, dh = k[0].shape[1:]
