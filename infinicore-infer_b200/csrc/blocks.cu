@@ -774,6 +774,23 @@ __device__ __forceinline__ void tile_product_split(const float *__restrict__ A, 
     }
 }
 
+// What earlier kernels wrote, read after the wait for them.  A plain load through a restricted pointer to constant data may be moved over
+// that wait, which is no barrier for data that the compiler takes for constant; these are not moved over other volatile statements.
+__device__ __forceinline__ int written_int(const int *p) {
+    int v;
+    asm volatile("ld.global.b32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ float written_float(const float *p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];\n" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void bulk_load(void *smem, const void *from, int bytes, unsigned long long *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
+                 ::"r"(smem_u32(smem)), "l"(from), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+
 // out[t, h * out_hs + n] = T(sum_k in[t, h * K + k] * w[h, n, k]) (* sigmoid(gate[t * gate_ld + h * N + n]), or with gate_head
 // sigmoid(gate[t * gate_ld + h]))
 template <typename T>
@@ -796,11 +813,81 @@ __global__ void __launch_bounds__(256) head_linear_kernel(const T *__restrict__ 
     }
 }
 
+// The same for few rows (bfloat16): a block a head, 32 features and 16 rows, a warp eight of the features.  Weights and rows come whole by bulk copies
+// (TMA), 16 bytes apart from row to row of shared memory so that ldmatrix meets every bank once; the weights before the kernel before has
+// ended.  The MMAs and their order are those of the tiles: the same bits.
+// What bounds it: latency, of one round of copies where the tiles wait for K / 32 of them.
+// B200, tiles of 64 x 64 -> this (us): 16 heads of 512 x 128, one row 4.9 -> 2.1, 16 5.2 -> 3.0, 64 7.8 -> 4.8; of 128 x 512 6.8 -> 2.3, 7.2 -> 2.8, 7.8 -> 4.0;
+// 40 of 512 x 128 5.6 -> 3.5, 64 rows 11.0 -> 8.0; 2 of 64 x 64 2.3 -> 1.4, 64 rows 2.8 -> 2.0.
+constexpr int HR_ROWS = 16, HR_FEATURES = 32, HR_THREADS = 32 * HR_FEATURES / 8;
+static size_t head_rows_smem(int K) { return (size_t)(HR_ROWS + HR_FEATURES) * (2 * K + 16) + 64; }
+static bool head_takes_rows(int rows, int K) { return rows <= 64 && K % 16 == 0 && head_rows_smem(K) <= 100 * 1024; }
+
+__global__ void __launch_bounds__(HR_THREADS) head_rows_kernel(const __nv_bfloat16 *in, const __nv_bfloat16 *w, __nv_bfloat16 *out, int rows, int H, int N, int K, int out_hs,
+                                                               const float *gate, int gate_ld, int gate_head) {
+    extern __shared__ __align__(128) unsigned char hr_smem[];
+    __shared__ unsigned long long full[2];
+    pdl_trigger();
+    const int h = blockIdx.y, n0 = blockIdx.x * HR_FEATURES, t0 = blockIdx.z * HR_ROWS, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pitch = 2 * K + 16;
+    unsigned char *xs = hr_smem, *ws = hr_smem + HR_ROWS * pitch;
+    if (threadIdx.x == 0) {
+        mbar_init(&full[0], 1);
+        mbar_init(&full[1], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncthreads();
+    const int count = min(HR_ROWS, rows - t0);
+    if (warp == 0) {
+        if (lane == 0) mbar_expect_tx(&full[0], HR_FEATURES * 2 * K);
+        __syncwarp();
+        bulk_load(ws + lane * pitch, w + ((size_t)h * N + min(n0 + lane, N - 1)) * K, 2 * K, &full[0]);
+    }
+    pdl_wait();
+    if (warp == 0) {
+        if (lane == 0) mbar_expect_tx(&full[1], count * 2 * K);
+        __syncwarp();
+        if (lane < count) bulk_load(xs + lane * pitch, in + ((size_t)(t0 + lane) * H + h) * K, 2 * K, &full[1]);
+    }
+    // a warp whose features lie behind the last one has nothing to do
+    const bool ok = mbar_wait(&full[0], 0) && mbar_wait(&full[1], 0);
+    if (n0 + warp * 8 >= N) return;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    const __nv_bfloat16 *a_at = reinterpret_cast<const __nv_bfloat16 *>(xs + (lane & 15) * pitch) + (lane >> 4) * 8;
+    const __nv_bfloat16 *b_at = reinterpret_cast<const __nv_bfloat16 *>(ws + (warp * 8 + (lane & 7)) * pitch) + (lane >> 3) * 8;
+#pragma unroll 4
+    for (int k = 0; k < K; k += 32) {           // weights of 32 columns at once
+        unsigned a0, a1, a2, a3, b0, b1, b2, b3;
+        ldmatrix_x4(b0, b1, b2, b3, b_at + k);
+        ldmatrix_x4(a0, a1, a2, a3, a_at + k);
+        mma_bf16_16816(acc, a0, a1, a2, a3, b0, b1);
+        if (k + 16 < K) {
+            ldmatrix_x4(a0, a1, a2, a3, a_at + k + 16);
+            mma_bf16_16816(acc, a0, a1, a2, a3, b2, b3);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = t0 + (lane >> 2) + 8 * (i >> 1), n = n0 + warp * 8 + 2 * (lane & 3) + (i & 1);
+        if (t >= rows || n >= N) continue;
+        float v = ok ? acc[i] : NAN;        // a wait that ran out does not pass for a result
+        if (gate != nullptr) v *= sigmoid_f(written_float(gate + (size_t)t * gate_ld + (gate_head ? (size_t)h : (size_t)h * N + n)));
+        out[((size_t)t * H + h) * out_hs + n] = __float2bfloat16_rn(v);
+    }
+}
+
 JK_EXPORT int jk_head_linear(const void *in, const void *w, void *out, int dtype, int rows, int H, int N, int K, int out_hs,
                              const float *gate, int gate_ld, int gate_head, cudaStream_t stream) {
     if (rows == 0) return JK_OK;
     JK_REQUIRE(in && w && out && rows > 0 && H > 0 && N > 0 && K > 0 && out_hs >= N, "head_linear: rows %d, heads %d, %d x %d into %d", rows, H, N, K, out_hs);
     JK_REQUIRE(H <= 65535, "head_linear: %d heads exceed one launch", H);
+    if (dtype == JK_BF16 && head_takes_rows(rows, K) && (((uintptr_t)in | (uintptr_t)w) & 15) == 0) {
+        const size_t smem = head_rows_smem(K);
+        if (smem > 46 * 1024) cudaFuncSetAttribute(head_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        jk_launch(head_rows_kernel, dim3((N + HR_FEATURES - 1) / HR_FEATURES, H, (rows + HR_ROWS - 1) / HR_ROWS), dim3(HR_THREADS), smem, stream, (const __nv_bfloat16 *)in,
+                  (const __nv_bfloat16 *)w, (__nv_bfloat16 *)out, rows, H, N, K, out_hs, gate, gate_ld, gate_head);
+        JK_CHECK_LAUNCH("head_linear");
+        return JK_OK;
+    }
     dim3 grid((rows + GT_M - 1) / GT_M, (N + GT_N - 1) / GT_N, H);
 #define LAUNCH(T) jk_launch(head_linear_kernel<T>, grid, dim3(256), 0, stream, (const T *)in, (const T *)w, (T *)out, rows, H, N, K, out_hs, gate, gate_ld, gate_head)
     BLOCKS_BY_DTYPE(dtype, "head_linear", LAUNCH);
@@ -2175,93 +2262,180 @@ __global__ void __launch_bounds__(256) expert_down_kernel(const T *__restrict__ 
     }
 }
 
-// Steps of few rows (decoding): an expert has a handful of entries, and its matrices only have to stream past them.  A
-// block of eight warps takes one expert and a slice of its output features; the expert's entries (up to ER_ROWS at a
-// time) wait in shared memory; a warp takes one feature at a time, its lanes 16 bytes of the weight row each
-// per pass, all loads of a row asked for before the sums start.  Float32 sums on the CUDA cores, in the order of K per
-// lane and then across lanes, whatever else the step holds.
-constexpr int ER_ROWS = 8, ER_FEATURES = 32;        // entries at a time; output features a block
+// Steps of few rows (decoding): an expert has a handful of entries, and its matrices only have to stream past them.  A block takes an
+// expert and 16 rows of its matrix: 16 features, or with GLU eight gate rows and the eight up rows that belong to them.  The rows come
+// whole by bulk copies (TMA), 4 KB of each at a time, and so do up to ER_ROWS entries; a warp takes two of the rows (a gate and its up row),
+// its lanes 16 bytes of each a pass.  More entries read the rows again, from shared memory where they fit.  With `eager` the copies of
+// the rows are asked for before the kernel before has ended, which pays where most experts have an entry.  Float32 sums on the CUDA cores, in
+// the order of K per lane and then across lanes, whatever else the step holds.
+// What bounds it: memory, with two to four blocks an SM that keep 130 KB in flight, and for experts of eight entries the multiply-adds.  m16n8k16
+// in their place took a tenth less, but another order of the sums turns a choice of experts further on where two are as good as tied.
+// Whole layers on a B200, the rows loaded by the warps as they need them -> this, the same bits (us): 2,048 x 1,408, 8 experts, 2 a row: one row 37 -> 25,
+// 8 57 -> 51, 16 89 -> 72, 32 131 -> 109; 64 experts, 6 a row: 63 -> 56, 8 rows 162 -> 158; 1,024 x 512, 32 experts, 4 a row 25 -> 21, 8 rows 38 -> 36,
+// 16 69 -> 53; 256 x 4,104, 4 experts 34 -> 23, 8 rows 86 -> 49; 512 x 128, 8 experts 19 -> 15, 32 rows 45 -> 31.  64 registers a thread: with 128 and two
+// blocks an SM at most 8 rows of 1,024 x 512 took 43.
+constexpr int ER_ROWS = 8, EF_BYTES = 4096;          // entries at a time; bytes of a row at a time
+__host__ __device__ constexpr int ef_chunk(int K, int elem) { return K * elem < EF_BYTES ? K * elem : EF_BYTES; }
+__host__ __device__ constexpr int ef_smem(int K, int elem) { return (16 + ER_ROWS) * ef_chunk(K, elem); }
 
-// the features of one block against ROWS staged entries (the caller picks the smallest ROWS that holds them)
-template <typename T, bool GLU, int ROWS>
-__device__ __forceinline__ void expert_rows_features(const T *__restrict__ er_rows, const T *__restrict__ we, void *__restrict__ out, int K, int N,
-                                                     int rows, size_t entry0, const float *__restrict__ entry_score, int actf, float limit) {
-    constexpr int V = Vec16<T>::N;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int f = warp; f < ER_FEATURES; f += 8) {
-        const int n = blockIdx.y * ER_FEATURES + f;
-        if (n >= N) break;
-        const T *wg = we + (size_t)n * K, *wu = we + (size_t)(N + n) * K;
+// The expert of the slot-th run of entries, or -1; a whole warp asks, for up to 256 experts at a time with one wait for memory.
+__device__ __forceinline__ int expert_with_entries(const int *starts, int E, int slot) {
+    const int lane = threadIdx.x & 31;
+    for (int base = 0; base < E; base += 256) {
+        int from[8], to[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int e = base + i * 32 + lane;
+            from[i] = e < E ? written_int(starts + e) : 0;
+            to[i] = e < E ? written_int(starts + e + 1) : 0;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const unsigned some = __ballot_sync(0xffffffffu, to[i] > from[i]);
+            if (slot < __popc(some)) return base + i * 32 + __fns(some, 0, slot + 1);
+            slot -= __popc(some);
+        }
+    }
+    return -1;
+}
+// GLU: act[entry, n] = T(actf(s g) (s u)) from rows of h picked by entry_row; else y[entry, n] = W[e][n] . in[entry].
+// in, starts, entry_row and entry_score are what earlier kernels wrote: no restricted pointers (written_int).  A grid has as many blocks along
+// x as experts, or as entries where those are fewer: then a block looks for its expert.
+struct ExpertRowsArgs {
+    const void *in, *w;
+    void *out;
+    int K, N, E;
+    const int *starts, *entry_row;
+    const float *entry_score;
+    int actf;
+    float limit;
+    int eager;
+    int *status;
+};
+struct ExpertRowsSmem {
+    unsigned char *w, *x;                       // 16 rows, ER_ROWS entries: a chunk of each
+    unsigned long long *w_full, *x_full;
+};
+template <typename T, bool GLU> struct ExpertRowsBlock {
+    const ExpertRowsArgs &a;
+    ExpertRowsSmem s;
+    int e, n0, chunk, chunks;                   // bytes a row at a time, how many times
+    unsigned w_phase = 0, x_phase = 0;          // of the chunk that is there, or on its way
+    bool ok = true, fresh = true;               // fresh: the rows' first chunk is asked for, and nothing else yet
+
+    __device__ __forceinline__ int bytes(int c) const { return min(EF_BYTES, a.K * (int)sizeof(T) - c * EF_BYTES); }
+    // warp 0: a chunk of the 16 rows (features behind N: the last one's, whose results are not stored)
+    __device__ __forceinline__ void bring_rows(int c) {
+        const int lane = threadIdx.x & 31;
+        if (lane == 0) mbar_expect_tx(s.w_full, 16 * bytes(c));
+        __syncwarp();
+        if (lane >= 16) return;
+        const size_t row = ((size_t)e * (GLU ? 2 : 1) + (GLU && lane >= 8 ? 1 : 0)) * a.N + min(n0 + lane % (GLU ? 8 : 16), a.N - 1);
+        bulk_load(s.w + lane * chunk, (const unsigned char *)((const T *)a.w + row * a.K) + (size_t)c * EF_BYTES, bytes(c), s.w_full);
+    }
+    // warp 0: a chunk of `rows` entries from entry `first` on
+    __device__ __forceinline__ void bring_entries(int c, int first, int rows) {
+        const int lane = threadIdx.x & 31;
+        if (lane == 0) mbar_expect_tx(s.x_full, rows * bytes(c));
+        __syncwarp();
+        if (lane >= rows) return;
+        const size_t row = (size_t)(GLU ? written_int(a.entry_row + first + lane) : first + lane);
+        bulk_load(s.x + lane * chunk, (const unsigned char *)((const T *)a.in + row * a.K) + (size_t)c * EF_BYTES, bytes(c), s.x_full);
+    }
+    // the block's features for ROWS entries (the caller picks the smallest ROWS that holds `rows`)
+    template <int ROWS> __device__ __forceinline__ void entries(int first, int rows) {
+        constexpr int V = Vec16<T>::N;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         float g[ROWS], u[ROWS];
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) { g[r] = 0.f; u[r] = 0.f; }
-#pragma unroll 4
-        for (int k = lane * V; k < K; k += 32 * V) {
-            float a[V], b[V];
-            unpack16<T>(*reinterpret_cast<const uint4 *>(wg + k), a);
-            if (GLU) unpack16<T>(*reinterpret_cast<const uint4 *>(wu + k), b);
+        for (int c = 0; c < chunks; ++c) {
+            if (!fresh) __syncthreads();        // what was there has been read
+            if (warp == 0) {
+                if (!fresh && chunks > 1) bring_rows(c);
+                bring_entries(c, first, rows);
+            }
+            if (!fresh) {
+                ++x_phase;
+                if (chunks > 1) ++w_phase;
+            }
+            fresh = false;
+            ok = mbar_wait(s.w_full, w_phase & 1) && ok;
+            ok = mbar_wait(s.x_full, x_phase & 1) && ok;
+            const int size = bytes(c);
+            const unsigned char *one = s.w + warp * chunk, *two = s.w + (warp + 8) * chunk;
+#pragma unroll 1
+            for (int k = lane * 16; k < size; k += 512) {
+                float p[V], q[V];
+                unpack16<T>(*reinterpret_cast<const uint4 *>(one + k), p);
+                unpack16<T>(*reinterpret_cast<const uint4 *>(two + k), q);
 #pragma unroll
-            for (int r = 0; r < ROWS; ++r) {
-                float x[V];
-                unpack16<T>(*reinterpret_cast<const uint4 *>(er_rows + r * K + k), x);
+                for (int r = 0; r < ROWS; ++r) {
+                    float x[V];
+                    unpack16<T>(*reinterpret_cast<const uint4 *>(s.x + r * chunk + k), x);
 #pragma unroll
-                for (int i = 0; i < V; ++i) {
-                    g[r] = fmaf(a[i], x[i], g[r]);
-                    if (GLU) u[r] = fmaf(b[i], x[i], u[r]);
+                    for (int i = 0; i < V; ++i) {
+                        g[r] = fmaf(p[i], x[i], g[r]);
+                        u[r] = fmaf(q[i], x[i], u[r]);
+                    }
                 }
             }
         }
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
             g[r] = warp_sum(g[r]);
-            if (GLU) u[r] = warp_sum(u[r]);
+            u[r] = warp_sum(u[r]);
         }
-        if (lane == 0) {
+        if (lane != 0) return;
+        const int n = n0 + warp;
 #pragma unroll
-            for (int r = 0; r < ROWS; ++r) {
-                if (r >= rows) break;
-                const size_t entry = entry0 + r;
-                if (GLU) {
-                    const float sc = entry_score ? entry_score[entry] : 1.f;
-                    ((T *)out)[entry * N + n] = from_f32<T>(expert_inner(actf, sc, g[r], u[r], limit));
-                } else {
-                    ((float *)out)[entry * N + n] = g[r];
-                }
+        for (int r = 0; r < ROWS; ++r) {
+            if (r >= rows) break;
+            const size_t at = (size_t)(first + r) * a.N + n;
+            if (GLU) {
+                if (n < a.N) ((T *)a.out)[at] = from_f32<T>(expert_inner(a.actf, a.entry_score ? written_float(a.entry_score + first + r) : 1.f, g[r], u[r], a.limit));
+            } else {
+                if (n < a.N) ((float *)a.out)[at] = g[r];
+                if (n + 8 < a.N) ((float *)a.out)[at + 8] = u[r];
             }
         }
     }
-}
+};
 
-// GLU: act[entry, n] = T(actf(s g) (s u)) from rows of h picked by entry_row; else y[entry, n] = W[e][n] . in[entry]
 template <typename T, bool GLU>
-__global__ void __launch_bounds__(256) expert_rows_kernel(const T *__restrict__ in, const T *__restrict__ w, void *__restrict__ out, int K, int N, int E,
-                                                          const int *__restrict__ starts, const int *__restrict__ entry_row,
-                                                          const float *__restrict__ entry_score, int actf, float limit) {
+__global__ void __launch_bounds__(256, 4) expert_rows_kernel(ExpertRowsArgs a) {
+    extern __shared__ __align__(128) unsigned char er_smem[];
+    __shared__ unsigned long long full[2];
     pdl_trigger();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, chunk = ef_chunk(a.K, sizeof(T));
+    if (threadIdx.x == 0) {
+        mbar_init(&full[0], 1);
+        mbar_init(&full[1], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncthreads();
+    ExpertRowsBlock<T, GLU> b{a, {er_smem, er_smem + 16 * chunk, &full[0], &full[1]}, (int)blockIdx.x, (int)blockIdx.y * (GLU ? 8 : 16), chunk,
+                              (a.K * (int)sizeof(T) + EF_BYTES - 1) / EF_BYTES};
+    if (a.eager && warp == 0) b.bring_rows(0);
     pdl_wait();
-    extern __shared__ __align__(16) unsigned char er_smem[];
-    T *er_rows = reinterpret_cast<T *>(er_smem);             // [ER_ROWS][K] as they are stored
-    const int e = blockIdx.x, first = starts[e], M = starts[e + 1] - first;
-    if (M <= 0) return;
-    constexpr int V = Vec16<T>::N;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const T *we = w + (size_t)e * (GLU ? 2 : 1) * N * K;
+    if (gridDim.x < a.E) {
+        b.e = expert_with_entries(a.starts, a.E, b.e);
+        if (b.e < 0) return;
+    }
+    const int first = written_int(a.starts + b.e), M = written_int(a.starts + b.e + 1) - first;
+    if (M <= 0) {
+        if (a.eager && warp == 0) mbar_wait(&full[0], 0);       // the copies end before the block does
+        return;
+    }
+    if (!a.eager && warp == 0) b.bring_rows(0);
     for (int r0 = 0; r0 < M; r0 += ER_ROWS) {
         const int rows = min(ER_ROWS, M - r0);
-        __syncthreads();
-        if (warp < rows) {      // warp r brings entry r: one look at where it lies, then 16 bytes a lane a pass
-            const T *src = in + (size_t)(GLU ? entry_row[first + r0 + warp] : first + r0 + warp) * K;
-#pragma unroll 4
-            for (int k = lane * V; k < K; k += 32 * V)
-                *reinterpret_cast<uint4 *>(er_rows + warp * K + k) = *reinterpret_cast<const uint4 *>(src + k);
-        }
-        __syncthreads();
-        const size_t entry0 = (size_t)(first + r0);
-        if (rows <= 1) expert_rows_features<T, GLU, 1>(er_rows, we, out, K, N, rows, entry0, entry_score, actf, limit);
-        else if (rows <= 2) expert_rows_features<T, GLU, 2>(er_rows, we, out, K, N, rows, entry0, entry_score, actf, limit);
-        else if (rows <= 4) expert_rows_features<T, GLU, 4>(er_rows, we, out, K, N, rows, entry0, entry_score, actf, limit);
-        else expert_rows_features<T, GLU, 8>(er_rows, we, out, K, N, rows, entry0, entry_score, actf, limit);
+        if (rows <= 1) b.template entries<1>(first + r0, rows);
+        else if (rows <= 2) b.template entries<2>(first + r0, rows);
+        else if (rows <= 4) b.template entries<4>(first + r0, rows);
+        else b.template entries<8>(first + r0, rows);
     }
+    if (!b.ok && lane == 0 && a.status != nullptr) atomicExch(a.status, 24);
 }
 
 // v[t] = (what waits in delta, times the row's gate, if `add`) + sum over the row's choices, in their order, of y[pair_entry[t *
@@ -2380,7 +2554,7 @@ JK_EXPORT int jk_routed_experts(const void *h, const float *router, const void *
     const float *in_score = score_form != 0 ? nullptr : entry_score, *out_scores = score_form != 0 ? scores : nullptr;
     const int per16 = dtype == JK_F32 ? 4 : 8;
     const bool stream_rows = pairs <= 64 && D % per16 == 0 && ff % per16 == 0 && (uintptr_t)w_gate_up % 16 == 0 && (uintptr_t)w_down % 16 == 0 &&
-                             (size_t)ER_ROWS * std::max(D, ff) * 4 <= 160 * 1024;
+                             (((uintptr_t)h | (uintptr_t)act) & 15) == 0;
     // Many rows an expert: tiles of 128 entries on tcgen05 (bfloat16, whole vectors, a status word for their waits).
     g_expert_launches = 0;
     const bool tc = dtype == JK_BF16 && !stream_rows && status != nullptr && E <= ET_MAX_EXPERTS && D % 8 == 0 && ff % 8 == 0 && jk::experts_take_tiles(pairs, E, D, ff) &&
@@ -2398,14 +2572,16 @@ JK_EXPORT int jk_routed_experts(const void *h, const float *router, const void *
         if (int rc = launch_expert_tc<false>((const __nv_bfloat16 *)act, (const __nv_bfloat16 *)w_down, dn, down * ((D + ET_BN - 1) / ET_BN), sms, stream)) return rc;
         g_expert_launches = 1;
     } else if (stream_rows) {
-        const size_t elem = dtype == JK_F32 ? 4 : 2, smem_up = (size_t)ER_ROWS * D * elem, smem_down = (size_t)ER_ROWS * ff * elem;
+        // (grids of fewer blocks than experts find out late which expert is theirs)
+        const int elem = dtype == JK_F32 ? 4 : 2, eager = pairs >= 2 * E, smem_up = ef_smem(D, elem), smem_down = ef_smem(ff, elem);
+        const ExpertRowsArgs up{h, w_gate_up, act, D, ff, E, starts, entry_row, in_score, actf, limit, eager, status};
+        const ExpertRowsArgs down{act, w_down, y, ff, D, E, starts, nullptr, nullptr, 0, 0.f, eager, status};
+        const int runs = std::min(E, pairs);
 #define LAUNCH(TT)                                                                                                                           \
-    if (smem_up > 46 * 1024) cudaFuncSetAttribute(expert_rows_kernel<TT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_up);  \
-    if (smem_down > 46 * 1024) cudaFuncSetAttribute(expert_rows_kernel<TT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_down); \
-    jk_launch(expert_rows_kernel<TT, true>, dim3(E, (ff + ER_FEATURES - 1) / ER_FEATURES), dim3(256), smem_up, stream, (const TT *)h,        \
-              (const TT *)w_gate_up, act, D, ff, E, (const int *)starts, (const int *)entry_row, in_score, actf, limit);          \
-    jk_launch(expert_rows_kernel<TT, false>, dim3(E, (D + ER_FEATURES - 1) / ER_FEATURES), dim3(256), smem_down, stream, (const TT *)act,    \
-              (const TT *)w_down, (void *)y, ff, D, E, (const int *)starts, (const int *)nullptr, (const float *)nullptr, 0, 0.f)
+    if (smem_up > 46 * 1024) cudaFuncSetAttribute(expert_rows_kernel<TT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_up);       \
+    if (smem_down > 46 * 1024) cudaFuncSetAttribute(expert_rows_kernel<TT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_down);  \
+    jk_launch(expert_rows_kernel<TT, true>, dim3(runs, (ff + 7) / 8), dim3(256), smem_up, stream, up);                                       \
+    jk_launch(expert_rows_kernel<TT, false>, dim3(runs, (D + 15) / 16), dim3(256), smem_down, stream, down)
         BLOCKS_BY_DTYPE(dtype, "expert rows", LAUNCH);
 #undef LAUNCH
         JK_CHECK_LAUNCH("expert rows");

@@ -161,6 +161,45 @@ def test_gemm_f32_tcgen05_what_the_split_does_not_carry(K, cuts):
     assert ((out - plain).abs()[ok] <= 1e-6 * plain.abs()[ok] + 2e-4).all()
 
 
+@pytest.mark.parametrize("heads,n,k", [(3, 33, 16), (2, 100, 48), (5, 8, 512), (2, 32, 144)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_head_linear_of_few_rows_has_the_tiles_bits(K, heads, n, k, gated):
+    """Rows, features and K at the edges of the few-row kernel's blocks, against 64 bits and against the tiles that many rows take."""
+    g = torch.Generator().manual_seed(n + k)
+    x, w = torch.randn(70, heads * k, generator=g).bfloat16().to(DEV), (torch.randn(heads, n, k, generator=g) * k ** -0.5).bfloat16().to(DEV)
+    gate = torch.randn(70, heads * n, generator=g).to(DEV) if gated else None
+    many = torch.empty(70, heads * n, dtype=torch.bfloat16, device=DEV)
+    K.head_linear(x, w, many, n, gate, heads * n)
+    want = torch.einsum("thk,hnk->thn", x.view(70, heads, k).double(), w.double()).reshape(70, -1) * (torch.sigmoid(gate.double()) if gated else 1.0)
+    assert ((many.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
+    for rows in (1, 15, 16, 17, 64):
+        few = torch.full((rows, heads * n), 7.0, dtype=torch.bfloat16, device=DEV)
+        K.head_linear(x[:rows], w, few, n, None if gate is None else gate[:rows], heads * n)
+        assert torch.equal(few, many[:rows])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,d,ff,experts,top", [(1, 8, 8, 5, 1), (3, 2056, 40, 9, 2), (9, 72, 2064, 2, 1), (21, 64, 24, 3, 3), (2, 64, 16, 300, 8)])
+def test_routed_experts_of_few_rows(K, dtype, rows, d, ff, experts, top):
+    """Rows of a matrix in one piece and in two, features at the edges of the blocks, more entries than run at a time, more experts than entries."""
+    g = torch.Generator().manual_seed(rows + d)
+    h, router = torch.randn(rows, d, generator=g).to(dtype).to(DEV), (torch.randn(experts, d, generator=g) * 2 * d ** -0.5).to(DEV)
+    up = (torch.randn(experts * 2 * ff, d, generator=g) * d ** -0.5).to(dtype).to(DEV)
+    down = (torch.randn(experts * d, ff, generator=g) * ff ** -0.5).to(dtype).to(DEV)
+    out = torch.full((rows, d), 7.0, device=DEV)
+    K.routed_experts(h, router, up, down, out, False, experts, top, 1)
+    K.check_gemm_status(DEV)
+    score, chosen = torch.sigmoid(h.double() @ router.double().T).topk(top, -1)
+    want = torch.zeros(rows, d, dtype=torch.float64, device=DEV)
+    for t in range(rows):
+        for s, e in zip(score[t], chosen[t].tolist()):
+            gate, rest = (up[e * 2 * ff + i * ff: e * 2 * ff + (i + 1) * ff].double() @ (s * h[t].double()) for i in range(2))
+            inner = (torch.nn.functional.silu(gate) * rest).to(dtype).double()      # rounded to the activation type, as it is stored
+            want[t] += down[e * d: (e + 1) * d].double() @ inner
+    # sums of ff terms below 1 in float32; in bfloat16 an inner activation may round the other way (2^-9 of it)
+    assert (out.double() - want).abs().max() <= (2e-5 if dtype == torch.float32 else 2.0 ** -8 * want.abs().max().item())
+
+
 def _scatter_pages(k, v, tables, page, num_pages, dtype, junk=7.0):
     """Dense per-request keys/values [len, nkvh, dh] -> pages [num_pages, nkvh, page, dh]."""
     nkvh, dh = k[0].shape[1:]
