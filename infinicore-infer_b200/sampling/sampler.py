@@ -13,6 +13,7 @@ from __future__ import annotations
 from dataclasses import dataclass
 from typing import List, Sequence
 
+import numpy as np
 import torch
 
 from ..kernels.host import uniform_for      # noqa: F401  (seed, absolute position) -> [0, 1): one rule, written in csrc/host_rules.h
@@ -47,9 +48,14 @@ class Sampler:
         if all(p.greedy for p in params):
             kernels.argmax(logits, out)
         else:
-            host = torch.tensor(
-                [[p.temperature, float(p.topk), p.topp, uniform_for(p.seed, i)] for p, i in zip(params, indices)],
-                dtype=torch.float32).t().contiguous()
-            dev = host.to(self.device)
-            kernels.sample(logits, dev[0], dev[1].to(torch.int32), dev[2], dev[3], out)
+            # One copy from pinned memory that does not wait: the draw is launched while the step still runs.  (A copy from pageable
+            # memory waited for the step, and the device then for this call's launches: a pass of the small named configuration 353 us, 329 so.)
+            host = torch.empty(4, n, dtype=torch.float32, pin_memory=self.device.type == "cuda")
+            rows, most = host.numpy(), 2 ** 31 - 1
+            rows[0] = [p.temperature for p in params]
+            rows[1].view(np.int32)[:] = [max(-most, min(most, int(p.topk))) for p in params]
+            rows[2] = [p.topp for p in params]
+            rows[3] = [uniform_for(p.seed, i) for p, i in zip(params, indices)]
+            dev = host.to(self.device, non_blocking=True)
+            kernels.sample(logits, dev[0], dev[1].view(torch.int32), dev[2], dev[3], out)
         return out.tolist()
