@@ -6,6 +6,9 @@
 // computed in float32 and rounded once when they are stored as bfloat16.
 #include "common.cuh"
 
+#include <algorithm>
+#include <type_traits>
+
 JK_DEFINE_ERROR_BUFFER(jk_elementwise)
 
 // ---------------------------------------------------------------------------------------
@@ -110,12 +113,11 @@ __global__ void add_rmsnorm_kernel(float *__restrict__ x, const TD *__restrict__
     }
 }
 
-// The same for steps of many rows: a warp per row, the row in registers (NV groups of four floats a lane), every load
-// of a row on its way before the first is used, no shared memory and no barrier (a prefill of 2,048 tokens of the 2B
-// shape: 9.94 -> 9.90 ms).
+// The same for steps of many rows of up to 1,024 columns: a warp per row, the row in registers (NV groups of four floats a lane), every load
+// of a row on its way before the first is used, no shared memory and no barrier.
 template <typename TD, typename TO, int NV>
 __global__ void __launch_bounds__(256)
-add_rmsnorm_rows_kernel(float *__restrict__ x, const TD *__restrict__ delta, float delta_scale, const float *__restrict__ w, float eps,
+add_rmsnorm_warp_kernel(float *__restrict__ x, const TD *__restrict__ delta, float delta_scale, const float *__restrict__ w, float eps,
                         float out_scale, TO *__restrict__ out, const int *__restrict__ rows, int nout, int d) {
     pdl_trigger();
     pdl_wait();
@@ -158,6 +160,62 @@ add_rmsnorm_rows_kernel(float *__restrict__ x, const TD *__restrict__ delta, flo
     }
 }
 
+// The same for steps of many rows of 1,024 to 3,072 columns: a block stays and walks over rows, a row in its registers (NV groups of four floats a thread), the norm's
+// weights read once, before the kernel before has ended, and the next row on its way while this one is reduced; one barrier a row.
+// What bounds it: memory, and below a thousand rows the latency of a row.  B200, a warp a row -> this, with a product to add (us): 532 rows of 1,536
+// 8.2 -> 3.3, 2,048 14.1 -> 10.2; 532 of 2,304 13.4 -> 4.6, 2,048 28.9 -> 14.3; 5,003 of 3,072 80 -> 43.  Without one there is
+// less to gain (532 of 1,536 3.0 -> 2.4, but 1,024 of 2,304 4.9 -> 5.8) and the warps keep it.  Narrower rows are left to the warps (5,003 of 256 4.9 -> 5.7), wider ones to a block a row through shared
+// memory (532 of 4,096 8.0 -> 8.5, of 8,192 14.1 -> 17.2).
+// (x and delta are not restricted: what is read ahead of the wait is the weights alone)
+template <typename TO, int NV>
+__global__ void __launch_bounds__(256)
+add_rmsnorm_rows_kernel(float *x, const float *delta, float delta_scale, const float *__restrict__ w, float eps, float out_scale, TO *out, const int *rows, int nout, int d) {
+    pdl_trigger();
+    __shared__ float sums[2][8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, first = threadIdx.x * 4, step = blockDim.x * 4;
+    float4 g[NV], v[NV], p[NV];
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) g[j] = first + j * step < d ? load4(w + first + j * step) : none;
+    pdl_wait();
+    int i = blockIdx.x;
+    size_t at = 0;
+    auto fetch = [&](int row) {
+        at = (size_t)(rows ? rows[row] : row) * d;
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int c = first + j * step;
+            v[j] = c < d ? load4(x + at + c) : none;
+            p[j] = c < d ? load4(delta + at + c) : none;
+        }
+    };
+    if (i < nout) fetch(i);
+    for (int turn = 0; i < nout; i += gridDim.x, turn ^= 1) {
+        float4 u[NV];
+        float ss = 0.f;
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            u[j] = make_float4(v[j].x + delta_scale * p[j].x, v[j].y + delta_scale * p[j].y, v[j].z + delta_scale * p[j].z, v[j].w + delta_scale * p[j].w);
+            const int c = first + j * step;
+            if (rows == nullptr && c < d) store4(x + at + c, u[j]);
+            ss += u[j].x * u[j].x + u[j].y * u[j].y + u[j].z * u[j].z + u[j].w * u[j].w;
+        }
+        if (i + gridDim.x < nout) fetch(i + gridDim.x);
+        ss = warp_sum(ss);
+        if (lane == 0) sums[turn][warp] = ss;
+        __syncthreads();            // the other half of `sums` is free: who reads it has not passed this barrier's predecessor
+        ss = 0.f;
+        for (int k = 0; k < warps; ++k) ss += sums[turn][k];
+        const float inv = rsqrtf(ss / (float)d + eps) * out_scale;
+        TO *o = out + (size_t)i * d;
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int c = first + j * step;
+            if (c < d) store4(o + c, make_float4(u[j].x * inv * g[j].x, u[j].y * inv * g[j].y, u[j].z * inv * g[j].z, u[j].w * inv * g[j].w));
+        }
+    }
+}
+
 template <typename TD, typename TO>
 static int launch_add_rmsnorm(float *x, const void *delta, float delta_scale, const float *w,
                               float eps, float out_scale, void *out, const int *rows, int nout,
@@ -171,11 +229,22 @@ static int launch_add_rmsnorm(float *x, const void *delta, float delta_scale, co
                             : cudaFuncSetAttribute(add_rmsnorm_kernel<TD, TO, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) JK_FAIL(JK_CUDA_ERROR, "add_rmsnorm: %s", cudaGetErrorString(e));
     }
-    if (vec && nout >= 256 && d <= 24 * 128) {
-        // many rows: a warp per row
+    if (vec && std::is_same<TD, float>::value && delta != nullptr && nout >= 256 && d >= 1024 && d <= 3072) {
+        const int threads = d <= 2048 ? 128 : 256, nv = (d / 4 + threads - 1) / threads, blocks = std::min(nout, 148 * 8);
+#define JK_ROWS_LAUNCH(NV_)                                                                                              \
+        jk_launch(add_rmsnorm_rows_kernel<TO, NV_>, dim3(blocks), dim3(threads), 0, stream, x, (const float *)delta, delta_scale, w, eps, \
+                  out_scale, (TO *)out, rows, nout, d)
+        if (nv == 2) JK_ROWS_LAUNCH(2);
+        else if (nv == 3) JK_ROWS_LAUNCH(3);
+        else JK_ROWS_LAUNCH(4);
+#undef JK_ROWS_LAUNCH
+        JK_CHECK_LAUNCH("add_rmsnorm");
+        return JK_OK;
+    }
+    if (vec && nout >= 256 && d <= 3072) {
         const int blocks = (nout + 7) / 8;
 #define JK_ROWS_LAUNCH(NV_)                                                                                              \
-        jk_launch(add_rmsnorm_rows_kernel<TD, TO, NV_>, dim3(blocks), dim3(256), 0, stream, x, (const TD *)delta, delta_scale, w, eps, \
+        jk_launch(add_rmsnorm_warp_kernel<TD, TO, NV_>, dim3(blocks), dim3(256), 0, stream, x, (const TD *)delta, delta_scale, w, eps, \
                   out_scale, (TO *)out, rows, nout, d)
         if (d <= 8 * 128) JK_ROWS_LAUNCH(8);
         else if (d <= 16 * 128) JK_ROWS_LAUNCH(16);
@@ -259,6 +328,21 @@ __global__ void swiglu_kernel(const TI *__restrict__ gu, TO *__restrict__ out, i
     }
 }
 
+// Four units a thread, a block a stretch of a row: no division, 16 bytes a load.  B200, a unit a thread with the row found by a division
+// -> this, the same bits (us): 532 rows of 3,840 to bfloat16 8.6 -> 5.3, 301 to float32 6.2 -> 3.8, 2,048 of 1,408 11.4 -> 6.7, 64 of 5,760 2.5 -> 1.8; below 48K units, or
+// in rows that leave half a block idle, the other way is the faster one (17 of 1,408 1.2 -> 1.3, 2,048 of 136 2.0 -> 2.5).
+template <typename TI, typename TO>
+__global__ void __launch_bounds__(256) swiglu4_kernel(const TI *gu, TO *out, int ntok, int di) {
+    pdl_trigger();
+    pdl_wait();
+    const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
+    if (c >= di) return;
+    for (size_t t = blockIdx.y; t < ntok; t += gridDim.y) {
+        const float4 g = load4(gu + t * 2 * di + c), u = load4(gu + t * 2 * di + di + c);
+        store4(out + t * di + c, make_float4(g.x / (1.f + expf(-g.x)) * u.x, g.y / (1.f + expf(-g.y)) * u.y, g.z / (1.f + expf(-g.z)) * u.z, g.w / (1.f + expf(-g.w)) * u.w));
+    }
+}
+
 JK_EXPORT int jk_swiglu(const void *gu, int in_dtype, void *out, int out_dtype, int ntok, int di,
                         cudaStream_t stream) {
     if (ntok == 0) return JK_OK;
@@ -267,6 +351,15 @@ JK_EXPORT int jk_swiglu(const void *gu, int in_dtype, void *out, int out_dtype, 
     const int threads = 256;
     size_t blocks = (total + threads - 1) / threads;
     if (blocks > 148 * 32) blocks = 148 * 32;
+    if (di % 4 == 0 && di >= 512 && total >= 48 * 1024 && (((uintptr_t)gu | (uintptr_t)out) & 15) == 0 && ((in_dtype == JK_F32) || (in_dtype == JK_BF16 && out_dtype == JK_BF16))) {
+        const dim3 grid((di / 4 + 255) / 256, std::min(ntok, 65535));
+        if (in_dtype == JK_F32 && out_dtype == JK_F32) jk_launch(swiglu4_kernel<float, float>, grid, dim3(256), 0, stream, (const float *)gu, (float *)out, ntok, di);
+        else if (in_dtype == JK_F32 && out_dtype == JK_BF16) jk_launch(swiglu4_kernel<float, __nv_bfloat16>, grid, dim3(256), 0, stream, (const float *)gu, (__nv_bfloat16 *)out, ntok, di);
+        else if (in_dtype == JK_BF16) jk_launch(swiglu4_kernel<__nv_bfloat16, __nv_bfloat16>, grid, dim3(256), 0, stream, (const __nv_bfloat16 *)gu, (__nv_bfloat16 *)out, ntok, di);
+        else JK_FAIL(JK_UNSUPPORTED, "swiglu: dtypes %d -> %d", in_dtype, out_dtype);
+        JK_CHECK_LAUNCH("swiglu");
+        return JK_OK;
+    }
     if (in_dtype == JK_F32 && out_dtype == JK_F32)
         jk_launch(swiglu_kernel<float, float>, dim3((int)blocks), dim3(threads), 0, stream, (const float *)gu, (float *)out, di, total);
     else if (in_dtype == JK_F32 && out_dtype == JK_BF16)

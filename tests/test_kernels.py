@@ -92,6 +92,34 @@ def test_swiglu(K, in_dtype, out_dtype, T, di):
     _close(out, a * torch.sigmoid(a) * b, out_dtype, scale=3.0)
 
 
+@pytest.mark.parametrize("T,d", [(256, 1024), (257, 1028), (300, 2052), (2400, 3072)])
+@pytest.mark.parametrize("delta", [False, True])
+@pytest.mark.parametrize("wanted", [False, True])
+def test_add_rmsnorm_of_many_rows(K, T, d, delta, wanted):
+    """Widths at the edges of the kernel that walks over rows, one and several rows a block, all rows and picked ones."""
+    g = torch.Generator().manual_seed(T + d)
+    x, p, w = torch.randn(T, d, generator=g), torch.randn(T, d, generator=g), torch.randn(d, generator=g)
+    rows = torch.randint(0, T, (T,), generator=g, dtype=torch.int32) if wanted else None
+    xd, out = x.to(DEV), torch.full((T, d), 7.0, device=DEV)
+    K.add_rmsnorm(xd, p.to(DEV) if delta else None, 0.25, w.to(DEV), 1e-5, out, 2.0, rows.to(DEV) if wanted else None)
+    v = x.double() + (0.25 * p.double() if delta else 0.0)
+    pick = v[rows.long()] if wanted else v
+    want = pick * torch.rsqrt(pick.square().mean(-1, keepdim=True) + 1e-5) * w.double() * 2.0
+    assert (out.cpu().double() - want).abs().max() <= 2e-6 * want.abs().max()
+    assert torch.equal(xd.cpu(), x + 0.25 * p if delta and not wanted else x) or (delta and not wanted and (xd.cpu().double() - v).abs().max() <= 2e-7 * v.abs().max())
+
+
+@pytest.mark.parametrize("T,di", [(96, 512), (100, 516), (13, 4100)])
+def test_swiglu_four_units_a_thread_has_the_same_bits(K, T, di):
+    """The vector form against the form that rows off 16 bytes take."""
+    g = torch.Generator().manual_seed(di)
+    gu = (torch.randn(T, 2 * di, generator=g) * 30).to(DEV)
+    fast, slow = torch.empty(T, di, device=DEV), torch.empty(T * di + 1, device=DEV)[1:].view(T, di)
+    K.swiglu(gu, fast)
+    K.swiglu(gu, slow)
+    assert torch.equal(fast, slow) and torch.isfinite(fast).all()
+
+
 @pytest.mark.parametrize("M,N,K_", [(1, 1, 1), (7, 301, 80), (65, 129, 33), (130, 64, 2304), (3, 1000, 17)])
 def test_gemm_f32_is_a_true_float32_product(K, M, N, K_):
     g = torch.Generator().manual_seed(M * N)
