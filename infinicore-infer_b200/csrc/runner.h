@@ -24,6 +24,9 @@ typedef int (*RopeKvFn)(const void *, int, int, const float *, const int *, cons
                         cudaStream_t);
 typedef int (*GemmF32Fn)(const float *, int, const float *, int, const float *, float *, int, int, int, int, cudaStream_t);
 typedef int (*GemmF32SplitFn)(const float *, int, const float *, int, const float *, float *, int, int, int, int, int, int, int *, cudaStream_t);
+typedef int (*AttentionF32Fn)(const float *, const float *, const float *, float *, const int *, int, const int *, const int *, const int *, int, int, int, int, int, float,
+                              cudaStream_t);
+typedef int (*Supports2Fn)(int, int);
 typedef int (*GemmF32SupportsFn)(const float *, int, const float *, int, int, int, int);
 typedef int (*LinearSmallFn)(const void *, const void *, void *, int, int, int, int, int, int, cudaStream_t);
 typedef int (*LinearSmallQkvFn)(const void *, const void *, int, int, void *, void *, void *, const float *, const float *,
@@ -196,6 +199,9 @@ struct RunnerFns {
     GemmF32SplitFn gemm_f32_tcgen05;
     GemmF32SupportsFn gemm_f32_tcgen05_supports;
     LastErrorFn err_gemm_f32_tcgen05;
+    // float32 attention in tiles of query rows (csrc/attention_f32.cu, part of the attention module); may be empty
+    AttentionF32Fn attention_f32;
+    Supports2Fn attention_f32_supports;
 };
 
 // ---- records ---------------------------------------------------------------------------------------------------

@@ -473,6 +473,18 @@ def _gate_args(gate: Optional[torch.Tensor], rows: int, nh: int):
     return _ptr(gate), _c_int(gate.stride(0))
 
 
+def attention_f32(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, out: torch.Tensor, tiles: torch.Tensor, ntiles: int, req_start, req_pos, block_table,
+                  nh: int, scale: float) -> torch.Tensor:
+    """Plain causal attention in float32, tiles of query rows: ``tiles`` int32 ``[ntiles, 2]`` (batch entry, first of up to 128 rows); heads of 64 or 128."""
+    for name, t in (("q", q), ("k_pages", k_pages), ("v_pages", v_pages), ("out", out)):
+        _need(t, name, torch.float32)
+    _, nkvh, page, dh = k_pages.shape
+    lib = _build.load("attention")
+    _check("attention", lib.jk_attention_f32(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _ptr(tiles), _c_int(ntiles), _ptr(req_start), _ptr(req_pos), _ptr(block_table),
+                                             _c_int(block_table.shape[1]), _c_int(page), _c_int(nh), _c_int(nkvh), _c_int(dh), _c_float(scale), _stream()))
+    return out
+
+
 def attention_rows(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, out: torch.Tensor,
                    positions: torch.Tensor, row_req: torch.Tensor, block_table: torch.Tensor, ntok: int,
                    nh: int, scale: float, window: int = 0, sink: bool = False,

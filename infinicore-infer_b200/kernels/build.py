@@ -24,7 +24,7 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 # module name -> its .cu sources (all may include the headers listed in HEADERS)
 MODULES: Dict[str, List[str]] = {
     "elementwise": ["elementwise.cu", "gemm_f32.cu"],
-    "attention": ["attention.cu"],
+    "attention": ["attention.cu", "attention_f32.cu"],
     "sampling": ["sampling.cu"],
     "linear_small": ["linear_small.cu"],
     "gemm_tcgen05": ["gemm_tcgen05.cu", "gemm_skinny.cu"],

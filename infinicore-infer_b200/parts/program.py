@@ -111,7 +111,8 @@ class _Fns(ctypes.Structure):
         "latent_attention_scratch", "causal_conv", "selective_scan", "routed_experts", "routed_experts_workspace",
         "routed_experts_launches", "softcap", "err_blocks", "linear_small_parts", "linear_small_parts_supports", "add_rows", "delta_rule", "delta_rule_scratch",
         "norm_pair", "embed_pair", "join_parts", "gated_recurrence", "gated_recurrence_scratch", "gated_recurrence_launches", "rotate_rows", "latent_gather", "selective_scan_scratch",
-        "attention_laid", "gemm_f32_tcgen05", "gemm_f32_tcgen05_supports", "err_gemm_f32_tcgen05")]
+        "attention_laid", "gemm_f32_tcgen05", "gemm_f32_tcgen05_supports", "err_gemm_f32_tcgen05",
+        "attention_f32", "attention_f32_supports")]
 
 
 def _addr(lib, name: str) -> int:
@@ -181,7 +182,8 @@ def runner_lib(gemm_tcgen05: bool = False, attention_tcgen05: bool = False, mixe
         gated_recurrence_launches=get("blocks", "jk_gated_recurrence_launches"), rotate_rows=get("mixers", "jk_rotate_rows"),
         latent_gather=get("blocks", "jk_latent_gather"), selective_scan_scratch=get("blocks", "jk_selective_scan_scratch_floats"), attention_laid=get("attention_tcgen05", "jk_attention_laid_tcgen05"),
         gemm_f32_tcgen05=get("gemm_f32_tcgen05", "jk_gemm_f32_tcgen05"), gemm_f32_tcgen05_supports=get("gemm_f32_tcgen05", "jk_gemm_f32_tcgen05_supports"),
-        err_gemm_f32_tcgen05=get("gemm_f32_tcgen05", "jk_gemm_f32_tcgen05_last_error"))
+        err_gemm_f32_tcgen05=get("gemm_f32_tcgen05", "jk_gemm_f32_tcgen05_last_error"),
+        attention_f32=get("attention", "jk_attention_f32"), attention_f32_supports=get("attention", "jk_attention_f32_supports"))
     if lib.jk_runner_bind(ctypes.byref(fns)):
         from ..kernels import KernelError
         raise KernelError(lib.jk_runner_last_error().decode(errors="replace"))

@@ -228,6 +228,93 @@ def test_routed_experts_of_few_rows(K, dtype, rows, d, ff, experts, top):
     assert (out.double() - want).abs().max() <= (2e-5 if dtype == torch.float32 else 2.0 ** -8 * want.abs().max().item())
 
 
+@pytest.mark.parametrize("nh,nkvh,dh,page", [(6, 2, 64, 16), (3, 1, 128, 8), (400, 400, 64, 16), (40, 8, 128, 64)])
+@pytest.mark.parametrize("reqs", [[(9, 0), (64, 3)], [(129, 60)], [(31, 200), (40, 0), (150, 129)]])
+def test_attention_f32_in_tiles_of_rows(K, nh, nkvh, dh, page, reqs):
+    """Both sizes of tiles (many heads take the large ones), rows and keys at their edges, histories, a value that is not finite behind some rows."""
+    g = torch.Generator().manual_seed(nh + dh)
+    T, blocks = sum(n for n, _ in reqs), max(-(-(n + h) // page) for n, h in reqs)
+    q = torch.randn(T, nh, dh, generator=g).to(DEV)
+    kp, vp = (torch.randn(blocks * len(reqs) + 1, nkvh, page, dh, generator=g).to(DEV) for _ in range(2))
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    table = ints([[1 + i * blocks + b for b in range(blocks)] for i in range(len(reqs))])
+    start = [0]
+    for n, _ in reqs:
+        start.append(start[-1] + n)
+    tiles = [[b, start[b] + t] for b, (n, _) in enumerate(reqs) for t in range(0, n, 128)]
+    n, h = reqs[-1]
+    last = (n + h - 1) // page
+    vp[table[-1, last], :, (n + h - 1) % page] = math.nan          # the last position's value: its own row's result alone
+    out = torch.full_like(q, 7.0)
+    K.attention_f32(q, kp, vp, out, ints(tiles), len(tiles), ints(start), ints([h for _, h in reqs]), table, nh, dh ** -0.5)
+    assert torch.isnan(out[-1]).all() and torch.isfinite(out[:-1]).all()
+    for b, (n, h) in enumerate(reqs):
+        flat = lambda p: p[table[b].long()].transpose(1, 2).reshape(-1, nkvh, dh)[: n + h].double().repeat_interleave(nh // nkvh, 1)
+        v = flat(vp).nan_to_num(0.0)
+        s = torch.einsum("thd,jhd->htj", q[start[b]: start[b + 1]].double(), flat(kp)) * dh ** -0.5
+        s = s.masked_fill(torch.arange(n + h, device=DEV)[None] > torch.arange(h, n + h, device=DEV)[:, None], -math.inf)
+        want = torch.einsum("htj,jhd->thd", s.softmax(-1), v)
+        rows = slice(start[b], start[b + 1] - (1 if b == len(reqs) - 1 else 0))
+        # scores of size 1 rounded 128 times, weights that sum to 1, values below 6
+        assert (out[rows].double() - want[: rows.stop - rows.start]).abs().max() <= 1e-5
+
+
+@pytest.mark.parametrize("T,heads,dv", [(256, 64, 128), (1100, 32, 64), (2100, 16, 64)])
+@pytest.mark.parametrize("per_head", [0, 1, 2])
+def test_norm_gate_of_many_rows(K, T, heads, dv, per_head):
+    g = torch.Generator().manual_seed(T)
+    n = heads * dv
+    o, u, w = (torch.randn(*s, generator=g).to(DEV) for s in ((T, n), (T, n + 8), (dv if per_head == 1 else n,)))
+    out = torch.empty(T, n, device=DEV)
+    K.norm_gate(o, u, 4, w, 1e-5, heads, dv, per_head, 1, out)
+    x = o.double().view(T, heads, dv) if per_head else o.double()
+    want = (x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-5)).reshape(T, n) * (w.double().repeat(heads) if per_head == 1 else w.double())
+    want = want * torch.nn.functional.silu(u[:, 4: 4 + n].double())
+    assert ((out.double() - want).abs() <= 4e-6 * want.abs() + 1e-6).all()
+
+
+def _off(t):
+    """The same numbers four bytes off a 16-byte boundary: the element-by-element forms."""
+    moved = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:].view(t.shape)
+    return moved.copy_(t)
+
+
+@pytest.mark.parametrize("has_kv", [False, True])
+def test_conv_qkv_four_channels_a_thread(K, has_kv):
+    """Three requests of several hundred rows: rows that look into the tail, and rows that do not, against the form an element at a time."""
+    g = torch.Generator().manual_seed(7)
+    H, G, dk, page, lens = 4, 2, 64, 16, [1, 200, 130]
+    T, nq, nk = sum(lens), H * dk, G * dk
+    C = nq + (2 * nk if has_kv else 0)
+    u, conv = torch.randn(T, nq + 2 * nk, generator=g).to(DEV), [torch.randn(c, 4, generator=g).to(DEV) for c in (nq, nk, nk)]
+    norm, freq, tail = [torch.randn(c, generator=g).to(DEV) for c in (nq, nk)], torch.rand(16, generator=g).to(DEV), torch.randn(3, 3, C, generator=g).to(DEV)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    pos, req, start = ints([i for n in lens for i in range(n)]), ints([r for r, n in enumerate(lens) for _ in range(n)]), ints([0, 1, 201, 331])
+    table = ints([[1 + 13 * r + b for b in range(13)] for r in range(3)])
+    got = []
+    for move in (lambda t: t, _off):
+        q, kp, vp, t = torch.zeros(T, nq, device=DEV), *(torch.zeros(40, G, page, dk, device=DEV) for _ in range(2)), tail.clone()
+        K.conv_qkv(move(u), (0, nq, nq + nk), H, G, dk, dk, has_kv, conv, 4, norm, 1e-5, freq, 32, t, pos, req, start, ints([0, 1, 2]), table, page, q, kp, vp)
+        got.append((q, kp, vp, t))
+    for a, b in zip(*got):          # only the squares' sums may differ, by their order
+        assert (a - b).abs().max() <= 2e-6 * b.abs().max()
+
+
+@pytest.mark.parametrize("dr,dims,half", [(64, 64, False), (64, 32, True), (0, 0, False)])
+def test_latent_qkv_four_elements_a_thread_has_the_same_bits(K, dr, dims, half):
+    g = torch.Generator().manual_seed(dr + dims)
+    T, H, dn, R, page = 37, 5, 24, 96, 8
+    u, w, freq = torch.randn(T, H * (dn + dr) + R + dr, generator=g).to(DEV), torch.randn(R, generator=g).to(DEV), torch.rand(max(1, dims // 2), generator=g).to(DEV)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    pos, req, table = ints(list(range(T))), ints([0] * T), ints([list(range(1, 6))])
+    got = []
+    for move in (lambda t: t, _off):
+        plain, full, pages = torch.zeros(T, H * dn, device=DEV).bfloat16(), torch.zeros(T, H * (R + dr), device=DEV).bfloat16(), torch.zeros(6, page, R + dr, device=DEV).bfloat16()
+        K.latent_qkv(move(u), 0, H * (dn + dr), H, dn, dr, R, dims, freq, 1.2, w, 1e-5, pos, req, table, page, plain, full, pages, rot_half=half)
+        got.append((plain, full, pages))
+    assert all(torch.equal(a, b) for a, b in zip(*got)) and got[0][0].abs().max() > 0
+
+
 def _scatter_pages(k, v, tables, page, num_pages, dtype, junk=7.0):
     """Dense per-request keys/values [len, nkvh, dh] -> pages [num_pages, nkvh, page, dh]."""
     nkvh, dh = k[0].shape[1:]
