@@ -216,6 +216,7 @@ JK_EXPORT int jk_glu(const float *gu, void *out, int dtype, int ntok, int di, in
 // row in the step moves forward here (a channel is one thread's); `conv_tail_kernel` does it for the others, after this
 // kernel has read them.
 // ---------------------------------------------------------------------------------------------------------------
+// What bounds it: the row's passes through shared memory and their barriers (2,048 rows of 16 + 4 + 4 heads of 128, half rotated: 70 -> 28 us with four taps a time and the table).  
 struct ConvQkvArgs {
     const float *u;             // [T, ld]
     int ld, q_off, k_off, v_off;
@@ -236,13 +237,14 @@ struct ConvQkvArgs {
     const int *positions, *row_req, *req_start, *slot_ids, *block_table;
     int max_blocks, page_size;
     void *q_out, *k_pages, *v_pages;
+    int four;                   // 1: four taps everywhere, everything in whole vectors of four, many rows: rows behind the third run four channels a thread
 };
 
 template <typename T>
 __global__ void conv_qkv_kernel(ConvQkvArgs a) {
     pdl_trigger();
     pdl_wait();
-    extern __shared__ __align__(16) float y[];      // [nq + nk + nv]
+    extern __shared__ __align__(16) float y[];      // [nq + nk + nv], then the row's sines and cosines [rot_dims / 2] each
     __shared__ float scratch[33];
     const int t = blockIdx.x;
     const int C = a.nq + a.nk + a.nv;
@@ -251,7 +253,36 @@ __global__ void conv_qkv_kernel(ConvQkvArgs a) {
     const int pos = a.positions[t];
     float *tail = a.tail ? a.tail + (size_t)a.slot_ids[req] * (a.taps - 1) * C : nullptr;
     const bool only_row = tail != nullptr && a.req_start[req + 1] - a.req_start[req] == 1;
+    // one angle a pair and row, whatever the number of heads
+    float *row_sin = y + C, *row_cos = row_sin + (a.rot_dims >> 1);
+    for (int i = threadIdx.x; i < (a.rot_dims >> 1); i += blockDim.x) {
+        float sn, cs;
+        sincosf((float)pos * a.freq[i], &sn, &cs);
+        row_sin[i] = sn * a.rot_mag;
+        row_cos[i] = cs * a.rot_mag;
+    }
     float ssq = 0.f, ssk = 0.f;
+    if (a.four && back >= 3) {      // four taps, four channels a thread: 8 loads of 16 bytes at once
+        auto taps4 = [](float4 w, float u0, float u1, float u2, float u3) { return fmaf(w.w, u3, fmaf(w.z, u2, fmaf(w.y, u1, fmaf(w.x, u0, 0.f)))); };
+#pragma unroll 2
+        for (int c = threadIdx.x * 4; c < C; c += blockDim.x * 4) {
+            const bool is_q = c < a.nq, is_k = !is_q && c < a.nq + a.nk;
+            const int from = is_q ? c : is_k ? c - a.nq : c - a.nq - a.nk;
+            const float4 *w = reinterpret_cast<const float4 *>(is_q ? a.conv_q : is_k ? a.conv_k : a.conv_v) + from;
+            const float *u = a.u + (size_t)(t - 3) * a.ld + (is_q ? a.q_off : is_k ? a.k_off : a.v_off) + from;
+            float4 r[4], f[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) r[j] = *reinterpret_cast<const float4 *>(u + (size_t)j * a.ld);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) f[j] = w[j];
+            const float4 v = make_float4(taps4(f[0], r[0].x, r[1].x, r[2].x, r[3].x), taps4(f[1], r[0].y, r[1].y, r[2].y, r[3].y),
+                                         taps4(f[2], r[0].z, r[1].z, r[2].z, r[3].z), taps4(f[3], r[0].w, r[1].w, r[2].w, r[3].w));
+            *reinterpret_cast<float4 *>(y + c) = v;
+            const float ss = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+            if (is_q) ssq += ss;
+            else if (is_k) ssk += ss;
+        }
+    } else
     for (int c = threadIdx.x; c < C; c += blockDim.x) {
         int col;
         const float *w;
@@ -284,6 +315,47 @@ __global__ void conv_qkv_kernel(ConvQkvArgs a) {
     const bool whole = a.head_norm != 2;        // the norm over a whole projection
     const float inv_q = (whole && a.norm_q) ? 1.f / sqrtf(sum_q / (float)a.nq + a.eps) : 1.f;
     const float inv_k = (whole && a.norm_k && a.nk > 0) ? 1.f / sqrtf(sum_k / (float)a.nk + a.eps) : 1.f;
+    if (a.four && !a.head_norm) {       // norm, rotation and stores of four channels a thread
+        struct __align__(4 * sizeof(T)) Four { T v[4]; };
+        const int page = a.nk > 0 ? a.block_table[(size_t)req * a.max_blocks + pos / a.page_size] : 0, half = a.rot_dims >> 1;
+        const size_t row = (size_t)page * a.kv_heads * a.page_size + (size_t)(pos % a.page_size);
+        for (int c = threadIdx.x * 4; c < C; c += blockDim.x * 4) {
+            float4 v = *reinterpret_cast<const float4 *>(y + c);
+            T *to;
+            if (c < a.nq + a.nk) {
+                const bool is_q = c < a.nq;
+                const int cc = is_q ? c : c - a.nq, head = cc / a.dk, e = cc - head * a.dk;
+                const float inv = is_q ? inv_q : inv_k, *nw = is_q ? a.norm_q : a.norm_k;
+                auto normed = [&](int at) {         // four of y from the projection's element `at` on
+                    const float4 z = *reinterpret_cast<const float4 *>(y + (c - cc) + at);
+                    const float4 f = nw ? *reinterpret_cast<const float4 *>(nw + at) : make_float4(1.f, 1.f, 1.f, 1.f);
+                    return make_float4(z.x * inv * f.x, z.y * inv * f.y, z.z * inv * f.z, z.w * inv * f.w);
+                };
+                v = normed(cc);
+                if (e < a.rot_dims) {
+                    if (a.rot_half) {
+                        const bool first = e < half;
+                        const int pair = first ? e : e - half;
+                        const float4 o = normed(first ? cc + half : cc - half);
+                        auto turn = [&](float p, float q, int k) { return first ? fmaf(p, row_cos[k], -q * row_sin[k]) : fmaf(p, row_cos[k], q * row_sin[k]); };
+                        v = make_float4(turn(v.x, o.x, pair), turn(v.y, o.y, pair + 1), turn(v.z, o.z, pair + 2), turn(v.w, o.w, pair + 3));
+                    } else {
+                        const float s0 = row_sin[e / 2], c0 = row_cos[e / 2], s1 = row_sin[e / 2 + 1], c1 = row_cos[e / 2 + 1];
+                        v = make_float4(fmaf(v.x, c0, -v.y * s0), fmaf(v.y, c0, v.x * s0), fmaf(v.z, c1, -v.w * s1), fmaf(v.w, c1, v.z * s1));
+                    }
+                }
+                if (is_q && a.temp) { const float f = a.temp[head]; v.x *= f; v.y *= f; v.z *= f; v.w *= f; }
+                to = is_q ? (T *)a.q_out + (size_t)t * a.nq + cc : (T *)a.k_pages + (row + (size_t)head * a.page_size) * a.dk + e;
+            } else {
+                const int cc = c - a.nq - a.nk, head = cc / a.dv;
+                to = (T *)a.v_pages + (row + (size_t)head * a.page_size) * a.dv + (cc - head * a.dv);
+            }
+            Four r;
+            r.v[0] = from_f32<T>(v.x); r.v[1] = from_f32<T>(v.y); r.v[2] = from_f32<T>(v.z); r.v[3] = from_f32<T>(v.w);
+            *reinterpret_cast<Four *>(to) = r;
+        }
+        return;
+    }
     for (int c = threadIdx.x; c < a.nq + a.nk; c += blockDim.x) {
         const bool is_q = c < a.nq;
         const int cc = is_q ? c : c - a.nq;
@@ -293,7 +365,6 @@ __global__ void conv_qkv_kernel(ConvQkvArgs a) {
     __syncthreads();
     // rotation and the stores; a thread reads its partner's element, nobody writes y any more
     T *q_out = (T *)a.q_out + (size_t)t * a.nq;
-    const float fpos = (float)pos;
     size_t k_row = 0, v_row = 0;
     if (a.nk > 0) {
         const int page = a.block_table[(size_t)req * a.max_blocks + pos / a.page_size];
@@ -320,9 +391,7 @@ __global__ void conv_qkv_kernel(ConvQkvArgs a) {
                         const bool first = a.rot_half ? e < half : !(e & 1);
                         const int pair = a.rot_half ? (first ? e : e - half) : e >> 1;
                         const float other = yh[a.rot_half ? (first ? e + half : e - half) : (first ? e + 1 : e - 1)];
-                        float sn, cs;
-                        sincosf(fpos * a.freq[pair], &sn, &cs);
-                        sn *= a.rot_mag; cs *= a.rot_mag;
+                        const float sn = row_sin[pair], cs = row_cos[pair];
                         val = first ? val * cs - other * sn : val * cs + other * sn;
                     }
                     const int c = hh * a.dk + e;
@@ -338,9 +407,7 @@ __global__ void conv_qkv_kernel(ConvQkvArgs a) {
                     const bool first = a.rot_half ? e < half : !(e & 1);
                     const int pair = a.rot_half ? (first ? e : e - half) : e >> 1;
                     const float other = yh[a.rot_half ? (first ? e + half : e - half) : (first ? e + 1 : e - 1)];
-                    float sn, cs;
-                    sincosf(fpos * a.freq[pair], &sn, &cs);
-                    sn *= a.rot_mag; cs *= a.rot_mag;
+                    const float sn = row_sin[pair], cs = row_cos[pair];
                     val = first ? val * cs - other * sn : val * cs + other * sn;
                 }
                 ss += val * val;
@@ -352,9 +419,7 @@ __global__ void conv_qkv_kernel(ConvQkvArgs a) {
                     const bool first = a.rot_half ? e < half : !(e & 1);
                     const int pair = a.rot_half ? (first ? e : e - half) : e >> 1;
                     const float other = yh[a.rot_half ? (first ? e + half : e - half) : (first ? e + 1 : e - 1)];
-                    float sn, cs;
-                    sincosf(fpos * a.freq[pair], &sn, &cs);
-                    sn *= a.rot_mag; cs *= a.rot_mag;
+                    const float sn = row_sin[pair], cs = row_cos[pair];
                     val = first ? val * cs - other * sn : val * cs + other * sn;
                 }
                 const int c = hh * a.dk + e;
@@ -374,10 +439,7 @@ __global__ void conv_qkv_kernel(ConvQkvArgs a) {
                 const int half = a.rot_dims >> 1;
                 const bool first = a.rot_half ? e < half : !(e & 1);
                 const int pair = a.rot_half ? (first ? e : e - half) : e >> 1;
-                const float ang = fpos * a.freq[pair];
-                float sn, cs;
-                sincosf(ang, &sn, &cs);
-                sn *= a.rot_mag; cs *= a.rot_mag;
+                const float sn = row_sin[pair], cs = row_cos[pair];
                 const float other = y[a.rot_half ? (first ? c + half : c - half) : (first ? c + 1 : c - 1)];
                 val = first ? fmaf(val, cs, -other * sn) : fmaf(val, cs, other * sn);
             }
@@ -433,17 +495,21 @@ JK_EXPORT int jk_conv_qkv(const float *u, int ld, int q_off, int k_off, int v_of
     a.positions = positions; a.row_req = row_req; a.req_start = req_start; a.slot_ids = slot_ids; a.block_table = block_table;
     a.max_blocks = max_blocks; a.page_size = page_size; a.q_out = q_out; a.k_pages = k_pages; a.v_pages = v_pages;
     const bool conv = conv_q || conv_k || conv_v;
+    a.four = T >= 256 && taps == 4 && conv_q && (!has_kv || (conv_k && conv_v)) && ld % 4 == 0 && q_off % 4 == 0 && (!has_kv || (k_off % 4 == 0 && v_off % 4 == 0)) &&
+             dk % 4 == 0 && (!has_kv || dv % 4 == 0) && rot_dims % (rot_half ? 8 : 4) == 0 &&
+             (((uintptr_t)q_out | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)norm_q | (uintptr_t)norm_k) & 15) == 0 && (((uintptr_t)u | (uintptr_t)conv_q | (uintptr_t)(has_kv ? conv_k : nullptr) | (uintptr_t)(has_kv ? conv_v : nullptr)) & 15) == 0;
     JK_REQUIRE(u && q_out && positions && row_req && req_start && heads > 0 && dk > 0, "conv_qkv: an argument is missing");
     JK_REQUIRE(!has_kv || (k_pages && v_pages && block_table && kv_heads > 0 && dv > 0 && page_size > 0), "conv_qkv: keys without a cache");
     JK_REQUIRE(!(conv && bias), "conv_qkv: a bias with a convolution is not built");
     JK_REQUIRE(!conv || (taps >= 1 && (taps == 1 || (tail && slot_ids))), "conv_qkv: a convolution of %d taps without its tails", taps);
     JK_REQUIRE(rot_dims >= 0 && rot_dims <= dk && rot_dims % 2 == 0 && (rot_dims == 0 || freq), "conv_qkv: rotation of %d of %d elements", rot_dims, dk);
     const int C = a.nq + a.nk + a.nv;
-    const size_t smem = (size_t)C * sizeof(float);
-    JK_REQUIRE(smem <= 200 * 1024, "conv_qkv: %d channels do not fit shared memory", C);
+    const size_t smem = (size_t)(C + rot_dims) * sizeof(float);
+    JK_REQUIRE((size_t)C * sizeof(float) <= 200 * 1024, "conv_qkv: %d channels do not fit shared memory", C);
     // a step of few rows has few blocks: more threads a row then, so that a thread's chain of channels is short
     int threads = C >= 2048 ? 512 : (C >= 512 ? 256 : 128);
     if (T <= 64) threads = std::min(1024, std::max(threads, (C / 2 + 31) / 32 * 32));
+    if (a.four) threads = C >= 1024 ? 256 : 128;
     if (dtype == JK_F32) {
         if (smem > 46 * 1024) cudaFuncSetAttribute(conv_qkv_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         jk_launch(conv_qkv_kernel<float>, dim3(T), dim3(threads), smem, stream, a);
@@ -1524,11 +1590,74 @@ __global__ void norm_gate_kernel(const float *__restrict__ o, const float *__res
     }
 }
 
+// The same for heads of 64 or 128 and rows of up to 16 elements a thread: everything of a row that is read is asked for at once and stays in
+// registers, 16 bytes a load.  What bounds it: memory.  B200, the form above -> this (us): 2,048
+// rows of 16 heads of 128 15.0 -> 11.0, of 32 of 64 17.9 -> 10.5, 512 rows of 64 of 128 16.6 -> 11.3.
+template <typename T, int DV>
+__global__ void __launch_bounds__(512) norm_gate_rows_kernel(const float *o, const float *u, int ld, int g_off, const float *__restrict__ w,
+                                                             float eps, int n, int per_head, int gate_act, T *out) {
+    pdl_trigger();
+    pdl_wait();
+    __shared__ float scratch[33];
+    const float *orow = o + (size_t)blockIdx.x * n, *grow = u + (size_t)blockIdx.x * ld + g_off;
+    T *dst = out + (size_t)blockIdx.x * n;
+    const int step = blockDim.x * 4, first = threadIdx.x * 4;
+    float4 x[4], g[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int c = first + j * step;
+        x[j] = c < n ? *reinterpret_cast<const float4 *>(orow + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        g[j] = c < n ? *reinterpret_cast<const float4 *>(grow + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float inv[4];
+    float all = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        float ss = x[j].x * x[j].x + x[j].y * x[j].y + x[j].z * x[j].z + x[j].w * x[j].w;
+        if (per_head) {             // the DV / 4 threads of a head are neighbours, and begin where a warp or half of one does
+#pragma unroll
+            for (int k = DV / 8; k > 0; k >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, k);
+            inv[j] = 1.f / sqrtf(ss / (float)DV + eps);
+        } else {
+            all += ss;
+        }
+    }
+    if (!per_head) {
+        all = 1.f / sqrtf(block_sum(all, scratch) / (float)n + eps);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) inv[j] = all;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int c = first + j * step;
+        if (c >= n) break;
+        const float4 f = w != nullptr ? *reinterpret_cast<const float4 *>(w + (per_head == 1 ? c % DV : c)) : make_float4(1.f, 1.f, 1.f, 1.f);
+        struct __align__(4 * sizeof(T)) Four { T v[4]; } r;
+        r.v[0] = from_f32<T>(x[j].x * inv[j] * f.x * apply_act(gate_act, g[j].x));
+        r.v[1] = from_f32<T>(x[j].y * inv[j] * f.y * apply_act(gate_act, g[j].y));
+        r.v[2] = from_f32<T>(x[j].z * inv[j] * f.z * apply_act(gate_act, g[j].z));
+        r.v[3] = from_f32<T>(x[j].w * inv[j] * f.w * apply_act(gate_act, g[j].w));
+        *reinterpret_cast<Four *>(dst + c) = r;
+    }
+}
+
 JK_EXPORT int jk_norm_gate(const float *o, const float *u, int ld, int g_off, const float *w, float eps, int heads, int dv,
                            int per_head, int gate_act, void *out, int dtype, int T, cudaStream_t stream) {
     if (T == 0) return JK_OK;
     JK_REQUIRE(o && u && out && heads > 0 && dv > 0, "norm_gate: an argument is missing");
     const int n = heads * dv;
+    // (512 rows of 2,048 5.2 -> 6.5 us, 2,048 of 1,024 8.3 -> 6.9, 256 of 8,192 14.1 -> 6.6)
+    if ((long long)T * n >= 1LL << 21 && T >= 256 && (dv == 64 || dv == 128) && n >= 512 && n <= 8192 && ld % 4 == 0 && g_off % 4 == 0 && (((uintptr_t)o | (uintptr_t)u | (uintptr_t)w | (uintptr_t)out) & 15) == 0 &&
+        (dtype == JK_F32 || dtype == JK_BF16)) {
+        const int wide = (n / 16 + 31) / 32 * 32;
+#define LAUNCH(TT, DV) jk_launch(norm_gate_rows_kernel<TT, DV>, dim3(T), dim3(wide), 0, stream, o, u, ld, g_off, w, eps, n, per_head, gate_act, (TT *)out)
+        if (dtype == JK_F32) { if (dv == 64) LAUNCH(float, 64); else LAUNCH(float, 128); }
+        else if (dv == 64) LAUNCH(__nv_bfloat16, 64);
+        else LAUNCH(__nv_bfloat16, 128);
+#undef LAUNCH
+        JK_CHECK_LAUNCH("norm_gate");
+        return JK_OK;
+    }
     const int threads = n >= 2048 ? 512 : (n >= 512 ? 256 : 128);
     if (dtype == JK_F32)
         jk_launch(norm_gate_kernel<float>, dim3(T), dim3(threads), 0, stream, o, u, ld, g_off, w, eps, heads, dv, per_head, gate_act, (float *)out);
