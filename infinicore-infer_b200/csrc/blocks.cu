@@ -139,6 +139,59 @@ __global__ void norm_add_kernel(const float *__restrict__ delta, float *__restri
     }
 }
 
+// The same for rows of up to NV = 2 vectors a thread: everything of a row in registers and asked for at once, the weights before the kernel before has ended.  The
+// same sums in the same order.  What bounds it: in steps of few rows two reductions and one round of loads, else memory.  B200, the form above -> this (us):
+// 8 rows of 2,048 2.5 -> 2.0, 300 4.8 -> 3.0, 2,048 10.2 -> 9.9, 300 of 4,096 5.9 -> 4.5, but 2,048 of 4,096 20.1 -> 21.8, which keep the other one.
+// (delta and x are not restricted: a load of theirs must not move over the wait)
+template <typename T>
+__global__ void __launch_bounds__(1024) norm_add_regs_kernel(const float *delta, float *x, const float *__restrict__ w, float eps, const float *__restrict__ w_next, float eps2, T *out,
+                                                             const float *__restrict__ w_next2, T *out2, int d) {
+    pdl_trigger();
+    __shared__ float scratch[33];
+    constexpr int NV = 2;
+    const size_t base = (size_t)blockIdx.x * d;
+    const int first = threadIdx.x * 4, step = blockDim.x * 4;
+    const float4 one = make_float4(1.f, 1.f, 1.f, 1.f), none = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 g[NV], n1[NV], n2[NV], v[NV], r[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int c = first + j * step;
+        g[j] = c < d ? *reinterpret_cast<const float4 *>(w + c) : none;
+        n1[j] = c < d && w_next != nullptr ? *reinterpret_cast<const float4 *>(w_next + c) : one;
+        n2[j] = c < d && out2 != nullptr ? *reinterpret_cast<const float4 *>(w_next2 + c) : one;
+    }
+    pdl_wait();
+    float ss = 0.f, ss2 = 0.f;
+    asm("" : "+f"(ss), "+f"(ss2));      // the compiler does not see that they start at 0: it would contract the first sums otherwise than a loop's
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int c = first + j * step;
+        v[j] = c < d ? *reinterpret_cast<const float4 *>(delta + base + c) : none;
+        r[j] = c < d ? *reinterpret_cast<const float4 *>(x + base + c) : none;
+    }
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+        if (first + j * step < d) ss += (v[j].x * v[j].x + v[j].y * v[j].y) + (v[j].z * v[j].z + v[j].w * v[j].w);
+    const float inv = 1.f / sqrtf(block_sum(ss, scratch) / (float)d + eps);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int c = first + j * step;
+        if (c >= d) continue;
+        v[j] = make_float4(r[j].x + v[j].x * inv * g[j].x, r[j].y + v[j].y * inv * g[j].y, r[j].z + v[j].z * inv * g[j].z, r[j].w + v[j].w * inv * g[j].w);
+        *reinterpret_cast<float4 *>(x + base + c) = v[j];
+        ss2 += (v[j].x * v[j].x + v[j].y * v[j].y) + (v[j].z * v[j].z + v[j].w * v[j].w);
+    }
+    if (out == nullptr) return;
+    const float inv2 = w_next != nullptr ? 1.f / sqrtf(block_sum(ss2, scratch) / (float)d + eps2) : 1.f;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int c = first + j * step;
+        if (c >= d) continue;
+        store4(out + base + c, w_next != nullptr ? make_float4(v[j].x * inv2 * n1[j].x, v[j].y * inv2 * n1[j].y, v[j].z * inv2 * n1[j].z, v[j].w * inv2 * n1[j].w) : v[j]);
+        if (out2 != nullptr) store4(out2 + base + c, make_float4(v[j].x * inv2 * n2[j].x, v[j].y * inv2 * n2[j].y, v[j].z * inv2 * n2[j].z, v[j].w * inv2 * n2[j].w));
+    }
+}
+
 JK_EXPORT int jk_norm_add(const float *delta, float *x, const float *w, float eps, const float *w_next, float eps2, void *out,
                           const float *w_next2, void *out2, int dtype, int rows, int d, cudaStream_t stream) {
     if (rows == 0) return JK_OK;
@@ -152,6 +205,14 @@ JK_EXPORT int jk_norm_add(const float *delta, float *x, const float *w, float ep
     // a step of few rows has few blocks: then a thread takes one vector of the row, so that a pass is one round of loads
     int threads = d >= 4096 ? 512 : (d >= 1024 ? 256 : 128);
     if (rows <= 64 && vec) threads = std::min(1024, std::max(threads, (d / 4 + 31) / 32 * 32));
+    if (vec && d <= 8 * threads && (rows <= 512 || d <= 2048)) {
+#define LAUNCH(T) \
+        jk_launch(norm_add_regs_kernel<T>, dim3(rows), dim3(threads), 0, stream, delta, x, w, eps, w_next, eps2, (T *)out, w_next2, (T *)out2, d)
+        BLOCKS_BY_DTYPE(dtype, "norm_add", LAUNCH);
+#undef LAUNCH
+        JK_CHECK_LAUNCH("norm_add");
+        return JK_OK;
+    }
 #define LAUNCH_V(T, V)                                                                                                              \
     do {                                                                                                                            \
         if (smem > 46 * 1024) cudaFuncSetAttribute(norm_add_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
@@ -459,6 +520,8 @@ __device__ __forceinline__ float latent_rotated(const LatentQkvArgs &a, const fl
     return first ? fmaf(val, cs, -other * sn) : fmaf(val, cs, other * sn);
 }
 
+// What bounds it: the row's passes; a sine and cosine per element, the same for every head, were most of it.  B200, 2,048 rows of 16 heads of
+// 128 + 64 over a latent of 512 33 -> 19 us, 8 rows 6.1 -> 4.6.
 template <typename T>
 __global__ void latent_qkv_kernel(LatentQkvArgs a) {
     pdl_trigger();
@@ -585,8 +648,6 @@ constexpr int GT_M = 64, GT_N = 64, GT_K = 16;
 template <typename T> struct OnTensorCores { static constexpr bool value = false; };
 template <> struct OnTensorCores<__nv_bfloat16> { static constexpr bool value = true; };
 
-// What bounds it: the row's passes; a sine and cosine per element, the same for every head, were most of it.  B200, 2,048 rows of 16 heads of
-// 128 + 64 over a latent of 512 33 -> 19 us, 8 rows 6.1 -> 4.6.
 template <typename T>
 __device__ __forceinline__ void tile_at(int e, int *row, int *col) {
     if (OnTensorCores<T>::value) {
@@ -2107,21 +2168,50 @@ struct RouteArgs {
     float score_scale;          // form 1: factor of the renormalised scores
 };
 
-template <typename T, int R>
-__global__ void route_topk_kernel(const T *__restrict__ h, RouteArgs a) {
+// A row a block, up to eight outputs: the outputs' weights are asked for before the kernel before has ended (EARLY, rows of up to ROUTE_AHEAD columns),
+// and the row's own elements all at once.  Four rows: four blocks an SM, so that 2,048 rows are one wave (17.0 -> 11.5 us with eight outputs of 2,048).
+constexpr int ROUTE_AHEAD = 2048;
+template <typename T, int R, bool EARLY = false>
+__global__ void __launch_bounds__(R == 1 && !EARLY ? 1024 : 256, R == 1 ? 1 : 4) route_topk_kernel(const T *h, RouteArgs a) {
     pdl_trigger();
-    pdl_wait();
     extern __shared__ float route_smem[];       // per row: [N] logits, then scores; [N] choice scores; [group_count] best of a group, kept
     const int N = a.N, D = a.D, row_floats = 2 * N + 2 * a.group_count;
     const int t0 = blockIdx.x * R, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     const bool vec = D % 8 == 0 && (uintptr_t)h % 16 == 0 && (uintptr_t)a.router % 16 == 0 && (uintptr_t)a.gate_w % 16 == 0;
+    const int outputs = a.gate_w != nullptr ? N + 1 : N;
+    const bool ahead = EARLY && vec && D <= ROUTE_AHEAD && warp < outputs;
+    float4 early[EARLY ? ROUTE_AHEAD / 128 : 1];
+    if (ahead) {
+        const float *w = warp < N ? a.router + (size_t)warp * D : a.gate_w;
+#pragma unroll
+        for (int i = 0; i < (EARLY ? ROUTE_AHEAD / 256 : 0); ++i) {
+            const int c = lane * 8 + i * 256;
+            if (c < D) {
+                early[2 * i] = __ldg(reinterpret_cast<const float4 *>(w + c));
+                early[2 * i + 1] = __ldg(reinterpret_cast<const float4 *>(w + c + 4));
+            }
+        }
+    }
+    pdl_wait();
     // output N: the row's gate on what the experts' sum is added to
-    for (int e = warp; e < (a.gate_w != nullptr ? N + 1 : N); e += nwarp) {
+    for (int e = warp; e < outputs; e += nwarp) {
         const float *w = e < N ? a.router + (size_t)e * D : a.gate_w;
         float dot[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) dot[r] = 0.f;
-        if (vec) {          // eight elements a lane a pass, the passes' loads independent of one another
+        if (ahead && e == warp) {
+            float x[EARLY ? ROUTE_AHEAD / 256 : 1][8];
+#pragma unroll
+            for (int i = 0; i < (EARLY ? ROUTE_AHEAD / 256 : 0); ++i)
+                if (lane * 8 + i * 256 < D) load8(h + (size_t)t0 * D + lane * 8 + i * 256, x[i]);
+#pragma unroll
+            for (int i = 0; i < (EARLY ? ROUTE_AHEAD / 256 : 0); ++i)
+                if (lane * 8 + i * 256 < D) {
+                    const float wv[8] = {early[2 * i].x, early[2 * i].y, early[2 * i].z, early[2 * i].w, early[2 * i + 1].x, early[2 * i + 1].y, early[2 * i + 1].z, early[2 * i + 1].w};
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) dot[0] = fmaf(wv[k], x[i][k], dot[0]);
+                }
+        } else if (vec) {          // eight elements a lane a pass, the passes' loads independent of one another
 #pragma unroll 4
             for (int c = lane * 8; c < D; c += 256) {
                 float wv[8];
@@ -2320,7 +2410,14 @@ __global__ void __launch_bounds__(256) expert_down_kernel(const T *__restrict__ 
 // blocks an SM at most 8 rows of 1,024 x 512 took 43.
 constexpr int ER_ROWS = 8, EF_BYTES = 4096;          // entries at a time; bytes of a row at a time
 __host__ __device__ constexpr int ef_chunk(int K, int elem) { return K * elem < EF_BYTES ? K * elem : EF_BYTES; }
-__host__ __device__ constexpr int ef_smem(int K, int elem) { return (16 + ER_ROWS) * ef_chunk(K, elem); }
+__host__ __device__ constexpr int ef_smem(int K, int elem, int groups) { return (16 * groups + ER_ROWS) * ef_chunk(K, elem); }
+// Groups of 16 rows a block: a short row's copy costs a block more than its bytes, so where blocks make several waves (four an SM) a block takes more of
+// them.  B200, 48 entries of 64 experts of 64 features over 2,048: 53.4 us with one group, 45.2 with four; but 2 entries of 512 18.5 and 20.6: one there.
+inline int ef_groups(int K, int elem, long long blocks) {
+    int groups = 1;
+    while (2 * groups * K * elem <= 2048 && groups < 4 && blocks / (2 * groups) >= 4 * 148) groups *= 2;
+    return groups;
+}
 
 // The expert of the slot-th run of entries, or -1; a whole warp asks, for up to 256 experts at a time with one wait for memory.
 __device__ __forceinline__ int expert_with_entries(const int *starts, int E, int slot) {
@@ -2353,7 +2450,7 @@ struct ExpertRowsArgs {
     const float *entry_score;
     int actf;
     float limit;
-    int eager;
+    int eager, groups;
     int *status;
 };
 struct ExpertRowsSmem {
@@ -2363,7 +2460,7 @@ struct ExpertRowsSmem {
 template <typename T, bool GLU> struct ExpertRowsBlock {
     const ExpertRowsArgs &a;
     ExpertRowsSmem s;
-    int e, n0, chunk, chunks;                   // bytes a row at a time, how many times
+    int e, n0, chunk, chunks, groups;           // bytes a row at a time, how many times; groups of 16 rows (more than one: one chunk)
     unsigned w_phase = 0, x_phase = 0;          // of the chunk that is there, or on its way
     bool ok = true, fresh = true;               // fresh: the rows' first chunk is asked for, and nothing else yet
 
@@ -2371,11 +2468,13 @@ template <typename T, bool GLU> struct ExpertRowsBlock {
     // warp 0: a chunk of the 16 rows (features behind N: the last one's, whose results are not stored)
     __device__ __forceinline__ void bring_rows(int c) {
         const int lane = threadIdx.x & 31;
-        if (lane == 0) mbar_expect_tx(s.w_full, 16 * bytes(c));
+        if (lane == 0) mbar_expect_tx(s.w_full, groups * 16 * bytes(c));
         __syncwarp();
-        if (lane >= 16) return;
-        const size_t row = ((size_t)e * (GLU ? 2 : 1) + (GLU && lane >= 8 ? 1 : 0)) * a.N + min(n0 + lane % (GLU ? 8 : 16), a.N - 1);
-        bulk_load(s.w + lane * chunk, (const unsigned char *)((const T *)a.w + row * a.K) + (size_t)c * EF_BYTES, bytes(c), s.w_full);
+        for (int i = lane; i < groups * 16; i += 32) {
+            const int n = n0 + (GLU ? i / 16 * 8 + i % 8 : i);
+            const size_t row = ((size_t)e * (GLU ? 2 : 1) + (GLU && i % 16 >= 8 ? 1 : 0)) * a.N + min(n, a.N - 1);
+            bulk_load(s.w + i * chunk, (const unsigned char *)((const T *)a.w + row * a.K) + (size_t)c * EF_BYTES, bytes(c), s.w_full);
+        }
     }
     // warp 0: a chunk of `rows` entries from entry `first` on
     __device__ __forceinline__ void bring_entries(int c, int first, int rows) {
@@ -2386,61 +2485,65 @@ template <typename T, bool GLU> struct ExpertRowsBlock {
         const size_t row = (size_t)(GLU ? written_int(a.entry_row + first + lane) : first + lane);
         bulk_load(s.x + lane * chunk, (const unsigned char *)((const T *)a.in + row * a.K) + (size_t)c * EF_BYTES, bytes(c), s.x_full);
     }
-    // the block's features for ROWS entries (the caller picks the smallest ROWS that holds `rows`)
+    // the block's features for ROWS entries (the caller picks the smallest ROWS that holds `rows`); short rows: one group of 16 after the other
     template <int ROWS> __device__ __forceinline__ void entries(int first, int rows) {
         constexpr int V = Vec16<T>::N;
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        float g[ROWS], u[ROWS];
+        for (int group = 0; group < groups; ++group) {
+            float g[ROWS], u[ROWS];
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r) { g[r] = 0.f; u[r] = 0.f; }
-        for (int c = 0; c < chunks; ++c) {
-            if (!fresh) __syncthreads();        // what was there has been read
-            if (warp == 0) {
-                if (!fresh && chunks > 1) bring_rows(c);
-                bring_entries(c, first, rows);
-            }
-            if (!fresh) {
-                ++x_phase;
-                if (chunks > 1) ++w_phase;
-            }
-            fresh = false;
-            ok = mbar_wait(s.w_full, w_phase & 1) && ok;
-            ok = mbar_wait(s.x_full, x_phase & 1) && ok;
-            const int size = bytes(c);
-            const unsigned char *one = s.w + warp * chunk, *two = s.w + (warp + 8) * chunk;
+            for (int r = 0; r < ROWS; ++r) { g[r] = 0.f; u[r] = 0.f; }
+            for (int c = 0; c < chunks; ++c) {
+                if (group == 0) {
+                    if (!fresh) __syncthreads();        // what was there has been read
+                    if (warp == 0) {
+                        if (!fresh && chunks > 1) bring_rows(c);
+                        bring_entries(c, first, rows);
+                    }
+                    if (!fresh) {
+                        ++x_phase;
+                        if (chunks > 1) ++w_phase;
+                    }
+                    fresh = false;
+                    ok = mbar_wait(s.w_full, w_phase & 1) && ok;
+                    ok = mbar_wait(s.x_full, x_phase & 1) && ok;
+                }
+                const int size = bytes(c);
+                const unsigned char *one = s.w + (group * 16 + warp) * chunk, *two = one + 8 * chunk;
 #pragma unroll 1
-            for (int k = lane * 16; k < size; k += 512) {
-                float p[V], q[V];
-                unpack16<T>(*reinterpret_cast<const uint4 *>(one + k), p);
-                unpack16<T>(*reinterpret_cast<const uint4 *>(two + k), q);
+                for (int k = lane * 16; k < size; k += 512) {
+                    float p[V], q[V];
+                    unpack16<T>(*reinterpret_cast<const uint4 *>(one + k), p);
+                    unpack16<T>(*reinterpret_cast<const uint4 *>(two + k), q);
 #pragma unroll
-                for (int r = 0; r < ROWS; ++r) {
-                    float x[V];
-                    unpack16<T>(*reinterpret_cast<const uint4 *>(s.x + r * chunk + k), x);
+                    for (int r = 0; r < ROWS; ++r) {
+                        float x[V];
+                        unpack16<T>(*reinterpret_cast<const uint4 *>(s.x + r * chunk + k), x);
 #pragma unroll
-                    for (int i = 0; i < V; ++i) {
-                        g[r] = fmaf(p[i], x[i], g[r]);
-                        u[r] = fmaf(q[i], x[i], u[r]);
+                        for (int i = 0; i < V; ++i) {
+                            g[r] = fmaf(p[i], x[i], g[r]);
+                            u[r] = fmaf(q[i], x[i], u[r]);
+                        }
                     }
                 }
             }
-        }
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r) {
-            g[r] = warp_sum(g[r]);
-            u[r] = warp_sum(u[r]);
-        }
-        if (lane != 0) return;
-        const int n = n0 + warp;
+            for (int r = 0; r < ROWS; ++r) {
+                g[r] = warp_sum(g[r]);
+                u[r] = warp_sum(u[r]);
+            }
+            if (lane != 0) continue;
+            const int n = n0 + group * (GLU ? 8 : 16) + warp;
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r) {
-            if (r >= rows) break;
-            const size_t at = (size_t)(first + r) * a.N + n;
-            if (GLU) {
-                if (n < a.N) ((T *)a.out)[at] = from_f32<T>(expert_inner(a.actf, a.entry_score ? written_float(a.entry_score + first + r) : 1.f, g[r], u[r], a.limit));
-            } else {
-                if (n < a.N) ((float *)a.out)[at] = g[r];
-                if (n + 8 < a.N) ((float *)a.out)[at + 8] = u[r];
+            for (int r = 0; r < ROWS; ++r) {
+                if (r >= rows) break;
+                const size_t at = (size_t)(first + r) * a.N + n;
+                if (GLU) {
+                    if (n < a.N) ((T *)a.out)[at] = from_f32<T>(expert_inner(a.actf, a.entry_score ? written_float(a.entry_score + first + r) : 1.f, g[r], u[r], a.limit));
+                } else {
+                    if (n < a.N) ((float *)a.out)[at] = g[r];
+                    if (n + 8 < a.N) ((float *)a.out)[at + 8] = u[r];
+                }
             }
         }
     }
@@ -2458,8 +2561,9 @@ __global__ void __launch_bounds__(256, 4) expert_rows_kernel(ExpertRowsArgs a) {
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
-    ExpertRowsBlock<T, GLU> b{a, {er_smem, er_smem + 16 * chunk, &full[0], &full[1]}, (int)blockIdx.x, (int)blockIdx.y * (GLU ? 8 : 16), chunk,
-                              (a.K * (int)sizeof(T) + EF_BYTES - 1) / EF_BYTES};
+    const int groups = a.groups;
+    ExpertRowsBlock<T, GLU> b{a, {er_smem, er_smem + 16 * groups * chunk, &full[0], &full[1]}, (int)blockIdx.x, (int)blockIdx.y * groups * (GLU ? 8 : 16), chunk,
+                              (a.K * (int)sizeof(T) + EF_BYTES - 1) / EF_BYTES, groups};
     if (a.eager && warp == 0) b.bring_rows(0);
     pdl_wait();
     if (gridDim.x < a.E) {
@@ -2586,6 +2690,7 @@ JK_EXPORT int jk_routed_experts(const void *h, const float *router, const void *
     const int many = T >= 512 && 4 * route_smem <= 40 * 1024, warps = many ? 8 : std::min(32, std::max(4, N));
 #define LAUNCH(TT)                                                                                                          \
     if (many) jk_launch(route_topk_kernel<TT, 4>, dim3((T + 3) / 4), dim3(32 * warps), 4 * route_smem, stream, (const TT *)h, ra); \
+    else if (warps <= 8) jk_launch(route_topk_kernel<TT, 1, true>, dim3(T), dim3(32 * warps), route_smem, stream, (const TT *)h, ra); \
     else jk_launch(route_topk_kernel<TT, 1>, dim3(T), dim3(32 * warps), route_smem, stream, (const TT *)h, ra)
     BLOCKS_BY_DTYPE(dtype, "route_topk", LAUNCH);
 #undef LAUNCH
@@ -2617,15 +2722,16 @@ JK_EXPORT int jk_routed_experts(const void *h, const float *router, const void *
         g_expert_launches = 1;
     } else if (stream_rows) {
         // (grids of fewer blocks than experts find out late which expert is theirs)
-        const int elem = dtype == JK_F32 ? 4 : 2, eager = pairs >= 2 * E, smem_up = ef_smem(D, elem), smem_down = ef_smem(ff, elem);
-        const ExpertRowsArgs up{h, w_gate_up, act, D, ff, E, starts, entry_row, in_score, actf, limit, eager, status};
-        const ExpertRowsArgs down{act, w_down, y, ff, D, E, starts, nullptr, nullptr, 0, 0.f, eager, status};
-        const int runs = std::min(E, pairs);
+        const int elem = dtype == JK_F32 ? 4 : 2, eager = pairs >= 2 * E, runs = std::min(E, pairs);
+        const int up_groups = ef_groups(D, elem, (long long)runs * ((ff + 7) / 8)), down_groups = ef_groups(ff, elem, (long long)runs * ((D + 15) / 16));
+        const int up_rows = 8 * up_groups, down_rows = 16 * down_groups, smem_up = ef_smem(D, elem, up_groups), smem_down = ef_smem(ff, elem, down_groups);
+        const ExpertRowsArgs up{h, w_gate_up, act, D, ff, E, starts, entry_row, in_score, actf, limit, eager, up_groups, status};
+        const ExpertRowsArgs down{act, w_down, y, ff, D, E, starts, nullptr, nullptr, 0, 0.f, eager, down_groups, status};
 #define LAUNCH(TT)                                                                                                                           \
     if (smem_up > 46 * 1024) cudaFuncSetAttribute(expert_rows_kernel<TT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_up);       \
     if (smem_down > 46 * 1024) cudaFuncSetAttribute(expert_rows_kernel<TT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_down);  \
-    jk_launch(expert_rows_kernel<TT, true>, dim3(runs, (ff + 7) / 8), dim3(256), smem_up, stream, up);                                       \
-    jk_launch(expert_rows_kernel<TT, false>, dim3(runs, (D + 15) / 16), dim3(256), smem_down, stream, down)
+    jk_launch(expert_rows_kernel<TT, true>, dim3(runs, (ff + up_rows - 1) / up_rows), dim3(256), smem_up, stream, up);                                       \
+    jk_launch(expert_rows_kernel<TT, false>, dim3(runs, (D + down_rows - 1) / down_rows), dim3(256), smem_down, stream, down)
         BLOCKS_BY_DTYPE(dtype, "expert rows", LAUNCH);
 #undef LAUNCH
         JK_CHECK_LAUNCH("expert rows");

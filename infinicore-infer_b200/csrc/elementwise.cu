@@ -65,6 +65,48 @@ __device__ __forceinline__ void store4(__nv_bfloat16 *p, float4 v) {
     *reinterpret_cast<uint2 *>(p) = raw;
 }
 
+// A row in registers, NV vectors a thread, the norm's weights asked for before the kernel before has ended: what steps of few rows take.  The sums are
+// those of the kernel below in their order.  What bounds it: the two reductions and one round of loads.  B200, with something to add, the form below -> this (us):
+// 8 rows of 2,048 2.35 -> 1.65, 64 of 2,304 2.92 -> 1.98, 64 of 4,096 2.89 -> 2.33, 200 of 4,096 4.32 -> 3.35, 200 of 2,048 2.9 and 3.0.
+// (x, delta and rows are not restricted: a load of theirs must not move over the wait)
+template <typename TD, typename TO, int NV>
+__global__ void __launch_bounds__(512) add_rmsnorm_regs_kernel(float *x, const TD *delta, float delta_scale, const float *__restrict__ w, float eps, float out_scale, TO *out,
+                                                               const int *rows, int d) {
+    pdl_trigger();
+    __shared__ float scratch[33];
+    const int first = threadIdx.x * 4, step = blockDim.x * 4, i = blockIdx.x;
+    float4 g[NV], v[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) g[j] = first + j * step < d ? load4(w + first + j * step) : make_float4(0.f, 0.f, 0.f, 0.f);
+    pdl_wait();
+    const size_t at = (size_t)(rows ? rows[i] : i) * d;
+    float4 p[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int c = first + j * step;
+        v[j] = c < d ? load4(x + at + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (delta != nullptr) p[j] = c < d ? load4(delta + at + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int c = first + j * step;
+        if (c >= d) continue;
+        if (delta != nullptr) {
+            v[j] = make_float4(v[j].x + delta_scale * p[j].x, v[j].y + delta_scale * p[j].y, v[j].z + delta_scale * p[j].z, v[j].w + delta_scale * p[j].w);
+            if (!rows) store4(x + at + c, v[j]);
+        }
+        ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
+    }
+    ss = block_sum(ss, scratch);
+    const float inv = rsqrtf(ss / (float)d + eps) * out_scale;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int c = first + j * step;
+        if (c < d) store4(out + (size_t)i * d + c, make_float4(v[j].x * inv * g[j].x, v[j].y * inv * g[j].y, v[j].z * inv * g[j].z, v[j].w * inv * g[j].w));
+    }
+}
+
 // VEC: the width is a multiple of 4 and rows are 16-byte aligned, so four elements move at a time.
 template <typename TD, typename TO, bool VEC>
 __global__ void add_rmsnorm_kernel(float *__restrict__ x, const TD *__restrict__ delta,
@@ -255,6 +297,15 @@ static int launch_add_rmsnorm(float *x, const void *delta, float delta_scale, co
     }
     if (vec) {
         const int threads = d >= 4096 ? 512 : (d >= 1024 ? 256 : 128);
+        if (nout < 256 && d <= 12 * threads) {
+#define JK_REGS_LAUNCH(NV_) jk_launch(add_rmsnorm_regs_kernel<TD, TO, NV_>, dim3(nout), dim3(threads), 0, stream, x, (const TD *)delta, delta_scale, w, eps, out_scale, (TO *)out, rows, d)
+            if (d <= 4 * threads) JK_REGS_LAUNCH(1);
+            else if (d <= 8 * threads) JK_REGS_LAUNCH(2);
+            else JK_REGS_LAUNCH(3);
+#undef JK_REGS_LAUNCH
+            JK_CHECK_LAUNCH("add_rmsnorm");
+            return JK_OK;
+        }
         jk_launch(add_rmsnorm_kernel<TD, TO, true>, dim3(nout), dim3(threads), smem, stream,
                   x, (const TD *)delta, delta_scale, w, eps, out_scale, (TO *)out, rows, d);
     } else {

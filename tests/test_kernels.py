@@ -109,6 +109,25 @@ def test_add_rmsnorm_of_many_rows(K, T, d, delta, wanted):
     assert torch.equal(xd.cpu(), x + 0.25 * p if delta and not wanted else x) or (delta and not wanted and (xd.cpu().double() - v).abs().max() <= 2e-7 * v.abs().max())
 
 
+@pytest.mark.parametrize("T,d", [(1, 4), (7, 1024), (7, 1540), (65, 4096), (64, 4100), (512, 4096), (513, 2052), (600, 1500), (600, 4096)])
+def test_norm_add_with_the_row_in_registers(K, T, d):
+    """Widths of one and two vectors a thread and a part of one, and the sizes next to them; one norm behind it, two, none."""
+    g = torch.Generator().manual_seed(T + d)
+    p, x = torch.randn(T, d, generator=g), torch.randn(T, d, generator=g)
+    w, w1, w2 = (1 + 0.1 * torch.randn(d, generator=g) for _ in range(3))
+    v = x.double() + plain_rmsnorm(p.double(), w.double(), 1e-5)
+    for outs in range(3):
+        got, h, h2 = x.to(DEV), torch.empty(T, d, device=DEV), torch.empty(T, d, device=DEV)
+        more = dict(next_weight=w1.to(DEV), next_eps=1e-4, out=h) if outs else {}
+        if outs == 2:
+            K.norm_add(p.to(DEV), got, w.to(DEV), 1e-5, w1.to(DEV), 1e-4, h, w2.to(DEV), h2)
+        else:
+            K.norm_add(p.to(DEV), got, w.to(DEV), 1e-5, **more)
+        # sums of d squares in a tree: a few roundings of 2^-24 each
+        for have, want in ((got, v), (h, plain_rmsnorm(v, w1.double(), 1e-4)), (h2, plain_rmsnorm(v, w2.double(), 1e-4)))[: 1 + outs]:
+            assert (have.cpu().double() - want).abs().max() <= 2e-6 * want.abs().max()
+
+
 @pytest.mark.parametrize("T,di", [(96, 512), (100, 516), (13, 4100)])
 def test_swiglu_four_units_a_thread_has_the_same_bits(K, T, di):
     """The vector form against the form that rows off 16 bytes take."""
@@ -207,9 +226,11 @@ def test_head_linear_of_few_rows_has_the_tiles_bits(K, heads, n, k, gated):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("rows,d,ff,experts,top", [(1, 8, 8, 5, 1), (3, 2056, 40, 9, 2), (9, 72, 2064, 2, 1), (21, 64, 24, 3, 3), (2, 64, 16, 300, 8)])
+@pytest.mark.parametrize("rows,d,ff,experts,top", [(1, 8, 8, 5, 1), (3, 2056, 40, 9, 2), (9, 72, 2064, 2, 1), (21, 64, 24, 3, 3), (2, 64, 16, 300, 8),
+                                                  (32, 3000, 24, 100, 2), (32, 72, 1000, 100, 2)])
 def test_routed_experts_of_few_rows(K, dtype, rows, d, ff, experts, top):
-    """Rows of a matrix in one piece and in two, features at the edges of the blocks, more entries than run at a time, more experts than entries."""
+    """Rows of a matrix in one piece and in two, features at the edges of the blocks, more entries than run at a time, more experts than entries,
+    several groups of short rows a block in either product."""
     g = torch.Generator().manual_seed(rows + d)
     h, router = torch.randn(rows, d, generator=g).to(dtype).to(DEV), (torch.randn(experts, d, generator=g) * 2 * d ** -0.5).to(DEV)
     up = (torch.randn(experts * 2 * ff, d, generator=g) * d ** -0.5).to(dtype).to(DEV)
