@@ -53,7 +53,7 @@ class Sampler:
             host = torch.empty(4, n, dtype=torch.float32, pin_memory=self.device.type == "cuda")
             rows, most = host.numpy(), 2 ** 31 - 1
             rows[0] = [p.temperature for p in params]
-            rows[1].view(np.int32)[:] = [max(-most, min(most, int(p.topk))) for p in params]
+            rows[1].view(np.int32)[:] = [int(max(-most, min(most, p.topk))) for p in params]
             rows[2] = [p.topp for p in params]
             rows[3] = [uniform_for(p.seed, i) for p, i in zip(params, indices)]
             dev = host.to(self.device, non_blocking=True)

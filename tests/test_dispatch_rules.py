@@ -109,3 +109,16 @@ def test_float32_products_on_the_tensor_cores(rows, n, k, tensor):
     # the blocks of clusters that run at once on 148 SMs, one a block: 33 of four, 14 of eight
     blocks = -(-rows // tile) * -(-n // 128) * cuts if tile else 0
     assert cuts in (1, 2, 4, 8) and (cuts == 1 or blocks <= {2: 148, 4: 132, 8: 112}[cuts])
+
+
+def test_sampling_parameters_beyond_their_types_are_clamped(monkeypatch):
+    """A top-k beyond 32 bits or infinite reaches the draw as the largest whole number."""
+    import torch
+
+    from infinicore_infer_b200 import kernels
+    from infinicore_infer_b200.sampling.sampler import Sampler, SamplingParams
+    seen = []
+    monkeypatch.setattr(kernels, "sample", lambda logits, t, k, p, u, out: (seen.append(k.tolist()), out.zero_()))
+    params = [SamplingParams(temperature=1.0, topk=k, topp=0.5) for k in (7, 2 ** 40, float("inf"), -2 ** 40)]
+    Sampler("cpu").sample(torch.zeros(4, 8), params, range(4))
+    assert seen == [[7, 2 ** 31 - 1, 2 ** 31 - 1, 1 - 2 ** 31]]
