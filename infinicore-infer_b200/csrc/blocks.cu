@@ -1917,7 +1917,7 @@ __global__ void __launch_bounds__(SS_THREADS) selective_scan_kernel(ScanArgs a) 
 // What bounds it: instructions (sixteen states: about 170 a row and channel, the exponentials half of them).  Eight lanes a
 // channel walking a prompt from end to end waited 600 cycles a row for one another and for the next rows.  B200, 2,048 rows,
 // 4,096 channels, 16 states, with the product of the step sizes: 589 -> 360 us, and with two
-// states an instruction, where they need no exponential, the same bits and 266 -> 238 us for the two launches (medians of three).
+// states an instruction, where they need no exponential, the same bits and 263 -> 238 us for the two launches (medians of three).
 constexpr int SP_THREADS = 128, SP_ROWS = jk::SELECTIVE_PIECE, SP_AHEAD = 4;
 struct PieceArgs {
     float *ends, *sums;         // [pieces, N, E] end states, [pieces, E] sums of step sizes
