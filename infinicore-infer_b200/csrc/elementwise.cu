@@ -155,8 +155,8 @@ __global__ void add_rmsnorm_kernel(float *__restrict__ x, const TD *__restrict__
     }
 }
 
-// The same for steps of many rows of up to 1,024 columns: a warp per row, the row in registers (NV groups of four floats a lane), every load
-// of a row on its way before the first is used, no shared memory and no barrier.
+// The same for steps of many rows of up to 3,072 columns, from 1,024 columns on only where there is no float32 product to add: a warp per row,
+// the row in registers (NV groups of four floats a lane), every load of a row on its way before the first is used, no shared memory and no barrier.
 template <typename TD, typename TO, int NV>
 __global__ void __launch_bounds__(256)
 add_rmsnorm_warp_kernel(float *__restrict__ x, const TD *__restrict__ delta, float delta_scale, const float *__restrict__ w, float eps,
@@ -203,18 +203,21 @@ add_rmsnorm_warp_kernel(float *__restrict__ x, const TD *__restrict__ delta, flo
 }
 
 // The same for steps of many rows of 1,024 to 3,072 columns: a block stays and walks over rows, a row in its registers (NV groups of four floats a thread), the norm's
-// weights read once, before the kernel before has ended, and the next row on its way while this one is reduced; one barrier a row.
+// weights read once, before the kernel before has ended, and the next row on its way while this one is reduced; one barrier a row.  The squares are
+// added in the order in which a lane of the kernel above adds its own, so the results are the same bits: a lane's sums of four lie
+// in shared memory, 128 columns a line, and every warp adds them up line by line.
 // What bounds it: memory, and below a thousand rows the latency of a row.  B200, a warp a row -> this, with a product to add (us): 532 rows of 1,536
 // 8.2 -> 3.3, 2,048 14.1 -> 10.2; 532 of 2,304 13.4 -> 4.6, 2,048 28.9 -> 14.3; 5,003 of 3,072 80 -> 43.  Without one there is
 // less to gain (532 of 1,536 3.0 -> 2.4, but 1,024 of 2,304 4.9 -> 5.8) and the warps keep it.  Narrower rows are left to the warps (5,003 of 256 4.9 -> 5.7), wider ones to a block a row through shared
 // memory (532 of 4,096 8.0 -> 8.5, of 8,192 14.1 -> 17.2).
 // (x and delta are not restricted: what is read ahead of the wait is the weights alone)
-template <typename TO, int NV>
-__global__ void __launch_bounds__(256)
+template <typename TO, int NV, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
 add_rmsnorm_rows_kernel(float *x, const float *delta, float delta_scale, const float *__restrict__ w, float eps, float out_scale, TO *out, const int *rows, int nout, int d) {
     pdl_trigger();
-    __shared__ float sums[2][8];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, first = threadIdx.x * 4, step = blockDim.x * 4;
+    constexpr int LINES = NV * WARPS, step = WARPS * 128;
+    __shared__ float sums[2][LINES * 32];
+    const int lane = threadIdx.x & 31, first = threadIdx.x * 4;
     float4 g[NV], v[NV], p[NV];
     const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
@@ -234,20 +237,19 @@ add_rmsnorm_rows_kernel(float *x, const float *delta, float delta_scale, const f
     if (i < nout) fetch(i);
     for (int turn = 0; i < nout; i += gridDim.x, turn ^= 1) {
         float4 u[NV];
-        float ss = 0.f;
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
             u[j] = make_float4(v[j].x + delta_scale * p[j].x, v[j].y + delta_scale * p[j].y, v[j].z + delta_scale * p[j].z, v[j].w + delta_scale * p[j].w);
             const int c = first + j * step;
             if (rows == nullptr && c < d) store4(x + at + c, u[j]);
-            ss += u[j].x * u[j].x + u[j].y * u[j].y + u[j].z * u[j].z + u[j].w * u[j].w;
+            sums[turn][j * WARPS * 32 + threadIdx.x] = c < d ? u[j].x * u[j].x + u[j].y * u[j].y + u[j].z * u[j].z + u[j].w * u[j].w : 0.f;
         }
         if (i + gridDim.x < nout) fetch(i + gridDim.x);
-        ss = warp_sum(ss);
-        if (lane == 0) sums[turn][warp] = ss;
         __syncthreads();            // the other half of `sums` is free: who reads it has not passed this barrier's predecessor
-        ss = 0.f;
-        for (int k = 0; k < warps; ++k) ss += sums[turn][k];
+        float ss = 0.f;
+#pragma unroll
+        for (int k = 0; k < LINES; ++k) ss += sums[turn][k * 32 + lane];
+        ss = warp_sum(ss);
         const float inv = rsqrtf(ss / (float)d + eps) * out_scale;
         TO *o = out + (size_t)i * d;
 #pragma unroll
@@ -272,13 +274,14 @@ static int launch_add_rmsnorm(float *x, const void *delta, float delta_scale, co
         if (e != cudaSuccess) JK_FAIL(JK_CUDA_ERROR, "add_rmsnorm: %s", cudaGetErrorString(e));
     }
     if (vec && std::is_same<TD, float>::value && delta != nullptr && nout >= 256 && d >= 1024 && d <= 3072) {
-        const int threads = d <= 2048 ? 128 : 256, nv = (d / 4 + threads - 1) / threads, blocks = std::min(nout, 148 * 8);
-#define JK_ROWS_LAUNCH(NV_)                                                                                              \
-        jk_launch(add_rmsnorm_rows_kernel<TO, NV_>, dim3(blocks), dim3(threads), 0, stream, x, (const float *)delta, delta_scale, w, eps, \
+        const int blocks = std::min(nout, 148 * 8);
+#define JK_ROWS_LAUNCH(NV_, WARPS_)                                                                                       \
+        jk_launch(add_rmsnorm_rows_kernel<TO, NV_, WARPS_>, dim3(blocks), dim3(WARPS_ * 32), 0, stream, x, (const float *)delta, delta_scale, w, eps, \
                   out_scale, (TO *)out, rows, nout, d)
-        if (nv == 2) JK_ROWS_LAUNCH(2);
-        else if (nv == 3) JK_ROWS_LAUNCH(3);
-        else JK_ROWS_LAUNCH(4);
+        if (d <= 1024) JK_ROWS_LAUNCH(2, 4);
+        else if (d <= 1536) JK_ROWS_LAUNCH(3, 4);
+        else if (d <= 2048) JK_ROWS_LAUNCH(4, 4);
+        else JK_ROWS_LAUNCH(3, 8);
 #undef JK_ROWS_LAUNCH
         JK_CHECK_LAUNCH("add_rmsnorm");
         return JK_OK;

@@ -109,6 +109,21 @@ def test_add_rmsnorm_of_many_rows(K, T, d, delta, wanted):
     assert torch.equal(xd.cpu(), x + 0.25 * p if delta and not wanted else x) or (delta and not wanted and (xd.cpu().double() - v).abs().max() <= 2e-7 * v.abs().max())
 
 
+@pytest.mark.parametrize("out_dtype", DTYPES)
+@pytest.mark.parametrize("T,d", [(256, 1024), (257, 1028), (532, 1536), (512, 2304), (2400, 2052), (1300, 3072)])
+@pytest.mark.parametrize("wanted", [False, True])
+def test_add_rmsnorm_of_many_rows_adds_in_one_order(K, out_dtype, T, d, wanted):
+    """The kernel that walks over rows with something to add, against the warp a row that takes the finished sum: the same bits."""
+    g = torch.Generator().manual_seed(T + d)
+    x, p, w = torch.randn(T, d, generator=g), torch.randn(T, d, generator=g), torch.randn(d, generator=g).to(DEV)
+    rows = torch.randint(0, T, (T,), generator=g, dtype=torch.int32).to(DEV) if wanted else None
+    added = (x + 0.25 * p).to(DEV)           # a quarter is exact: one rounding, as in the kernel
+    out, want = (torch.full((T, d), 7.0, dtype=out_dtype, device=DEV) for _ in range(2))
+    K.add_rmsnorm(x.to(DEV), p.to(DEV), 0.25, w, 1e-5, out, 2.0, rows)
+    K.add_rmsnorm(added, None, 1.0, w, 1e-5, want, 2.0, rows)
+    assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("T,d", [(1, 4), (7, 1024), (7, 1540), (65, 4096), (64, 4100), (512, 4096), (513, 2052), (600, 1500), (600, 4096)])
 def test_norm_add_with_the_row_in_registers(K, T, d):
     """Widths of one and two vectors a thread and a part of one, and the sizes next to them; one norm behind it, two, none."""
