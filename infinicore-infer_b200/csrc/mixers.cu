@@ -216,7 +216,7 @@ JK_EXPORT int jk_glu(const float *gu, void *out, int dtype, int ntok, int di, in
 // row in the step moves forward here (a channel is one thread's); `conv_tail_kernel` does it for the others, after this
 // kernel has read them.
 // ---------------------------------------------------------------------------------------------------------------
-// What bounds it: the row's passes through shared memory and their barriers (2,048 rows of 16 + 4 + 4 heads of 128, half rotated: 70 -> 28 us with four taps a time and the table).  
+// What bounds it: the row's passes through shared memory and their barriers (2,048 rows of 16 + 4 + 4 heads of 128, half rotated: 70 -> 29 us with four taps a time and the table).
 struct ConvQkvArgs {
     const float *u;             // [T, ld]
     int ld, q_off, k_off, v_off;
@@ -237,8 +237,30 @@ struct ConvQkvArgs {
     const int *positions, *row_req, *req_start, *slot_ids, *block_table;
     int max_blocks, page_size;
     void *q_out, *k_pages, *v_pages;
-    int four;                   // 1: four taps everywhere, everything in whole vectors of four, many rows: rows behind the third run four channels a thread
+    int four;                   // 1: four taps everywhere, everything in whole vectors of four, many rows: four channels a thread
 };
+
+// warp_sum and block_sum where a thread stands for four neighbours (eight lanes for a warp): the same sums, bit for bit.
+__device__ __forceinline__ float warp_sum_of_four(float4 v) {
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {           // lanes 16, 8 and 4 apart
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, o); v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+        v.z += __shfl_xor_sync(0xffffffffu, v.z, o); v.w += __shfl_xor_sync(0xffffffffu, v.w, o);
+    }
+    return (v.x + v.z) + (v.y + v.w);           // 2 and 1 apart
+}
+__device__ __forceinline__ float block_sum_of_four(float4 v, float *scratch) {
+    const float s = warp_sum_of_four(v);
+    __syncthreads();
+    if (threadIdx.x % 8 == 0) scratch[threadIdx.x / 8] = s;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const float t = warp_sum(threadIdx.x < blockDim.x / 8 ? scratch[threadIdx.x] : 0.f);
+        if (threadIdx.x == 0) scratch[32] = t;
+    }
+    __syncthreads();
+    return scratch[32];
+}
 
 template <typename T>
 __global__ void conv_qkv_kernel(ConvQkvArgs a) {
@@ -261,57 +283,65 @@ __global__ void conv_qkv_kernel(ConvQkvArgs a) {
         row_sin[i] = sn * a.rot_mag;
         row_cos[i] = cs * a.rot_mag;
     }
-    float ssq = 0.f, ssk = 0.f;
-    if (a.four && back >= 3) {      // four taps, four channels a thread: 8 loads of 16 bytes at once
+    float sum_q, sum_k;
+    if (a.four) {      // four taps, four channels a thread: 8 loads of 16 bytes at once
         auto taps4 = [](float4 w, float u0, float u1, float u2, float u3) { return fmaf(w.w, u3, fmaf(w.z, u2, fmaf(w.y, u1, fmaf(w.x, u0, 0.f)))); };
+        float4 sq = make_float4(0.f, 0.f, 0.f, 0.f), sk = sq;
 #pragma unroll 2
         for (int c = threadIdx.x * 4; c < C; c += blockDim.x * 4) {
             const bool is_q = c < a.nq, is_k = !is_q && c < a.nq + a.nk;
             const int from = is_q ? c : is_k ? c - a.nq : c - a.nq - a.nk;
             const float4 *w = reinterpret_cast<const float4 *>(is_q ? a.conv_q : is_k ? a.conv_k : a.conv_v) + from;
-            const float *u = a.u + (size_t)(t - 3) * a.ld + (is_q ? a.q_off : is_k ? a.k_off : a.v_off) + from;
+            const float *u = a.u + (size_t)t * a.ld + (is_q ? a.q_off : is_k ? a.k_off : a.v_off) + from;
             float4 r[4], f[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) r[j] = *reinterpret_cast<const float4 *>(u + (size_t)j * a.ld);
+            for (int j = 0; j < 4; ++j) r[j] = *reinterpret_cast<const float4 *>(3 - j <= back ? u - (size_t)(3 - j) * a.ld : tail + (size_t)(j + back) * C + c);
 #pragma unroll
             for (int j = 0; j < 4; ++j) f[j] = w[j];
+            if (only_row)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) *reinterpret_cast<float4 *>(tail + (size_t)j * C + c) = r[j + 1];
             const float4 v = make_float4(taps4(f[0], r[0].x, r[1].x, r[2].x, r[3].x), taps4(f[1], r[0].y, r[1].y, r[2].y, r[3].y),
                                          taps4(f[2], r[0].z, r[1].z, r[2].z, r[3].z), taps4(f[3], r[0].w, r[1].w, r[2].w, r[3].w));
             *reinterpret_cast<float4 *>(y + c) = v;
-            const float ss = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-            if (is_q) ssq += ss;
-            else if (is_k) ssk += ss;
+            auto add = [&](float4 &s) { s = make_float4(fmaf(v.x, v.x, s.x), fmaf(v.y, v.y, s.y), fmaf(v.z, v.z, s.z), fmaf(v.w, v.w, s.w)); };
+            if (is_q) add(sq);
+            else if (is_k) add(sk);
         }
-    } else
-    for (int c = threadIdx.x; c < C; c += blockDim.x) {
-        int col;
-        const float *w;
-        if (c < a.nq) { col = a.q_off + c; w = a.conv_q ? a.conv_q + (size_t)c * a.taps : nullptr; }
-        else if (c < a.nq + a.nk) { col = a.k_off + c - a.nq; w = a.conv_k ? a.conv_k + (size_t)(c - a.nq) * a.taps : nullptr; }
-        else { col = a.v_off + c - a.nq - a.nk; w = a.conv_v ? a.conv_v + (size_t)(c - a.nq - a.nk) * a.taps : nullptr; }
-        float acc;
-        if (w == nullptr) {
-            acc = a.u[(size_t)t * a.ld + col] + (a.bias ? a.bias[col] : 0.f);
-        } else {
-            acc = 0.f;
-            for (int j = 0; j < a.taps; ++j) {
-                const int d = a.taps - 1 - j;       // how many rows back
-                float uv;
-                if (d <= back) uv = a.u[(size_t)(t - d) * a.ld + col];
-                else uv = tail[(size_t)(a.taps - 1 + back - d) * C + c];
-                acc = fmaf(w[j], uv, acc);
+        sum_q = block_sum_of_four(sq, scratch);
+        sum_k = a.nk > 0 ? block_sum_of_four(sk, scratch) : 0.f;
+    } else {
+        float ssq = 0.f, ssk = 0.f;
+        for (int c = threadIdx.x; c < C; c += blockDim.x) {
+            int col;
+            const float *w;
+            if (c < a.nq) { col = a.q_off + c; w = a.conv_q ? a.conv_q + (size_t)c * a.taps : nullptr; }
+            else if (c < a.nq + a.nk) { col = a.k_off + c - a.nq; w = a.conv_k ? a.conv_k + (size_t)(c - a.nq) * a.taps : nullptr; }
+            else { col = a.v_off + c - a.nq - a.nk; w = a.conv_v ? a.conv_v + (size_t)(c - a.nq - a.nk) * a.taps : nullptr; }
+            float acc;
+            if (w == nullptr) {
+                acc = a.u[(size_t)t * a.ld + col] + (a.bias ? a.bias[col] : 0.f);
+            } else {
+                acc = 0.f;
+                for (int j = 0; j < a.taps; ++j) {
+                    const int d = a.taps - 1 - j;       // how many rows back
+                    float uv;
+                    if (d <= back) uv = a.u[(size_t)(t - d) * a.ld + col];
+                    else uv = tail[(size_t)(a.taps - 1 + back - d) * C + c];
+                    acc = fmaf(w[j], uv, acc);
+                }
+                if (only_row) {
+                    for (int s = 0; s + 2 < a.taps; ++s) tail[(size_t)s * C + c] = tail[(size_t)(s + 1) * C + c];
+                    if (a.taps > 1) tail[(size_t)(a.taps - 2) * C + c] = a.u[(size_t)t * a.ld + col];
+                }
             }
-            if (only_row) {
-                for (int s = 0; s + 2 < a.taps; ++s) tail[(size_t)s * C + c] = tail[(size_t)(s + 1) * C + c];
-                if (a.taps > 1) tail[(size_t)(a.taps - 2) * C + c] = a.u[(size_t)t * a.ld + col];
-            }
+            y[c] = acc;
+            if (c < a.nq) ssq += acc * acc;
+            else if (c < a.nq + a.nk) ssk += acc * acc;
         }
-        y[c] = acc;
-        if (c < a.nq) ssq += acc * acc;
-        else if (c < a.nq + a.nk) ssk += acc * acc;
+        sum_q = block_sum(ssq, scratch);
+        sum_k = a.nk > 0 ? block_sum(ssk, scratch) : 0.f;
     }
-    const float sum_q = block_sum(ssq, scratch);
-    const float sum_k = a.nk > 0 ? block_sum(ssk, scratch) : 0.f;
     const bool whole = a.head_norm != 2;        // the norm over a whole projection
     const float inv_q = (whole && a.norm_q) ? 1.f / sqrtf(sum_q / (float)a.nq + a.eps) : 1.f;
     const float inv_k = (whole && a.norm_k && a.nk > 0) ? 1.f / sqrtf(sum_k / (float)a.nk + a.eps) : 1.f;
@@ -497,7 +527,7 @@ JK_EXPORT int jk_conv_qkv(const float *u, int ld, int q_off, int k_off, int v_of
     const bool conv = conv_q || conv_k || conv_v;
     a.four = T >= 256 && taps == 4 && conv_q && (!has_kv || (conv_k && conv_v)) && ld % 4 == 0 && q_off % 4 == 0 && (!has_kv || (k_off % 4 == 0 && v_off % 4 == 0)) &&
              dk % 4 == 0 && (!has_kv || dv % 4 == 0) && rot_dims % (rot_half ? 8 : 4) == 0 &&
-             (((uintptr_t)q_out | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)norm_q | (uintptr_t)norm_k) & 15) == 0 && (((uintptr_t)u | (uintptr_t)conv_q | (uintptr_t)(has_kv ? conv_k : nullptr) | (uintptr_t)(has_kv ? conv_v : nullptr)) & 15) == 0;
+             (((uintptr_t)q_out | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)norm_q | (uintptr_t)norm_k) & 15) == 0 && (((uintptr_t)u | (uintptr_t)conv_q | (uintptr_t)(has_kv ? conv_k : nullptr) | (uintptr_t)(has_kv ? conv_v : nullptr) | (uintptr_t)tail) & 15) == 0;
     JK_REQUIRE(u && q_out && positions && row_req && req_start && heads > 0 && dk > 0, "conv_qkv: an argument is missing");
     JK_REQUIRE(!has_kv || (k_pages && v_pages && block_table && kv_heads > 0 && dv > 0 && page_size > 0), "conv_qkv: keys without a cache");
     JK_REQUIRE(!(conv && bias), "conv_qkv: a bias with a convolution is not built");
@@ -509,7 +539,7 @@ JK_EXPORT int jk_conv_qkv(const float *u, int ld, int q_off, int k_off, int v_of
     // a step of few rows has few blocks: more threads a row then, so that a thread's chain of channels is short
     int threads = C >= 2048 ? 512 : (C >= 512 ? 256 : 128);
     if (T <= 64) threads = std::min(1024, std::max(threads, (C / 2 + 31) / 32 * 32));
-    if (a.four) threads = C >= 1024 ? 256 : 128;
+    if (a.four) threads /= 4;           // a thread stands for four: the order of the squares' sums stays
     if (dtype == JK_F32) {
         if (smem > 46 * 1024) cudaFuncSetAttribute(conv_qkv_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         jk_launch(conv_qkv_kernel<float>, dim3(T), dim3(threads), smem, stream, a);

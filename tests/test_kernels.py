@@ -336,6 +336,30 @@ def test_conv_qkv_four_channels_a_thread(K, has_kv):
         assert (a - b).abs().max() <= 2e-6 * b.abs().max()
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("H,G,rot,half,temp,head_norm", [(4, 2, 32, False, False, 0), (16, 4, 64, True, True, 0), (5, 1, 16, True, False, 0), (16, 4, 32, False, True, 1),
+                                                        (12, 12, 64, True, True, 2), (3, 1, 0, False, True, 0)])
+def test_conv_qkv_four_channels_a_thread_has_the_same_bits(K, dtype, H, G, rot, half, temp, head_norm):
+    """Each way of norm and rotation with and without what the heads are scaled by, in both types, against the form an element at a time."""
+    g = torch.Generator().manual_seed(H + rot)
+    dk, page, lens = 64, 16, [1, 200, 130]
+    T, nq, nk = sum(lens), H * dk, G * dk
+    C = nq + 2 * nk
+    u, conv = torch.randn(T, C, generator=g).to(DEV), [torch.randn(c, 4, generator=g).to(DEV) for c in (nq, nk, nk)]
+    norm, freq, tail = [torch.randn(dk if head_norm == 2 else c, generator=g).to(DEV) for c in (nq, nk)], torch.rand(32, generator=g).to(DEV), torch.randn(3, 3, C, generator=g).to(DEV)
+    scale = torch.rand(H, generator=g).to(DEV) if temp else None
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    pos, req, start = ints([i for n in lens for i in range(n)]), ints([r for r, n in enumerate(lens) for _ in range(n)]), ints([0, 1, 201, 331])
+    table = ints([[1 + 13 * r + b for b in range(13)] for r in range(3)])
+    got = []
+    for move in (lambda t: t, _off):
+        q, kp, vp, t = torch.zeros(T, nq, device=DEV).to(dtype), *(torch.zeros(40, G, page, dk, device=DEV).to(dtype) for _ in range(2)), tail.clone()
+        K.conv_qkv(move(u), (0, nq, nq + nk), H, G, dk, dk, True, conv, 4, norm, 1e-5, freq if rot else None, rot, t, pos, req, start, ints([0, 1, 2]), table, page, q, kp, vp,
+                   temp=scale, rot_half=half, head_norm=head_norm)
+        got.append((q, kp, vp, t))
+    assert all(torch.equal(a, b) for a, b in zip(*got)) and got[0][0].float().abs().max() > 0
+
+
 @pytest.mark.parametrize("dr,dims,half", [(64, 64, False), (64, 32, True), (0, 0, False)])
 def test_latent_qkv_four_elements_a_thread_has_the_same_bits(K, dr, dims, half):
     g = torch.Generator().manual_seed(dr + dims)
