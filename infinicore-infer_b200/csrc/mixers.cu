@@ -1620,10 +1620,12 @@ __global__ void norm_gate_kernel(const float *__restrict__ o, const float *__res
     }
 }
 
-// The same for heads of 64 or 128 and rows of up to 16 elements a thread: everything of a row that is read is asked for at once and stays in
-// registers, 16 bytes a load.  What bounds it: memory.  B200, the form above -> this (us): 2,048
-// rows of 16 heads of 128 15.0 -> 11.0, of 32 of 64 17.9 -> 10.5, 512 rows of 64 of 128 16.6 -> 11.3.
-template <typename T, int DV>
+// The same for heads of 64 or 128 and many rows: everything of a row that is read is asked for at once and stays in registers, 16 bytes a
+// load.  The squares are added in the order of the form above, so the results are the same bits: with a mean a head (DV > 0) eight lanes
+// stand for a warp's 32; with one mean for the row a thread stands for four of the block's, or rows that are too long for that pass
+// through shared memory, from where the block's threads take their own.  What bounds it: memory.  B200, the form above -> this
+// (us): 2,048 rows of 16 heads of 128 15.0 -> 10.0, of 32 of 64 17.9 -> 10.0, 512 rows of 64 of 128 16.6 -> 10.1 (one mean: 12.9).
+template <typename T, int DV, bool LONG>
 __global__ void __launch_bounds__(512) norm_gate_rows_kernel(const float *o, const float *u, int ld, int g_off, const float *__restrict__ w,
                                                              float eps, int n, int per_head, int gate_act, T *out) {
     pdl_trigger();
@@ -1631,42 +1633,46 @@ __global__ void __launch_bounds__(512) norm_gate_rows_kernel(const float *o, con
     __shared__ float scratch[33];
     const float *orow = o + (size_t)blockIdx.x * n, *grow = u + (size_t)blockIdx.x * ld + g_off;
     T *dst = out + (size_t)blockIdx.x * n;
-    const int step = blockDim.x * 4, first = threadIdx.x * 4;
-    float4 x[4], g[4];
+    constexpr int NV = 4, PER = DV > 0 ? DV / 32 : NV;          // vectors of a head that a lane has
+    auto place = [&](int j) { return DV > 0 ? (int)((threadIdx.x >> 3) + j / PER * (blockDim.x >> 3)) * DV + j % PER * 32 + (int)(threadIdx.x & 7) * 4 : (int)(threadIdx.x + j * blockDim.x) * 4; };
+    float4 x[NV], g[NV];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int c = first + j * step;
+    for (int j = 0; j < NV; ++j) {
+        const int c = place(j);
         x[j] = c < n ? *reinterpret_cast<const float4 *>(orow + c) : make_float4(0.f, 0.f, 0.f, 0.f);
         g[j] = c < n ? *reinterpret_cast<const float4 *>(grow + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    float inv[4];
-    float all = 0.f;
+    float inv[NV / PER];
+    auto add = [](float4 s, float4 v) { return make_float4(fmaf(v.x, v.x, s.x), fmaf(v.y, v.y, s.y), fmaf(v.z, v.z, s.z), fmaf(v.w, v.w, s.w)); };
+    if (LONG) {
+        extern __shared__ __align__(16) float row[];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        float ss = x[j].x * x[j].x + x[j].y * x[j].y + x[j].z * x[j].z + x[j].w * x[j].w;
-        if (per_head) {             // the DV / 4 threads of a head are neighbours, and begin where a warp or half of one does
+        for (int j = 0; j < NV; ++j)
+            if (place(j) < n) *reinterpret_cast<float4 *>(row + place(j)) = x[j];
+        __syncthreads();
+        float ss = 0.f;
+        for (int c = threadIdx.x; c < n; c += blockDim.x) ss = fmaf(row[c], row[c], ss);
+        inv[0] = 1.f / sqrtf(block_sum(ss, scratch) / (float)n + eps);
+    } else {
 #pragma unroll
-            for (int k = DV / 8; k > 0; k >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, k);
-            inv[j] = 1.f / sqrtf(ss / (float)DV + eps);
-        } else {
-            all += ss;
+        for (int j = 0; j < NV; j += PER) {
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int k = 0; k < PER; ++k) s = add(s, x[j + k]);
+            inv[j / PER] = 1.f / sqrtf(DV > 0 ? warp_sum_of_four(s) / (float)DV + eps : block_sum_of_four(s, scratch) / (float)n + eps);
         }
     }
-    if (!per_head) {
-        all = 1.f / sqrtf(block_sum(all, scratch) / (float)n + eps);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) inv[j] = all;
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int c = first + j * step;
-        if (c >= n) break;
-        const float4 f = w != nullptr ? *reinterpret_cast<const float4 *>(w + (per_head == 1 ? c % DV : c)) : make_float4(1.f, 1.f, 1.f, 1.f);
+    for (int j = 0; j < NV; ++j) {
+        const int c = place(j);
+        if (c >= n) continue;
+        const float i = inv[j / PER];
+        const float4 f = w != nullptr ? *reinterpret_cast<const float4 *>(w + (DV > 0 && per_head == 1 ? c % max(DV, 1) : c)) : make_float4(1.f, 1.f, 1.f, 1.f);
         struct __align__(4 * sizeof(T)) Four { T v[4]; } r;
-        r.v[0] = from_f32<T>(x[j].x * inv[j] * f.x * apply_act(gate_act, g[j].x));
-        r.v[1] = from_f32<T>(x[j].y * inv[j] * f.y * apply_act(gate_act, g[j].y));
-        r.v[2] = from_f32<T>(x[j].z * inv[j] * f.z * apply_act(gate_act, g[j].z));
-        r.v[3] = from_f32<T>(x[j].w * inv[j] * f.w * apply_act(gate_act, g[j].w));
+        r.v[0] = from_f32<T>(x[j].x * i * f.x * apply_act(gate_act, g[j].x));
+        r.v[1] = from_f32<T>(x[j].y * i * f.y * apply_act(gate_act, g[j].y));
+        r.v[2] = from_f32<T>(x[j].z * i * f.z * apply_act(gate_act, g[j].z));
+        r.v[3] = from_f32<T>(x[j].w * i * f.w * apply_act(gate_act, g[j].w));
         *reinterpret_cast<Four *>(dst + c) = r;
     }
 }
@@ -1676,19 +1682,28 @@ JK_EXPORT int jk_norm_gate(const float *o, const float *u, int ld, int g_off, co
     if (T == 0) return JK_OK;
     JK_REQUIRE(o && u && out && heads > 0 && dv > 0, "norm_gate: an argument is missing");
     const int n = heads * dv;
-    // (512 rows of 2,048 5.2 -> 6.5 us, 2,048 of 1,024 8.3 -> 6.9, 256 of 8,192 14.1 -> 6.6)
-    if ((long long)T * n >= 1LL << 21 && T >= 256 && (dv == 64 || dv == 128) && n >= 512 && n <= 8192 && ld % 4 == 0 && g_off % 4 == 0 && (((uintptr_t)o | (uintptr_t)u | (uintptr_t)w | (uintptr_t)out) & 15) == 0 &&
-        (dtype == JK_F32 || dtype == JK_BF16)) {
-        const int wide = (n / 16 + 31) / 32 * 32;
-#define LAUNCH(TT, DV) jk_launch(norm_gate_rows_kernel<TT, DV>, dim3(T), dim3(wide), 0, stream, o, u, ld, g_off, w, eps, n, per_head, gate_act, (TT *)out)
-        if (dtype == JK_F32) { if (dv == 64) LAUNCH(float, 64); else LAUNCH(float, 128); }
-        else if (dv == 64) LAUNCH(__nv_bfloat16, 64);
-        else LAUNCH(__nv_bfloat16, 128);
+    const int threads = n >= 2048 ? 512 : (n >= 512 ? 256 : 128);
+    // (512 rows of 2,048 5.2 -> 6.5 us, 2,048 of 1,024 8.3 -> 6.9, 256 of 8,192 14.1 -> 6.6; with one mean, 2,048 rows of 1,536 11.3 -> 12.5)
+    if ((long long)T * n >= 1LL << 21 && (per_head || n <= 1024 || n >= 2048) && T >= 256 && (dv == 64 || dv == 128) && n >= 512 && n <= 8192 && ld % 4 == 0 && g_off % 4 == 0 &&
+        (((uintptr_t)o | (uintptr_t)u | (uintptr_t)w | (uintptr_t)out) & 15) == 0 && (dtype == JK_F32 || dtype == JK_BF16)) {
+        // with one mean for the row the threads of the form above set the order of the sum
+        const bool whole = !per_head, lengthy = whole && n > 4 * threads;
+        const int wide = whole ? (lengthy ? threads : threads / 4) : (n / 16 + 31) / 32 * 32;
+#define LAUNCH(TT, DV, LONG) jk_launch(norm_gate_rows_kernel<TT, DV, LONG>, dim3(T), dim3(wide), LONG ? n * sizeof(float) : 0, stream, o, u, ld, g_off, w, eps, n, per_head, gate_act, (TT *)out)
+#define BY_HEAD(TT)                               \
+    do {                                          \
+        if (lengthy) LAUNCH(TT, 0, true);         \
+        else if (whole) LAUNCH(TT, 0, false);     \
+        else if (dv == 64) LAUNCH(TT, 64, false); \
+        else LAUNCH(TT, 128, false);              \
+    } while (0)
+        if (dtype == JK_F32) BY_HEAD(float);
+        else BY_HEAD(__nv_bfloat16);
+#undef BY_HEAD
 #undef LAUNCH
         JK_CHECK_LAUNCH("norm_gate");
         return JK_OK;
     }
-    const int threads = n >= 2048 ? 512 : (n >= 512 ? 256 : 128);
     if (dtype == JK_F32)
         jk_launch(norm_gate_kernel<float>, dim3(T), dim3(threads), 0, stream, o, u, ld, g_off, w, eps, heads, dv, per_head, gate_act, (float *)out);
     else if (dtype == JK_BF16)

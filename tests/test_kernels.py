@@ -309,6 +309,22 @@ def test_norm_gate_of_many_rows(K, T, heads, dv, per_head):
     assert ((out.double() - want).abs() <= 4e-6 * want.abs() + 1e-6).all()
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("T,heads,dv", [(256, 64, 128), (300, 63, 128), (1100, 33, 64), (2100, 16, 64), (1100, 16, 128), (1400, 25, 64)])
+@pytest.mark.parametrize("per_head,act", [(0, 1), (1, 0), (2, 1)])
+def test_norm_gate_of_many_rows_has_the_bits_of_few(K, dtype, T, heads, dv, per_head, act):
+    """Rows in registers against the form that steps of fewer than 256 rows take: heads in pairs and one over, one mean or many."""
+    g = torch.Generator().manual_seed(T + heads)
+    n = heads * dv
+    o, u, w = (torch.randn(*s, generator=g).to(DEV) for s in ((T, n), (T, n + 8), (dv if per_head == 1 else n,)))
+    out, want = (torch.full((T, n), 7.0, dtype=dtype, device=DEV) for _ in range(2))
+    K.norm_gate(o, u, 4, w, 1e-5, heads, dv, per_head, act, out)
+    for at in range(0, T, 200):
+        rows = slice(at, min(T, at + 200))
+        K.norm_gate(o[rows], u[rows], 4, w, 1e-5, heads, dv, per_head, act, want[rows])
+    assert torch.equal(out, want)
+
+
 def _off(t):
     """The same numbers four bytes off a 16-byte boundary: the element-by-element forms."""
     moved = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:].view(t.shape)
