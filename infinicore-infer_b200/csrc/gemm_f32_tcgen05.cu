@@ -1,13 +1,15 @@
 // The float32 matrix product of steps of many rows on the 5th-generation tensor cores:  C[M, N] = A[M, K] * W[N, K]^T (+ bias[N]).
 //
-// A float32 number is the sum of three bfloat16 ones (round to nearest, twice the remainder: 8 + 8 + 8 bits and signs, so
-// nothing is lost), and a product of two float32 numbers the sum of nine products of those, each exact in float32.  Six of
-// them are made, smallest first: m m, h l, l h, h m, m h, h h.  What is left out (m l, l m, l l) is below 2^-26 of |a||w|.
+// A float32 number is the sum of three bfloat16 ones (round to nearest, twice the remainder: 8 + 8 + 8 bits and signs), and a product of two
+// float32 numbers the sum of nine products of those, each exact in float32.  Six of them are made, smallest first: m m, h l, l h, h m, m h,
+// h h.  What is left out (m l, l m, l l) is at most about 2^-24 of |a||w|, and 2^-27.4 in the mean (root of the mean square, normal operands).
+// bfloat16 has float32's exponents but not its smallest numbers: below 2^-110 the parts of a number would be cut off.  So both operands are
+// taken times 2^16, which makes every float32 number's parts whole, and the sums times 2^-32.
 // The tensor core adds the products of FS_BK = 64 columns of K into tensor memory; these sums go to registers and are added
 // up there by float32 additions, since the tensor core's own additions cut off instead of rounding, which adds up over a long
 // chain.  Error against 64 bits (2-norm of the difference over that of the result, normal operands): K 1,536 1.0e-7 to 1.2e-7, the
 // multiply-adds of gemm_f32.cu 2.5e-7; K 3,840 1.1e-7 to 1.6e-7 and 4.0e-7; K 96 0.8e-7 and 0.8e-7.
-// Numbers that the split does not carry (infinities, NaN, magnitudes that round to infinity in bfloat16) leave a result that
+// Numbers that this does not carry (infinities, NaN, operands from 2^111 and results from 2^95 on) leave a result that
 // is not finite: such outputs are computed again from the operands by float32 multiply-adds, so they are what those give.
 //
 // The weights are on the MMA's M side (128 features a tile), tokens on its N side (BN of them), so that a prompt's odd number
@@ -34,6 +36,7 @@ JK_DEFINE_ERROR_BUFFER(jk_gemm_f32_tcgen05)
 namespace {
 
 constexpr int FS_BK = 64, FS_ADDERS = 8, FS_LOADERS = 6, FS_THREADS = 32 * (FS_ADDERS + FS_LOADERS + 1), FS_STAGES = 2;
+constexpr float FS_SCALE = 65536.f, FS_UNSCALE = 1.f / (FS_SCALE * FS_SCALE);
 
 struct FsArgs {
     const float *A, *W, *bias;
@@ -76,12 +79,23 @@ __device__ __forceinline__ unsigned bf16_pair(float lo, float hi) {
 __device__ __forceinline__ float pair_lo(unsigned p) { return __uint_as_float(p << 16); }
 __device__ __forceinline__ float pair_hi(unsigned p) { return __uint_as_float(p & 0xffff0000u); }
 
+// two numbers times FS_SCALE in one instruction
+__device__ __forceinline__ void scale_pair(float &x, float &y) {
+    asm("{ .reg .b64 a, b;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %2};\n\tmul.rn.f32x2 a, a, b;\n\tmov.b64 {%0, %1}, a; }" : "+f"(x), "+f"(y) : "f"(FS_SCALE));
+}
+// two numbers rounded to bfloat16, and what is left of them
+__device__ __forceinline__ unsigned split_pair(float &x, float &y) {
+    const unsigned h = bf16_pair(x, y);
+    asm("{ .reg .b64 a, b, c;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\tmov.b64 c, {%4, %4};\n\tfma.rn.f32x2 a, b, c, a;\n\tmov.b64 {%0, %1}, a; }"
+        : "+f"(x), "+f"(y) : "f"(pair_lo(h)), "f"(pair_hi(h)), "f"(-1.f));
+    return h;
+}
 // four consecutive floats into the three tiles (`plane` bytes apart)
 __device__ __forceinline__ void split_store(unsigned char *dst, int plane, float4 x) {
-    const unsigned h0 = bf16_pair(x.x, x.y), h1 = bf16_pair(x.z, x.w);
-    x.x -= pair_lo(h0); x.y -= pair_hi(h0); x.z -= pair_lo(h1); x.w -= pair_hi(h1);
-    const unsigned m0 = bf16_pair(x.x, x.y), m1 = bf16_pair(x.z, x.w);
-    x.x -= pair_lo(m0); x.y -= pair_hi(m0); x.z -= pair_lo(m1); x.w -= pair_hi(m1);
+    scale_pair(x.x, x.y);
+    scale_pair(x.z, x.w);
+    const unsigned h0 = split_pair(x.x, x.y), h1 = split_pair(x.z, x.w);
+    const unsigned m0 = split_pair(x.x, x.y), m1 = split_pair(x.z, x.w);
     *reinterpret_cast<uint2 *>(dst) = make_uint2(h0, h1);
     *reinterpret_cast<uint2 *>(dst + plane) = make_uint2(m0, m1);
     *reinterpret_cast<uint2 *>(dst + 2 * plane) = make_uint2(bf16_pair(x.x, x.y), bf16_pair(x.z, x.w));
@@ -223,18 +237,16 @@ __global__ void __launch_bounds__(FS_THREADS, 1) gemm_f32_tcgen05_kernel(const _
                 float v[16];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const float4 x = *reinterpret_cast<const float4 *>(from + (((4 * p + i) ^ (row & 7)) << 4));
+                    float4 x = *reinterpret_cast<const float4 *>(from + (((4 * p + i) ^ (row & 7)) << 4));
+                    scale_pair(x.x, x.y);
+                    scale_pair(x.z, x.w);
                     v[4 * i] = x.x; v[4 * i + 1] = x.y; v[4 * i + 2] = x.z; v[4 * i + 3] = x.w;
                 }
 #pragma unroll
                 for (int part = 0; part < 3; ++part) {
                     unsigned b[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        b[i] = bf16_pair(v[2 * i], v[2 * i + 1]);
-                        v[2 * i] -= pair_lo(b[i]);
-                        v[2 * i + 1] -= pair_hi(b[i]);
-                    }
+                    for (int i = 0; i < 8; ++i) b[i] = part < 2 ? split_pair(v[2 * i], v[2 * i + 1]) : bf16_pair(v[2 * i], v[2 * i + 1]);
                     tmem_st8(to + part * 32 + p * 8, b);
                 }
             }
@@ -267,7 +279,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) gemm_f32_tcgen05_kernel(const _
 #pragma unroll
             for (int j = 0; j < HALF; ++j) {
                 finite = finite && isfinite(acc[j]);
-                if (m + j < a.M) to[(size_t)j * a.ldc] = acc[j] + bias;
+                if (m + j < a.M) to[(size_t)j * a.ldc] = fmaf(acc[j], FS_UNSCALE, bias);
             }
             if (!finite)
                 for (int j = 0; j < HALF && m + j < a.M; ++j)
@@ -283,7 +295,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) gemm_f32_tcgen05_kernel(const _
             for (int r = 1; r < a.cuts; ++r) v += load_cluster(cluster_addr(share + i, r));
             const int m = m0 + i / TG_BM, n = n0 + i % TG_BM;
             if (m >= a.M || n >= a.N) continue;
-            if (isfinite(v)) a.C[(size_t)m * a.ldc + n] = v + (a.bias != nullptr ? a.bias[n] : 0.f);
+            if (isfinite(v)) a.C[(size_t)m * a.ldc + n] = fmaf(v, FS_UNSCALE, a.bias != nullptr ? a.bias[n] : 0.f);
             else store_plain(a, m, n);
         }
         cluster_sync();      // no block leaves while another reads its share

@@ -223,6 +223,32 @@ def test_gemm_f32_tcgen05_what_the_split_does_not_carry(K, cuts):
     assert ((out - plain).abs()[ok] <= 1e-6 * plain.abs()[ok] + 2e-4).all()
 
 
+@pytest.mark.parametrize("what", ["tiny and large", "below the normal numbers", "results below the normal numbers", "large", "one sign", "columns of uneven size", "rows of uneven size"])
+@pytest.mark.parametrize("cuts", [1, 4])
+def test_gemm_f32_tcgen05_of_operands_that_are_not_of_size_one(K, what, cuts):
+    """Operands whose last bits lie below bfloat16's smallest number, large ones, sums that grow, terms of very unlike sizes: no further off than float32."""
+    g = torch.Generator().manual_seed(8)
+    M, N, K_ = 40, 136, 1536
+    a, w = torch.randn(M, K_, generator=g), torch.randn(N, K_, generator=g)
+    if what == "tiny and large": a, w = a * 1e-37, w * 1e30
+    elif what == "below the normal numbers": a, w = a * 1e30, w * 1e-41
+    elif what == "results below the normal numbers": a, w = a * 1e-20, w * 1e-20
+    elif what == "large": a, w = a * 1e32, w * 1e-8
+    elif what == "one sign": a, w = a.abs(), w.abs()
+    elif what == "columns of uneven size": a, w = a * 2.0 ** torch.randint(-40, 40, (K_,), generator=g), w * 2.0 ** torch.randint(-8, 8, (K_,), generator=g)
+    else: a, w = a * 2.0 ** torch.randint(-90, 60, (M, 1), generator=g), w * 2.0 ** torch.randint(-40, 20, (N, 1), generator=g)
+    a, w = a.to(DEV), w.to(DEV)
+    out, plain = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    K.gemm_f32_tcgen05(a, w, out, tile=64, cuts=cuts)
+    K.gemm_f32(a, w, plain)
+    want = a.double() @ w.double().T
+    # each output by the sizes of its two operands, so that all of them count alike
+    unit = a.double().norm(dim=1)[:, None] * w.double().norm(dim=1)[None] * K_ ** -0.5
+    off = lambda x: ((x.double() - want) / unit).norm()
+    # three units in the last place of the outputs' sizes beside what the multiply-adds are off by, and the spacing of the smallest numbers
+    assert off(out) <= off(plain) + 3 * 2.0 ** -24 * (want / unit).norm() + (2.0 ** -149 / unit).norm()
+
+
 @pytest.mark.parametrize("heads,n,k", [(3, 33, 16), (2, 100, 48), (5, 8, 512), (2, 32, 144)])
 @pytest.mark.parametrize("gated", [False, True])
 def test_head_linear_of_few_rows_has_the_tiles_bits(K, heads, n, k, gated):
