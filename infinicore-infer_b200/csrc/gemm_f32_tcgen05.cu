@@ -10,7 +10,7 @@
 // chain.  Error against 64 bits (2-norm of the difference over that of the result, normal operands): K 1,536 1.0e-7 to 1.2e-7, the
 // multiply-adds of gemm_f32.cu 2.5e-7; K 3,840 1.1e-7 to 1.6e-7 and 4.0e-7; K 96 0.8e-7 and 0.8e-7.
 // Numbers that this does not carry (infinities, NaN, operands from 2^111 and results from 2^95 on) leave a result that
-// is not finite: such outputs are computed again from the operands by float32 multiply-adds, so they are what those give.
+// is not finite: such outputs are made again from the operands by the multiply-adds of gemm_f32.cu, in its order.
 //
 // The weights are on the MMA's M side (128 features a tile), tokens on its N side (BN of them), so that a prompt's odd number
 // of rows costs no more than its last tile of BN.  K is cut over the blocks of a cluster where tiles alone leave SMs idle;
@@ -100,12 +100,34 @@ __device__ __forceinline__ void split_store(unsigned char *dst, int plane, float
     *reinterpret_cast<uint2 *>(dst + plane) = make_uint2(m0, m1);
     *reinterpret_cast<uint2 *>(dst + 2 * plane) = make_uint2(bf16_pair(x.x, x.y), bf16_pair(x.z, x.w));
 }
-// an output that came out infinite or not a number, from the operands themselves
-__device__ __noinline__ void store_plain(const FsArgs &a, int m, int n) {
-    const float *x = a.A + (size_t)m * a.lda, *w = a.W + (size_t)n * a.ldw;
-    float sum = 0.f;
-    for (int k = 0; k < a.K; ++k) sum = fmaf(x[k], w[k], sum);
-    a.C[(size_t)m * a.ldc + n] = sum + (a.bias != nullptr ? a.bias[n] : 0.f);
+// The outputs of row m that came out infinite or not a number (`bad`), from the operands themselves, a warp a row and a lane an output: what
+// gemm_f32.cu gives, its sums in its order.  A row of A that holds a NaN, the usual cause, is known by one look at it.  301 x 7,680 x 1,536 with
+// one row of NaN takes 70 us where it takes 45 without, with an infinity in one row 145, all rows NaN some 250 (a thread an output by itself: 175, 170 and 17,000).
+__device__ __noinline__ void store_plain(const FsArgs &a, int m, int n, bool bad) {
+    const float *x = a.A + (size_t)m * a.lda;
+    bool nan = false;
+    for (int k = (threadIdx.x & 31) * 4; k < a.K; k += 128) {
+        const float4 v = *reinterpret_cast<const float4 *>(x + k);
+        nan = nan || isnan(v.x) || isnan(v.y) || isnan(v.z) || isnan(v.w);
+    }
+    nan = __any_sync(0xffffffffu, nan);
+    if (!bad) return;
+    float sum = NAN;
+    if (!nan) {
+        const float *w = a.W + (size_t)n * a.ldw;
+        float even[4] = {0.f, 0.f, 0.f, 0.f}, odd[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int k0 = 0; k0 < a.K; k0 += 64)
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int k = k0 + 4 * i, g = i / 4;
+                if (k >= a.K) break;
+                const float4 p = *reinterpret_cast<const float4 *>(x + k), q = *reinterpret_cast<const float4 *>(w + k);
+                even[g] = fmaf(p.z, q.z, fmaf(p.x, q.x, even[g]));
+                odd[g] = fmaf(p.w, q.w, fmaf(p.y, q.y, odd[g]));
+            }
+        sum = ((even[0] + odd[0]) + (even[1] + odd[1])) + ((even[2] + odd[2]) + (even[3] + odd[3])) + (a.bias != nullptr ? a.bias[n] : 0.f);
+    }
+    a.C[(size_t)m * a.ldc + n] = sum;
 }
 __device__ __forceinline__ float load_cluster(unsigned addr) {
     float v;
@@ -272,18 +294,21 @@ __global__ void __launch_bounds__(FS_THREADS, 1) gemm_f32_tcgen05_kernel(const _
             // every product of this block is complete (its last sums were read), so the ring is free to hold its share
 #pragma unroll
             for (int j = 0; j < HALF; ++j) share[(half * HALF + j) * TG_BM + quarter * 32 + lane] = acc[j];
-        } else if (n < a.N) {
-            const float bias = a.bias != nullptr ? a.bias[n] : 0.f;
+        } else {
+            const bool mine = n < a.N;
+            const float bias = mine && a.bias != nullptr ? a.bias[n] : 0.f;
             float *to = a.C + (size_t)m * a.ldc + n;
             bool finite = true;
 #pragma unroll
             for (int j = 0; j < HALF; ++j) {
                 finite = finite && isfinite(acc[j]);
-                if (m + j < a.M) to[(size_t)j * a.ldc] = fmaf(acc[j], FS_UNSCALE, bias);
+                if (mine && m + j < a.M) to[(size_t)j * a.ldc] = fmaf(acc[j], FS_UNSCALE, bias);
             }
-            if (!finite)
-                for (int j = 0; j < HALF && m + j < a.M; ++j)
-                    if (!isfinite(to[(size_t)j * a.ldc])) store_plain(a, m + j, n);
+            if (__any_sync(0xffffffffu, mine && !finite))
+                for (int j = 0; j < HALF && m + j < a.M; ++j) {
+                    const bool bad = mine && !isfinite(to[(size_t)j * a.ldc]);
+                    if (__any_sync(0xffffffffu, bad)) store_plain(a, m + j, n, bad);
+                }
         }
     }
     if (a.cuts > 1) {
@@ -293,10 +318,10 @@ __global__ void __launch_bounds__(FS_THREADS, 1) gemm_f32_tcgen05_kernel(const _
         for (int i = begin + threadIdx.x; i < end; i += FS_THREADS) {
             float v = load_cluster(cluster_addr(share + i, 0));
             for (int r = 1; r < a.cuts; ++r) v += load_cluster(cluster_addr(share + i, r));
-            const int m = m0 + i / TG_BM, n = n0 + i % TG_BM;
-            if (m >= a.M || n >= a.N) continue;
-            if (isfinite(v)) a.C[(size_t)m * a.ldc + n] = fmaf(v, FS_UNSCALE, a.bias != nullptr ? a.bias[n] : 0.f);
-            else store_plain(a, m, n);
+            const int m = m0 + i / TG_BM, n = n0 + i % TG_BM;          // a warp: 32 features of one row
+            const bool mine = m < a.M && n < a.N;
+            if (mine && isfinite(v)) a.C[(size_t)m * a.ldc + n] = fmaf(v, FS_UNSCALE, a.bias != nullptr ? a.bias[n] : 0.f);
+            if (__any_sync(0xffffffffu, mine && !isfinite(v))) store_plain(a, m, n, mine && !isfinite(v));
         }
         cluster_sync();      // no block leaves while another reads its share
     }

@@ -249,6 +249,25 @@ def test_gemm_f32_tcgen05_of_operands_that_are_not_of_size_one(K, what, cuts):
     assert off(out) <= off(plain) + 3 * 2.0 ** -24 * (want / unit).norm() + (2.0 ** -149 / unit).norm()
 
 
+@pytest.mark.parametrize("tile,cuts", [(32, 1), (32, 4), (160, 1)])
+def test_gemm_f32_tcgen05_makes_what_is_not_finite_with_the_multiply_adds_bits(K, tile, cuts):
+    """Rows with an infinity or a NaN, weights beyond what the split holds: what the product on the CUDA cores gives, and nothing else is touched."""
+    g = torch.Generator().manual_seed(6)
+    a, w, bias = torch.randn(70, 580, generator=g), torch.randn(200, 580, generator=g), torch.randn(200, generator=g)
+    clean = torch.empty(70, 200, device=DEV)
+    K.gemm_f32_tcgen05(a.to(DEV), w.to(DEV), clean, bias.to(DEV), tile=tile, cuts=cuts)
+    a[3, 5], a[33, 579], a[34, 64], w[11, 7], w[130, 0] = math.inf, math.nan, -3e36, 2e37, -math.inf
+    a, w, bias = a.to(DEV), w.to(DEV), bias.to(DEV)
+    out, plain = torch.empty(70, 200, device=DEV), torch.empty(70, 200, device=DEV)
+    K.gemm_f32_tcgen05(a, w, out, bias, tile=tile, cuts=cuts)
+    K.gemm_f32(a, w, plain, bias)
+    rows, cols = torch.ones(70, dtype=torch.bool, device=DEV), torch.ones(200, dtype=torch.bool, device=DEV)
+    rows[[3, 33, 34]] = cols[[11, 130]] = False
+    again = ~(rows[:, None] & cols[None])
+    assert torch.equal(out[again].nan_to_num(7.0), plain[again].nan_to_num(7.0)) and torch.equal(out[again].isnan(), plain[again].isnan())
+    assert torch.equal(out[~again], clean[~again])
+
+
 @pytest.mark.parametrize("heads,n,k", [(3, 33, 16), (2, 100, 48), (5, 8, 512), (2, 32, 144)])
 @pytest.mark.parametrize("gated", [False, True])
 def test_head_linear_of_few_rows_has_the_tiles_bits(K, heads, n, k, gated):
