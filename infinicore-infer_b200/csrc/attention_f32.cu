@@ -3,13 +3,15 @@
 // The row kernel of attention.cu gives a warp whole (row, head) pairs: a score is one lane's chain over the head, and the weighted
 // values one slice of it.  Here a block takes 32 or 64 rows of one request and head and 64 keys at a time: a lane makes two or four rows x 8
 // keys of scores, and two or four rows x 4 or 8 columns of every 32 of the output, so that a vector read from shared memory serves several
-// multiply-adds, two of them an instruction.  Float32 throughout: scores, weights by expf, running maximum and sums.
+// multiply-adds, two of them an instruction (two rows' scores, two columns' sums).  Float32 throughout, each sum in the row kernel's order: a
+// score is one chain over the head, chunks of 32 keys from position 0 on set the running maximum and add their weights as
+// a warp's tree does.  So a row's result is the same bits in either kernel, and does not depend on how its prompt was cut.
 // What bounds it: shared memory (a read of 16 bytes a lane takes four cycles of the SM's one port, whatever lanes share), and in short
-// prompts the chain of one block's tiles.  B200, row kernel -> this (us): 24 heads of 64 over 8, a prompt of 64 rows 15 -> 9, 301 61 -> 35, 1,200
-// 440 -> 227, 128 rows after 2,000 378 -> 181; 36 heads, 301 rows 87 -> 40; 32 heads of 128 over 2, 301 rows 113 -> 63; 8 of 128, 1,200 rows
-// 404 -> 191.  Error against 64 bits as the row kernel's or a fifth smaller.
+// prompts the chain of one block's tiles.  B200, row kernel -> this (us): 24 heads of 64 over 8, a prompt of 64 rows 15.5 -> 8.2, 301 62 -> 33, 600
+// 148 -> 82, 1,200 437 -> 232, 128 rows after 2,000 381 -> 191; 36 heads, 301 rows 88 -> 40; 32 heads of 128 over 2, 200 rows 64 -> 44, 301
+// 113 -> 67; 8 of 128, 1,200 rows 409 -> 207.
 //
-// Keys that a row does not see have weight 0; where one of their values is infinite or not a number, the tile's products leave them out.
+// Keys that a row does not see have weight 0; where one of their values is infinite or not a number, the chunk's products leave them out.
 #include "common.cuh"
 #include "host_rules.h"
 
@@ -23,7 +25,7 @@ struct AfArgs {
     const float *q, *k_pages, *v_pages;
     float *out;
     const int *tiles, *req_start, *req_pos, *block_table;
-    int nh, nkvh, page_size, page_shift, max_blocks;
+    int nh, nkvh, page_shift, max_blocks;
     float scale;
 };
 
@@ -44,7 +46,8 @@ __device__ __forceinline__ float af_hi(unsigned long long v) { return __uint_as_
 
 template <int DH, int RL> struct AfSmem {
     static constexpr int LD = DH + 4;        // eight lanes that read eight rows touch every bank once
-    float q[16 * RL * LD], k[2][AF_KEYS * LD], v[2][AF_KEYS * DH], p[AF_WARPS][4 * RL * AF_P];
+    static constexpr int LDQ = 2 * DH + 4;   // two rows of q, element by element side by side
+    float q[8 * RL * LDQ], k[2][AF_KEYS * LD], v[2][AF_KEYS * DH], p[AF_WARPS][4 * RL * AF_P];
 };
 
 // RL: rows a lane
@@ -54,7 +57,7 @@ __global__ void __launch_bounds__(AF_WARPS * 32) attention_f32_kernel(AfArgs a) 
     pdl_wait();
     extern __shared__ __align__(16) unsigned char af_raw[];
     using Smem = AfSmem<DH, RL>;
-    constexpr int AF_ROWS = 16 * RL, WR = 4 * RL, LD = Smem::LD, CHUNKS = DH / 4, PASS = AF_WARPS * 32 / CHUNKS, CN = DH / 32;
+    constexpr int AF_ROWS = 16 * RL, WR = 4 * RL, LD = Smem::LD, LDQ = Smem::LDQ, CHUNKS = DH / 4, PASS = AF_WARPS * 32 / CHUNKS, CN = DH / 32;
     Smem &s = *reinterpret_cast<Smem *>(af_raw);
     const int *tile = a.tiles + 2 * (blockIdx.x / (jk::TILE_ROWS / AF_ROWS));
     const int req = tile[0], row0 = tile[1] + blockIdx.x % (jk::TILE_ROWS / AF_ROWS) * AF_ROWS;
@@ -65,30 +68,33 @@ __global__ void __launch_bounds__(AF_WARPS * 32) attention_f32_kernel(AfArgs a) 
     const int *bt = a.block_table + (size_t)req * a.max_blocks;
     const int chunk = threadIdx.x % CHUNKS * 4, line = threadIdx.x / CHUNKS;
     // a lane looks up the page of two keys of a tile, one tile ahead of its copies
-    auto block_of = [&](int j) { return a.page_shift >= 0 ? j >> a.page_shift : j / a.page_size; };
     int page[2];
     auto look = [&](int j0) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) page[i] = bt[block_of(min(j0 + lane + 32 * i, last))];
+        for (int i = 0; i < 2; ++i) page[i] = bt[min(j0 + lane + 32 * i, last) >> a.page_shift];
     };
     auto bring = [&](int stage, int j0) {
 #pragma unroll
         for (int i = 0; i < AF_KEYS / PASS; ++i) {
             const int r = line + i * PASS, j = min(j0 + r, last);
             const int where = __shfl_sync(0xffffffffu, i * PASS < 32 ? page[0] : page[1], r & 31);
-            const size_t at = (((size_t)where * a.nkvh + hk) * a.page_size + (j - block_of(j) * a.page_size)) * DH + chunk;
+            const size_t at = ((((size_t)where * a.nkvh + hk) << a.page_shift) + (j & ((1 << a.page_shift) - 1))) * DH + chunk;
             af_copy16(s.k[stage] + r * LD + chunk, a.k_pages + at, j0 + r <= last);
             af_copy16(s.v[stage] + r * DH + chunk, a.v_pages + at, j0 + r <= last);
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
-    for (int i = 0; i < AF_ROWS / PASS; ++i) {
-        const int r = line + i * PASS;
-        af_copy16(s.q + r * LD + chunk, a.q + ((size_t)(row0 + min(r, rows - 1)) * a.nh + h) * DH + chunk, true);
-    }
     look(0);
     bring(0, 0);
     look(AF_KEYS);
+    for (int i = line; i < AF_ROWS / 2; i += PASS) {
+        const float *from = a.q + ((size_t)row0 * a.nh + h) * DH + chunk;
+        const float4 x = *reinterpret_cast<const float4 *>(from + (size_t)min(2 * i, rows - 1) * a.nh * DH);
+        const float4 y = *reinterpret_cast<const float4 *>(from + (size_t)min(2 * i + 1, rows - 1) * a.nh * DH);
+        float4 *to = reinterpret_cast<float4 *>(s.q + i * LDQ + 2 * chunk);
+        to[0] = make_float4(x.x, y.x, x.y, y.y);
+        to[1] = make_float4(x.z, y.z, x.w, y.w);
+    }
     const int rg = lane >> 3, cg = lane & 7, mine = warp * WR + rg * RL;      // this lane's rows of the tile, RL from here on
     float m[RL], l[RL];
     unsigned long long o[RL][2 * CN];
@@ -109,99 +115,115 @@ __global__ void __launch_bounds__(AF_WARPS * 32) attention_f32_kernel(AfArgs a) 
         else asm volatile("cp.async.commit_group;\n" ::: "memory");
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         __syncthreads();
-        const bool masked = j0 + AF_KEYS - 1 > pos0 + warp * WR;      // some row of the warp does not see all of the tile
-        if (j0 <= pos0 + warp * WR + WR - 1) {
-            const float *ks = s.k[stage] + cg * LD, *qs = s.q + mine * LD;
-            unsigned long long sc[RL][8];
+        const int top_pos = pos0 + warp * WR + WR - 1;      // of the warp's last row
+        if (j0 <= top_pos) {
+            const float *ks = s.k[stage] + cg * LD, *qs = s.q + mine / 2 * LDQ;
+            unsigned long long sc[RL / 2][8];               // two rows side by side
 #pragma unroll
-            for (int r = 0; r < RL; ++r)
+            for (int r = 0; r < RL / 2; ++r)
 #pragma unroll
                 for (int j = 0; j < 8; ++j) sc[r][j] = 0ull;
-#pragma unroll 4
-            for (int e = 0; e < DH; e += 4) {
-                ulonglong2 q[RL];
-#pragma unroll
-                for (int r = 0; r < RL; ++r) q[r] = *reinterpret_cast<const ulonglong2 *>(qs + r * LD + e);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const ulonglong2 k = *reinterpret_cast<const ulonglong2 *>(ks + j * 8 * LD + e);
-#pragma unroll
-                    for (int r = 0; r < RL; ++r) af_fma2(sc[r][j], q[r].x, k.x);
-#pragma unroll
-                    for (int r = 0; r < RL; ++r) af_fma2(sc[r][j], q[r].y, k.y);
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < RL; ++r) {
-                const int pos = pos0 + mine + r;
-                float x[8], top = -INFINITY;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    x[j] = (af_lo(sc[r][j]) + af_hi(sc[r][j])) * a.scale;
-                    if (masked && j0 + cg + 8 * j > pos) x[j] = -INFINITY;
-                    top = fmaxf(top, x[j]);
-                }
-#pragma unroll
-                for (int k = 4; k > 0; k >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, k));
-                const float m_new = fmaxf(m[r], top), corr = expf(m[r] - m_new);
-                m[r] = m_new;
-                float sum = 0.f;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const float w = masked && j0 + cg + 8 * j > pos ? 0.f : expf(x[j] - m_new);
-                    p[(rg * RL + r) * AF_P + cg + 8 * j] = w;
-                    sum += w;
-                }
-                l[r] = l[r] * corr + sum;
-                const unsigned long long c2 = af_pair(corr);
-#pragma unroll
-                for (int c = 0; c < 2 * CN; ++c) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(o[r][c]) : "l"(c2));
-            }
-            __syncwarp();
-            const float *vs = s.v[stage] + cg * 4, *ps = p + rg * RL * AF_P;
-            bool whole = true;
-            if (masked) {
-                float sum[4] = {0.f, 0.f, 0.f, 0.f};                 // stay 0 unless a value is infinite or not a number
-#pragma unroll 8
-                for (int i = lane * 4; i < AF_KEYS * DH; i += 128) {
-                    const float4 v = *reinterpret_cast<const float4 *>(s.v[stage] + i);
-                    sum[0] = fmaf(v.x, 0.f, sum[0]); sum[1] = fmaf(v.y, 0.f, sum[1]);
-                    sum[2] = fmaf(v.z, 0.f, sum[2]); sum[3] = fmaf(v.w, 0.f, sum[3]);
-                }
-                whole = __all_sync(0xffffffffu, (sum[0] + sum[1]) + (sum[2] + sum[3]) == 0.f);
-            }
-            if (whole) {
 #pragma unroll 2
-                for (int j = 0; j < AF_KEYS; j += 4) {
-                    float w[RL][4];
+            for (int e = 0; e < DH; e += 4) {
+                ulonglong2 q[RL / 2][2];
 #pragma unroll
-                    for (int r = 0; r < RL; ++r) *reinterpret_cast<float4 *>(w[r]) = *reinterpret_cast<const float4 *>(ps + r * AF_P + j);
+                for (int r = 0; r < RL / 2; ++r)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
+                    for (int i = 0; i < 2; ++i) q[r][i] = *reinterpret_cast<const ulonglong2 *>(qs + r * LDQ + 2 * e + 4 * i);
 #pragma unroll
-                        for (int c = 0; c < CN; ++c) {
-                            const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(vs + (j + i) * DH + 32 * c);
+                for (int j = 0; j < 8; ++j) {
+                    const float4 k = *reinterpret_cast<const float4 *>(ks + j * 8 * LD + e);
+                    const unsigned long long k0 = af_pair(k.x), k1 = af_pair(k.y), k2 = af_pair(k.z), k3 = af_pair(k.w);
 #pragma unroll
-                            for (int r = 0; r < RL; ++r) {
-                                const unsigned long long w2 = af_pair(w[r][i]);
-                                af_fma2(o[r][2 * c], w2, v.x);
-                                af_fma2(o[r][2 * c + 1], w2, v.y);
-                            }
-                        }
+                    for (int r = 0; r < RL / 2; ++r) af_fma2(sc[r][j], q[r][0].x, k0);
+#pragma unroll
+                    for (int r = 0; r < RL / 2; ++r) af_fma2(sc[r][j], q[r][0].y, k1);
+#pragma unroll
+                    for (int r = 0; r < RL / 2; ++r) af_fma2(sc[r][j], q[r][1].x, k2);
+#pragma unroll
+                    for (int r = 0; r < RL / 2; ++r) af_fma2(sc[r][j], q[r][1].y, k3);
                 }
-            } else {
-                for (int j = 0; j < AF_KEYS; ++j)
+            }
+            // the row kernel's chunks of 32 keys, one after the other
 #pragma unroll
-                    for (int r = 0; r < RL; ++r)
-                        if (j0 + j <= pos0 + mine + r) {
-                            const unsigned long long w = af_pair(ps[r * AF_P + j]);
+            for (int part = 0; part < 2; ++part) {
+                const int k0 = j0 + 32 * part;
+                if (k0 > top_pos) break;
+                const bool masked = k0 + 31 > pos0 + warp * WR;       // some row of the warp does not see all of the chunk
+#pragma unroll
+                for (int r = 0; r < RL; ++r) {
+                    const int pos = pos0 + mine + r;
+                    float x[4], top = -INFINITY;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const unsigned long long both = sc[r / 2][4 * part + j];
+                        x[j] = __fmul_rn(r % 2 ? af_hi(both) : af_lo(both), a.scale);
+                        if (!masked || k0 + cg + 8 * j <= pos) top = fmaxf(top, x[j]);
+                    }
+#pragma unroll
+                    for (int k = 4; k > 0; k >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, k));
+                    const float m_new = fmaxf(m[r], top), corr = expf(__fsub_rn(m[r], m_new));
+                    m[r] = m_new;
+                    float w[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        w[j] = masked && k0 + cg + 8 * j > pos ? 0.f : expf(__fsub_rn(x[j], m_new));
+                        p[(rg * RL + r) * AF_P + 32 * part + cg + 8 * j] = w[j];
+                    }
+                    float sum = (w[0] + w[2]) + (w[1] + w[3]);        // a warp's tree over the 32 keys
+#pragma unroll
+                    for (int k = 4; k > 0; k >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, k);
+                    l[r] = fmaf(l[r], corr, sum);
+                    const unsigned long long c2 = af_pair(corr);
+#pragma unroll
+                    for (int c = 0; c < 2 * CN; ++c) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(o[r][c]) : "l"(c2));
+                }
+                __syncwarp();
+                const float *vs = s.v[stage] + 32 * part * DH + cg * 4, *ps = p + rg * RL * AF_P + 32 * part;
+                bool whole = true;
+                if (masked) {
+                    float sum[4] = {0.f, 0.f, 0.f, 0.f};                 // stay 0 unless a value is infinite or not a number
+#pragma unroll 8
+                    for (int i = lane * 4; i < 32 * DH; i += 128) {
+                        const float4 v = *reinterpret_cast<const float4 *>(s.v[stage] + 32 * part * DH + i);
+                        sum[0] = fmaf(v.x, 0.f, sum[0]); sum[1] = fmaf(v.y, 0.f, sum[1]);
+                        sum[2] = fmaf(v.z, 0.f, sum[2]); sum[3] = fmaf(v.w, 0.f, sum[3]);
+                    }
+                    whole = __all_sync(0xffffffffu, (sum[0] + sum[1]) + (sum[2] + sum[3]) == 0.f);
+                }
+                if (whole) {
+#pragma unroll 2
+                    for (int j = 0; j < 32; j += 4) {
+                        float w[RL][4];
+#pragma unroll
+                        for (int r = 0; r < RL; ++r) *reinterpret_cast<float4 *>(w[r]) = *reinterpret_cast<const float4 *>(ps + r * AF_P + j);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
 #pragma unroll
                             for (int c = 0; c < CN; ++c) {
-                                const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(vs + j * DH + 32 * c);
-                                af_fma2(o[r][2 * c], w, v.x);
-                                af_fma2(o[r][2 * c + 1], w, v.y);
+                                const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(vs + (j + i) * DH + 32 * c);
+#pragma unroll
+                                for (int r = 0; r < RL; ++r) {
+                                    const unsigned long long w2 = af_pair(w[r][i]);
+                                    af_fma2(o[r][2 * c], w2, v.x);
+                                    af_fma2(o[r][2 * c + 1], w2, v.y);
+                                }
                             }
-                        }
+                    }
+                } else {
+                    for (int j = 0; j < 32; ++j)
+#pragma unroll
+                        for (int r = 0; r < RL; ++r)
+                            if (k0 + j <= pos0 + mine + r) {
+                                const unsigned long long w = af_pair(ps[r * AF_P + j]);
+#pragma unroll
+                                for (int c = 0; c < CN; ++c) {
+                                    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(vs + j * DH + 32 * c);
+                                    af_fma2(o[r][2 * c], w, v.x);
+                                    af_fma2(o[r][2 * c + 1], w, v.y);
+                                }
+                            }
+                }
             }
         }
         __syncthreads();
@@ -209,8 +231,6 @@ __global__ void __launch_bounds__(AF_WARPS * 32) attention_f32_kernel(AfArgs a) 
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 #pragma unroll
     for (int r = 0; r < RL; ++r) {
-#pragma unroll
-        for (int k = 4; k > 0; k >>= 1) l[r] += __shfl_xor_sync(0xffffffffu, l[r], k);
         if (mine + r >= rows) continue;
         const float inv = 1.f / l[r];
         float *to = a.out + ((size_t)(row0 + mine + r) * a.nh + h) * DH + cg * 4;
@@ -227,12 +247,12 @@ JK_EXPORT int jk_attention_f32(const float *q, const float *k_pages, const float
                                const int *block_table, int max_blocks, int page_size, int nh, int nkvh, int dh, float scale, cudaStream_t stream) {
     if (ntiles == 0) return JK_OK;
     JK_REQUIRE(q && k_pages && v_pages && out && tiles && req_start && req_pos && block_table, "attention_f32: an argument is missing");
-    JK_REQUIRE(jk_attention_f32_supports(dh, dh) && ntiles > 0 && nkvh > 0 && nh % nkvh == 0 && nh <= 65535 && page_size > 0 && max_blocks > 0,
+    JK_REQUIRE(jk_attention_f32_supports(dh, dh) && ntiles > 0 && nkvh > 0 && nh % nkvh == 0 && nh <= 65535 && page_size > 0 && (page_size & (page_size - 1)) == 0 && max_blocks > 0,
                "attention_f32: heads %d/%d of %d, page size %d", nh, nkvh, dh, page_size);
     JK_REQUIRE((((uintptr_t)q | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)out) & 15) == 0, "attention_f32: operands must be 16-byte aligned");
     int shift = 0;
     while ((1 << shift) < page_size) ++shift;
-    const AfArgs a{q, k_pages, v_pages, out, tiles, req_start, req_pos, block_table, nh, nkvh, page_size, (1 << shift) == page_size ? shift : -1, max_blocks, scale};
+    const AfArgs a{q, k_pages, v_pages, out, tiles, req_start, req_pos, block_table, nh, nkvh, shift, max_blocks, scale};
     // four rows a lane where tiles of 64 rows are enough blocks: fewer reads a multiply-add, half the blocks.  B200, two -> four rows a lane (us):
     // 24 heads of 64 over 600 rows 87 -> 93, over 1,200 255 -> 227; 36 over 600 113 -> 106; 8 heads of 128 over 600 72 -> 102, over 1,200 220 -> 191;
     // 32 over 200 47 -> 43

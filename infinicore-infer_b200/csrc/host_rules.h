@@ -319,10 +319,10 @@ inline bool attention_rows_walk(int T, int nreq, int context, int nh, int nkvh, 
     return single && n <= 8 && context <= 512;
 }
 
-// Whether a float32 attention without options runs in tiles of query rows (csrc/attention_f32.cu): every request brings more rows than go one
-// by one, and there are enough of them.  B200, by rows -> in tiles (us): 24 heads of 64 over 8, 9 rows 6.0 -> 7.4, 24 rows 7.2 -> 7.4, 40 rows 10 -> 8, 10
-// requests of 20 rows after 100 46 -> 17; 4 heads over 1, 40 rows 8.2 -> 6.7, 32 rows after 1,000 76 -> 75; pages that are no power of two: 3 heads, 200
-// rows 20 -> 22, 32 rows after 1,000 76 -> 85.
+// Whether a float32 attention without options runs in tiles of query rows (csrc/attention_f32.cu, the same bits): every request brings more rows than
+// go one by one, and there are enough of them.  B200, by rows -> in tiles (us): 24 heads of 64 over 8, 9 rows 6.0 -> 7.4, 24 rows 7.2 -> 7.4, 40 rows 10 -> 8, 10
+// requests of 20 rows after 100 46 -> 17; 4 heads over 1, 40 rows 8.2 -> 6.7, 32 rows after 1,000 76 -> 75; pages that are no power of two it
+// does not take (with a division a key: 3 heads, 200 rows 20 -> 22, 32 rows after 1,000 76 -> 85).
 inline bool attention_f32_takes(int rows, int n_short, int n_tiles, int page_size) {
     return n_short == 0 && n_tiles > 0 && rows >= 32 && page_size > 0 && (page_size & (page_size - 1)) == 0;
 }

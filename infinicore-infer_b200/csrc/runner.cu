@@ -299,7 +299,8 @@ int run_attention(Run &r, const RunnerOp &op) {
     if (dv != dh && !jk::attention_unlike_heads(dh, dv)) fast = false;
     if (fast && n_tiles > 0 && !(tc || (dv == dh && g_fns.attention_prefill_supports(dh)))) fast = false;
     if (r.env.dtype == JK_F32 && !r.env.plain_attention && g_fns.attention_f32 != nullptr && g_fns.attention_f32_supports(dh, dv) && op.window == 0 && !op.sink && !op.gated &&
-        op.cap == 0.f && op.keep_first == 0 && jk::attention_f32_takes(T, n_short, n_tiles, page)) {
+        op.cap == 0.f && op.keep_first == 0 && jk::attention_f32_takes(T, n_short, n_tiles, page) &&
+        (((uintptr_t)q | (uintptr_t)op.k_pages | (uintptr_t)op.v_pages | (uintptr_t)o) & 15) == 0) {
         RUN(attention, g_fns.attention_f32((const float *)q, (const float *)op.k_pages, (const float *)op.v_pages, (float *)o, tiles, n_tiles, r.st.req_start, r.st.req_pos, table,
                                            r.env.max_blocks, page, nh, nkvh, dh, op.softmax_scale, r.stream));
         return JK_OK;

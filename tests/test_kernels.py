@@ -340,6 +340,28 @@ def test_attention_f32_in_tiles_of_rows(K, nh, nkvh, dh, page, reqs):
         assert (out[rows].double() - want[: rows.stop - rows.start]).abs().max() <= 1e-5
 
 
+@pytest.mark.parametrize("nh,nkvh,dh,page", [(6, 2, 64, 16), (3, 1, 128, 8), (200, 200, 64, 16), (40, 8, 128, 64)])
+@pytest.mark.parametrize("reqs", [[(9, 0), (64, 3)], [(129, 60)], [(31, 200), (40, 0), (150, 129)], [(63, 1), (1, 95)]])
+def test_attention_f32_in_tiles_has_the_row_kernel_s_bits(K, nh, nkvh, dh, page, reqs):
+    """Rows and chunks of 32 keys at the edges of the tiles, both tile sizes, a value that is not finite among the keys of some rows."""
+    g = torch.Generator().manual_seed(nh + dh + len(reqs))
+    T, blocks = sum(n for n, _ in reqs), max(-(-(n + h) // page) for n, h in reqs)
+    q = (torch.randn(T, nh, dh, generator=g) * 2).to(DEV)
+    kp, vp = (torch.randn(blocks * len(reqs) + 1, nkvh, page, dh, generator=g).to(DEV) for _ in range(2))
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    table = ints([[1 + i * blocks + b for b in range(blocks)] for i in range(len(reqs))])
+    start = [0]
+    for n, _ in reqs:
+        start.append(start[-1] + n)
+    tiles = [[b, start[b] + t] for b, (n, _) in enumerate(reqs) for t in range(0, n, 128)]
+    n, h = reqs[0]
+    vp[table[0, (n + h - 1) // page], :, (n + h - 1) % page] = math.inf
+    out, rows = torch.full_like(q, 7.0), torch.full_like(q, 7.0)
+    K.attention_f32(q, kp, vp, out, ints(tiles), len(tiles), ints(start), ints([h for _, h in reqs]), table, nh, dh ** -0.5)
+    K.attention_rows(q, kp, vp, rows, ints([h + i for n, h in reqs for i in range(n)]), ints([r for r, (n, _) in enumerate(reqs) for _ in range(n)]), table, T, nh, dh ** -0.5)
+    assert torch.equal(out.nan_to_num(5.0, 6.0, -6.0), rows.nan_to_num(5.0, 6.0, -6.0)) and torch.isfinite(out[start[1]:]).all()
+
+
 @pytest.mark.parametrize("T,heads,dv", [(256, 64, 128), (1100, 32, 64), (2100, 16, 64)])
 @pytest.mark.parametrize("per_head", [0, 1, 2])
 def test_norm_gate_of_many_rows(K, T, heads, dv, per_head):
