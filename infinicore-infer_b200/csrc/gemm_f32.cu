@@ -1,5 +1,5 @@
-// The float32 matrix product on the CUDA cores:  C[M, N] = A[M, K] * W[N, K]^T (+ bias[N]).  Steps of few rows and short sums take it;
-// the others go to gemm_f32_tcgen05.cu (jk::f32_plan).
+// The float32 matrix product on the CUDA cores:  C[M, N] = A[M, K] * W[N, K]^T (+ bias[N]).  Short sums take it, and
+// operands off 16 bytes; the others go to gemm_f32_tcgen05.cu (jk::f32_plan).
 //
 // Fused multiply-adds in float32: no tensor cores, hence no TF32 rounding of the operands.
 // (reference: the products at jiuge.cpp:200, :236, :247, :249, :264 go to a library.)

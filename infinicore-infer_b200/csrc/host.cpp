@@ -100,7 +100,7 @@ JK_HOST_EXPORT int jk_f32_plan(long long rows, long long n, long long k, int sms
     const jk::F32Plan p = jk::f32_plan(rows, n, k, sms);
     return p.tile << 8 | p.cuts;
 }
-JK_HOST_EXPORT int jk_f32_tensor_rows() { return jk::F32_TENSOR_ROWS; }
+JK_HOST_EXPORT int jk_attention_f32_takes(int rows, int n_short, int n_tiles, int page_size) { return jk::attention_f32_takes(rows, n_short, n_tiles, page_size) ? 1 : 0; }
 JK_HOST_EXPORT void jk_rotary_tables(double theta, int half, int positions, double angle_scale, float *cos_out, float *sin_out) {
     jk::rotary_tables(theta, half, positions, angle_scale, cos_out, sin_out);
 }

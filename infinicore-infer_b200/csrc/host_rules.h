@@ -469,28 +469,55 @@ inline int f32_tile(long long M, long long N, int sms, double *us) {
 // tile's time; fitted to 1,700 launches of 18 shapes with 16 to 2,048 rows, nine of ten within 8 %, and what the fit chooses is within
 // 12 % of the fastest form everywhere.  A block fills an SM, and clusters of four or eight leave some SMs of a chip of 148 without a block:
 // 33 and 14 of them run at once (three tiles of 96 x 12 of 128, four cuts, 36 clusters: 29 us where 24 clusters take 20).
-// From F32_TENSOR_ROWS rows on, so that steps of few rows (decoding) add in an order that does not depend on the batch, and from K 512:
-// below, a launch costs what it saves.  CUDA cores -> tensor cores (us): 301 rows, 7,680 x 1,536 199 -> 45, 2,560 x 1,536 73 -> 27, 1,536 x 1,536
-// 46 -> 20, 1,536 x 3,840 108 -> 33; 24 rows, 1,536 x 1,536 20 -> 10; 48 rows, 2,560 x 1,536 23 -> 14; 2,048 rows, 4,608 x 4,096 1,768 -> 397.
+// From K 512: below, a launch costs what it saves.  CUDA cores -> tensor cores (us): 301 rows, 7,680 x 1,536 199 -> 45, 2,560 x 1,536 73 -> 27,
+// 1,536 x 1,536 46 -> 20, 1,536 x 3,840 108 -> 33; 48 rows, 2,560 x 1,536 23 -> 14; 2,048 rows, 4,608 x 4,096 1,768 -> 402.
+//
+// The cuts set the order of the sums (the tile does not).  Below F32_ONE_ORDER_ROWS rows, where the norms of a step add in one order too,
+// way and cuts follow from N and K alone, so that a row's result depends neither on what else is in the step nor on how its prompt
+// was cut.  One choice for all of them: the cuts that are cheapest for two steps of 32 rows (decoding) and one of 255.
+// It costs steps of 161 to 255 rows up to a third of a product, and few rows of products that are wide (CUDA cores -> tensor cores, 8 rows:
+// 11,520 x 2,304 37 -> 48, 73,440 x 1,536 89 -> 137), where the others gain (7,680 x 1,536 26 -> 21, 2,560 x 1,536 16 -> 13, 1,536 x 3,840
+// 34 -> 16, 4,096 x 16,384 134 -> 84).
 struct F32Plan { int tile, cuts; };
-constexpr int F32_TENSOR_ROWS = 24, F32_TENSOR_K = 512;
-inline F32Plan f32_plan(long long M, long long N, long long K, int sms) {
-    F32Plan best = {0, 1};
-    if (M < F32_TENSOR_ROWS || K < F32_TENSOR_K || sms <= 0) return best;
+constexpr int F32_ONE_ORDER_ROWS = 256, F32_TENSOR_K = 512;
+// microseconds of the best tile for the given cuts, and that tile; `waves`: how often it fills the chip
+inline double f32_tensor_cost(long long M, long long N, long long K, int sms, int cuts, int *tile, long long *waves) {
     constexpr int TILES[5] = {32, 64, 96, 128, 160};
     constexpr double CHUNK[5] = {1.25, 1.30, 1.30, 1.42, 1.57};
-    double least = 0.;
-    if (f32_tile(M, N, sms, &least) < 0) least = 1e30;
-    least = least * (double)K / 1536. + 2.;
+    const int at_once = std::max(1, cuts == 8 ? sms * 14 / 148 : cuts == 4 ? sms * 33 / 148 : sms / cuts);
+    double least = -1.;
+    for (int i = 0; i < 5; ++i) {
+        const long long tiles = (M + TILES[i] - 1) / TILES[i] * ((N + 127) / 128), w = (tiles + at_once - 1) / at_once;
+        if (tiles * cuts > (1LL << 30)) continue;
+        const double cost = (double)w * (0.8 + (cuts > 1 ? 2.8 : 0.) + 0.036 * TILES[i] + CHUNK[i] * (double)(((K + 63) / 64 + cuts - 1) / cuts));
+        if (least < 0. || cost < least) { least = cost; *tile = TILES[i]; *waves = w; }
+    }
+    return least;
+}
+inline F32Plan f32_plan(long long M, long long N, long long K, int sms) {
+    F32Plan best = {0, 1};
+    if (M < 1 || K < F32_TENSOR_K || sms <= 0) return best;
     const long long chunks = (K + 63) / 64;
-    for (int i = 0; i < 5; ++i)
-        for (int cuts = 1; cuts <= 8; cuts *= 2) {
-            const long long blocks = (M + TILES[i] - 1) / TILES[i] * ((N + 127) / 128) * cuts;
-            if (blocks > (1LL << 30) || (cuts > 1 && (chunks < 2 * cuts || blocks > (cuts == 8 ? sms * 112 / 148 : cuts == 4 ? sms * 132 / 148 : sms)))) continue;
-            const double cost = (double)((blocks + sms - 1) / sms) *
-                                (0.8 + (cuts > 1 ? 2.8 : 0.) + 0.036 * TILES[i] + CHUNK[i] * (double)((chunks + cuts - 1) / cuts));
-            if (cost < least) { least = cost; best = {TILES[i], cuts}; }
+    const bool one_order = M < F32_ONE_ORDER_ROWS;
+    double least = -1.;
+    if (!one_order && f32_tile(M, N, sms, &least) >= 0) least = least * (double)K / 1536. + 2.;
+    for (int cuts = 1; cuts <= 8; cuts *= 2) {
+        if (cuts > 1 && chunks < 2 * cuts) continue;
+        int tile = 0;
+        long long waves = 0;
+        double cost;
+        if (one_order) {
+            const double few = f32_tensor_cost(32, N, K, sms, cuts, &tile, &waves), many = f32_tensor_cost(F32_ONE_ORDER_ROWS - 1, N, K, sms, cuts, &tile, &waves);
+            if (few < 0. || many < 0.) continue;
+            cost = 2. * few + many;
+        } else {
+            cost = f32_tensor_cost(M, N, K, sms, cuts, &tile, &waves);
+            if (cost < 0. || (cuts > 1 && waves > 1)) continue;
         }
+        if (least < 0. || cost < least) { least = cost; best = {tile, cuts}; }
+    }
+    long long waves = 0;
+    if (one_order && best.tile > 0) f32_tensor_cost(M, N, K, sms, best.cuts, &best.tile, &waves);
     return best;
 }
 

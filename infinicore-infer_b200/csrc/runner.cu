@@ -3,8 +3,9 @@
 // One call launches every kernel of a run of records (for the standard stack: the whole step, embedding to logits)
 // where Python would make a dozen calls a layer.  Which kernel runs a record is decided here and nowhere else:
 //
-//   float32       products of few rows on the CUDA cores (gemm_f32), of many rows on the tensor cores with every operand split into
-//                 three bfloat16 parts (gemm_f32_tcgen05), by jk::f32_plan; attention by the row kernel
+//   float32       products of short sums on the CUDA cores (gemm_f32), the others on the tensor cores with every operand split into
+//                 three bfloat16 parts (gemm_f32_tcgen05), by jk::f32_plan; attention by the row kernel, or in tiles of query
+//                 rows with the same bits where every request brings many (attention_f32, by jk::attention_f32_takes)
 //   bfloat16      products by the rules of host_rules.h (jk::product_route):
 //                   rows <= 16          the weight-streaming kernels of linear_small.cu (q/k/v with rotation and cache
 //                                       write in the epilogue, gate/up with SwiGLU in the epilogue)
@@ -1208,6 +1209,19 @@ JK_EXPORT int jk_runner_needs_gemm_tcgen05(const RunnerEnv *env, const RunnerOp 
                 if (rt2 == jk::ROUTE_SKINNY || rt2 == jk::ROUTE_TCGEN05) return 1;
             }
     }
+    return 0;
+}
+
+// Whether records [0, count) can reach the split float32 product (its way follows from N and K, whatever the step's rows).
+JK_EXPORT int jk_runner_needs_gemm_f32_tcgen05(const RunnerEnv *env, const RunnerOp *ops, int count) {
+    if (!env || !ops || env->dtype != JK_F32 || env->routing.library_only) return 0;
+    for (int i = 0; i < count; ++i)
+        switch (ops[i].kind) {
+            case OP_QKV: case OP_LINEAR: case OP_REINJECT: case OP_RESIDUAL: case OP_GATE_UP:
+                if (ops[i].k >= jk::F32_TENSOR_K) return 1;
+                break;
+            default: break;
+        }
     return 0;
 }
 

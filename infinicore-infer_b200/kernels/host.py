@@ -30,6 +30,7 @@ def lib() -> ctypes.CDLL:
         h.jk_pool_is_held.argtypes = [_c_p, _c_int]
         h.jk_decode_scratch_floats.restype = ctypes.c_longlong
         h.jk_uniform_for.restype = ctypes.c_float
+        h.jk_f32_plan.argtypes = [ctypes.c_longlong] * 3 + [_c_int]
         h.jk_uniform_for.argtypes = [ctypes.c_ulonglong, ctypes.c_ulonglong]
         h.jk_rotary_tables.argtypes = [ctypes.c_double, _c_int, _c_int, ctypes.c_double, _c_p, _c_p]
         h.jk_rotary_tables.restype = None
@@ -193,9 +194,9 @@ def f32_plan(rows: int, n: int, k: int, sms: int = 148):
     return plan >> 8, plan & 255
 
 
-def f32_tensor_rows() -> int:
-    """Fewest rows of a float32 product on the tensor cores."""
-    return lib().jk_f32_tensor_rows()
+def attention_f32_takes(rows: int, n_short: int, n_tiles: int, page_size: int) -> bool:
+    """Whether a plain float32 attention runs in tiles of query rows."""
+    return bool(lib().jk_attention_f32_takes(rows, n_short, n_tiles, page_size))
 
 
 # ---- tables and uniforms -----------------------------------------------------------------------------------------------

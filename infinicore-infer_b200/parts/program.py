@@ -360,7 +360,7 @@ def modules_needed(env: RunnerEnv, ops, count: int, max_rows: int) -> Dict[str, 
                 op.kind == OP["attention"] and _host.attention_tcgen05_takes(op.head_dim, env.page_size, op.v_head_dim) for op in records)),
             "mixers": any(op.kind in _MIXERS_OPS or (op.kind == OP["gate_up"] and op.act > ACT["silu"]) for op in records),
             "blocks": any(op.kind in _BLOCKS_OPS for op in records),
-            "gemm_f32_tcgen05": env.dtype == _dtype_code(torch.float32) and not env.routing.library_only and max_rows >= _host.f32_tensor_rows()}
+            "gemm_f32_tcgen05": bool(_build.load("runner").jk_runner_needs_gemm_f32_tcgen05(ctypes.byref(env), ops, count))}
 
 
 def free_bytes(device) -> int:
@@ -424,8 +424,7 @@ class ProgramRunner:
         if rt.routing_key() != self._routing_key:       # a test moved a threshold or a switch
             self._routing_key = rt.routing_key()
             self.env = rt.env(prog.page_size, prog.max_blocks)
-            need_gemm = bool(prog.lib.jk_runner_needs_gemm_tcgen05(ctypes.byref(self.env), prog.ops, prog.count, self.max_rows))
-            runner_lib(need_gemm, _bound["attention_tcgen05"])
+            runner_lib(**modules_needed(self.env, prog.ops, prog.count, self.max_rows))
         T = ctx.ntok
         if T > self.max_rows:
             raise kernels.KernelError(f"the step's buffers hold {self.max_rows} rows, the step has {T}")

@@ -97,11 +97,11 @@ def test_way_of_a_latent_attention(dim, rot, rank, requests, window, heads):
 
 @pytest.mark.parametrize("rows,n,k,tensor", [
     # microseconds: on the CUDA cores, on the tensor cores
-    (16, 2560, 1536, False), (23, 7680, 1536, False),               # few rows keep the order of sums that single rows have
+    (16, 2560, 1536, True), (23, 7680, 1536, True),                 # 16, 13; 26, 21: below 256 rows K alone decides
     (24, 1536, 1536, True), (32, 11264, 2048, True),                # 20, 10; 52, 45
     (301, 7680, 1536, True), (301, 1536, 3840, True),               # 199, 45; 108, 33
     (64, 64, 2048, True), (2048, 512, 512, True),                   # 19, 9; 35, 14
-    (32, 512, 512, False), (64, 512, 512, False),                   # 7, 7; 7, 7
+    (32, 512, 512, True), (64, 512, 512, True), (64, 512, 508, False),      # 7, 7; 7, 7
     (301, 288, 96, False), (640, 1024, 256, False)])                # 3, 5; 15, 9: short sums stay
 def test_float32_products_on_the_tensor_cores(rows, n, k, tensor):
     tile, cuts = host.f32_plan(rows, n, k)
@@ -109,6 +109,20 @@ def test_float32_products_on_the_tensor_cores(rows, n, k, tensor):
     # the blocks of clusters that run at once on 148 SMs, one a block: 33 of four, 14 of eight
     blocks = -(-rows // tile) * -(-n // 128) * cuts if tile else 0
     assert cuts in (1, 2, 4, 8) and (cuts == 1 or blocks <= {2: 148, 4: 132, 8: 112}[cuts])
+
+
+@pytest.mark.parametrize("n,k,cuts", [(2560, 1536, 4), (1536, 1536, 4), (7680, 1536, 2), (1536, 3840, 8), (11520, 2304, 1), (4096, 16384, 4), (64, 2048, 8),
+                                      (512, 512, 4), (73440, 1536, 1), (1, 512, 4), (300, 511, 0)])
+def test_float32_products_of_few_rows_add_in_one_order(n, k, cuts):
+    """Below 256 rows neither the way nor the cuts of K, which set the order of a row's sums, depend on the rows; the tile may."""
+    plans = [host.f32_plan(rows, n, k) for rows in range(1, 256)]
+    assert {c if t else 0 for t, c in plans} == {cuts}
+
+
+@pytest.mark.parametrize("rows,short,tiles,page,takes", [(31, 0, 1, 16, False), (32, 0, 1, 16, True), (32, 1, 1, 16, False), (300, 0, 0, 16, False), (300, 0, 3, 24, False),
+                                                         (300, 0, 3, 1, True), (300, 0, 3, 256, True)])
+def test_float32_attention_in_tiles(rows, short, tiles, page, takes):
+    assert host.attention_f32_takes(rows, short, tiles, page) == takes
 
 
 def test_sampling_parameters_beyond_their_types_are_clamped(monkeypatch):
