@@ -929,7 +929,7 @@ static size_t head_rows_smem(int K) { return (size_t)(HR_ROWS + HR_FEATURES) * (
 static bool head_takes_rows(int rows, int K) { return rows <= 64 && K % 16 == 0 && head_rows_smem(K) <= 100 * 1024; }
 
 __global__ void __launch_bounds__(HR_THREADS) head_rows_kernel(const __nv_bfloat16 *in, const __nv_bfloat16 *w, __nv_bfloat16 *out, int rows, int H, int N, int K, int out_hs,
-                                                               const float *gate, int gate_ld, int gate_head) {
+                                                               const float *gate, int gate_ld, int gate_head, int *status) {
     extern __shared__ __align__(128) unsigned char hr_smem[];
     __shared__ unsigned long long full[2];
     pdl_trigger();
@@ -955,6 +955,7 @@ __global__ void __launch_bounds__(HR_THREADS) head_rows_kernel(const __nv_bfloat
     }
     // a warp whose features lie behind the last one has nothing to do
     const bool ok = mbar_wait(&full[0], 0) && mbar_wait(&full[1], 0);
+    if (!ok && lane == 0 && status != nullptr) atomicExch(status, 25);
     if (n0 + warp * 8 >= N) return;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     const __nv_bfloat16 *a_at = reinterpret_cast<const __nv_bfloat16 *>(xs + (lane & 15) * pitch) + (lane >> 4) * 8;
@@ -981,7 +982,7 @@ __global__ void __launch_bounds__(HR_THREADS) head_rows_kernel(const __nv_bfloat
 }
 
 JK_EXPORT int jk_head_linear(const void *in, const void *w, void *out, int dtype, int rows, int H, int N, int K, int out_hs,
-                             const float *gate, int gate_ld, int gate_head, cudaStream_t stream) {
+                             const float *gate, int gate_ld, int gate_head, int *status, cudaStream_t stream) {
     if (rows == 0) return JK_OK;
     JK_REQUIRE(in && w && out && rows > 0 && H > 0 && N > 0 && K > 0 && out_hs >= N, "head_linear: rows %d, heads %d, %d x %d into %d", rows, H, N, K, out_hs);
     JK_REQUIRE(H <= 65535, "head_linear: %d heads exceed one launch", H);
@@ -989,7 +990,7 @@ JK_EXPORT int jk_head_linear(const void *in, const void *w, void *out, int dtype
         const size_t smem = head_rows_smem(K);
         if (smem > 46 * 1024) cudaFuncSetAttribute(head_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         jk_launch(head_rows_kernel, dim3((N + HR_FEATURES - 1) / HR_FEATURES, H, (rows + HR_ROWS - 1) / HR_ROWS), dim3(HR_THREADS), smem, stream, (const __nv_bfloat16 *)in,
-                  (const __nv_bfloat16 *)w, (__nv_bfloat16 *)out, rows, H, N, K, out_hs, gate, gate_ld, gate_head);
+                  (const __nv_bfloat16 *)w, (__nv_bfloat16 *)out, rows, H, N, K, out_hs, gate, gate_ld, gate_head, status);
         JK_CHECK_LAUNCH("head_linear");
         return JK_OK;
     }
@@ -2557,6 +2558,7 @@ template <typename T, bool GLU> struct ExpertRowsBlock {
             for (int r = 0; r < ROWS; ++r) {
                 if (r >= rows) break;
                 const size_t at = (size_t)(first + r) * a.N + n;
+                if (!ok) { g[r] = NAN; u[r] = NAN; }          // a wait that ran out does not pass for a result
                 if (GLU) {
                     if (n < a.N) ((T *)a.out)[at] = from_f32<T>(expert_inner(a.actf, a.entry_score ? written_float(a.entry_score + first + r) : 1.f, g[r], u[r], a.limit));
                 } else {

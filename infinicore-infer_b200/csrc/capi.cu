@@ -438,7 +438,7 @@ int check_status(JkModel *m) {
         if (status == 4)
             JK_FAIL(JK_CUDA_ERROR, "batch: a row's sum of squares is beyond the range of the fixed-point counters; the results "
                                    "of this batch are invalid (JK_NO_FUSED_NORM=1 keeps the norm kernels, which have no such limit)");
-        JK_FAIL(JK_CUDA_ERROR, "batch: a tcgen05 kernel gave up a bounded wait (status %d); the results of this batch are invalid", status);
+        JK_FAIL(JK_CUDA_ERROR, "batch: a kernel gave up a bounded wait (status %d); the results of this batch are invalid", status);
     }
     return JK_OK;
 }

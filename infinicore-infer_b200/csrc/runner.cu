@@ -690,7 +690,7 @@ int run_head_linear(Run &r, const RunnerOp &op) {
         if (int rc = r.slot(SLOT_TMP, 4LL * T * op.ld, &u, "the projection that holds the gate")) return rc;
         gate = (const float *)u + op.g_off;
     }
-    RUN(blocks, g_fns.head_linear(in, op.w, out, r.env.dtype, T, op.heads, op.n, op.k, op.out_hs, gate, op.ld, op.gated == 2, r.stream));
+    RUN(blocks, g_fns.head_linear(in, op.w, out, r.env.dtype, T, op.heads, op.n, op.k, op.out_hs, gate, op.ld, op.gated == 2, r.env.status, r.stream));
     return JK_OK;
 }
 

@@ -76,7 +76,7 @@ typedef int (*ConcatCastFn)(const float *, const float *, void *, int, int, int,
 typedef int (*AddBiasRowsFn)(float *, const float *, int, int, cudaStream_t);
 typedef int (*LatentQkvFn)(const float *, int, int, int, int, int, int, int, int, const float *, float, const float *, float, const int *,
                            const int *, const int *, int, int, void *, void *, void *, int, int, const float *, int, int, cudaStream_t);
-typedef int (*HeadLinearFn)(const void *, const void *, void *, int, int, int, int, int, int, const float *, int, int, cudaStream_t);
+typedef int (*HeadLinearFn)(const void *, const void *, void *, int, int, int, int, int, int, const float *, int, int, int *, cudaStream_t);
 typedef int (*LatentAttentionFn)(const void *, const void *, void *, float *, int, const int *, const int *, const int *, int, int, int,
                                  int, int, int, float, int, const int *, int, int, const float *, cudaStream_t);
 typedef long long (*LatentScratchFn)(int, int, int, int);

@@ -385,15 +385,24 @@ def check_gemm_status(device) -> None:
         code = int(_tg_status[key].item())
         if code:
             _tg_status[key].zero_()
-            if code == 4:
-                raise KernelError("linear_small: a row's sum of squares is beyond the range of the fixed-point counters "
-                                  "(activations of several thousand on average); the step's results are not valid; "
-                                  "JK_NO_FUSED_NORM=1 keeps the norm kernels, which have no such limit")
-            if 31 <= code <= 33:
-                raise KernelError(f"gemm_f32_tcgen05: a bounded wait ran out (role {code - 30}: 1 MMA, 2 tokens, 3 weights and sums); "
-                                  "the step's results are not valid")
-            raise KernelError(f"gemm_tcgen05: a bounded wait ran out (role {code}: 1 TMA, 2 MMA, 3 epilogue); "
-                              "the step's results are not valid")
+            raise KernelError(_status_message(code))
+
+
+# who writes which codes into the status word, from the first one on, and what waited
+_STATUS_CODES = ((1, "gemm_tcgen05", ("TMA", "MMA", "epilogue")), (11, "attention_tcgen05", ("TMA", "MMA", "softmax", "misaligned shared memory")),
+                 (21, "routed_experts of many rows", ("TMA", "MMA", "epilogue")), (24, "routed_experts of few rows", ("copies",)),
+                 (25, "head_linear of few rows", ("copies",)), (31, "gemm_f32_tcgen05", ("MMA", "tokens", "weights and sums")))
+
+
+def _status_message(code: int) -> str:
+    if code == 4:
+        return ("linear_small: a row's sum of squares is beyond the range of the fixed-point counters "
+                "(activations of several thousand on average); the step's results are not valid; "
+                "JK_NO_FUSED_NORM=1 keeps the norm kernels, which have no such limit")
+    for first, kernel, roles in _STATUS_CODES:
+        if first <= code < first + len(roles):
+            return f"{kernel}: a bounded wait ran out ({roles[code - first]}, code {code}); the step's results are not valid"
+    return f"a kernel left status code {code}; the step's results are not valid"
 
 
 def gemm_tcgen05_supports(m: int, n: int, k: int) -> bool:
@@ -823,7 +832,8 @@ def head_linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, out_head_st
     H, n, k = w.shape
     lib = _build.load("blocks")
     _check("blocks", lib.jk_head_linear(_ptr(x), _ptr(w), _ptr(out), _c_int(dtype_code(x.dtype)), _c_int(x.shape[0]), _c_int(H), _c_int(n),
-                                        _c_int(k), _c_int(out_head_stride), _ptr(gate), _c_int(gate_ld), _c_int(1 if gate_head else 0), _stream()))
+                                        _c_int(k), _c_int(out_head_stride), _ptr(gate), _c_int(gate_ld), _c_int(1 if gate_head else 0),
+                                        _ptr(gemm_status(x.device)), _stream()))
     return out
 
 

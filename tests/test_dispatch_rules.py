@@ -125,6 +125,25 @@ def test_float32_attention_in_tiles(rows, short, tiles, page, takes):
     assert host.attention_f32_takes(rows, short, tiles, page) == takes
 
 
+@pytest.mark.parametrize("code,words", [(1, "gemm_tcgen05: a bounded wait ran out (TMA"), (4, "linear_small: a row's sum of squares"), (14, "attention_tcgen05"),
+                                        (23, "routed_experts of many rows"), (24, "routed_experts of few rows: a bounded wait ran out (copies"),
+                                        (25, "head_linear of few rows: a bounded wait ran out (copies"), (33, "gemm_f32_tcgen05: a bounded wait ran out (weights and sums"),
+                                        (99, "status code 99")])
+def test_a_status_word_names_its_kernel(monkeypatch, code, words):
+    """The word as a kernel leaves it: the check raises with the kernel's own name, and clears it."""
+    import torch
+
+    from infinicore_infer_b200 import kernels
+    word = torch.tensor([code], dtype=torch.int32)
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda device=None: None)
+    monkeypatch.setattr(kernels._build, "_loaded", {})
+    monkeypatch.setitem(kernels._tg_status, "a device", word)
+    with pytest.raises(kernels.KernelError) as e:
+        kernels.check_gemm_status("a device")
+    assert words in str(e.value) and int(word) == 0
+    kernels.check_gemm_status("a device")
+
+
 def test_sampling_parameters_beyond_their_types_are_clamped(monkeypatch):
     """A top-k beyond 32 bits or infinite reaches the draw as the largest whole number."""
     import torch
