@@ -253,11 +253,6 @@ JK_EXPORT int jk_attention_f32(const float *q, const float *k_pages, const float
     int shift = 0;
     while ((1 << shift) < page_size) ++shift;
     const AfArgs a{q, k_pages, v_pages, out, tiles, req_start, req_pos, block_table, nh, nkvh, shift, max_blocks, scale};
-    // four rows a lane where tiles of 64 rows are enough blocks: fewer reads a multiply-add, half the blocks.  B200, two -> four rows a lane (us):
-    // 24 heads of 64 over 600 rows 87 -> 93, over 1,200 255 -> 227; 36 over 600 113 -> 106; 8 heads of 128 over 600 72 -> 102, over 1,200 220 -> 191;
-    // 32 over 200 47 -> 43
-    const long long blocks = 2LL * ntiles * nh;
-    const bool four = blocks >= (dh == 64 ? 350 : 120);
     auto run = [&](auto kernel, size_t smem, int rows) -> int {
         const dim3 grid(ntiles * (jk::TILE_ROWS / rows), nh);
         const cudaError_t e = cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -266,6 +261,6 @@ JK_EXPORT int jk_attention_f32(const float *q, const float *k_pages, const float
         JK_CHECK_LAUNCH("attention_f32");
         return JK_OK;
     };
-    if (four) return dh == 64 ? run(attention_f32_kernel<64, 4>, sizeof(AfSmem<64, 4>), 64) : run(attention_f32_kernel<128, 4>, sizeof(AfSmem<128, 4>), 64);
+    if (jk::attention_f32_tall(2LL * ntiles * nh, dh)) return dh == 64 ? run(attention_f32_kernel<64, 4>, sizeof(AfSmem<64, 4>), 64) : run(attention_f32_kernel<128, 4>, sizeof(AfSmem<128, 4>), 64);
     return dh == 64 ? run(attention_f32_kernel<64, 2>, sizeof(AfSmem<64, 2>), 32) : run(attention_f32_kernel<128, 2>, sizeof(AfSmem<128, 2>), 32);
 }

@@ -924,9 +924,7 @@ __global__ void __launch_bounds__(256) head_linear_kernel(const T *__restrict__ 
 // What bounds it: latency, of one round of copies where the tiles wait for K / 32 of them.
 // B200, tiles of 64 x 64 -> this (us): 16 heads of 512 x 128, one row 4.9 -> 2.1, 16 5.2 -> 3.0, 64 7.8 -> 4.8; of 128 x 512 6.8 -> 2.3, 7.2 -> 2.8, 7.8 -> 4.0;
 // 40 of 512 x 128 5.6 -> 3.5, 64 rows 11.0 -> 8.0; 2 of 64 x 64 2.3 -> 1.4, 64 rows 2.8 -> 2.0.
-constexpr int HR_ROWS = 16, HR_FEATURES = 32, HR_THREADS = 32 * HR_FEATURES / 8;
-static size_t head_rows_smem(int K) { return (size_t)(HR_ROWS + HR_FEATURES) * (2 * K + 16) + 64; }
-static bool head_takes_rows(int rows, int K) { return rows <= 64 && K % 16 == 0 && head_rows_smem(K) <= 100 * 1024; }
+constexpr int HR_ROWS = jk::HEAD_ROWS, HR_FEATURES = jk::HEAD_FEATURES, HR_THREADS = 32 * HR_FEATURES / 8;
 
 __global__ void __launch_bounds__(HR_THREADS) head_rows_kernel(const __nv_bfloat16 *in, const __nv_bfloat16 *w, __nv_bfloat16 *out, int rows, int H, int N, int K, int out_hs,
                                                                const float *gate, int gate_ld, int gate_head, int *status) {
@@ -986,8 +984,8 @@ JK_EXPORT int jk_head_linear(const void *in, const void *w, void *out, int dtype
     if (rows == 0) return JK_OK;
     JK_REQUIRE(in && w && out && rows > 0 && H > 0 && N > 0 && K > 0 && out_hs >= N, "head_linear: rows %d, heads %d, %d x %d into %d", rows, H, N, K, out_hs);
     JK_REQUIRE(H <= 65535, "head_linear: %d heads exceed one launch", H);
-    if (dtype == JK_BF16 && head_takes_rows(rows, K) && (((uintptr_t)in | (uintptr_t)w) & 15) == 0) {
-        const size_t smem = head_rows_smem(K);
+    if (dtype == JK_BF16 && jk::head_takes_rows(rows, K) && (((uintptr_t)in | (uintptr_t)w) & 15) == 0) {
+        const size_t smem = (size_t)jk::head_rows_bytes(K);
         if (smem > 46 * 1024) cudaFuncSetAttribute(head_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         jk_launch(head_rows_kernel, dim3((N + HR_FEATURES - 1) / HR_FEATURES, H, (rows + HR_ROWS - 1) / HR_ROWS), dim3(HR_THREADS), smem, stream, (const __nv_bfloat16 *)in,
                   (const __nv_bfloat16 *)w, (__nv_bfloat16 *)out, rows, H, N, K, out_hs, gate, gate_ld, gate_head, status);
@@ -2431,14 +2429,6 @@ __global__ void __launch_bounds__(256) expert_down_kernel(const T *__restrict__ 
 constexpr int ER_ROWS = 8, EF_BYTES = 4096;          // entries at a time; bytes of a row at a time
 __host__ __device__ constexpr int ef_chunk(int K, int elem) { return K * elem < EF_BYTES ? K * elem : EF_BYTES; }
 __host__ __device__ constexpr int ef_smem(int K, int elem, int groups) { return (16 * groups + ER_ROWS) * ef_chunk(K, elem); }
-// Groups of 16 rows a block: a short row's copy costs a block more than its bytes, so where blocks make several waves (four an SM) a block takes more of
-// them.  B200, 48 entries of 64 experts of 64 features over 2,048: 53.4 us with one group, 45.2 with four; but 2 entries of 512 18.5 and 20.6: one there.
-inline int ef_groups(int K, int elem, long long blocks) {
-    int groups = 1;
-    while (2 * groups * K * elem <= 2048 && groups < 4 && blocks / (2 * groups) >= 4 * 148) groups *= 2;
-    return groups;
-}
-
 // The expert of the slot-th run of entries, or -1; a whole warp asks, for up to 256 experts at a time with one wait for memory.
 __device__ __forceinline__ int expert_with_entries(const int *starts, int E, int slot) {
     const int lane = threadIdx.x & 31;
@@ -2744,7 +2734,7 @@ JK_EXPORT int jk_routed_experts(const void *h, const float *router, const void *
     } else if (stream_rows) {
         // (grids of fewer blocks than experts find out late which expert is theirs)
         const int elem = dtype == JK_F32 ? 4 : 2, eager = pairs >= 2 * E, runs = std::min(E, pairs);
-        const int up_groups = ef_groups(D, elem, (long long)runs * ((ff + 7) / 8)), down_groups = ef_groups(ff, elem, (long long)runs * ((D + 15) / 16));
+        const int up_groups = jk::expert_row_groups(D, elem, (long long)runs * ((ff + 7) / 8)), down_groups = jk::expert_row_groups(ff, elem, (long long)runs * ((D + 15) / 16));
         const int up_rows = 8 * up_groups, down_rows = 16 * down_groups, smem_up = ef_smem(D, elem, up_groups), smem_down = ef_smem(ff, elem, down_groups);
         const ExpertRowsArgs up{h, w_gate_up, act, D, ff, E, starts, entry_row, in_score, actf, limit, eager, up_groups, status};
         const ExpertRowsArgs down{act, w_down, y, ff, D, E, starts, nullptr, nullptr, 0, 0.f, eager, down_groups, status};

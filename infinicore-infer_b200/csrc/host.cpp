@@ -101,6 +101,9 @@ JK_HOST_EXPORT int jk_f32_plan(long long rows, long long n, long long k, int sms
     return p.tile << 8 | p.cuts;
 }
 JK_HOST_EXPORT int jk_attention_f32_takes(int rows, int n_short, int n_tiles, int page_size) { return jk::attention_f32_takes(rows, n_short, n_tiles, page_size) ? 1 : 0; }
+JK_HOST_EXPORT int jk_attention_f32_tall(long long blocks, int dh) { return jk::attention_f32_tall(blocks, dh) ? 1 : 0; }
+JK_HOST_EXPORT int jk_head_takes_rows(int rows, int k) { return jk::head_takes_rows(rows, k) ? 1 : 0; }
+JK_HOST_EXPORT int jk_expert_row_groups(int k, int elem, long long blocks) { return jk::expert_row_groups(k, elem, blocks); }
 JK_HOST_EXPORT void jk_rotary_tables(double theta, int half, int positions, double angle_scale, float *cos_out, float *sin_out) {
     jk::rotary_tables(theta, half, positions, angle_scale, cos_out, sin_out);
 }

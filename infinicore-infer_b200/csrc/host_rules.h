@@ -327,6 +327,25 @@ inline bool attention_f32_takes(int rows, int n_short, int n_tiles, int page_siz
     return n_short == 0 && n_tiles > 0 && rows >= 32 && page_size > 0 && (page_size & (page_size - 1)) == 0;
 }
 
+// Whether its tiles have 64 rows, four a lane, instead of 32: where `blocks` tiles of 64 are enough.  Fewer reads a multiply-add, half the blocks.
+// B200, two -> four rows a lane (us): 24 heads of 64 over 600 rows 87 -> 93, over 1,200 255 -> 227; 36 over 600 113 -> 106; 8 heads of 128 over
+// 600 72 -> 102, over 1,200 220 -> 191; 32 over 200 47 -> 43.
+inline bool attention_f32_tall(long long blocks, int dh) { return blocks >= (dh == 64 ? 350 : 120); }
+
+// ---- routed experts and heads' products of few rows (csrc/blocks.cu) ---------------------------------------------------------------
+// Bytes of shared memory of a block of a per-head product of few rows, and whether that form takes `rows` rows with K columns.
+constexpr int HEAD_ROWS = 16, HEAD_FEATURES = 32;
+inline long long head_rows_bytes(int K) { return (long long)(HEAD_ROWS + HEAD_FEATURES) * (2LL * K + 16) + 64; }
+inline bool head_takes_rows(int rows, int K) { return rows <= 64 && K % 16 == 0 && head_rows_bytes(K) <= 100 * 1024; }
+// Groups of 16 rows of its matrix that a block of an expert's product of few rows takes, for K columns of `elem` bytes and `blocks` blocks of one
+// group: a short row's copy costs a block more than its bytes, so where blocks make several waves (four an SM) a block takes more of
+// them.  B200, 48 entries of 64 experts of 64 features over 2,048: 53.4 us with one group, 45.2 with four; but 2 entries of 512 18.5 and 20.6: one there.
+inline int expert_row_groups(int K, int elem, long long blocks) {
+    int groups = 1;
+    while (2 * groups * K * elem <= 2048 && groups < 4 && blocks / (2 * groups) >= 4 * 148) groups *= 2;
+    return groups;
+}
+
 // Whether a causal convolution over `rows` rows of `nreq` requests walks eight rows a thread (csrc/blocks.cu) instead of making an element
 // a thread: a walk is a chain that takes a large launch to hide, the more so where every row is a request of its own and reads and
 // moves its own tail.  B200, element a thread -> rows (us): 64 channels, 128 to 2,048 rows 9 -> 13; 512 channels, 512 rows 11 to 13 -> 13,

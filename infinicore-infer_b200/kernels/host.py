@@ -31,6 +31,8 @@ def lib() -> ctypes.CDLL:
         h.jk_decode_scratch_floats.restype = ctypes.c_longlong
         h.jk_uniform_for.restype = ctypes.c_float
         h.jk_f32_plan.argtypes = [ctypes.c_longlong] * 3 + [_c_int]
+        h.jk_attention_f32_tall.argtypes = [ctypes.c_longlong, _c_int]
+        h.jk_expert_row_groups.argtypes = [_c_int, _c_int, ctypes.c_longlong]
         h.jk_uniform_for.argtypes = [ctypes.c_ulonglong, ctypes.c_ulonglong]
         h.jk_rotary_tables.argtypes = [ctypes.c_double, _c_int, _c_int, ctypes.c_double, _c_p, _c_p]
         h.jk_rotary_tables.restype = None
@@ -197,6 +199,21 @@ def f32_plan(rows: int, n: int, k: int, sms: int = 148):
 def attention_f32_takes(rows: int, n_short: int, n_tiles: int, page_size: int) -> bool:
     """Whether a plain float32 attention runs in tiles of query rows."""
     return bool(lib().jk_attention_f32_takes(rows, n_short, n_tiles, page_size))
+
+
+def attention_f32_tall(blocks: int, dh: int) -> bool:
+    """Whether its tiles have 64 rows instead of 32, ``blocks`` of them."""
+    return bool(lib().jk_attention_f32_tall(blocks, dh))
+
+
+def head_takes_rows(rows: int, k: int) -> bool:
+    """Whether a per-head product of bfloat16 streams its weights past few rows."""
+    return bool(lib().jk_head_takes_rows(rows, k))
+
+
+def expert_row_groups(k: int, elem: int, blocks: int) -> int:
+    """Groups of 16 matrix rows that a block of an expert's product of few rows takes."""
+    return lib().jk_expert_row_groups(k, elem, blocks)
 
 
 # ---- tables and uniforms -----------------------------------------------------------------------------------------------

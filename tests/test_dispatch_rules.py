@@ -125,6 +125,23 @@ def test_float32_attention_in_tiles(rows, short, tiles, page, takes):
     assert host.attention_f32_takes(rows, short, tiles, page) == takes
 
 
+@pytest.mark.parametrize("blocks,dh,tall", [(349, 64, False), (350, 64, True), (119, 128, False), (120, 128, True)])
+def test_tiles_of_the_float32_attention(blocks, dh, tall):
+    assert host.attention_f32_tall(blocks, dh) == tall
+
+
+@pytest.mark.parametrize("rows,k,takes", [(64, 512, True), (65, 512, False), (1, 16, True), (1, 24, False), (16, 1040, True), (16, 1072, False)])
+def test_heads_products_of_few_rows(rows, k, takes):
+    """Whole steps of 16 columns, and two blocks an SM."""
+    assert host.head_takes_rows(rows, k) == takes
+
+
+@pytest.mark.parametrize("k,elem,blocks,groups", [(2048, 2, 10 ** 6, 1), (512, 2, 1183, 1), (512, 2, 1184, 2), (256, 2, 2368, 4), (256, 2, 2367, 2), (64, 4, 10 ** 6, 4), (512, 4, 10 ** 6, 1)])
+def test_groups_of_an_experts_rows_a_block(k, elem, blocks, groups):
+    """More than one only where that many rows of 16 are 2 KB at most and the grid stays at four blocks an SM."""
+    assert host.expert_row_groups(k, elem, blocks) == groups
+
+
 @pytest.mark.parametrize("code,words", [(1, "gemm_tcgen05: a bounded wait ran out (TMA"), (4, "linear_small: a row's sum of squares"), (14, "attention_tcgen05"),
                                         (23, "routed_experts of many rows"), (24, "routed_experts of few rows: a bounded wait ran out (copies"),
                                         (25, "head_linear of few rows: a bounded wait ran out (copies"), (33, "gemm_f32_tcgen05: a bounded wait ran out (weights and sums"),

@@ -109,6 +109,37 @@ def test_add_rmsnorm_of_many_rows(K, T, d, delta, wanted):
     assert torch.equal(xd.cpu(), x + 0.25 * p if delta and not wanted else x) or (delta and not wanted and (xd.cpu().double() - v).abs().max() <= 2e-7 * v.abs().max())
 
 
+@pytest.mark.parametrize("in_dtype,out_dtype", [(torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16)])
+@pytest.mark.parametrize("T,di", [(96, 512), (13, 4100), (12, 4096)])
+def test_swiglu_four_units_a_thread_in_the_types_of_the_models(K, in_dtype, out_dtype, T, di):
+    """Sums in float32 or operands in bfloat16, rounded once: the bits of the form that rows off 16 bytes take, and 64 bits."""
+    g = torch.Generator().manual_seed(di + T)
+    gu = (torch.randn(T, 2 * di, generator=g) * 3).to(in_dtype)
+    out, slow = torch.empty(T, di, dtype=out_dtype, device=DEV), torch.empty(T * di + 1, dtype=out_dtype, device=DEV)[1:].view(T, di)
+    K.swiglu(gu.to(DEV), out)
+    K.swiglu(gu.to(DEV), slow)
+    a, b = gu.double().split(di, 1)
+    _close(out, a * torch.sigmoid(a) * b, out_dtype, scale=3.0)
+    assert torch.equal(out, slow)
+
+
+@pytest.mark.parametrize("out_dtype", DTYPES)
+@pytest.mark.parametrize("delta_dtype", [None, torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,d", [(1, 1536), (64, 2048), (255, 4096), (7, 1028), (200, 2052), (3, 132), (2, 6144)])
+def test_add_rmsnorm_of_few_rows_in_registers(K, out_dtype, delta_dtype, T, d):
+    """One, two and three vectors a thread, whole and in part, all rows and picked ones."""
+    g = torch.Generator().manual_seed(T + d)
+    x, w = torch.randn(T, d, generator=g) * 3, 1 + 0.1 * torch.randn(d, generator=g)
+    delta = None if delta_dtype is None else torch.randn(T, d, generator=g).to(delta_dtype)
+    v = x.double() + (0 if delta is None else 0.7 * delta.double())
+    rows = torch.randint(0, T, (T,), generator=g, dtype=torch.int32)
+    for pick in (None, rows):
+        xd, out = x.to(DEV), torch.empty(T, d, dtype=out_dtype, device=DEV)
+        K.add_rmsnorm(xd, None if delta is None else delta.to(DEV), 0.7, w.to(DEV), 1e-5, out, 4.0, None if pick is None else pick.to(DEV))
+        _close(xd, x.double() if pick is not None else v, torch.float32)
+        _close(out, 4.0 * plain_rmsnorm(v if pick is None else v[pick.long()], w.double(), 1e-5), out_dtype, scale=4.0)
+
+
 @pytest.mark.parametrize("out_dtype", DTYPES)
 @pytest.mark.parametrize("T,d", [(256, 1024), (257, 1028), (532, 1536), (512, 2304), (2400, 2052), (1300, 3072)])
 @pytest.mark.parametrize("wanted", [False, True])
