@@ -65,6 +65,9 @@ __device__ __forceinline__ void store4(__nv_bfloat16 *p, float4 v) {
     *reinterpret_cast<uint2 *>(p) = raw;
 }
 
+// Four squares, added as every form of the norm adds them: written out, since the compiler contracts the sum in one way here and in another there.
+__device__ __forceinline__ float squares(float4 v) { return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.x, v.x, __fmul_rn(v.y, v.y)))); }
+
 // A row in registers, NV vectors a thread, the norm's weights asked for before the kernel before has ended: what steps of few rows take.  The sums are
 // those of the kernel below in their order.  What bounds it: the two reductions and one round of loads.  B200, with something to add, the form below -> this (us):
 // 8 rows of 2,048 2.35 -> 1.65, 64 of 2,304 2.92 -> 1.98, 64 of 4,096 2.89 -> 2.33, 200 of 4,096 4.32 -> 3.35, 200 of 2,048 2.9 and 3.0.
@@ -96,7 +99,7 @@ __global__ void __launch_bounds__(512) add_rmsnorm_regs_kernel(float *x, const T
             v[j] = make_float4(v[j].x + delta_scale * p[j].x, v[j].y + delta_scale * p[j].y, v[j].z + delta_scale * p[j].z, v[j].w + delta_scale * p[j].w);
             if (!rows) store4(x + at + c, v[j]);
         }
-        ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
+        ss += squares(v[j]);
     }
     ss = block_sum(ss, scratch);
     const float inv = rsqrtf(ss / (float)d + eps) * out_scale;
@@ -131,7 +134,7 @@ __global__ void add_rmsnorm_kernel(float *__restrict__ x, const TD *__restrict__
                 if (!rows) store4(xr + c, v);
             }
             store4(row_buf + c, v);
-            ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+            ss += squares(v);
         }
     } else {
         for (int c = threadIdx.x; c < d; c += blockDim.x) {
@@ -188,7 +191,7 @@ add_rmsnorm_warp_kernel(float *__restrict__ x, const TD *__restrict__ delta, flo
     }
     float ss = 0.f;
 #pragma unroll
-    for (int j = 0; j < NV; ++j) ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
+    for (int j = 0; j < NV; ++j) ss += squares(v[j]);
     ss = warp_sum(ss);
     const float inv = rsqrtf(ss / (float)d + eps) * out_scale;
     TO *o = out + (size_t)i * d;
@@ -242,7 +245,7 @@ add_rmsnorm_rows_kernel(float *x, const float *delta, float delta_scale, const f
             u[j] = make_float4(v[j].x + delta_scale * p[j].x, v[j].y + delta_scale * p[j].y, v[j].z + delta_scale * p[j].z, v[j].w + delta_scale * p[j].w);
             const int c = first + j * step;
             if (rows == nullptr && c < d) store4(x + at + c, u[j]);
-            sums[turn][j * WARPS * 32 + threadIdx.x] = c < d ? u[j].x * u[j].x + u[j].y * u[j].y + u[j].z * u[j].z + u[j].w * u[j].w : 0.f;
+            sums[turn][j * WARPS * 32 + threadIdx.x] = c < d ? squares(u[j]) : 0.f;
         }
         if (i + gridDim.x < nout) fetch(i + gridDim.x);
         __syncthreads();            // the other half of `sums` is free: who reads it has not passed this barrier's predecessor

@@ -140,6 +140,43 @@ def test_add_rmsnorm_of_few_rows_in_registers(K, out_dtype, delta_dtype, T, d):
         _close(out, 4.0 * plain_rmsnorm(v if pick is None else v[pick.long()], w.double(), 1e-5), out_dtype, scale=4.0)
 
 
+def _norm_in_order(v, w, eps, threads):
+    """The norm of float32 rows as a block of ``threads`` adds: four squares, a thread's vectors, a warp's tree, the warps' tree."""
+    T, d = v.shape
+    n = -(-d // (4 * threads))
+    q = torch.zeros(T, n * threads * 4, dtype=torch.float64, device=DEV)
+    q[:, :d] = v
+    q, once, lanes = q.view(T, n, threads, 4), lambda x: x.float().double(), torch.arange(32, device=DEV)
+    four = once(q[..., 3] ** 2 + once(q[..., 2] ** 2 + once(q[..., 0] ** 2 + once(q[..., 1] ** 2))))      # 64 bits hold a square, so each step rounds once
+    total = torch.zeros(T, threads, device=DEV)
+    for j in range(n):
+        total = total + four[:, j].float()
+    total = total.view(T, -1, 32)
+    for o in (16, 8, 4, 2, 1):
+        total = total + total[..., lanes ^ o]
+    total = torch.nn.functional.pad(total[..., 0], (0, 32 - threads // 32))
+    for o in (16, 8, 4, 2, 1):
+        total = total + total[:, lanes ^ o]
+    return v * torch.rsqrt(total[:, :1] / d + eps) * w
+
+
+@pytest.mark.parametrize("T", [12, 300])
+@pytest.mark.parametrize("delta_dtype", [None, torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("d,threads", [(512, 128), (1024, 256), (4096, 512)])
+def test_add_rmsnorm_adds_in_the_order_of_its_block(K, T, delta_dtype, d, threads):
+    """One and two vectors a thread, in registers (few rows) and through shared memory: the same bits, which do not depend on how it was compiled.
+    (Widths whose reciprocal is exact; many rows of up to 3,072 columns add a warp a row.)"""
+    if T >= 256 and d <= 3072:
+        pytest.skip("a warp a row")
+    g = torch.Generator().manual_seed(T + d)
+    x, w = torch.randn(T, d, generator=g).to(DEV), torch.randn(d, generator=g).to(DEV)
+    delta = None if delta_dtype is None else torch.randn(T, d, generator=g).to(DEV).to(delta_dtype)
+    v = x if delta is None else x + 0.5 * delta.float()         # a half is exact: one rounding, as in the kernel
+    out = torch.empty(T, d, device=DEV)
+    K.add_rmsnorm(x.clone(), delta, 0.5, w, 1e-5, out)
+    assert torch.equal(out, _norm_in_order(v, w, 1e-5, threads))
+
+
 @pytest.mark.parametrize("out_dtype", DTYPES)
 @pytest.mark.parametrize("T,d", [(256, 1024), (257, 1028), (532, 1536), (512, 2304), (2400, 2052), (1300, 3072)])
 @pytest.mark.parametrize("wanted", [False, True])
