@@ -493,10 +493,10 @@ inline int f32_tile(long long M, long long N, int sms, double *us) {
 //
 // The cuts set the order of the sums (the tile does not).  Below F32_ONE_ORDER_ROWS rows, where the norms of a step add in one order too,
 // way and cuts follow from N and K alone, so that a row's result depends neither on what else is in the step nor on how its prompt
-// was cut.  One choice for all of them: the cuts that are cheapest for two steps of 32 rows (decoding) and one of 255.
-// It costs steps of 161 to 255 rows up to a third of a product, and few rows of products that are wide (CUDA cores -> tensor cores, 8 rows:
-// 11,520 x 2,304 37 -> 48, 73,440 x 1,536 89 -> 137), where the others gain (7,680 x 1,536 26 -> 21, 2,560 x 1,536 16 -> 13, 1,536 x 3,840
-// 34 -> 16, 4,096 x 16,384 134 -> 84).
+// was cut.  One choice for all of them: the cuts that are cheapest for three steps of 32 rows (decoding, short prompts) and one of 255.
+// What it costs and gives, whole steps of the 1B shape against cuts by the rows and CUDA cores below 24 rows (us): prompts of 24 rows 4,454 -> 4,508, 64
+// 4,863 -> 4,955, 160 6,820 -> 6,868, 200 8,453 -> 10,494, 255 8,617 -> 10,736; one decoding row 8,724 -> 4,524, 24 4,932 -> 4,962.  (With eight cuts of
+// 1,536 x 1,536; with four 64 rows took 5,245 and 200 10,063.)  Wide products of few rows lose: 8 rows, 11,520 x 2,304 37 -> 48, 73,440 x 1,536 89 -> 137.
 struct F32Plan { int tile, cuts; };
 constexpr int F32_ONE_ORDER_ROWS = 256, F32_TENSOR_K = 512;
 // microseconds of the best tile for the given cuts, and that tile; `waves`: how often it fills the chip
@@ -528,7 +528,7 @@ inline F32Plan f32_plan(long long M, long long N, long long K, int sms) {
         if (one_order) {
             const double few = f32_tensor_cost(32, N, K, sms, cuts, &tile, &waves), many = f32_tensor_cost(F32_ONE_ORDER_ROWS - 1, N, K, sms, cuts, &tile, &waves);
             if (few < 0. || many < 0.) continue;
-            cost = 2. * few + many;
+            cost = 3. * few + many;
         } else {
             cost = f32_tensor_cost(M, N, K, sms, cuts, &tile, &waves);
             if (cost < 0. || (cuts > 1 && waves > 1)) continue;
