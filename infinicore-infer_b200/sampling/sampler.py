@@ -49,13 +49,15 @@ class Sampler:
             kernels.argmax(logits, out)
         else:
             # One copy from pinned memory that does not wait: the draw is launched while the step still runs.  (A copy from pageable
-            # memory waited for the step, and the device then for this call's launches: a pass of the small named configuration 353 us, 329 so.)
+            # memory waited for the step, and the device then for this call's launches: a pass of the small named configuration 350 us, 326 with
+            # this and norms of rows in registers.)
             host = torch.empty(4, n, dtype=torch.float32, pin_memory=self.device.type == "cuda")
             rows, most = host.numpy(), 2 ** 31 - 1
-            rows[0] = [p.temperature for p in params]
-            rows[1].view(np.int32)[:] = [int(max(-most, min(most, p.topk))) for p in params]
-            rows[2] = [p.topp for p in params]
-            rows[3] = [uniform_for(p.seed, i) for p, i in zip(params, indices)]
+            with np.errstate(over="ignore"):         # a number beyond float32 is infinite, as in a tensor
+                rows[0] = [p.temperature for p in params]
+                rows[1].view(np.int32)[:] = [int(max(-most, min(most, p.topk))) for p in params]
+                rows[2] = [p.topp for p in params]
+                rows[3] = [uniform_for(p.seed, i) for p, i in zip(params, indices)]
             dev = host.to(self.device, non_blocking=True)
             kernels.sample(logits, dev[0], dev[1].view(torch.int32), dev[2], dev[3], out)
         return out.tolist()

@@ -172,3 +172,15 @@ def test_sampling_parameters_beyond_their_types_are_clamped(monkeypatch):
     params = [SamplingParams(temperature=1.0, topk=k, topp=0.5) for k in (7, 2 ** 40, float("inf"), -2 ** 40)]
     Sampler("cpu").sample(torch.zeros(4, 8), params, range(4))
     assert seen == [[7, 2 ** 31 - 1, 2 ** 31 - 1, 1 - 2 ** 31]]
+
+
+@pytest.mark.filterwarnings("error")
+def test_sampling_parameters_beyond_float32_are_infinite(monkeypatch):
+    import torch
+
+    from infinicore_infer_b200 import kernels
+    from infinicore_infer_b200.sampling.sampler import Sampler, SamplingParams
+    seen = []
+    monkeypatch.setattr(kernels, "sample", lambda logits, t, k, p, u, out: (seen.append(t.tolist()), out.zero_()))
+    Sampler("cpu").sample(torch.zeros(2, 8), [SamplingParams(temperature=t, topk=5, topp=0.5) for t in (1e300, 0.5)], range(2))
+    assert seen == [[float("inf"), 0.5]]
