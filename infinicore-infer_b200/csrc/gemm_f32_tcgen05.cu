@@ -1,4 +1,4 @@
-// The float32 matrix product of steps of many rows on the 5th-generation tensor cores:  C[M, N] = A[M, K] * W[N, K]^T (+ bias[N]).
+// The float32 matrix product on the 5th-generation tensor cores:  C[M, N] = A[M, K] * W[N, K]^T (+ bias[N]).
 //
 // A float32 number is the sum of three bfloat16 ones (round to nearest, twice the remainder: 8 + 8 + 8 bits and signs), and a product of two
 // float32 numbers the sum of nine products of those, each exact in float32.  Six of them are made, smallest first: m m, h l, l h, h m, m h,
@@ -11,6 +11,7 @@
 // multiply-adds of gemm_f32.cu 2.5e-7; K 3,840 1.1e-7 to 1.6e-7 and 4.0e-7; K 96 0.8e-7 and 0.8e-7.
 // Numbers that this does not carry (infinities, NaN, operands from 2^111 and results from 2^95 on) leave a result that
 // is not finite: such outputs are made again from the operands by the multiply-adds of gemm_f32.cu, in its order.
+// A row's result depends on the row and on the cuts of K, not on the tile nor on the other rows (jk::f32_plan says who sets the cuts).
 //
 // The weights are on the MMA's M side (128 features a tile), tokens on its N side (BN of them), so that a prompt's odd number
 // of rows costs no more than its last tile of BN.  K is cut over the blocks of a cluster where tiles alone leave SMs idle;
@@ -18,7 +19,7 @@
 //
 // What bounds it: the MMAs (six where bfloat16 has one; 65 cycles each up to 128 tokens, 80 at 160: a chunk takes 1,560 to 1,920) and, by a
 // little more, the chain from raw weights to split ones and from tensor memory to the sums, which two stages only half hide (1.2 to 1.5 us
-// a chunk).  Shared memory would hold both of an MMA's operands as a rule, and 24 MMAs a chunk would read 216 KB of it at BN = 160,
+// a chunk; 301 x 7,680 x 1,536: the tensor pipe is active for two thirds of the cycles of an SM that has a block, issue slots are used for three quarters).  Shared memory would hold both of an MMA's operands as a rule, and 24 MMAs a chunk would read 216 KB of it at BN = 160,
 // as long as they take; so the weights' three parts go to tensor memory, from where an MMA takes its A operand as well.  Splitting
 // weights and tokens in registers on their way to shared memory measured 89 us for 301 x 7,680 x 1,536 where this takes 45.
 //

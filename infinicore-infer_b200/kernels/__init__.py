@@ -179,7 +179,7 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional
 
 def gemm_f32_tcgen05(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None, tile: int = 0, cuts: int = 1) -> torch.Tensor:
     """The same product with the operands split into three bfloat16 parts on the tensor cores: errors as ``gemm_f32``'s or smaller, sums
-    in an order that depends on ``tile`` (tokens: 32, 64, 96, 128 or 160; 0: by the rule, or 96) and ``cuts`` of K (1, 2, 4 or 8)."""
+    in an order that depends on ``cuts`` of K (1, 2, 4 or 8) alone; ``tile``: 32, 64, 96, 128 or 160 tokens, or 0: tile and cuts by the rule (or 96 and 1)."""
     _need(a, "a", torch.float32); _need(w, "w", torch.float32); _need(out, "out", torch.float32)
     m, k = a.shape
     n = w.shape[0]

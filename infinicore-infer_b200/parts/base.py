@@ -60,8 +60,8 @@ def part_class(family: str, spec) -> type:
 class Runtime:
     """The precision and device a model runs in, and the switches of the native step.
 
-    ``dtype`` float32: every product has the precision of float32 operands and sums: few rows on the CUDA
-    cores, many on the tensor cores with each operand as the sum of three bfloat16 numbers (no TF32).  ``dtype``
+    ``dtype`` float32: every product has the precision of float32 operands and sums: short sums on the CUDA
+    cores, the others on the tensor cores with each operand as the sum of three bfloat16 numbers (no TF32).  ``dtype``
     bfloat16: operands are bfloat16, accumulation and (where asked) the output are float32; a product goes to this
     package's own kernels or to the library, as the reference sends its products to one
     (src/models/inference_context.cpp:59-79).  Which kernel takes which product is decided in ONE place, the native
