@@ -119,6 +119,21 @@ def test_float32_products_of_few_rows_add_in_one_order(n, k, cuts):
     assert {c if t else 0 for t, c in plans} == {cuts}
 
 
+@pytest.mark.parametrize("kind,k,dtype,library,needs", [("linear", 512, "float32", 0, True), ("residual", 511, "float32", 0, False), ("gate_up", 2048, "float32", 0, True),
+                                                        ("norm_add", 2048, "float32", 0, False), ("linear", 2048, "float32", 1, False), ("linear", 2048, "bfloat16", 0, False)])
+@pytest.mark.parametrize("rows", [1, 23, 4096])
+def test_a_model_binds_the_split_float32_product_where_its_records_reach_it(kind, k, dtype, library, needs, rows):
+    """By the records alone, as the product's way: an engine of small steps would else run it or not by what another engine has bound."""
+    import torch
+
+    from infinicore_infer_b200.kernels import dtype_code
+    from infinicore_infer_b200.parts import program
+    env = program.RunnerEnv(dtype=dtype_code(getattr(torch, dtype)), page_size=16, max_blocks=4)
+    env.routing.sms, env.routing.library_only = 148, library
+    ops = (program.RunnerOp * 1)(program.record(kind, "h", "act", n=256, k=k))
+    assert program.modules_needed(env, ops, 1, rows)["gemm_f32_tcgen05"] == needs
+
+
 @pytest.mark.parametrize("rows,short,tiles,page,takes", [(31, 0, 1, 16, False), (32, 0, 1, 16, True), (32, 1, 1, 16, False), (300, 0, 0, 16, False), (300, 0, 3, 24, False),
                                                          (300, 0, 3, 1, True), (300, 0, 3, 256, True)])
 def test_float32_attention_in_tiles(rows, short, tiles, page, takes):
